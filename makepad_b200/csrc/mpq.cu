@@ -17,11 +17,13 @@
 #include <new>
 #include <string>
 
+#include "checksum.cuh"
 #include "nvfp4.cuh"
 #include "per_device.h"
 #include "q4.cuh"
 #include "q4_rect.cuh"
 #include "q4_umma.cuh"
+#include "upload.h"
 
 using namespace mpq;
 
@@ -59,6 +61,8 @@ struct mpq_context {
     int q4_pre;               // stages copied before the dependency resolves (the rest right after the activation loads)
     bool q4_slab4;            // M > 4 as slabs of four rows through the streaming kernel
     Nvfp4Scratch fp4;
+    StagedUpload upload;      // pinned slots through which weights travel to the device
+    cudaStream_t upload_stream;
 };
 
 struct mpq_weight {
@@ -152,6 +156,7 @@ extern "C" int32_t mpq_context_create(int32_t device, mpq_context** out)
     c->q4_rect_partial_bytes = 0;
     c->q4_partials_ctas = 0;
     c->q4_status = nullptr;
+    c->upload_stream = nullptr;
     if (cudaSetDevice(device) != cudaSuccess || cudaGetDeviceProperties(&c->prop, device) != cudaSuccess) {
         delete c;
         return MPQ_ERR_CUDA;
@@ -159,6 +164,10 @@ extern "C" int32_t mpq_context_create(int32_t device, mpq_context** out)
     if (c->prop.major != 10) {   // sm_100a code only; no other path exists
         delete c;
         return MPQ_ERR_UNSUPPORTED;
+    }
+    if (cudaStreamCreateWithFlags(&c->upload_stream, cudaStreamNonBlocking) != cudaSuccess) {
+        delete c;
+        return MPQ_ERR_CUDA;
     }
     const char* e = getenv("MPQ_PDL");
     c->pdl = !(e && e[0] == '0');
@@ -202,6 +211,8 @@ extern "C" int32_t mpq_context_destroy(mpq_context* ctx)
     cudaFree(ctx->q4_rect_partial);
     cudaFree(ctx->q4_status);
     ctx->fp4.release();
+    ctx->upload.release();
+    cudaStreamDestroy(ctx->upload_stream);
     ctx->magic = 0;
     delete ctx;
     return MPQ_OK;
@@ -231,7 +242,7 @@ extern "C" int64_t mpq_context_launch_count(const mpq_context* ctx) { return ctx
 // Q4 weights
 // ---------------------------------------------------------------------------
 static int32_t q4_build(mpq_context* ctx, int64_t Nfull, int64_t Kfull, const uint8_t* codes_dev, const uint16_t* scales_dev,
-                        int64_t row0, int64_t k0, int64_t N, int64_t K, mpq_weight** out)
+                        int64_t row0, int64_t k0, int64_t N, int64_t K, cudaStream_t s, mpq_weight** out)
 {
     mpq_weight* w = new (std::nothrow) mpq_weight();
     if (!w) return fail(ctx, MPQ_ERR_CUDA, "out of host memory");
@@ -251,12 +262,13 @@ static int32_t q4_build(mpq_context* ctx, int64_t Nfull, int64_t Kfull, const ui
         return fail(ctx, MPQ_ERR_CUDA, "cudaMalloc of %zu weight bytes failed: %s", q.bytes(), cudaGetErrorString(e));
     }
     int64_t words = (int64_t)q.nrp * q.nchunks * 256, halves = (int64_t)q.nrp * q.nchunks * 64;
-    q4_repack_codes_kernel<<<(unsigned)((words + 255) / 256), 256>>>(codes_dev, Kfull, row0, k0, N, K, q.nrp, q.nchunks,
+    q4_repack_codes_kernel<<<(unsigned)((words + 255) / 256), 256, 0, s>>>(codes_dev, Kfull, row0, k0, N, K, q.nrp, q.nchunks,
                                                                       reinterpret_cast<uint32_t*>(q.stream));
-    q4_repack_scales_kernel<<<(unsigned)((halves + 255) / 256), 256>>>(scales_dev, Kfull / 32, row0, k0 / 32, N, K / 32, q.nrp,
+    q4_repack_scales_kernel<<<(unsigned)((halves + 255) / 256), 256, 0, s>>>(scales_dev, Kfull / 32, row0, k0 / 32, N, K / 32, q.nrp,
                                                                         q.nchunks, reinterpret_cast<uint16_t*>(q.stream));
     ctx->launches += 2;
-    e = cudaDeviceSynchronize();
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {
         cudaFree(q.stream);
         delete w;
@@ -303,14 +315,14 @@ extern "C" int32_t mpq_q4_weight_create(mpq_context* ctx, int64_t N, int64_t K, 
     uint16_t* ds = nullptr;
     CU_TRY(ctx, cudaMalloc(&dc, cb));
     cudaError_t e = cudaMalloc(&ds, sb);
-    if (e == cudaSuccess) e = cudaMemcpy(dc, codes_host + (size_t)row0 * (K / 2), cb, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(ds, scales_host + (size_t)row0 * (K / 32), sb, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) ctx->upload.run(ctx->device, dc, codes_host + (size_t)row0 * (K / 2), -1, 0, cb, ctx->upload_stream, &e);
+    if (e == cudaSuccess) ctx->upload.run(ctx->device, ds, scales_host + (size_t)row0 * (K / 32), -1, 0, sb, ctx->upload_stream, &e);
     if (e != cudaSuccess) {
         cudaFree(dc);
         cudaFree(ds);
         return fail(ctx, MPQ_ERR_CUDA, "upload of canonical Q4 arrays failed: %s", cudaGetErrorString(e));
     }
-    st = q4_build(ctx, n, K, dc, ds, 0, k0, n, k, out);
+    st = q4_build(ctx, n, K, dc, ds, 0, k0, n, k, ctx->upload_stream, out);
     cudaFree(dc);
     cudaFree(ds);
     return st;
@@ -325,7 +337,7 @@ extern "C" int32_t mpq_q4_weight_create_dev(mpq_context* ctx, int64_t N, int64_t
     if (N <= 0 || K <= 0 || K % 32) return fail(ctx, MPQ_ERR_SHAPE, "Q4 needs N > 0 and K a positive multiple of 32 (N=%lld K=%lld)", (long long)N, (long long)K);
     if (N > (1LL << 30) || K > (1LL << 30)) return fail(ctx, MPQ_ERR_UNSUPPORTED, "dimension above 2^30");
     CU_TRY(ctx, cudaSetDevice(ctx->device));
-    return q4_build(ctx, N, K, codes_dev, scales_dev, 0, 0, N, K, out);
+    return q4_build(ctx, N, K, codes_dev, scales_dev, 0, 0, N, K, 0, out);      // the arrays are the caller's: the legacy stream waits for their writers
 }
 
 // ---------------------------------------------------------------------------
@@ -1369,15 +1381,16 @@ struct FileHeader {                                        // 128 bytes, little 
 };
 static_assert(sizeof(FileHeader) == 128, "container header is 128 bytes");
 
-static uint64_t fnv1a64(const uint8_t* p, size_t n, uint64_t h = 0xCBF29CE484222325ull)
+static const uint64_t FNV_START = 0xCBF29CE484222325ull;
+static uint64_t fnv1a64(const uint8_t* p, size_t n, uint64_t h = FNV_START)
 {
     for (size_t i = 0; i < n; ++i) { h ^= p[i]; h *= 0x100000001B3ull; }
     return h;
 }
 
-static int32_t file_write(const char* path, FileHeader& h, const void* a, const void* b)
+// h.checksum is the caller's to fill in
+static int32_t file_write(const char* path, const FileHeader& h, const void* a, const void* b)
 {
-    h.checksum = fnv1a64(static_cast<const uint8_t*>(b), (size_t)h.bytes_b, fnv1a64(static_cast<const uint8_t*>(a), (size_t)h.bytes_a));
     FILE* f = fopen(path, "wb");
     if (!f) return MPQ_ERR_IO;
     bool ok = fwrite(&h, sizeof h, 1, f) == 1 && (h.bytes_a == 0 || fwrite(a, (size_t)h.bytes_a, 1, f) == 1) &&
@@ -1439,6 +1452,7 @@ extern "C" int32_t mpq_canonical_save(const char* path, int32_t fmt, int64_t N, 
     h.N = N; h.K = K; h.tensor_scale = fmt == MPQ_FMT_Q4 ? 1.f : tensor_scale;
     h.bytes_a = N * (K / 2);
     h.bytes_b = fmt == MPQ_FMT_Q4 ? N * (K / 32) * 2 : N * (K / 16);
+    h.checksum = fnv1a64(static_cast<const uint8_t*>(scales_host), (size_t)h.bytes_b, fnv1a64(codes_host, (size_t)h.bytes_a));
     return file_write(path, h, codes_host, scales_host);
 }
 
@@ -1480,6 +1494,10 @@ extern "C" int32_t mpq_weight_save(mpq_context* ctx, const mpq_weight* w, const 
     if (!host) return fail(ctx, MPQ_ERR_CUDA, "out of host memory");
     cudaError_t e = cudaMemcpy(host, da, (size_t)h.bytes_a, cudaMemcpyDeviceToHost);        // synchronises with prior work
     if (e == cudaSuccess && h.bytes_b) e = cudaMemcpy(host + h.bytes_a, db, (size_t)h.bytes_b, cudaMemcpyDeviceToHost);
+    // the checksum is taken where the bytes lie: the legacy stream runs after the copies above
+    h.checksum = FNV_START;
+    if (e == cudaSuccess) e = fnv1a64_device(da, h.bytes_a, &h.checksum, 0);
+    if (e == cudaSuccess) e = fnv1a64_device(db, h.bytes_b, &h.checksum, 0);
     int32_t st = e == cudaSuccess ? file_write(path, h, host, host + h.bytes_a) : MPQ_ERR_CUDA;
     free(host);
     if (st == MPQ_ERR_CUDA) return fail(ctx, st, "device-to-host copy failed: %s", cudaGetErrorString(e));
@@ -1513,31 +1531,37 @@ extern "C" int32_t mpq_weight_load(mpq_context* ctx, const char* path, mpq_weigh
         fclose(f);
         return fail(ctx, MPQ_ERR_FORMAT, "%s: device layout of another build (rebuild the weight from its canonical arrays)", path);
     }
-    uint8_t* host = static_cast<uint8_t*>(malloc((size_t)(h.bytes_a + h.bytes_b) + 1));
-    if (!host) { fclose(f); return fail(ctx, MPQ_ERR_CUDA, "out of host memory"); }
-    st = file_read_payload(f, h, host, host + h.bytes_a);
-    if (st) { free(host); return fail(ctx, st, "%s: %s", path, st == MPQ_ERR_IO ? "read failed" : "checksum mismatch"); }
     cudaError_t e = cudaSetDevice(ctx->device);
     mpq_weight* w = new (std::nothrow) mpq_weight();
-    if (!w) { free(host); return fail(ctx, MPQ_ERR_CUDA, "out of host memory"); }
+    if (!w) { fclose(f); return fail(ctx, MPQ_ERR_CUDA, "out of host memory"); }
     w->magic = W_MAGIC; w->fmt = (int)h.fmt; w->device = ctx->device;
     if (h.fmt == MPQ_FMT_Q4) {
         w->q4.N = h.N; w->q4.K = h.K; w->q4.nrp = h.nrp; w->q4.nchunks = h.nchunks;
         if (e == cudaSuccess) e = cudaMalloc(&w->q4.stream, (size_t)h.bytes_a);
-        if (e == cudaSuccess) e = cudaMemcpy(w->q4.stream, host, (size_t)h.bytes_a, cudaMemcpyHostToDevice);
     } else {
         w->fp4.N = h.N; w->fp4.K = h.K; w->fp4.tensor_scale = h.tensor_scale; w->fp4.sf_tiled_bytes = (size_t)h.bytes_b;
         if (e == cudaSuccess) e = cudaMalloc(&w->fp4.codes, (size_t)h.bytes_a);
         if (e == cudaSuccess) e = cudaMalloc(&w->fp4.sf_tiled, (size_t)h.bytes_b);
-        if (e == cudaSuccess) e = cudaMemcpy(w->fp4.codes, host, (size_t)h.bytes_a, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(w->fp4.sf_tiled, host + h.bytes_a, (size_t)h.bytes_b, cudaMemcpyHostToDevice);
     }
-    free(host);
-    if (e != cudaSuccess) {
+    // The payload goes straight to where the weight lives; the checksum is taken there, of what arrived, and no weight is
+    // handed out before it agrees.
+    void* part[2] = {h.fmt == MPQ_FMT_Q4 ? static_cast<void*>(w->q4.stream) : w->fp4.codes, w->fp4.sf_tiled};
+    const int64_t bytes[2] = {h.bytes_a, h.bytes_b};
+    uint64_t sum = FNV_START;
+    int64_t at = (int64_t)sizeof h;
+    for (int i = 0; i < 2 && e == cudaSuccess && st == MPQ_OK; at += bytes[i], ++i) {
+        if (!bytes[i]) continue;
+        if (ctx->upload.run(ctx->device, part[i], nullptr, fileno(f), at, (size_t)bytes[i], ctx->upload_stream, &e) == StagedUpload::READ_FAILED) st = MPQ_ERR_IO;
+        if (st == MPQ_OK && e == cudaSuccess) e = fnv1a64_device(part[i], bytes[i], &sum, ctx->upload_stream);
+    }
+    fclose(f);
+    if (st == MPQ_OK && e == cudaSuccess && sum != h.checksum) st = MPQ_ERR_FORMAT;
+    if (st != MPQ_OK || e != cudaSuccess) {
         cudaFree(w->q4.stream);
         w->fp4.release();
         delete w;
-        return fail(ctx, MPQ_ERR_CUDA, "upload of %s failed: %s", path, cudaGetErrorString(e));
+        if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "upload of %s failed: %s", path, cudaGetErrorString(e));
+        return fail(ctx, st, "%s: %s", path, st == MPQ_ERR_IO ? "read failed" : "checksum mismatch");
     }
     *out = w;
     return MPQ_OK;

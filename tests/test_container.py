@@ -111,3 +111,31 @@ def test_stale_or_damaged_cache_files_are_refused(ctx, tmp_path):
         assert ctx.lib.mpq_weight_load(ctx.h, p.encode(), C.byref(h)) == _lib.ERR_FORMAT, mutate
         assert not h.value
     assert ctx.lib.mpq_weight_load(ctx.h, str(tmp_path / "nope").encode(), C.byref(h)) == _lib.ERR_IO
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N, K", [(1, 32), (33, 288), (96, 1216), (1000, 2112), (4097, 4096), (12320, 4096)])
+def test_device_checksum_is_the_host_loop(ctx, tmp_path, N, K):
+    """The checksum taken on the GPU against the host's byte loop over the same payload (below one chunk of 4096 bytes, across
+    chunks, across groups of 64 chunks, and across 64 groups), and a payload byte flipped anywhere is refused."""
+    import makepad_b200
+    w = makepad_b200.Q4Weight(ctx, *synth.q4_weight(N, K, seed=N))
+    path, ref = str(tmp_path / "w.q4d"), str(tmp_path / "ref.q4c")
+    w.save(path)
+    raw = bytearray(open(path, "rb").read())
+    payload = np.frombuffer(bytes(raw[128:]), dtype=np.uint8)
+    # a tile stream of 1152-byte units is as long as the canonical arrays of the padded shape, whose file the host sums
+    n, k = (N + 31) // 32 * 32, (K + 255) // 256 * 256
+    cut = n * k // 2
+    assert payload.size == n * k * 9 // 16
+    makepad_b200.save_canonical(ref, _lib.FMT_Q4, payload[:cut].reshape(n, k // 2), payload[cut:].view(np.uint16).reshape(n, k // 32))
+    assert raw[56:64] == open(ref, "rb").read()[56:64]
+    want = w.dequantize()
+    assert np.array_equal(makepad_b200.load_weight(ctx, path).dequantize().cpu().numpy(), want.cpu().numpy())
+    for at in (128, len(raw) // 2, len(raw) - 1):
+        bad = bytearray(raw)
+        bad[at] ^= 0x80
+        open(path, "wb").write(bad)
+        with pytest.raises(makepad_b200.MpqError) as err:
+            makepad_b200.load_weight(ctx, path)
+        assert err.value.status == _lib.ERR_FORMAT
