@@ -133,16 +133,25 @@ __global__ void __launch_bounds__(FNV_GROUP) fnv_sum_kernel(const uint8_t* __res
     }
 }
 
-// *h = FNV-1a 64 of buf[0, bytes) continued from *h.  buf: 16-byte aligned device memory.  Waits for the stream.
-inline cudaError_t fnv1a64_device(const void* buf, int64_t bytes, uint64_t* h, cudaStream_t s)
+// device memory fnv1a64_device wants: 1/32 of the buffer
+inline size_t fnv1a64_scratch_bytes(int64_t bytes)
+{
+    const int64_t chunks = (bytes + FNV_CHUNK - 1) / FNV_CHUNK, groups = (chunks + FNV_GROUP - 1) / FNV_GROUP;
+    return ((size_t)groups * 8 + 127) / 128 * 128 + (size_t)groups * 129 + (size_t)chunks * 128;
+}
+
+// *h = FNV-1a 64 of buf[0, bytes) continued from *h.  buf: 16-byte aligned device memory; scratch: fnv1a64_scratch_bytes, or
+// null to allocate it here.  Waits for the stream.
+inline cudaError_t fnv1a64_device(const void* buf, int64_t bytes, uint64_t* h, uint8_t* scratch, cudaStream_t s)
 {
     if (bytes <= 0) return cudaSuccess;
     const int64_t chunks = (bytes + FNV_CHUNK - 1) / FNV_CHUNK, groups = (chunks + FNV_GROUP - 1) / FNV_GROUP;
     // sums (8 B per group) | group maps (128 B) | chunk maps (128 B) | group starts (1 B)
     const size_t off_gmap = ((size_t)groups * 8 + 127) / 128 * 128, off_map = off_gmap + (size_t)groups * 128, off_start = off_map + (size_t)chunks * 128;
-    uint8_t* scratch = nullptr;
-    cudaError_t e = cudaMalloc(&scratch, off_start + (size_t)groups);
+    uint8_t* own = nullptr;
+    cudaError_t e = scratch ? cudaSuccess : cudaMalloc(&own, off_start + (size_t)groups);
     if (e != cudaSuccess) return e;
+    if (!scratch) scratch = own;
     const uint8_t* b = static_cast<const uint8_t*>(buf);
     uint64_t* sum = reinterpret_cast<uint64_t*>(scratch);
     uint32_t* map = reinterpret_cast<uint32_t*>(scratch + off_map);
@@ -164,7 +173,7 @@ inline cudaError_t fnv1a64_device(const void* buf, int64_t bytes, uint64_t* h, c
         *h = (*h - host_l[g]) * pn + host[g];
     }
     free(host);
-    cudaFree(scratch);
+    if (own) cudaFree(own);
     return e;
 }
 

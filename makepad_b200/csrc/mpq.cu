@@ -241,12 +241,11 @@ extern "C" int64_t mpq_context_launch_count(const mpq_context* ctx) { return ctx
 // ---------------------------------------------------------------------------
 // Q4 weights
 // ---------------------------------------------------------------------------
-static int32_t q4_build(mpq_context* ctx, int64_t Nfull, int64_t Kfull, const uint8_t* codes_dev, const uint16_t* scales_dev,
-                        int64_t row0, int64_t k0, int64_t N, int64_t K, cudaStream_t s, mpq_weight** out)
+// the weight with its device memory, not yet filled
+static int32_t q4_alloc(mpq_context* ctx, int64_t N, int64_t K, mpq_weight** out)
 {
     mpq_weight* w = new (std::nothrow) mpq_weight();
     if (!w) return fail(ctx, MPQ_ERR_CUDA, "out of host memory");
-    (void)Nfull;
     w->magic = W_MAGIC;
     w->fmt = MPQ_FMT_Q4;
     w->device = ctx->device;
@@ -261,21 +260,23 @@ static int32_t q4_build(mpq_context* ctx, int64_t Nfull, int64_t Kfull, const ui
         delete w;
         return fail(ctx, MPQ_ERR_CUDA, "cudaMalloc of %zu weight bytes failed: %s", q.bytes(), cudaGetErrorString(e));
     }
-    int64_t words = (int64_t)q.nrp * q.nchunks * 256, halves = (int64_t)q.nrp * q.nchunks * 64;
-    q4_repack_codes_kernel<<<(unsigned)((words + 255) / 256), 256, 0, s>>>(codes_dev, Kfull, row0, k0, N, K, q.nrp, q.nchunks,
-                                                                      reinterpret_cast<uint32_t*>(q.stream));
-    q4_repack_scales_kernel<<<(unsigned)((halves + 255) / 256), 256, 0, s>>>(scales_dev, Kfull / 32, row0, k0 / 32, N, K / 32, q.nrp,
-                                                                        q.nchunks, reinterpret_cast<uint16_t*>(q.stream));
-    ctx->launches += 2;
-    e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) {
-        cudaFree(q.stream);
-        delete w;
-        return fail(ctx, MPQ_ERR_CUDA, "Q4 repack failed: %s", cudaGetErrorString(e));
-    }
     *out = w;
     return MPQ_OK;
+}
+
+// Repacks the rows rp0 * 32 .. of the weight from canonical arrays whose row 0 is the first of them; `rows` of them exist.
+static cudaError_t q4_repack(mpq_context* ctx, const Q4Dev& q, int rp0, int64_t rows, int64_t Kfull, const uint8_t* codes_dev,
+                             const uint16_t* scales_dev, int64_t k0, cudaStream_t s)
+{
+    const int nrp = (int)((rows + 31) / 32);
+    const int64_t words = (int64_t)nrp * q.nchunks * 256, halves = (int64_t)nrp * q.nchunks * 64;
+    unsigned char* to = reinterpret_cast<unsigned char*>(q.stream) + (size_t)rp0 * q.nchunks * Q4_UNIT_BYTES;
+    q4_repack_codes_kernel<<<(unsigned)((words + 255) / 256), 256, 0, s>>>(codes_dev, Kfull, 0, k0, rows, q.K, nrp, q.nchunks,
+                                                                           reinterpret_cast<uint32_t*>(to));
+    q4_repack_scales_kernel<<<(unsigned)((halves + 255) / 256), 256, 0, s>>>(scales_dev, Kfull / 32, 0, k0 / 32, rows, q.K / 32, nrp,
+                                                                             q.nchunks, reinterpret_cast<uint16_t*>(to));
+    ctx->launches += 2;
+    return cudaGetLastError();
 }
 
 static int32_t q4_shard(mpq_context* ctx, int64_t N, int64_t K, int32_t tp_mode, int32_t rank, int32_t world,
@@ -309,23 +310,34 @@ extern "C" int32_t mpq_q4_weight_create(mpq_context* ctx, int64_t N, int64_t K, 
     int32_t st = q4_shard(ctx, N, K, tp_mode, rank, world, &row0, &k0, &n, &k);
     if (st) return st;
     CU_TRY(ctx, cudaSetDevice(ctx->device));
-    // upload only the rows the shard needs (all K of them; the K slice is cut by the repack)
-    size_t cb = (size_t)n * (K / 2), sb = (size_t)n * (K / 32) * 2;
-    uint8_t* dc = nullptr;
-    uint16_t* ds = nullptr;
-    CU_TRY(ctx, cudaMalloc(&dc, cb));
-    cudaError_t e = cudaMalloc(&ds, sb);
-    if (e == cudaSuccess) ctx->upload.run(ctx->device, dc, codes_host + (size_t)row0 * (K / 2), -1, 0, cb, ctx->upload_stream, &e);
-    if (e == cudaSuccess) ctx->upload.run(ctx->device, ds, scales_host + (size_t)row0 * (K / 32), -1, 0, sb, ctx->upload_stream, &e);
+    mpq_weight* w = nullptr;
+    if ((st = q4_alloc(ctx, n, k, &w))) return st;
+    // Upload only the rows the shard needs (all K of them; the K slice is cut by the repack), as many at a time as the staging
+    // memory takes; the stream keeps a slab's repack in front of the next slab's copy.
+    const size_t row_codes = (size_t)K / 2, row_scales = (size_t)K / 32 * 2, row_bytes = row_codes + row_scales;
+    const int64_t slab = std::min<int64_t>((n + 31) / 32, std::max<int64_t>(1, (int64_t)(StagedUpload::STAGING_MOST / (32 * row_bytes)))) * 32;
+    std::lock_guard<std::mutex> staging_held(ctx->upload.staging_lock());
+    uint8_t* own = nullptr;                                // 32 rows that do not fit the kept staging memory
+    uint8_t* dc = ctx->upload.staging((size_t)slab * row_bytes);
+    cudaError_t e = dc ? cudaSuccess : cudaMalloc(&own, (size_t)slab * row_bytes);
+    if (!dc) dc = own;
+    uint16_t* ds = reinterpret_cast<uint16_t*>(dc + (size_t)slab * row_codes);          // 32 rows x 16 bytes and up: aligned
+    for (int64_t r = 0; r < n && e == cudaSuccess; r += slab) {
+        const int64_t rows = std::min(slab, n - r);
+        ctx->upload.run(ctx->device, dc, codes_host + (size_t)(row0 + r) * row_codes, -1, 0, (size_t)rows * row_codes, ctx->upload_stream, &e);
+        if (e == cudaSuccess) ctx->upload.run(ctx->device, ds, scales_host + (size_t)(row0 + r) * (K / 32), -1, 0, (size_t)rows * row_scales, ctx->upload_stream, &e);
+        if (e == cudaSuccess) e = q4_repack(ctx, w->q4, (int)(r / 32), rows, K, dc, ds, k0, ctx->upload_stream);
+    }
+    const cudaError_t done = cudaStreamSynchronize(ctx->upload_stream);
+    if (e == cudaSuccess) e = done;
+    if (own) cudaFree(own);
     if (e != cudaSuccess) {
-        cudaFree(dc);
-        cudaFree(ds);
+        cudaFree(w->q4.stream);
+        delete w;
         return fail(ctx, MPQ_ERR_CUDA, "upload of canonical Q4 arrays failed: %s", cudaGetErrorString(e));
     }
-    st = q4_build(ctx, n, K, dc, ds, 0, k0, n, k, ctx->upload_stream, out);
-    cudaFree(dc);
-    cudaFree(ds);
-    return st;
+    *out = w;
+    return MPQ_OK;
 }
 
 extern "C" int32_t mpq_q4_weight_create_dev(mpq_context* ctx, int64_t N, int64_t K, const uint8_t* codes_dev,
@@ -337,7 +349,19 @@ extern "C" int32_t mpq_q4_weight_create_dev(mpq_context* ctx, int64_t N, int64_t
     if (N <= 0 || K <= 0 || K % 32) return fail(ctx, MPQ_ERR_SHAPE, "Q4 needs N > 0 and K a positive multiple of 32 (N=%lld K=%lld)", (long long)N, (long long)K);
     if (N > (1LL << 30) || K > (1LL << 30)) return fail(ctx, MPQ_ERR_UNSUPPORTED, "dimension above 2^30");
     CU_TRY(ctx, cudaSetDevice(ctx->device));
-    return q4_build(ctx, N, K, codes_dev, scales_dev, 0, 0, N, K, 0, out);      // the arrays are the caller's: the legacy stream waits for their writers
+    mpq_weight* w = nullptr;
+    const int32_t st = q4_alloc(ctx, N, K, &w);
+    if (st) return st;
+    cudaError_t e = q4_repack(ctx, w->q4, 0, N, K, codes_dev, scales_dev, 0, 0);      // the arrays are the caller's: the legacy stream waits for their writers
+    const cudaError_t done = cudaDeviceSynchronize();
+    if (e == cudaSuccess) e = done;
+    if (e != cudaSuccess) {
+        cudaFree(w->q4.stream);
+        delete w;
+        return fail(ctx, MPQ_ERR_CUDA, "Q4 repack failed: %s", cudaGetErrorString(e));
+    }
+    *out = w;
+    return MPQ_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -1496,8 +1520,8 @@ extern "C" int32_t mpq_weight_save(mpq_context* ctx, const mpq_weight* w, const 
     if (e == cudaSuccess && h.bytes_b) e = cudaMemcpy(host + h.bytes_a, db, (size_t)h.bytes_b, cudaMemcpyDeviceToHost);
     // the checksum is taken where the bytes lie: the legacy stream runs after the copies above
     h.checksum = FNV_START;
-    if (e == cudaSuccess) e = fnv1a64_device(da, h.bytes_a, &h.checksum, 0);
-    if (e == cudaSuccess) e = fnv1a64_device(db, h.bytes_b, &h.checksum, 0);
+    if (e == cudaSuccess) e = fnv1a64_device(da, h.bytes_a, &h.checksum, nullptr, 0);
+    if (e == cudaSuccess) e = fnv1a64_device(db, h.bytes_b, &h.checksum, nullptr, 0);
     int32_t st = e == cudaSuccess ? file_write(path, h, host, host + h.bytes_a) : MPQ_ERR_CUDA;
     free(host);
     if (st == MPQ_ERR_CUDA) return fail(ctx, st, "device-to-host copy failed: %s", cudaGetErrorString(e));
@@ -1547,12 +1571,13 @@ extern "C" int32_t mpq_weight_load(mpq_context* ctx, const char* path, mpq_weigh
     // handed out before it agrees.
     void* part[2] = {h.fmt == MPQ_FMT_Q4 ? static_cast<void*>(w->q4.stream) : w->fp4.codes, w->fp4.sf_tiled};
     const int64_t bytes[2] = {h.bytes_a, h.bytes_b};
+    std::lock_guard<std::mutex> staging_held(ctx->upload.staging_lock());
     uint64_t sum = FNV_START;
     int64_t at = (int64_t)sizeof h;
     for (int i = 0; i < 2 && e == cudaSuccess && st == MPQ_OK; at += bytes[i], ++i) {
         if (!bytes[i]) continue;
         if (ctx->upload.run(ctx->device, part[i], nullptr, fileno(f), at, (size_t)bytes[i], ctx->upload_stream, &e) == StagedUpload::READ_FAILED) st = MPQ_ERR_IO;
-        if (st == MPQ_OK && e == cudaSuccess) e = fnv1a64_device(part[i], bytes[i], &sum, ctx->upload_stream);
+        if (st == MPQ_OK && e == cudaSuccess) e = fnv1a64_device(part[i], bytes[i], &sum, ctx->upload.staging(fnv1a64_scratch_bytes(bytes[i])), ctx->upload_stream);
     }
     fclose(f);
     if (st == MPQ_OK && e == cudaSuccess && sum != h.checksum) st = MPQ_ERR_FORMAT;

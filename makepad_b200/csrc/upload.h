@@ -2,7 +2,7 @@
 //
 // cudaMemcpy from pageable memory is one thread's memcpy into the driver's staging (about 7 GB/s here); a file adds a
 // read into fresh pages before it.  Several threads fill pinned slots (memcpy or pread) while the slots filled before
-// are on their way.  The slots belong to a context: made by its first upload, at most 8 x 1 MiB, freed with it.
+// are on their way.  The slots belong to a context: made by its first upload, at most 16 x 512 KiB, freed with it.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -19,8 +19,8 @@ namespace mpq {
 
 class StagedUpload {
 public:
-    static constexpr int THREADS = 4, SLOTS = 2;               // slots per thread: one is filled while the other travels
-    static constexpr size_t PIECE = (size_t)1 << 20;
+    static constexpr int THREADS = 8, SLOTS = 2;               // slots per thread: one is filled while the other travels
+    static constexpr size_t PIECE = (size_t)1 << 19;
     enum Result { OK = 0, READ_FAILED, CUDA_FAILED };
 
     // One upload at a time per context (several host threads may build weights).  Returns when the bytes are in device
@@ -72,8 +72,31 @@ public:
         return (Result)result.load();
     }
 
+    // Device memory for what an upload needs beside its destination, kept with the slots (a cudaMalloc and its cudaFree cost
+    // 0.4 ms each): a buffer of at least `bytes`, at most STAGING_MOST.  Null when it cannot be had.
+    static constexpr size_t STAGING_MOST = (size_t)32 << 20;
+    uint8_t* staging(size_t bytes)
+    {
+        if (bytes > STAGING_MOST) return nullptr;
+        if (staging_bytes_ < bytes) {
+            cudaFree(staging_);
+            staging_bytes_ = 0;
+            if (cudaMalloc(&staging_, bytes) != cudaSuccess) {
+                cudaGetLastError();
+                staging_ = nullptr;
+                return nullptr;
+            }
+            staging_bytes_ = bytes;
+        }
+        return staging_;
+    }
+    std::mutex& staging_lock() { return staging_lock_; }       // held from staging() until its use has been waited for
+
     void release()
     {
+        cudaFree(staging_);
+        staging_ = nullptr;
+        staging_bytes_ = 0;
         for (Slot& s : slots_) {
             if (s.mem) cudaFreeHost(s.mem);
             if (s.done) cudaEventDestroy(s.done);
@@ -83,7 +106,9 @@ public:
 
 private:
     struct Slot { void* mem = nullptr; cudaEvent_t done = nullptr; };
-    std::mutex lock_;
+    std::mutex lock_, staging_lock_;
+    uint8_t* staging_ = nullptr;
+    size_t staging_bytes_ = 0;
     Slot slots_[THREADS * SLOTS];
 };
 
