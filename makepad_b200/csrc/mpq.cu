@@ -21,6 +21,7 @@
 #include "nvfp4.cuh"
 #include "per_device.h"
 #include "q4.cuh"
+#include "q4_gemm.cuh"
 #include "q4_rect.cuh"
 #include "q4_umma.cuh"
 #include "upload.h"
@@ -47,6 +48,7 @@ struct mpq_context {
     int q4_umma_min;          // fewest activation rows routed to the tcgen05 kernel (0 = never)
     float* q4_rect_partial;   // [K slices][M][N] partial outputs of the rectangle kernel (grown on demand)
     size_t q4_rect_partial_bytes;
+    int q4_gemm_min;          // fewest activation rows routed to the CTA-pair kernel (0 = never: slabs of 64 through the tcgen05 kernel)
     bool q4_rect;             // use the rectangle kernel for 5..16 rows (else slabs of <= 4 rows through the streaming kernel)
     int q4_stream_max_m;      // most activation rows mpq_q4_linear_forward gives to the streaming kernel (1..4)
     int q4_rect_nks;          // experiment: at least so many K slices in the rectangle kernel (0 = the plan's choice)
@@ -183,6 +185,8 @@ extern "C" int32_t mpq_context_create(int32_t device, mpq_context** out)
     c->q4_pre = (e && e[0] >= '0' && e[0] <= '8') ? e[0] - '0' : 1;
     e = getenv("MPQ_Q4_UMMA_MIN");
     c->q4_umma_min = e ? atoi(e) : 17;         // measured: above 16 rows (two passes of the rectangle kernel) the tcgen05 kernel is faster
+    e = getenv("MPQ_Q4_GEMM_MIN");
+    c->q4_gemm_min = e ? atoi(e) : 65;
     e = getenv("MPQ_Q4_RECT");
     c->q4_rect = !(e && e[0] == '0');
     e = getenv("MPQ_Q4_STREAM_MAX_M");
@@ -839,6 +843,127 @@ static int32_t q4_umma_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
     return MPQ_OK;
 }
 
+// ---------------------------------------------------------------------------
+// the CTA-pair kernel: more than 64 rows
+// ---------------------------------------------------------------------------
+static size_t q4_gemm_smem(int Mt)
+{
+    // rings, barriers, alignment; at least 116 KiB, so that two CTAs never share an SM (each allocates all of its tensor memory)
+    return std::max<size_t>((size_t)Q4G_XSTAGES * Mt * 128 + (size_t)Q4G_WSTAGES * Q4U_WSTAGE_BYTES + 512 + 1024, (size_t)116 * 1024);
+}
+
+// CTA pairs the device keeps resident (0: clusters of two cannot be scheduled)
+static int q4_gemm_pairs(const mpq_context* ctx)
+{
+    static int cached[PerDeviceOnce::MAX_DEVICES];
+    static PerDeviceOnce known;
+    if (ctx->device < 0 || ctx->device >= PerDeviceOnce::MAX_DEVICES) return 0;
+    if (!known.needs(ctx->device)) return cached[ctx->device];
+    int n = 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(ctx->prop.multiProcessorCount & ~1));
+    cfg.blockDim = dim3(Q4G_THREADS);
+    cfg.dynamicSmemBytes = q4_gemm_smem(Q4G_MT_MAX);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(q4_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) != cudaSuccess ||
+        cudaFuncSetAttribute(q4g_xstage_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess ||
+        cudaFuncSetAttribute(q4g_xstage_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, q4_gemm_pair_kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    cached[ctx->device] = n;
+    known.mark(ctx->device);
+    return n;
+}
+
+// y = x . W^T for M > 64 rows; with swiglu x is [M][2K] = [gate | up].  One slab's staged rows take M * K * 4 bytes of scratch.
+static int32_t q4_gemm_forward(mpq_context* ctx, const Q4Dev& q, const float* x, bool swiglu, int M, float* y, int64_t ldy, int pairs_max, cudaStream_t s)
+{
+    int32_t st = q4_status_word(ctx);
+    if (st) return st;
+    // as few activation tiles as possible (each expands the weights again), as equal as possible, in steps of 32 rows (a
+    // quarter of the rows, eight or more, is what a team drains)
+    const int nt = (M + Q4G_MT_MAX - 1) / Q4G_MT_MAX, Mt = ((M + nt - 1) / nt + 31) / 32 * 32;
+    const int nb = (q.nrp + 7) / 8;
+    const int64_t total = (int64_t)nb * nt * q.nchunks;
+    const int W = (int)std::max<int64_t>((total + pairs_max - 1) / pairs_max, std::min<int64_t>(Q4G_MIN_W, total));
+    const int pairs = (int)((total + W - 1) / W);
+    const size_t xs_bytes = (size_t)nt * q.nchunks * 2 * Mt * 128, need = xs_bytes + (size_t)M * sizeof(float);
+    if (ctx->q4u_xs_bytes < need) {
+        CU_TRY(ctx, cudaDeviceSynchronize());
+        cudaFree(ctx->q4u_xs);
+        ctx->q4u_xs = nullptr;
+        ctx->q4u_xs_bytes = 0;
+        CU_TRY(ctx, cudaMalloc(&ctx->q4u_xs, need));
+        ctx->q4u_xs_bytes = need;
+    }
+    float* inv_sc = reinterpret_cast<float*>(ctx->q4u_xs + xs_bytes);
+    const bool cut = W % q.nchunks != 0;                   // some tile lies in more than one range
+    if (cut && (st = q4_partial_scratch(ctx, (size_t)pairs * 2 * Q4G_SLOT * sizeof(float)))) return st;
+    CUtensorMap map_x;
+    if (!make_rows128_map(&map_x, ctx->q4u_xs, (int64_t)nt * q.nchunks * 2 * Mt, Mt / 2)) return fail(ctx, MPQ_ERR_CUDA, "cuTensorMapEncodeTiled failed for the staged activations");
+
+    cudaLaunchAttribute at[1];
+    cudaLaunchConfig_t cfg = {};
+    const int cached = (size_t)q.K * 4 <= (size_t)200 * 1024;
+    cfg.gridDim = dim3((unsigned)(nt * Mt));
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = cached ? (size_t)q.K * 4 : 0;
+    cfg.stream = s;
+    launch_pdl(cfg, at, ctx->pdl);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, swiglu ? q4g_xstage_kernel<true> : q4g_xstage_kernel<false>, x, M, Mt, (int)q.K, q.nchunks, cached, ctx->q4u_xs, inv_sc);
+    ctx->launches += 1;
+    if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4g_xstage_kernel launch failed: %s", cudaGetErrorString(e));
+
+    Q4GemmLaunch p;
+    p.stream = q.stream; p.inv_sc = inv_sc; p.Y = y; p.partial = ctx->q4_rect_partial;
+    p.M = M; p.Mt = Mt; p.N = (int)q.N; p.nt = nt; p.ldy = ldy; p.nchunks = q.nchunks; p.nrp = q.nrp; p.W = W; p.total = total;
+    p.status = ctx->q4_status;
+    cfg = {};
+    cfg.gridDim = dim3((unsigned)(2 * pairs));
+    cfg.blockDim = dim3(Q4G_THREADS);
+    cfg.dynamicSmemBytes = q4_gemm_smem(Mt);
+    cfg.stream = s;
+    launch_pdl(cfg, at, ctx->pdl);
+    e = cudaLaunchKernelEx(&cfg, q4_gemm_pair_kernel, map_x, p);
+    ctx->launches += 1;
+    if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4_gemm_pair_kernel launch failed: %s", cudaGetErrorString(e));
+    if (cut) {
+        cfg = {};
+        cfg.gridDim = dim3((unsigned)std::min<int64_t>(((int64_t)nb * nt * Mt + 3) / 4, (int64_t)ctx->prop.multiProcessorCount * 16));
+        cfg.blockDim = dim3(256);
+        cfg.stream = s;
+        launch_pdl(cfg, at, ctx->pdl);
+        e = cudaLaunchKernelEx(&cfg, q4g_reduce_kernel, (const float*)ctx->q4_rect_partial, M, Mt, (int)q.N, nt, q.nchunks, W, nb * nt, y, ldy);
+        ctx->launches += 1;
+        if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4g_reduce_kernel launch failed: %s", cudaGetErrorString(e));
+    }
+    return MPQ_OK;
+}
+
+// Slabs of rows through the pair kernel: at most 2048, fewer where K is so long that the staged rows would pass 256 MB.
+static int32_t q4_gemm_slabs(mpq_context* ctx, const Q4Dev& q, const float* x, bool swiglu, int64_t M, float* y, int64_t ldy, int pairs_max, cudaStream_t s)
+{
+    const int64_t slab = std::max<int64_t>(Q4G_MT_MAX, std::min<int64_t>(2048, ((int64_t)1 << 26) / q.K / Q4G_MT_MAX * Q4G_MT_MAX));
+    for (int64_t m0 = 0; m0 < M; m0 += slab) {
+        const int32_t st = q4_gemm_forward(ctx, q, x + (size_t)m0 * q.K * (swiglu ? 2 : 1), swiglu, (int)std::min<int64_t>(slab, M - m0),
+                                           y + (size_t)m0 * ldy, ldy, pairs_max, s);
+        if (st) return st;
+    }
+    return MPQ_OK;
+}
+
+// rows that go to the pair kernel: all above 64 where the tcgen05 path is on and clusters of two can be scheduled (else 0)
+static int q4_gemm_route(const mpq_context* ctx, int64_t M)
+{
+    return (ctx->q4_gemm_min > 0 && M >= ctx->q4_gemm_min && ctx->q4_umma_min > 0 && M >= ctx->q4_umma_min) ? q4_gemm_pairs(ctx) : 0;
+}
+
 // The streaming kernel stages ALL of x in every CTA, the rectangle kernel only a K slice of it: measured on the 7B shapes,
 // from about 16 K staged elements (4 rows of K = 4096, 2 rows of K = 11008) the rectangle kernel is the faster one for
 // several rows (4096 x 11008 at 4 rows: 11.9 against 22.8 us).  One row always streams.
@@ -907,6 +1032,7 @@ static int q4_slab_rows(const mpq_context* ctx, const Q4Dev& q, int64_t M)
 static int32_t q4_forward_checked(mpq_context* ctx, const mpq_weight* w, const float* x_dev, int64_t M, float* y_dev,
                                   int64_t ldy, cudaStream_t s)
 {
+    if (const int pairs = q4_gemm_route(ctx, M)) return q4_gemm_slabs(ctx, w->q4, x_dev, false, M, y_dev, ldy, pairs, s);
     if (ctx->q4_umma_min > 0 && M >= ctx->q4_umma_min) {       // slabs of up to 64 rows on the tcgen05 path
         for (int64_t m0 = 0; m0 < M; m0 += 64) {
             int m = (int)std::min<int64_t>(64, M - m0);
@@ -1004,6 +1130,7 @@ extern "C" int32_t mpq_q4_linear_forward_swiglu(mpq_context* ctx, const mpq_weig
         p.swiglu = 1;
         return q4_stream_enqueue(ctx, pl, p, grid, s);
     }
+    if (const int pairs = q4_gemm_route(ctx, M)) return q4_gemm_slabs(ctx, q, gate_up_dev, true, M, y_dev, q.N, pairs, s);
     const size_t need = (size_t)M * q.K * sizeof(float);
     if (ctx->swiglu_bytes < need) {
         CU_TRY(ctx, cudaDeviceSynchronize());

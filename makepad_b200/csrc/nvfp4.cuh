@@ -4,6 +4,7 @@
 // No reference source exists for this path (the makepad/makepad snapshot has no
 // quantised-linear code); the operator is specified by the task configuration.
 #pragma once
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -45,6 +46,9 @@ size_t nvfp4_sf_tiled_bytes(int64_t N, int64_t K);
 void nvfp4_weight_dequant_launch(const Nvfp4Dev& w, float* out, cudaStream_t s);
 int32_t nvfp4_gemm_launch(Nvfp4Scratch& scratch, const Nvfp4Dev& w, const uint8_t* a_codes, const uint8_t* a_sf, float ta,
                           int64_t M, uint16_t* c, int device, int sm_count, cudaStream_t s, int* launches, std::string& err);
+
+// TMA map of an array of 128-byte rows, box = box_rows of them, dense (false: the driver's encoder is missing or refuses)
+bool make_rows128_map(CUtensorMap* map, const void* base, int64_t rows, int box_rows);
 
 // launches the tensor-pipe ceiling probe (see nvfp4_mma_probe_kernel); *flop = the flop it executes
 int32_t nvfp4_mma_probe_launch(Nvfp4Scratch& scratch, int device, int sm_count, int mmas, cudaStream_t s, double* flop, std::string& err);

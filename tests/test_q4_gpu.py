@@ -379,3 +379,30 @@ def test_f16_mma_issue_probe(ctx):
     assert 31.0 <= got[4] < got[1] < 400.0, got
     assert ctx.lib.mpq_probe_f16_mma(ctx.h, 24, 1, 1024, C.byref(cyc)) == _lib.ERR_INVALID_ARG
     assert ctx.lib.mpq_context_poll_status(ctx.h) == _lib.OK
+
+
+# one ragged tile; tiles of 32 x 3; a pair-tile short of a group; whole tiles and cut ones; one chunk per segment; long K (many
+# pieces of one tile); several activation tiles with a ragged last one; more rows than one launch stages
+@pytest.mark.parametrize("N,K,M", [(1, 32, 65), (40, 160, 65), (257, 1120, 96), (1000, 2112, 300), (4096, 4096, 256), (20000, 64, 129),
+                                   (96, 28672, 70), (4096, 11008, 128), (2500, 1056, 513), (33, 288, 2100)])
+def test_pair_kernel_above_64_rows(ctx, orc, N, K, M):
+    """The CTA-pair kernel against the binary64 oracle (the bound of the other tcgen05 kernel: the arithmetic is the same),
+    nothing written outside the output, the same bits twice, and the SwiGLU form equal to the unfused one bit for bit."""
+    import makepad_b200
+    torch = _torch()
+    codes, scales = synth.q4_weight(N, K, seed=15)
+    lin = makepad_b200.QuantLinear(makepad_b200.Q4Weight(ctx, codes, scales))
+    x = synth.activations(M, K, seed=16)
+    buf = torch.full((M * N + 256,), 777.0, device="cuda")
+    y = buf[128:128 + M * N].view(M, N)
+    xd = torch.from_numpy(x).cuda()
+    lin.forward(xd, out=y)
+    torch.cuda.synchronize()
+    rep = orc.err_report(y.cpu().numpy(), orc.q4_matmul_f64(codes, scales, x))
+    assert rep["floored_1e-2_rms"] < TOL and rep["max_abs_over_rms"] < 2e-5, rep
+    assert (buf[:128] == 777.0).all() and (buf[128 + M * N:] == 777.0).all()
+    assert torch.equal(y, lin(xd))
+    gate_up = torch.from_numpy(synth.activations(M, 2 * K, seed=17)).cuda()
+    assert torch.equal(lin.forward_swiglu(gate_up), lin(makepad_b200.swiglu(ctx, gate_up)))
+    torch.cuda.synchronize()
+    assert ctx.lib.mpq_context_poll_status(ctx.h) == _lib.OK
