@@ -9,7 +9,10 @@
 // tile one expansion feeds 12 MMAs of N = 256 = 1536 cycles of tensor pipe, and the kernel is bound by the tensor pipe.
 // One SM would have to fetch 64 KB of staged activations per 1536 cycles, about what L2 delivers when every SM asks; the
 // pair (tcgen05 cta_group::2, M = 256) fetches half the tile per SM.
-// <MEASURED>
+// Measured, 22016 x 4096, slabs of 64 rows / this kernel: 112 / 86 us at 96 rows, 118 / 88 at 128, 236 / 119 at 256,
+// 475 / 217 at 512 (1280 TFLOP/s of fp16 products, 92% of what a plain bf16 GEMM sustains under the power limit); 4096 x 11008:
+// 94 / 58 at 128, 380 / 116 at 512; 57344 x 8192 at 96 / 128 / 256 rows: 343 / 353, 367 / 358, 757 / 501.  Below 65 rows one pass
+// of the other kernel is the faster one (60 / 83 us at 64 rows): here the MMAs of a chunk cost the same for any Mt up to 128.
 //
 // WORK.  Tile = 256 weight rows x Mt activation rows, numbered activation tile fastest; the (tile, chunk) sequence is cut
 // into equal ranges of W chunks, one per pair, so that any shape fills the SMs.  A tile inside one range is stored to y; the
@@ -110,10 +113,11 @@ __device__ __forceinline__ uint32_t q4g_map_to_leader(uint32_t addr)
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(0u));
     return r;
 }
-// arrive on a barrier of the pair's leader; what it hands over went through tcgen05 fences (tensor memory)
+// Arrive on a barrier of the pair's leader.  What it hands over went through tcgen05 fences (tensor memory), so it is
+// relaxed: a release at cluster scope waits for the thread's stores to y as well (about 2000 cycles per hand-off)
 __device__ __forceinline__ void q4g_arrive_leader(uint32_t cluster_addr)
 {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ void q4g_cluster_sync()
 {
@@ -228,30 +232,46 @@ q4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             x.next(p.nchunks);
         }
     } else if (warp == 17) {
-        // ---------------- MMA issue: one thread of the leader ----------------
-        if (rank == 0 && lane == 0) {
+        // ---------------- MMA issue: a warp of the leader ----------------
+        // (a lane that is alone in its branch issues an MMA every 110 cycles, an elected lane of a whole warp every 45)
+        if (rank == 0) {
             const uint32_t idesc = (1u << 4) | ((uint32_t)(p.Mt >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);      // f16 x f16 -> f32, K-major both, 256 x Mt
             int xs = 0, as = 0, drains = 0;
-            uint32_t xph = 0, aph = 0;
+            uint32_t xph = 0, aph = 0, x_seen = 0, a_seen = 0;                   // the current chunk's barriers were seen complete
             for (Q4GWalk w(L_begin, count, p.nchunks); w.left; w.next(p.nchunks)) {
-                if (!q4u_bar_wait(x_full + 8 * xs, xph)) { atomicExch(p.status, 43); s_abort = 1; break; }
-                if (!q4u_bar_wait(a_full + 8 * as, aph)) { atomicExch(p.status, 44); s_abort = 1; break; }
+                if (!x_seen && !q4u_bar_wait(x_full + 8 * xs, xph)) { if (lane == 0) { atomicExch(p.status, 43); s_abort = 1; } break; }
+                if (!a_seen && !q4u_bar_wait(a_full + 8 * as, aph)) { if (lane == 0) { atomicExch(p.status, 44); s_abort = 1; } break; }
                 // a new segment overwrites the accumulator: both CTAs must have drained the last one
-                if (w.seg_n == 0 && drains > 0 && !q4u_bar_wait(d_empty, (uint32_t)(drains - 1) & 1u)) { atomicExch(p.status, 45); s_abort = 1; break; }
+                if (w.seg_n == 0 && drains > 0 && !q4u_bar_wait(d_empty, (uint32_t)(drains - 1) & 1u)) { if (lane == 0) { atomicExch(p.status, 45); s_abort = 1; } break; }
                 q4u_fence_after();
                 const uint64_t bhi = q4u_desc_sw128(xring + xs * xstage_bytes), blo = q4u_desc_sw128(xring + xs * xstage_bytes + xstage_bytes / 2);
                 const uint32_t a = tmem + Q4U_A_COL + (uint32_t)as * 64;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {                                    // K steps of 16: +32 bytes along K = +2 in the descriptor
-                    q4g_mma_pair(tmem, a + j * 16, bhi + 2 * j, idesc, (w.seg_n > 0 || j > 0) ? 1u : 0u);
-                    q4g_mma_pair(tmem, a + j * 16, blo + 2 * j, idesc, 1u);
-                    q4g_mma_pair(tmem, a + j * 16 + 8, bhi + 2 * j, idesc, 1u);
-                }
-                q4g_commit_pair(a_empty + 8 * as);
-                q4g_commit_pair(x_empty + 8 * xs);
-                if (w.seg_last(p.nchunks)) { q4g_commit_pair(d_full); ++drains; }
+                const uint32_t x_now = x_empty + 8 * xs, a_now = a_empty + 8 * as;
+                const bool last = w.seg_last(p.nchunks);
                 if (++xs == Q4G_XSTAGES) { xs = 0; xph ^= 1u; }
                 if (++as == Q4G_ASTAGES) { as = 0; aph ^= 1u; }
+                if (q4u_elect_one()) {
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) {                                // K steps of 16: +32 bytes along K = +2 in the descriptor
+                        q4g_mma_pair(tmem, a + j * 16, bhi + 2 * j, idesc, (w.seg_n > 0 || j > 0) ? 1u : 0u);
+                        q4g_mma_pair(tmem, a + j * 16, blo + 2 * j, idesc, 1u);
+                        q4g_mma_pair(tmem, a + j * 16 + 8, bhi + 2 * j, idesc, 1u);
+                    }
+                }
+                __syncwarp();
+                // a test's round trip is longer than an MMA's issue: the next chunk's barriers are looked at in between
+                x_seen = q4u_bar_test(x_full + 8 * xs, xph);
+                a_seen = q4u_bar_test(a_full + 8 * as, aph);
+                if (q4u_elect_one()) {
+                    q4g_mma_pair(tmem, a + 48, bhi + 6, idesc, 1u);
+                    q4g_mma_pair(tmem, a + 48, blo + 6, idesc, 1u);
+                    q4g_mma_pair(tmem, a + 56, bhi + 6, idesc, 1u);
+                    q4g_commit_pair(a_now);
+                    q4g_commit_pair(x_now);
+                    if (last) q4g_commit_pair(d_full);
+                }
+                __syncwarp();
+                drains += last;
             }
         }
     } else {
@@ -354,26 +374,26 @@ q4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 __syncwarp();
                 if (lane == 0) q4g_arrive_leader(lead_d_empty);                      // the next segment may overwrite the accumulator
                 if (pending_piece) {
-                // the piece's sums: to y when this range holds the whole tile, else to the range's slot
-                if (!waited) {
-                    asm volatile("griddepcontrol.wait;" ::: "memory");               // inv_sc, and y and the slots may still be read
-                    waited = true;
-                }
-                const int b = pending_tile / p.nt, t = pending_tile - b * p.nt, m0 = t * p.Mt + team * cpt;
-                const float isc0 = lane < cpt && m0 + lane < p.M ? p.inv_sc[m0 + lane] : 0.f;
-                const float isc1 = lane + 32 < cpt && m0 + lane + 32 < p.M ? p.inv_sc[m0 + lane + 32] : 0.f;
-                const int col = (int)rank * 128 + qd * 32 + lane, nrow = b * 256 + col;
-                const bool whole = (int64_t)pending_tile * p.nchunks >= L_begin && ((int64_t)pending_tile + 1) * p.nchunks <= L_end;
-                float* out = whole ? p.Y + (size_t)m0 * p.ldy + nrow
-                                   : p.partial + ((size_t)pair * 2 + (pending_tile != first_tile)) * Q4G_SLOT + (size_t)team * cpt * 256 + col;
-                const int64_t ld = whole ? p.ldy : 256;
-                const bool mine = !whole || nrow < p.N;
+                    // the piece's sums: to y when this range holds the whole tile, else to the range's slot
+                    if (!waited) {
+                        asm volatile("griddepcontrol.wait;" ::: "memory");               // inv_sc, and y and the slots may still be read
+                        waited = true;
+                    }
+                    const int b = pending_tile / p.nt, t = pending_tile - b * p.nt, m0 = t * p.Mt + team * cpt;
+                    const float isc0 = lane < cpt && m0 + lane < p.M ? p.inv_sc[m0 + lane] : 0.f;
+                    const float isc1 = lane + 32 < cpt && m0 + lane + 32 < p.M ? p.inv_sc[m0 + lane + 32] : 0.f;
+                    const int col = (int)rank * 128 + qd * 32 + lane, nrow = b * 256 + col;
+                    const bool whole = (int64_t)pending_tile * p.nchunks >= L_begin && ((int64_t)pending_tile + 1) * p.nchunks <= L_end;
+                    float* out = whole ? p.Y + (size_t)m0 * p.ldy + nrow
+                                       : p.partial + ((size_t)pair * 2 + (pending_tile != first_tile)) * Q4G_SLOT + (size_t)team * cpt * 256 + col;
+                    const int64_t ld = whole ? p.ldy : 256;
+                    const bool mine = !whole || nrow < p.N;
 #pragma unroll
-                for (int i = 0; i < Q4G_MT_MAX / 4; ++i) {
-                    const float sc = __shfl_sync(0xFFFFFFFFu, i < 32 ? isc0 : isc1, i & 31);
-                    if (i < cpt && mine && m0 + i < p.M) out[(size_t)i * ld] = racc[i] * sc;
-                    racc[i] = 0.f;
-                }
+                    for (int i = 0; i < Q4G_MT_MAX / 4; ++i) {
+                        const float sc = __shfl_sync(0xFFFFFFFFu, i < 32 ? isc0 : isc1, i & 31);
+                        if (i < cpt && mine && m0 + i < p.M) out[(size_t)i * ld] = racc[i] * sc;
+                        racc[i] = 0.f;
+                    }
                 }
             }
             if (!w.left) break;
@@ -396,7 +416,7 @@ q4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     }
 }
 
-// y of the tiles that were cut: their pieces' slots added in order.  One warp per (tile, row): 64 lanes x float4 would be two.
+// y of the tiles that were cut: their pieces' slots added in order.  64 threads x float4 per (tile, row).
 __global__ void __launch_bounds__(256) q4g_reduce_kernel(const float* __restrict__ partial, int M, int Mt, int N, int nt, int nchunks, int W, int ntiles,
                                                           float* __restrict__ Y, int64_t ldy)
 {
