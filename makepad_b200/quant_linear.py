@@ -28,6 +28,13 @@ def _np_ptr(a: np.ndarray):
     return C.c_void_p(a.ctypes.data)
 
 
+def _stream() -> int:
+    """The current stream of the current device.  (The stream object that torch.cuda.current_stream() builds costs more host
+    time than the launch itself.)"""
+    import torch
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
 class Context:
     """One per (process, GPU)."""
 
@@ -41,7 +48,7 @@ class Context:
         self.device = device
 
     def check(self, st: int):
-        if st != _lib.OK:
+        if st:                                                 # anything but OK (0)
             raise MpqError(st, f"{self.lib.mpq_status_string(st).decode()}: {self.lib.mpq_last_error(self.h).decode()}")
 
     def info(self) -> _lib.DeviceInfo:
@@ -80,8 +87,7 @@ class _Weight:
         """Exact fp32 [N][K] export read back from the device layout (torch tensor on the GPU)."""
         import torch
         out = torch.empty((self.N, self.K), dtype=torch.float32, device=f"cuda:{self.ctx.device}")
-        self.ctx.check(self.ctx.lib.mpq_weight_dequantize(self.ctx.h, self.h, C.c_void_p(out.data_ptr()),
-                                                          C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        self.ctx.check(self.ctx.lib.mpq_weight_dequantize(self.ctx.h, self.h, out.data_ptr(), _stream()))
         return out
 
     def save(self, path: str):
@@ -195,18 +201,15 @@ class QuantLinear:
                 return y
             if x.dtype != torch.float32 or not x.is_cuda or not x.is_contiguous():
                 raise MpqError(_lib.ERR_INVALID_ARG, "x must be a contiguous fp32 CUDA tensor")
-            x2 = x.reshape(-1, w.K)
+            x2 = x if x.dim() == 2 and x.shape[1] == w.K else x.reshape(-1, w.K)
             y = torch.empty((x2.shape[0], w.N), dtype=torch.float32, device=x.device) if out is None else out
-            ctx.check(ctx.lib.mpq_q4_linear_forward(ctx.h, w.h, C.c_void_p(x2.data_ptr()), x2.shape[0],
-                                                    C.c_void_p(y.data_ptr()),
-                                                    C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+            ctx.check(ctx.lib.mpq_q4_linear_forward(ctx.h, w.h, x2.data_ptr(), x2.shape[0], y.data_ptr(), _stream()))
             return y
         codes, sf, ts = x
         M = codes.shape[0]
         y = torch.empty((M, w.N), dtype=torch.bfloat16, device=codes.device) if out is None else out
-        ctx.check(ctx.lib.mpq_nvfp4_gemm_forward(ctx.h, w.h, C.c_void_p(codes.data_ptr()), C.c_void_p(sf.data_ptr()),
-                                                 C.c_float(ts), M, C.c_void_p(y.data_ptr()),
-                                                 C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        ctx.check(ctx.lib.mpq_nvfp4_gemm_forward(ctx.h, w.h, codes.data_ptr(), sf.data_ptr(),
+                                                 C.c_float(ts), M, y.data_ptr(), _stream()))
         return y
 
     __call__ = forward
@@ -220,10 +223,9 @@ class QuantLinear:
             raise MpqError(_lib.ERR_INVALID_ARG, "forward_swiglu is for Q4 weights")
         if gate_up.dtype != torch.float32 or not gate_up.is_cuda or not gate_up.is_contiguous():
             raise MpqError(_lib.ERR_INVALID_ARG, "gate_up must be a contiguous fp32 CUDA tensor")
-        g2 = gate_up.reshape(-1, 2 * w.K)
+        g2 = gate_up if gate_up.dim() == 2 and gate_up.shape[1] == 2 * w.K else gate_up.reshape(-1, 2 * w.K)
         y = torch.empty((g2.shape[0], w.N), dtype=torch.float32, device=gate_up.device) if out is None else out
-        ctx.check(ctx.lib.mpq_q4_linear_forward_swiglu(ctx.h, w.h, C.c_void_p(g2.data_ptr()), g2.shape[0], C.c_void_p(y.data_ptr()),
-                                                       C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        ctx.check(ctx.lib.mpq_q4_linear_forward_swiglu(ctx.h, w.h, g2.data_ptr(), g2.shape[0], y.data_ptr(), _stream()))
         return y
 
 
@@ -232,8 +234,7 @@ def swiglu(ctx: Context, gate_up):
     import torch
     M, F2 = gate_up.shape
     out = torch.empty((M, F2 // 2), dtype=torch.float32, device=gate_up.device)
-    ctx.check(ctx.lib.mpq_swiglu(ctx.h, C.c_void_p(gate_up.data_ptr()), M, F2 // 2, C.c_void_p(out.data_ptr()),
-                                 C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    ctx.check(ctx.lib.mpq_swiglu(ctx.h, gate_up.data_ptr(), M, F2 // 2, out.data_ptr(), _stream()))
     return out
 
 
@@ -246,6 +247,6 @@ def nvfp4_quantize(ctx: Context, x, tensor_scale: float = 1.0, swiglu_fused: boo
     codes = torch.empty((M, K // 2), dtype=torch.uint8, device=x.device)
     sf = torch.empty((M, K // 16), dtype=torch.uint8, device=x.device)
     fn = ctx.lib.mpq_nvfp4_quantize_swiglu if swiglu_fused else ctx.lib.mpq_nvfp4_quantize_activations
-    ctx.check(fn(ctx.h, C.c_void_p(x.data_ptr()), 1 if x.dtype == torch.bfloat16 else 0, M, K, C.c_float(tensor_scale),
-                 C.c_void_p(codes.data_ptr()), C.c_void_p(sf.data_ptr()), C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    ctx.check(fn(ctx.h, x.data_ptr(), 1 if x.dtype == torch.bfloat16 else 0, M, K, C.c_float(tensor_scale),
+                 codes.data_ptr(), sf.data_ptr(), _stream()))
     return codes, sf
