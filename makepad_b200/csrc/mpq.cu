@@ -328,8 +328,8 @@ extern "C" int32_t mpq_q4_weight_create(mpq_context* ctx, int64_t N, int64_t K, 
     uint16_t* ds = reinterpret_cast<uint16_t*>(dc + (size_t)slab * row_codes);          // 32 rows x 16 bytes and up: aligned
     for (int64_t r = 0; r < n && e == cudaSuccess; r += slab) {
         const int64_t rows = std::min(slab, n - r);
-        ctx->upload.run(ctx->device, dc, codes_host + (size_t)(row0 + r) * row_codes, -1, 0, (size_t)rows * row_codes, ctx->upload_stream, &e);
-        if (e == cudaSuccess) ctx->upload.run(ctx->device, ds, scales_host + (size_t)(row0 + r) * (K / 32), -1, 0, (size_t)rows * row_scales, ctx->upload_stream, &e);
+        ctx->upload.run(dc, codes_host + (size_t)(row0 + r) * row_codes, -1, 0, (size_t)rows * row_codes, ctx->upload_stream, &e);
+        if (e == cudaSuccess) ctx->upload.run(ds, scales_host + (size_t)(row0 + r) * (K / 32), -1, 0, (size_t)rows * row_scales, ctx->upload_stream, &e);
         if (e == cudaSuccess) e = q4_repack(ctx, w->q4, (int)(r / 32), rows, K, dc, ds, k0, ctx->upload_stream);
     }
     const cudaError_t done = cudaStreamSynchronize(ctx->upload_stream);
@@ -1703,7 +1703,7 @@ extern "C" int32_t mpq_weight_load(mpq_context* ctx, const char* path, mpq_weigh
     int64_t at = (int64_t)sizeof h;
     for (int i = 0; i < 2 && e == cudaSuccess && st == MPQ_OK; at += bytes[i], ++i) {
         if (!bytes[i]) continue;
-        if (ctx->upload.run(ctx->device, part[i], nullptr, fileno(f), at, (size_t)bytes[i], ctx->upload_stream, &e) == StagedUpload::READ_FAILED) st = MPQ_ERR_IO;
+        if (ctx->upload.run(part[i], nullptr, fileno(f), at, (size_t)bytes[i], ctx->upload_stream, &e) == StagedUpload::READ_FAILED) st = MPQ_ERR_IO;
         if (st == MPQ_OK && e == cudaSuccess) e = fnv1a64_device(part[i], bytes[i], &sum, ctx->upload.staging(fnv1a64_scratch_bytes(bytes[i])), ctx->upload_stream);
     }
     fclose(f);
