@@ -1458,7 +1458,7 @@ extern "C" int32_t mpq_nvfp4_gemm_forward(mpq_context* ctx, const mpq_weight* w,
     std::string err;
     int launches = 0;
     int32_t st = nvfp4_gemm_launch(ctx->fp4, w->fp4, a_codes_dev, a_sf_dev, a_tensor_scale, M, c_bf16_dev, ctx->device,
-                                   ctx->prop.multiProcessorCount, (cudaStream_t)stream, &launches, err);
+                                   ctx->prop.multiProcessorCount, ctx->pdl, (cudaStream_t)stream, &launches, err);
     ctx->launches += launches;
     if (st) return fail(ctx, st, "%s", err.c_str());
     return MPQ_OK;
@@ -1488,7 +1488,7 @@ extern "C" int32_t mpq_nvfp4_quantize_activations(mpq_context* ctx, const void* 
     CU_TRY(ctx, cudaSetDevice(ctx->device));
     nvfp4_quantize_launch(x_dev, x_is_bf16 != 0, false, M, K, tensor_scale, codes_dev, sf_dev, (cudaStream_t)stream);
     ctx->launches += 1;
-    CU_TRY(ctx, cudaGetLastError());
+    CU_TRY(ctx, nvfp4_quantize_launch(gate_up_dev, x_is_bf16 != 0, true, M, F, tensor_scale, codes_dev, sf_dev, ctx->pdl, (cudaStream_t)stream));
     return MPQ_OK;
 }
 
@@ -1503,7 +1503,7 @@ extern "C" int32_t mpq_nvfp4_quantize_swiglu(mpq_context* ctx, const void* gate_
     CU_TRY(ctx, cudaSetDevice(ctx->device));
     nvfp4_quantize_launch(gate_up_dev, x_is_bf16 != 0, true, M, F, tensor_scale, codes_dev, sf_dev, (cudaStream_t)stream);
     ctx->launches += 1;
-    CU_TRY(ctx, cudaGetLastError());
+    CU_TRY(ctx, nvfp4_quantize_launch(x_dev, x_is_bf16 != 0, false, M, K, tensor_scale, codes_dev, sf_dev, ctx->pdl, (cudaStream_t)stream));
     return MPQ_OK;
 }
 

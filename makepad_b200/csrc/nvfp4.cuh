@@ -31,21 +31,23 @@ struct Nvfp4Dev {
 struct Nvfp4Scratch {
     uint8_t* sfa_tiled = nullptr;      // activation scale factors re-tiled per call
     size_t sfa_bytes = 0;
+    float* partial = nullptr;          // fp32 sums of tiles cut along K (at most one wave of tiles: 17 MB)
+    size_t partial_bytes = 0;
     int* status = nullptr;             // set non-zero when a bounded wait in the GEMM kernel ran out
-    void release() { cudaFree(sfa_tiled); cudaFree(status); sfa_tiled = nullptr; status = nullptr; sfa_bytes = 0; }
+    void release() { cudaFree(sfa_tiled); cudaFree(status); cudaFree(partial); sfa_tiled = nullptr; status = nullptr; partial = nullptr; sfa_bytes = partial_bytes = 0; }
 };
 
 void nvfp4_dequant_launch(const uint8_t* codes, const uint8_t* sf, float ts, int64_t R, int64_t K, float* out, cudaStream_t s);
 int32_t nvfp4_weight_build(Nvfp4Dev& w, int64_t N, int64_t K, const uint8_t* codes_host, const uint8_t* sf_host, float ts,
                            int* launches, std::string& err);
 // fp32 (or bf16) rows -> canonical NVFP4 codes [R][K/2] and e4m3 scales [R][K/16]
-void nvfp4_quantize_launch(const void* x, bool bf16, bool swiglu, int64_t R, int64_t K, float ts, uint8_t* codes, uint8_t* sf, cudaStream_t s);
+cudaError_t nvfp4_quantize_launch(const void* x, bool bf16, bool swiglu, int64_t R, int64_t K, float ts, uint8_t* codes, uint8_t* sf, bool pdl, cudaStream_t s);
 // bytes of a weight's tiled scale factors in the current layout
 size_t nvfp4_sf_tiled_bytes(int64_t N, int64_t K);
 // exact fp32 export [N][K] of a weight, its scale factors read back from the tiled device layout
 void nvfp4_weight_dequant_launch(const Nvfp4Dev& w, float* out, cudaStream_t s);
 int32_t nvfp4_gemm_launch(Nvfp4Scratch& scratch, const Nvfp4Dev& w, const uint8_t* a_codes, const uint8_t* a_sf, float ta,
-                          int64_t M, uint16_t* c, int device, int sm_count, cudaStream_t s, int* launches, std::string& err);
+                          int64_t M, uint16_t* c, int device, int sm_count, bool pdl, cudaStream_t s, int* launches, std::string& err);
 
 // TMA map of an array of 128-byte rows, box = box_rows of them, dense (false: the driver's encoder is missing or refuses)
 bool make_rows128_map(CUtensorMap* map, const void* base, int64_t rows, int box_rows);

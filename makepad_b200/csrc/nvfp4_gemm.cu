@@ -117,6 +117,25 @@ __device__ __forceinline__ uint32_t f32_to_e2m1_sat(float f)
     return sign | m;
 }
 
+// |v| / d for 2^-73 <= d <= 2^73 and r = 1/d correctly rounded, as e2m1 sees it.  The quotient of a multiplication by r,
+// corrected once by its exact remainder, is the correctly rounded quotient (P. Markstein, "Computation of elementary functions
+// on the IBM RISC System/6000 processor", 1990) unless something leaves the exponent range: a tiny |v| stays far below the
+// grid's first step (0.25), an infinite or overflowing product ends as NaN and is taken as 8, which saturates.
+__device__ __forceinline__ float e2m1_quotient(float v, float d, float r)
+{
+    const float x = fabsf(v), q = x * r;
+    return copysignf(fminf(fmaf(fmaf(-q, d, x), r, q), 8.f), v);
+}
+// f32_to_e2m1_sat(v0 / d) | f32_to_e2m1_sat(v1 / d) << 4, by the conversion instruction (ties to even, saturating).  A NaN
+// gives +6, whatever its sign, as the quotient of a NaN has no sign.
+__device__ __forceinline__ uint32_t e2m1x2_div_sat(float v0, float v1, float d, float r)
+{
+    const float q0 = v0 == v0 ? e2m1_quotient(v0, d, r) : 8.f, q1 = v1 == v1 ? e2m1_quotient(v1, d, r) : 8.f;
+    uint32_t out;
+    asm("{\n\t.reg .b8 b;\n\tcvt.rn.satfinite.e2m1x2.f32 b, %2, %1;\n\tcvt.u32.u8 %0, b;\n\t}" : "=r"(out) : "f"(q0), "f"(q1));
+    return out;
+}
+
 // 16 consecutive elements starting at element `at` of a row-major fp32 or bf16 array
 template <bool BF16>
 __device__ __forceinline__ void nvfp4_load16(const void* xin, int64_t at, float (&v)[16])
@@ -143,11 +162,16 @@ __device__ __forceinline__ void nvfp4_load16(const void* xin, int64_t at, float 
     }
 }
 
+// Bound by instruction issue: with a division and seven comparisons per element 1000 x 14336 took 21.6 us (fp32; bf16 21.2,
+// SwiGLU of bf16 33.3); with one reciprocal per block and the conversion instruction 9.4 (8.8, 20.6); 2048 x 4096 bf16
+// 13.4 -> 5.6.  (These times include what launching beside the kernel before saves, about 2 us of each.)
 // SWIGLU: the input is [R][2K] = [gate | up] and what is quantised is silu(gate) * up (fp32), never written to memory.
 template <bool BF16, bool SWIGLU>
 __global__ void nvfp4_quantize_kernel(const void* __restrict__ xin, int64_t R, int64_t K, float ts, uint8_t* __restrict__ codes,
                                       uint8_t* __restrict__ sf)
 {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int64_t blk = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (blk >= R * (K / 16)) return;
     float v[16];
@@ -167,7 +191,15 @@ __global__ void nvfp4_quantize_kernel(const void* __restrict__ xin, int64_t R, i
     const uint32_t s8 = f32_to_e4m3_sat(__fdiv_rn(amax, 6.0f * ts));
     const float d = e4m3_value(s8) * ts;
     uint32_t lo = 0, hi = 0;
-    if (d > 0.f) {
+    if (d > 0.f && ts >= 0x1p-64f && ts <= 0x1p64f) {
+        // One reciprocal per block instead of sixteen divisions; the same codes (see e2m1x2_div_sat).
+        const float r = __frcp_rn(d);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            lo |= e2m1x2_div_sat(v[2 * i], v[2 * i + 1], d, r) << (8 * i);
+            hi |= e2m1x2_div_sat(v[8 + 2 * i], v[9 + 2 * i], d, r) << (8 * i);
+        }
+    } else if (d > 0.f) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             lo |= f32_to_e2m1_sat(__fdiv_rn(v[i], d)) << (4 * i);
@@ -178,17 +210,20 @@ __global__ void nvfp4_quantize_kernel(const void* __restrict__ xin, int64_t R, i
     sf[blk] = (uint8_t)s8;
 }
 
-void nvfp4_quantize_launch(const void* x, bool bf16, bool swiglu, int64_t R, int64_t K, float ts, uint8_t* codes, uint8_t* sf, cudaStream_t s)
+cudaError_t nvfp4_quantize_launch(const void* x, bool bf16, bool swiglu, int64_t R, int64_t K, float ts, uint8_t* codes, uint8_t* sf, bool pdl, cudaStream_t s)
 {
-    const int64_t blocks = R * (K / 16);
-    const unsigned grid = (unsigned)((blocks + 255) / 256);
-    if (swiglu) {
-        if (bf16) nvfp4_quantize_kernel<true, true><<<grid, 256, 0, s>>>(x, R, K, ts, codes, sf);
-        else nvfp4_quantize_kernel<false, true><<<grid, 256, 0, s>>>(x, R, K, ts, codes, sf);
-    } else {
-        if (bf16) nvfp4_quantize_kernel<true, false><<<grid, 256, 0, s>>>(x, R, K, ts, codes, sf);
-        else nvfp4_quantize_kernel<false, false><<<grid, 256, 0, s>>>(x, R, K, ts, codes, sf);
-    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((R * (K / 16) + 255) / 256));
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = pdl ? 1u : 0u;
+    auto kern = swiglu ? (bf16 ? nvfp4_quantize_kernel<true, true> : nvfp4_quantize_kernel<false, true>)
+                       : (bf16 ? nvfp4_quantize_kernel<true, false> : nvfp4_quantize_kernel<false, false>);
+    return cudaLaunchKernelEx(&cfg, kern, x, R, K, ts, codes, sf);
 }
 
 // ---------------------------------------------------------------------------
@@ -765,7 +800,22 @@ struct PairParams {
     float scale;
     int* status;
     int sfa_direct;          // 1: the activations' scale factors are read from their canonical [M][K/16] array (K % 256 == 0)
+    int whole, splits;       // items [0, whole) are whole tiles; behind them every tile is `splits` items, cut along K
+    int items;
+    float* partial;          // [items - whole][256][BN] fp32 sums of the cut tiles' items
 };
+
+// item -> tile and its range of K blocks
+__device__ __forceinline__ int pair_item(const PairParams& p, int item, int* kb0, int* kb1)
+{
+    *kb0 = 0;
+    *kb1 = p.k_blocks;
+    if (item < p.whole) return item;
+    const int r = item - p.whole, t = r / p.splits, s = r - t * p.splits;
+    *kb0 = p.k_blocks * s / p.splits;
+    *kb1 = p.k_blocks * (s + 1) / p.splits;
+    return p.whole + t;
+}
 
 // ---------------------------------------------------------------------------
 // the default kernel where clusters of two can be scheduled
@@ -783,6 +833,7 @@ constexpr int Q_STAGE_BYTES = A_BYTES + P_BH_BYTES + SFA_BYTES + SFB_BYTES;     
 constexpr int Q_OUT_COLS = 16;                                                  // columns per TMA store of one epilogue warp
 constexpr int Q_OUT_BYTES = 32 * Q_OUT_COLS * 2;                                // 1024: 32 rows of bf16, dense
 constexpr int Q_SMEM_BYTES = Q_STAGES * Q_STAGE_BYTES + 8 * Q_OUT_BYTES + 1024 + 256;
+constexpr int SPLIT_MIN_BLOCKS = 2;                                             // fewest K blocks of an item of a tile that is cut along K
 static_assert(V2_EPI_COLS % Q_OUT_COLS == 0 && (Q_OUT_COLS * 2) % 16 == 0, "store boxes tile the epilogue columns in 16-byte units");
 static_assert(V2_SF_COL + Q_STAGES * V2_SF_COLS <= TMEM_COLS, "scale-factor buffers must fit beside the accumulator");
 
@@ -804,7 +855,6 @@ nvfp4_gemm_pair_kernel_v2(const __grid_constant__ CUtensorMap map_a, const __gri
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();                 // 0 = leader of the pair
     const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
-    const int total_tiles = p.m_pairs * p.n_tiles;
     constexpr uint32_t AB_BYTES = A_BYTES + P_BH_BYTES, SF_BYTES = SFA_BYTES + SFB_BYTES;
 
     if (threadIdx.x == 0) {
@@ -828,18 +878,21 @@ nvfp4_gemm_pair_kernel_v2(const __grid_constant__ CUtensorMap map_a, const __gri
     cluster_sync_all();                                      // both CTAs' barriers exist before anyone signals them
     tc_fence_after();
     const uint32_t tmem = s_tmem_base;
+    asm volatile("griddepcontrol.launch_dependents;");
 
     if (warp == 0) {
         // ---------------- producer (both CTAs; the leader arms the shared full barrier) ----------------
         if (lane == 0) {
             int stage = 0;
             uint32_t phase = 0;
-            for (int tile = pair; tile < total_tiles && !s_abort; tile += npairs) {
-                const int nt = tile / p.m_pairs, mp = tile - nt * p.m_pairs;
+            asm volatile("griddepcontrol.wait;" ::: "memory");     // A and its scale factors are the kernel's before this one
+            for (int item = pair; item < p.items && !s_abort; item += npairs) {
+                int kb0, kb1;
+                const int tile = pair_item(p, item, &kb0, &kb1), nt = tile / p.m_pairs, mp = tile - nt * p.m_pairs;
                 const int mt128 = 2 * mp + (int)rank;
                 const uint8_t* sfa_t = sfa + (size_t)mt128 * p.ksteps_pad * 512;
                 const uint8_t* sfb_t = sfb + (size_t)nt * p.ksteps_pad * 1024;
-                for (int kb = 0; kb < p.k_blocks; ++kb) {
+                for (int kb = kb0; kb < kb1; ++kb) {
                     if (!bar_spin(bar_empty + 8 * stage, phase ^ 1u, SPIN_LIMIT)) { atomicExch(p.status, 13); s_abort = 1; break; }
                     const uint32_t st = smem0 + stage * Q_STAGE_BYTES, full = bar_full + 8 * stage, sf_full = bar_sf_full + 8 * stage;
                     bar_expect_tx(sf_full, SF_BYTES);
@@ -857,19 +910,19 @@ nvfp4_gemm_pair_kernel_v2(const __grid_constant__ CUtensorMap map_a, const __gri
         // ---------------- MMA issuer: the leader only ----------------
         if (lane == 0 && rank == 0) {
             const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
-            const int my_tiles = pair < total_tiles ? (total_tiles - 1 - pair) / npairs + 1 : 0;
-            const long long total_kb = (long long)my_tiles * p.k_blocks;
-            long long done_kb = 0;
+            const int my_items = pair < p.items ? (p.items - 1 - pair) / npairs + 1 : 0;
             int stage = 0;
             uint32_t phase = 0;
             bool seen = false, ok = true;
             const uint64_t adesc0 = smem_desc_sw128(smem0), bdesc0 = smem_desc_sw128(smem0 + A_BYTES);
             const uint32_t sfc0 = tmem + V2_SF_COL;
             uint32_t soff = 0, sfoff = 0;              // stage * (Q_STAGE_BYTES >> 4), stage * V2_SF_COLS
-            for (int local = 0; local < my_tiles && ok && !s_abort; ++local) {
+            for (int local = 0; local < my_items && ok && !s_abort; ++local) {
+                int kb0, kb1;
+                pair_item(p, pair + local * npairs, &kb0, &kb1);
                 if (local > 0 && !bar_spin(bar_acc_empty, (uint32_t)(local - 1) & 1u, SPIN_LIMIT)) { atomicExch(p.status, 14); s_abort = 1; break; }
                 tc_fence_after();
-                for (int kb = 0; kb < p.k_blocks; ++kb) {
+                for (int kb = kb0; kb < kb1; ++kb) {
                     if (!seen) {
                         ok = bar_spin(bar_sf_ready + 8 * stage, phase, SPIN_LIMIT);
                         ok = ok && bar_spin(bar_full + 8 * stage, phase, SPIN_LIMIT);
@@ -881,12 +934,11 @@ nvfp4_gemm_pair_kernel_v2(const __grid_constant__ CUtensorMap map_a, const __gri
                     // the next K block's two barriers and the fence are spread over the gaps, the address arithmetic is a few adds.
                     const uint64_t adesc = adesc0 + soff, bdesc = bdesc0 + soff;
                     const uint32_t sfb_c = sfc0 + sfoff, sfa_c = sfb_c + 32;
-                    ++done_kb;
                     int nstage = stage + 1;
                     uint32_t nphase = phase;
                     if (nstage == Q_STAGES) { nstage = 0; nphase ^= 1u; }
-                    const bool more = done_kb < total_kb;
-                    tc_mma_nvf4_pair(tmem, adesc, bdesc, idesc, sfa_c, sfb_c, kb ? 1u : 0u);
+                    const bool more = kb + 1 < kb1 || local + 1 < my_items;
+                    tc_mma_nvf4_pair(tmem, adesc, bdesc, idesc, sfa_c, sfb_c, kb > kb0 ? 1u : 0u);
                     const bool r1 = more && bar_test(bar_sf_ready + 8 * nstage, nphase);
                     tc_mma_nvf4_pair(tmem, adesc + 2, bdesc + 2, idesc, sfa_c + 4, sfb_c + 8, 1u);        // +32 bytes along K = +2
                     const bool r2 = r1 && bar_test(bar_full + 8 * nstage, nphase);
@@ -915,8 +967,10 @@ nvfp4_gemm_pair_kernel_v2(const __grid_constant__ CUtensorMap map_a, const __gri
         int stage = 0;
         uint32_t phase = 0;
         bool live = true;
-        for (int tile = pair; tile < total_tiles && live && !s_abort; tile += npairs) {
-            for (int kb = 0; kb < p.k_blocks; ++kb) {
+        for (int item = pair; item < p.items && live && !s_abort; item += npairs) {
+            int kb0, kb1;
+            pair_item(p, item, &kb0, &kb1);
+            for (int kb = kb0; kb < kb1; ++kb) {
                 if (!bar_spin(bar_sf_full + 8 * stage, phase, SPIN_LIMIT)) { if (lane == 0) { atomicExch(p.status, 18); s_abort = 1; } live = false; break; }
                 const unsigned char* src = sf_smem + stage * Q_STAGE_BYTES;
                 uint32_t r[48];
@@ -942,8 +996,10 @@ nvfp4_gemm_pair_kernel_v2(const __grid_constant__ CUtensorMap map_a, const __gri
         const int quarter = warp & 3, half = (warp - 2) >> 2;
         const uint32_t leader_acc_empty = map_to_cta(bar_acc_empty, 0);
         int local = 0;
-        for (int tile = pair; tile < total_tiles && !s_abort; tile += npairs, ++local) {
-            const int nt = tile / p.m_pairs, mp = tile - nt * p.m_pairs;
+        asm volatile("griddepcontrol.wait;" ::: "memory");         // C and the partial sums may still be read by the kernel before
+        for (int item = pair; item < p.items && !s_abort; item += npairs, ++local) {
+            int kb0, kb1;
+            const int tile = pair_item(p, item, &kb0, &kb1), nt = tile / p.m_pairs, mp = tile - nt * p.m_pairs;
             if (!bar_spin(bar_acc_full, (uint32_t)local & 1u, SPIN_LIMIT)) { if (lane == 0) { atomicExch(p.status, 16); s_abort = 1; } break; }
             tc_fence_after();
             const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + half * V2_EPI_COLS;
@@ -958,6 +1014,14 @@ nvfp4_gemm_pair_kernel_v2(const __grid_constant__ CUtensorMap map_a, const __gri
             if (lane == 0) {                                       // the leader's MMA thread waits for all sixteen warps
                 if (rank == 0) bar_arrive(bar_acc_empty);
                 else bar_arrive_cluster_relaxed(leader_acc_empty);
+            }
+            if (item >= p.whole) {                                 // fp32 sums: this thread's row, half of its columns
+                float4* out = reinterpret_cast<float4*>(p.partial + ((size_t)(item - p.whole) * 256 + rank * 128 + quarter * 32 + lane) * BN + half * V2_EPI_COLS);
+                if ((2 * mp + (int)rank) * BM + quarter * 32 + lane < p.M)
+#pragma unroll
+                    for (int v = 0; v < V2_EPI_COLS / 4; ++v)
+                        out[v] = make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]), __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3]));
+                continue;
             }
             // Stores: one lane per row would touch 32 rows with every instruction, and all CTAs store at the same time
             // (the tile boundaries coincide): measured, that stalls the next tile's loads for 2-3 us.  So the tile goes
@@ -993,6 +1057,27 @@ nvfp4_gemm_pair_kernel_v2(const __grid_constant__ CUtensorMap map_a, const __gri
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+    }
+}
+
+// C of the tiles that were cut along K: their items' sums added in order, scaled, rounded once.  56 threads x four columns per row.
+__global__ void __launch_bounds__(224) nvfp4_pair_reduce_kernel(const PairParams p)
+{
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int q = threadIdx.x % 56, rows = (p.items - p.whole) / p.splits * 256;
+    for (int i = blockIdx.x * 4 + threadIdx.x / 56; i < rows; i += gridDim.x * 4) {
+        const int t = i >> 8, r = i & 255, tile = p.whole + t, nt = tile / p.m_pairs, mp = tile - nt * p.m_pairs;
+        const int m = mp * 256 + r, n = nt * BN + 4 * q;
+        if (m >= p.M || n >= p.N) continue;                        // (N is a multiple of 8)
+        const float4* src = reinterpret_cast<const float4*>(p.partial + ((size_t)t * p.splits * 256 + r) * BN) + q;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int s = 0; s < p.splits; ++s) {
+            const float4 u = __ldcs(src + (size_t)s * (256 * BN / 4));
+            v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+        }
+        const __nv_bfloat162 h0 = __floats2bfloat162_rn(v.x * p.scale, v.y * p.scale), h1 = __floats2bfloat162_rn(v.z * p.scale, v.w * p.scale);
+        *reinterpret_cast<uint2*>(p.C + (size_t)m * p.N + n) = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
     }
 }
 
@@ -1176,7 +1261,7 @@ static int pair_v2_clusters(int device, int sm_count)
 }
 
 int32_t nvfp4_gemm_launch(Nvfp4Scratch& scratch, const Nvfp4Dev& w, const uint8_t* a_codes, const uint8_t* a_sf, float ta,
-                          int64_t M, uint16_t* c, int device, int sm_count, cudaStream_t s, int* launches, std::string& err)
+                          int64_t M, uint16_t* c, int device, int sm_count, bool pdl, cudaStream_t s, int* launches, std::string& err)
 {
     *launches = 0;
     const int64_t N = w.N, K = w.K;
@@ -1225,10 +1310,61 @@ int32_t nvfp4_gemm_launch(Nvfp4Scratch& scratch, const Nvfp4Dev& w, const uint8_
         pp.scale = ta * w.tensor_scale;
         pp.status = scratch.status;
         pp.sfa_direct = direct ? 1 : 0;
-        int grid = 2 * std::min(nclusters, pp.m_pairs * pp.n_tiles);
-        nvfp4_gemm_pair_kernel_v2<<<grid, V2_THREADS, Q_SMEM_BYTES, s>>>(map_a, map_bh, map_sfa, map_c, pp, scratch.sfa_tiled, w.sf_tiled);
+        // Full waves of tiles go whole; a last wave that leaves pairs idle may be cut along K.  The cut that costs least, by
+        // rates measured on 74 pairs (microseconds: a K block of a pair; the launch that adds the items and the fp32 epilogue;
+        // writing and adding the rows of one item); uncut unless it gains a microsecond.  1000 x 4096 x 14336 (2 tiles of 76 in
+        // the second wave): 48.6 -> 40.5 us; 16 x 1024 x 8192 (5 tiles): 17.2 -> 9.6; but 700 x 11008 x 4096 (2 of 150) cut into
+        // eighths of 16 K blocks: 24.9 -> 28.7, left whole.
+        const int tiles = pp.m_pairs * pp.n_tiles, last = tiles % nclusters;
+        const double rows = (double)M / (256.0 * pp.m_pairs);
+        int splits = 1;
+        double best = 0.42 * pp.k_blocks - 1.0;
+        for (int c = 2; last && c <= std::min(nclusters / last, pp.k_blocks / SPLIT_MIN_BLOCKS); ++c) {
+            const double cost = 0.42 * ((pp.k_blocks + c - 1) / c) + 5.0 + 0.08 * rows * last * c;
+            if (cost < best) { best = cost; splits = c; }
+        }
+        if (splits > 1 && scratch.partial_bytes < (size_t)last * splits * 256 * BN * sizeof(float)) {
+            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;      // nothing can be allocated while a stream captures
+            if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+                cudaGetLastError();
+                splits = 1;
+            }
+        }
+        pp.splits = splits;
+        pp.whole = splits > 1 ? tiles - last : tiles;
+        pp.items = pp.whole + (tiles - pp.whole) * splits;
+        if (splits > 1) {
+            const size_t need = (size_t)(pp.items - pp.whole) * 256 * BN * sizeof(float);
+            if (scratch.partial_bytes < need) {
+                cudaDeviceSynchronize();                           // nobody may still be using the old array
+                cudaFree(scratch.partial);
+                scratch.partial = nullptr;
+                scratch.partial_bytes = 0;
+                e = cudaMalloc(&scratch.partial, need);
+                if (e != cudaSuccess) { err = std::string("scratch allocation failed: ") + cudaGetErrorString(e); return MPQ_ERR_CUDA; }
+                scratch.partial_bytes = need;
+            }
+        }
+        pp.partial = scratch.partial;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(2 * std::min(nclusters, pp.items)));
+        cfg.blockDim = dim3(V2_THREADS);
+        cfg.dynamicSmemBytes = Q_SMEM_BYTES;
+        cfg.stream = s;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = pdl ? 1u : 0u;
+        e = cudaLaunchKernelEx(&cfg, nvfp4_gemm_pair_kernel_v2, map_a, map_bh, map_sfa, map_c, pp, (const uint8_t*)scratch.sfa_tiled, (const uint8_t*)w.sf_tiled);
         *launches += 1;
-        e = cudaGetLastError();
+        if (e == cudaSuccess && splits > 1) {
+            cfg.gridDim = dim3((unsigned)std::min(sm_count * 8, last * 64));
+            cfg.blockDim = dim3(224);
+            cfg.dynamicSmemBytes = 0;
+            e = cudaLaunchKernelEx(&cfg, nvfp4_pair_reduce_kernel, pp);
+            *launches += 1;
+        }
         if (e != cudaSuccess) { err = std::string("nvfp4_gemm_pair_kernel_v2 launch failed: ") + cudaGetErrorString(e); return MPQ_ERR_CUDA; }
         return MPQ_OK;
     }

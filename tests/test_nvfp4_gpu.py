@@ -288,3 +288,56 @@ def test_quantise_then_gemm(ctx, orc):
     c32, _ = orc.nvfp4_gemm(a_c, a_s, 1.0, b, sfb, 1.0)
     _check(orc, y.view(torch.int16).cpu().numpy().view(np.uint16), c32)
     w.destroy()
+
+
+@pytest.mark.parametrize("ts", [1.0, 0.37, 2.0 ** -64, 2.0 ** 64, 1e-25, 3e20])
+def test_quantisation_at_the_rounding_boundaries(ctx, orc, ts):
+    """Quotients on and a few ulp beside every boundary of the e2m1 grid, for every positive e4m3 scale, on the path with one
+    reciprocal per block (tensor scale within 2^+-64) and on the path with divisions; then infinities and NaN."""
+    import torch
+    import makepad_b200
+    ts = np.float32(ts)
+    rows = []
+    for s8 in range(1, 0x7F):
+        e, m = s8 >> 3, s8 & 7
+        d = np.float32((m * 2.0 ** -9 if e == 0 else (8 + m) * 2.0 ** (e - 10))) * ts
+        for t in (0.25, 0.75, 1.25, 1.75, 2.5, 3.5, 5.0):
+            x = np.float32(d) * np.float32(t)
+            near = [x]
+            for _ in range(3):
+                near += [np.nextafter(near[-1], np.float32(np.inf), dtype=np.float32)]
+            for _ in range(3):
+                near += [np.nextafter(near[0] if len(near) == 4 else near[-1], np.float32(0), dtype=np.float32)]
+            rows.append([np.float32(6) * d] + near + [-v for v in near] + [np.float32(-0.0)])
+    x = np.array(rows, dtype=np.float32)
+    codes, sf = makepad_b200.nvfp4_quantize(ctx, torch.from_numpy(x).cuda(), float(ts))
+    want_c, want_s = orc.nvfp4_quantize(x, float(ts))
+    assert np.array_equal(sf.cpu().numpy(), want_s) and np.array_equal(codes.cpu().numpy(), want_c)
+    if ts == 1.0:
+        x = np.zeros((2, 16), dtype=np.float32)
+        x[0, :4] = [np.inf, -np.inf, 100.0, -0.0]                      # the scale saturates at 448
+        x[1, :4] = [np.nan, -np.nan, 12.0, -np.inf * 0]                # a NaN does not count for the scale and becomes +6
+        codes, sf = makepad_b200.nvfp4_quantize(ctx, torch.from_numpy(x).cuda(), 1.0)
+        assert codes[:, :2].cpu().tolist() == [[0xF7, 0x80], [0x77, 0x77]] and sf.flatten().cpu().tolist() == [0x7E, 0x40]
+
+
+@pytest.mark.parametrize("M,N,K", [(1000, 4096, 14336), (300, 1024, 8192), (1, 4096, 8192), (257, 232, 6176)])
+def test_tiles_split_along_k(ctx, orc, M, N, K):
+    """Shapes whose last (or only) wave of tiles is cut along K: sampled rows against the oracle, nothing written outside the
+    output, the same bits twice."""
+    import torch
+    import makepad_b200
+    a, sfa = synth.nvfp4_tensor(M, K, seed=31, stream=0)
+    b, sfb = synth.nvfp4_tensor(N, K, seed=31, stream=1)
+    lin = makepad_b200.QuantLinear(makepad_b200.Nvfp4Weight(ctx, b, sfb, 2.0))
+    ad, sd = torch.from_numpy(a).cuda(), torch.from_numpy(sfa).cuda()
+    buf = torch.full((M * N + 128,), 7.0, dtype=torch.bfloat16, device="cuda")
+    y = buf[64:64 + M * N].view(M, N)
+    lin.forward((ad, sd, 0.5), out=y)
+    assert torch.equal(y, lin((ad, sd, 0.5)))
+    torch.cuda.synchronize()
+    assert ctx.lib.mpq_context_poll_status(ctx.h) == _lib.OK
+    assert (buf[:64] == 7.0).all() and (buf[64 + M * N:] == 7.0).all()
+    rows = sorted({0, M - 1} | set(np.random.default_rng(3).integers(0, M, 6).tolist()))
+    c32, _ = orc.nvfp4_gemm(a[rows], sfa[rows], 0.5, b, sfb, 2.0)
+    _check(orc, y[rows].view(torch.int16).cpu().numpy().view(np.uint16), c32)
