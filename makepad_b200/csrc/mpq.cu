@@ -881,30 +881,53 @@ static int q4_gemm_pairs(const mpq_context* ctx)
     return n;
 }
 
+// How one slab of M rows is cut, and the scratch that takes.
+struct Q4GemmPlan { int nt, Mt, W, pairs; int64_t total; bool cut; size_t xs_bytes, need_xs, need_partial; };
+static Q4GemmPlan q4_gemm_plan(const Q4Dev& q, int M, int pairs_max)
+{
+    Q4GemmPlan pl;
+    // as few activation tiles as possible (each expands the weights again), as equal as possible, in steps of 32 rows (a
+    // quarter of the rows, eight or more, is what a team drains)
+    pl.nt = (M + Q4G_MT_MAX - 1) / Q4G_MT_MAX;
+    pl.Mt = ((M + pl.nt - 1) / pl.nt + 31) / 32 * 32;
+    pl.total = (int64_t)((q.nrp + 7) / 8) * pl.nt * q.nchunks;
+    pl.W = (int)std::max<int64_t>((pl.total + pairs_max - 1) / pairs_max, std::min<int64_t>(Q4G_MIN_W, pl.total));
+    pl.pairs = (int)((pl.total + pl.W - 1) / pl.W);
+    pl.cut = pl.W % q.nchunks != 0;                        // some tile lies in more than one range
+    pl.xs_bytes = (size_t)pl.nt * q.nchunks * 2 * pl.Mt * 128;
+    pl.need_xs = pl.xs_bytes + (size_t)M * sizeof(float);
+    pl.need_partial = pl.cut ? (size_t)pl.pairs * 2 * Q4G_SLOT * sizeof(float) : 0;
+    return pl;
+}
+
+// true when the stream must not see an allocation now
+static bool stream_captures(cudaStream_t s)
+{
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return cs != cudaStreamCaptureStatusNone;
+}
+
 // y = x . W^T for M > 64 rows; with swiglu x is [M][2K] = [gate | up].  One slab's staged rows take M * K * 4 bytes of scratch.
 static int32_t q4_gemm_forward(mpq_context* ctx, const Q4Dev& q, const float* x, bool swiglu, int M, float* y, int64_t ldy, int pairs_max, cudaStream_t s)
 {
     int32_t st = q4_status_word(ctx);
     if (st) return st;
-    // as few activation tiles as possible (each expands the weights again), as equal as possible, in steps of 32 rows (a
-    // quarter of the rows, eight or more, is what a team drains)
-    const int nt = (M + Q4G_MT_MAX - 1) / Q4G_MT_MAX, Mt = ((M + nt - 1) / nt + 31) / 32 * 32;
-    const int nb = (q.nrp + 7) / 8;
-    const int64_t total = (int64_t)nb * nt * q.nchunks;
-    const int W = (int)std::max<int64_t>((total + pairs_max - 1) / pairs_max, std::min<int64_t>(Q4G_MIN_W, total));
-    const int pairs = (int)((total + W - 1) / W);
-    const size_t xs_bytes = (size_t)nt * q.nchunks * 2 * Mt * 128, need = xs_bytes + (size_t)M * sizeof(float);
-    if (ctx->q4u_xs_bytes < need) {
+    const Q4GemmPlan pl = q4_gemm_plan(q, M, pairs_max);
+    const int nt = pl.nt, Mt = pl.Mt, W = pl.W, nb = (q.nrp + 7) / 8;
+    if (ctx->q4u_xs_bytes < pl.need_xs) {
         CU_TRY(ctx, cudaDeviceSynchronize());
         cudaFree(ctx->q4u_xs);
         ctx->q4u_xs = nullptr;
         ctx->q4u_xs_bytes = 0;
-        CU_TRY(ctx, cudaMalloc(&ctx->q4u_xs, need));
-        ctx->q4u_xs_bytes = need;
+        CU_TRY(ctx, cudaMalloc(&ctx->q4u_xs, pl.need_xs));
+        ctx->q4u_xs_bytes = pl.need_xs;
     }
-    float* inv_sc = reinterpret_cast<float*>(ctx->q4u_xs + xs_bytes);
-    const bool cut = W % q.nchunks != 0;                   // some tile lies in more than one range
-    if (cut && (st = q4_partial_scratch(ctx, (size_t)pairs * 2 * Q4G_SLOT * sizeof(float)))) return st;
+    float* inv_sc = reinterpret_cast<float*>(ctx->q4u_xs + pl.xs_bytes);
+    if (pl.cut && (st = q4_partial_scratch(ctx, pl.need_partial))) return st;
     CUtensorMap map_x;
     if (!make_rows128_map(&map_x, ctx->q4u_xs, (int64_t)nt * q.nchunks * 2 * Mt, Mt / 2)) return fail(ctx, MPQ_ERR_CUDA, "cuTensorMapEncodeTiled failed for the staged activations");
 
@@ -922,10 +945,10 @@ static int32_t q4_gemm_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
 
     Q4GemmLaunch p;
     p.stream = q.stream; p.inv_sc = inv_sc; p.Y = y; p.partial = ctx->q4_rect_partial;
-    p.M = M; p.Mt = Mt; p.N = (int)q.N; p.nt = nt; p.ldy = ldy; p.nchunks = q.nchunks; p.nrp = q.nrp; p.W = W; p.total = total;
+    p.M = M; p.Mt = Mt; p.N = (int)q.N; p.nt = nt; p.ldy = ldy; p.nchunks = q.nchunks; p.nrp = q.nrp; p.W = W; p.total = pl.total;
     p.status = ctx->q4_status;
     cfg = {};
-    cfg.gridDim = dim3((unsigned)(2 * pairs));
+    cfg.gridDim = dim3((unsigned)(2 * pl.pairs));
     cfg.blockDim = dim3(Q4G_THREADS);
     cfg.dynamicSmemBytes = q4_gemm_smem(Mt);
     cfg.stream = s;
@@ -933,7 +956,7 @@ static int32_t q4_gemm_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
     e = cudaLaunchKernelEx(&cfg, q4_gemm_pair_kernel, map_x, p);
     ctx->launches += 1;
     if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4_gemm_pair_kernel launch failed: %s", cudaGetErrorString(e));
-    if (cut) {
+    if (pl.cut) {
         cfg = {};
         cfg.gridDim = dim3((unsigned)std::min<int64_t>(((int64_t)nb * nt * Mt + 3) / 4, (int64_t)ctx->prop.multiProcessorCount * 16));
         cfg.blockDim = dim3(256);
@@ -946,10 +969,15 @@ static int32_t q4_gemm_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
     return MPQ_OK;
 }
 
-// Slabs of rows through the pair kernel: at most 2048, fewer where K is so long that the staged rows would pass 256 MB.
+// Rows per launch of the pair kernel: at most 2048, fewer where K is so long that the staged rows would pass 256 MB.
+static int64_t q4_gemm_slab(const Q4Dev& q)
+{
+    return std::max<int64_t>(Q4G_MT_MAX, std::min<int64_t>(2048, ((int64_t)1 << 26) / q.K / Q4G_MT_MAX * Q4G_MT_MAX));
+}
+
 static int32_t q4_gemm_slabs(mpq_context* ctx, const Q4Dev& q, const float* x, bool swiglu, int64_t M, float* y, int64_t ldy, int pairs_max, cudaStream_t s)
 {
-    const int64_t slab = std::max<int64_t>(Q4G_MT_MAX, std::min<int64_t>(2048, ((int64_t)1 << 26) / q.K / Q4G_MT_MAX * Q4G_MT_MAX));
+    const int64_t slab = q4_gemm_slab(q);
     for (int64_t m0 = 0; m0 < M; m0 += slab) {
         const int32_t st = q4_gemm_forward(ctx, q, x + (size_t)m0 * q.K * (swiglu ? 2 : 1), swiglu, (int)std::min<int64_t>(slab, M - m0),
                                            y + (size_t)m0 * ldy, ldy, pairs_max, s);
@@ -958,10 +986,25 @@ static int32_t q4_gemm_slabs(mpq_context* ctx, const Q4Dev& q, const float* x, b
     return MPQ_OK;
 }
 
-// rows that go to the pair kernel: all above 64 where the tcgen05 path is on and clusters of two can be scheduled (else 0)
-static int q4_gemm_route(const mpq_context* ctx, int64_t M)
+// Pairs to run a call on, or 0 for the kernels of 64 rows and fewer: all calls above 64 rows go to the pair kernel (measured:
+// equal to two slabs of 64 on 57344 x 8192 at 65..96 rows, faster everywhere else) where the tcgen05 path is on and clusters of
+// two can be scheduled.  Slabs of 64 rows want no more scratch than a call of 64 rows; so a capture after such a warm-up,
+// in which nothing can be allocated, keeps to them.
+static int q4_gemm_route(const mpq_context* ctx, const Q4Dev& q, int64_t M, cudaStream_t s)
 {
-    return (ctx->q4_gemm_min > 0 && M >= ctx->q4_gemm_min && ctx->q4_umma_min > 0 && M >= ctx->q4_umma_min) ? q4_gemm_pairs(ctx) : 0;
+    if (ctx->q4_gemm_min <= 0 || M < ctx->q4_gemm_min || ctx->q4_umma_min <= 0 || M < ctx->q4_umma_min) return 0;
+    const int pairs = q4_gemm_pairs(ctx);
+    if (!pairs) return 0;
+    const int64_t slab = q4_gemm_slab(q);
+    size_t need_xs = 0, need_partial = 0;
+    for (const int64_t rows : {std::min(M, slab), M % slab}) {
+        if (!rows) continue;
+        const Q4GemmPlan pl = q4_gemm_plan(q, (int)rows, pairs);
+        need_xs = std::max(need_xs, pl.need_xs);
+        need_partial = std::max(need_partial, pl.need_partial);
+    }
+    if ((ctx->q4u_xs_bytes < need_xs || ctx->q4_rect_partial_bytes < need_partial) && stream_captures(s)) return 0;
+    return pairs;
 }
 
 // The streaming kernel stages ALL of x in every CTA, the rectangle kernel only a K slice of it: measured on the 7B shapes,
@@ -1032,7 +1075,7 @@ static int q4_slab_rows(const mpq_context* ctx, const Q4Dev& q, int64_t M)
 static int32_t q4_forward_checked(mpq_context* ctx, const mpq_weight* w, const float* x_dev, int64_t M, float* y_dev,
                                   int64_t ldy, cudaStream_t s)
 {
-    if (const int pairs = q4_gemm_route(ctx, M)) return q4_gemm_slabs(ctx, w->q4, x_dev, false, M, y_dev, ldy, pairs, s);
+    if (const int pairs = q4_gemm_route(ctx, w->q4, M, s)) return q4_gemm_slabs(ctx, w->q4, x_dev, false, M, y_dev, ldy, pairs, s);
     if (ctx->q4_umma_min > 0 && M >= ctx->q4_umma_min) {       // slabs of up to 64 rows on the tcgen05 path
         for (int64_t m0 = 0; m0 < M; m0 += 64) {
             int m = (int)std::min<int64_t>(64, M - m0);
@@ -1130,7 +1173,7 @@ extern "C" int32_t mpq_q4_linear_forward_swiglu(mpq_context* ctx, const mpq_weig
         p.swiglu = 1;
         return q4_stream_enqueue(ctx, pl, p, grid, s);
     }
-    if (const int pairs = q4_gemm_route(ctx, M)) return q4_gemm_slabs(ctx, q, gate_up_dev, true, M, y_dev, q.N, pairs, s);
+    if (const int pairs = q4_gemm_route(ctx, q, M, s)) return q4_gemm_slabs(ctx, q, gate_up_dev, true, M, y_dev, q.N, pairs, s);
     const size_t need = (size_t)M * q.K * sizeof(float);
     if (ctx->swiglu_bytes < need) {
         CU_TRY(ctx, cudaDeviceSynchronize());
@@ -1486,9 +1529,8 @@ extern "C" int32_t mpq_nvfp4_quantize_activations(mpq_context* ctx, const void* 
     if (!(tensor_scale > 0.f)) return fail(ctx, MPQ_ERR_INVALID_ARG, "tensor_scale must be positive");
     if (!aligned16(x_dev) || (reinterpret_cast<uintptr_t>(codes_dev) & 7u)) return fail(ctx, MPQ_ERR_ALIGN, "x must be 16-byte, codes 8-byte aligned");
     CU_TRY(ctx, cudaSetDevice(ctx->device));
-    nvfp4_quantize_launch(x_dev, x_is_bf16 != 0, false, M, K, tensor_scale, codes_dev, sf_dev, (cudaStream_t)stream);
     ctx->launches += 1;
-    CU_TRY(ctx, nvfp4_quantize_launch(gate_up_dev, x_is_bf16 != 0, true, M, F, tensor_scale, codes_dev, sf_dev, ctx->pdl, (cudaStream_t)stream));
+    CU_TRY(ctx, nvfp4_quantize_launch(x_dev, x_is_bf16 != 0, false, M, K, tensor_scale, codes_dev, sf_dev, ctx->pdl, (cudaStream_t)stream));
     return MPQ_OK;
 }
 
@@ -1501,9 +1543,8 @@ extern "C" int32_t mpq_nvfp4_quantize_swiglu(mpq_context* ctx, const void* gate_
     if (!(tensor_scale > 0.f)) return fail(ctx, MPQ_ERR_INVALID_ARG, "tensor_scale must be positive");
     if (!aligned16(gate_up_dev) || (reinterpret_cast<uintptr_t>(codes_dev) & 7u)) return fail(ctx, MPQ_ERR_ALIGN, "gate_up must be 16-byte, codes 8-byte aligned");
     CU_TRY(ctx, cudaSetDevice(ctx->device));
-    nvfp4_quantize_launch(gate_up_dev, x_is_bf16 != 0, true, M, F, tensor_scale, codes_dev, sf_dev, (cudaStream_t)stream);
     ctx->launches += 1;
-    CU_TRY(ctx, nvfp4_quantize_launch(x_dev, x_is_bf16 != 0, false, M, K, tensor_scale, codes_dev, sf_dev, ctx->pdl, (cudaStream_t)stream));
+    CU_TRY(ctx, nvfp4_quantize_launch(gate_up_dev, x_is_bf16 != 0, true, M, F, tensor_scale, codes_dev, sf_dev, ctx->pdl, (cudaStream_t)stream));
     return MPQ_OK;
 }
 

@@ -406,3 +406,31 @@ def test_pair_kernel_above_64_rows(ctx, orc, N, K, M):
     assert torch.equal(lin.forward_swiglu(gate_up), lin(makepad_b200.swiglu(ctx, gate_up)))
     torch.cuda.synchronize()
     assert ctx.lib.mpq_context_poll_status(ctx.h) == _lib.OK
+
+
+def test_capture_above_64_rows_after_a_warm_up_of_64(orc):
+    """A capture cannot allocate: with the scratch of a 64-row warm-up the call keeps to slabs of 64 rows, with that of a full
+    warm-up it takes the pair kernel; both replay to the oracle's result."""
+    import makepad_b200
+    torch = _torch()
+    N, K, M = 500, 1056, 300
+    codes, scales = synth.q4_weight(N, K, seed=21)
+    x = synth.activations(M, K, seed=22)
+    xd = torch.from_numpy(x).cuda()
+    ref = orc.q4_matmul_f64(codes, scales, x)
+    for warm in (64, M):
+        c2 = makepad_b200.Context(0)
+        lin = makepad_b200.QuantLinear(makepad_b200.Q4Weight(c2, codes, scales))
+        lin(xd[:warm])
+        torch.cuda.synchronize()
+        y = torch.empty((M, N), device="cuda")
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            lin.forward(xd, out=y)
+        y.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert orc.err_report(y.cpu().numpy(), ref)["max_abs_over_rms"] < 2e-5
+        assert c2.lib.mpq_context_poll_status(c2.h) == _lib.OK
+        del graph, lin
+        c2.close()
