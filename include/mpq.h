@@ -200,7 +200,7 @@ int32_t mpq_q4_linear_forward_allreduce(mpq_context* ctx, const mpq_weight* w, m
 int32_t mpq_swiglu(mpq_context* ctx, const float* gate_up_dev, int64_t M, int64_t F, float* out_dev, void* stream);
 /* Y[M][N] = swiglu(gate_up)[M][K] * W^T with gate_up[M][2K]: the down projection with the SwiGLU fused into
  * the kernel's activation staging where mpq_q4_linear_forward would use the streaming kernel (one row, or
- * up to four rows of a short K) or that of CTA pairs (above 64 rows): the intermediate never exists in memory;
+ * up to four rows of a short K) or a tcgen05 kernel (from 17 rows): the intermediate never exists in memory;
  * otherwise mpq_swiglu runs into scratch the context owns, then mpq_q4_linear_forward.  Same bits as the two calls. */
 int32_t mpq_q4_linear_forward_swiglu(mpq_context* ctx, const mpq_weight* w, const float* gate_up_dev, int64_t M,
                                      float* y_dev, void* stream);

@@ -761,7 +761,8 @@ static cudaError_t launch_pdl(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, 
     return cudaSuccess;
 }
 
-static int32_t q4_umma_forward(mpq_context* ctx, const Q4Dev& q, const float* x, int M, float* y, int64_t ldy, cudaStream_t s)
+// swiglu: x is [M][2K] = [gate | up]
+static int32_t q4_umma_forward(mpq_context* ctx, const Q4Dev& q, const float* x, bool swiglu, int M, float* y, int64_t ldy, cudaStream_t s)
 {
     const int sms = ctx->prop.multiProcessorCount;
     const int Mp = (M + 15) / 16 * 16;
@@ -793,13 +794,20 @@ static int32_t q4_umma_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
     }
     if (maxp > 1 && (st = q4_partial_scratch(ctx, (size_t)maxp * M * q.N * sizeof(float)))) return st;
 
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)Mp, (unsigned)std::max(1, std::min(8, 2 * sms / Mp)));     // a row is shared by several CTAs: about two per SM
+    const int parts = std::max(1, std::min(8, 2 * sms / Mp));            // a row is shared by the CTAs of a cluster: about two per SM
+    const size_t part_bytes = (size_t)((q.nchunks * 16 + parts - 1) / parts) * sizeof(float4);
+    const int cached = part_bytes <= (size_t)47 * 1024;                  // (the shared memory any kernel gets; K up to 96 K with 8 parts)
+    cfg.gridDim = dim3((unsigned)Mp, (unsigned)parts);
     cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = cached ? part_bytes : 0;
     cfg.stream = s;
     launch_pdl(cfg, at, ctx->pdl);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, q4u_xstage_kernel, x, M, Mp, (int)q.K, q.nchunks, ctx->q4u_xs, inv_sc);
+    at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    at[cfg.numAttrs].val.clusterDim.x = 1; at[cfg.numAttrs].val.clusterDim.y = (unsigned)parts; at[cfg.numAttrs].val.clusterDim.z = 1;
+    cfg.numAttrs += 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, swiglu ? q4u_xstage_kernel<true> : q4u_xstage_kernel<false>, x, M, Mp, (int)q.K, q.nchunks, cached, ctx->q4u_xs, inv_sc);
     ctx->launches += 1;
     if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4u_xstage_kernel launch failed: %s", cudaGetErrorString(e));
 
@@ -1071,18 +1079,22 @@ static int q4_slab_rows(const mpq_context* ctx, const Q4Dev& q, int64_t M)
     }
     return 16;
 }
+static int32_t q4_umma_slabs(mpq_context* ctx, const Q4Dev& q, const float* x, bool swiglu, int64_t M, float* y, int64_t ldy, cudaStream_t s)
+{
+    for (int64_t m0 = 0; m0 < M; m0 += 64) {
+        const int32_t st = q4_umma_forward(ctx, q, x + (size_t)m0 * q.K * (swiglu ? 2 : 1), swiglu, (int)std::min<int64_t>(64, M - m0), y + (size_t)m0 * ldy, ldy, s);
+        if (st) return st;
+    }
+    return MPQ_OK;
+}
+
 
 static int32_t q4_forward_checked(mpq_context* ctx, const mpq_weight* w, const float* x_dev, int64_t M, float* y_dev,
                                   int64_t ldy, cudaStream_t s)
 {
     if (const int pairs = q4_gemm_route(ctx, w->q4, M, s)) return q4_gemm_slabs(ctx, w->q4, x_dev, false, M, y_dev, ldy, pairs, s);
     if (ctx->q4_umma_min > 0 && M >= ctx->q4_umma_min) {       // slabs of up to 64 rows on the tcgen05 path
-        for (int64_t m0 = 0; m0 < M; m0 += 64) {
-            int m = (int)std::min<int64_t>(64, M - m0);
-            int32_t st = q4_umma_forward(ctx, w->q4, x_dev + (size_t)m0 * w->q4.K, m, y_dev + (size_t)m0 * ldy, ldy, s);
-            if (st) return st;
-        }
-        return MPQ_OK;
+        return q4_umma_slabs(ctx, w->q4, x_dev, false, M, y_dev, ldy, s);
     }
     const int slab = q4_slab_rows(ctx, w->q4, M);
     for (int64_t m0 = 0; m0 < M; m0 += slab) {
@@ -1153,8 +1165,8 @@ extern "C" int32_t mpq_swiglu(mpq_context* ctx, const float* gate_up_dev, int64_
     return swiglu_launch(ctx, gate_up_dev, M, F, out_dev, (cudaStream_t)stream);
 }
 
-// y = W * swiglu(gate_up): fused into the streaming kernel's activation staging for M <= 4 (the intermediate never
-// exists in memory); above that the SwiGLU runs as its own kernel into scratch the context owns.
+// y = W * swiglu(gate_up): fused into the activation staging of the streaming kernel and of the tcgen05 kernels (the
+// intermediate never exists in memory); for the rectangle kernel the SwiGLU runs as its own kernel into scratch the context owns.
 extern "C" int32_t mpq_q4_linear_forward_swiglu(mpq_context* ctx, const mpq_weight* w, const float* gate_up_dev, int64_t M,
                                                 float* y_dev, void* stream)
 {
@@ -1173,6 +1185,7 @@ extern "C" int32_t mpq_q4_linear_forward_swiglu(mpq_context* ctx, const mpq_weig
         p.swiglu = 1;
         return q4_stream_enqueue(ctx, pl, p, grid, s);
     }
+    if (ctx->q4_umma_min > 0 && M >= ctx->q4_umma_min) return q4_umma_slabs(ctx, q, gate_up_dev, true, M, y_dev, q.N, s);
     if (const int pairs = q4_gemm_route(ctx, q, M, s)) return q4_gemm_slabs(ctx, q, gate_up_dev, true, M, y_dev, q.N, pairs, s);
     const size_t need = (size_t)M * q.K * sizeof(float);
     if (ctx->swiglu_bytes < need) {

@@ -85,23 +85,38 @@ __host__ __device__ __forceinline__ void q4u_pieces(int b, int nchunks, int W, i
 // ---------------------------------------------------------------------------
 // activation staging: fp32 rows -> hi/lo fp16 tiles in the order the MMA's shared-memory descriptor wants
 // ---------------------------------------------------------------------------
-// gridDim.x = staged rows (rows >= M are zeros), gridDim.y = parts of a row.  Row m of a chunk's tile lies at (m/8)*1024 + (m%8)*128 bytes;
-// inside the row the 16-byte group j (8 halves) is stored at group j ^ (m % 8) (SWIZZLE_128B, K-major).
-__global__ void __launch_bounds__(256) q4u_xstage_kernel(const float* __restrict__ X, int M, int Mp, int K, int nchunks,
+// gridDim.x = staged rows (rows >= M are zeros), gridDim.y = parts of a row = one cluster.  Row m of a chunk's tile lies at
+// (m/8)*1024 + (m%8)*128 bytes; inside the row the 16-byte group j (8 halves) is stored at group j ^ (m % 8) (SWIZZLE_128B,
+// K-major).  SWIGLU: X is [M][2K] = [gate | up] and silu(gate) * up is what gets staged.
+// Bound by latency (64 rows are 256 CTAs of a few loads each).  Each CTA finds the largest magnitude of its own part, keeps
+// the part in shared memory (cached) and takes the maximum over the cluster; when every CTA read the whole row for it, the
+// SwiGLU needed a kernel and a pass over memory of its own.  70B feed-forward
+// block at 64 rows: 346 -> 339 us.
+template <bool SWIGLU>
+__global__ void __launch_bounds__(256) q4u_xstage_kernel(const float* __restrict__ X, int M, int Mp, int K, int nchunks, int cached,
                                                           unsigned char* __restrict__ XS, float* __restrict__ inv_sc)
 {
-    __shared__ uint32_t s_max[8];
+    extern __shared__ float4 s_part[];
+    __shared__ uint32_t s_max[8], s_all;
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int m = blockIdx.x, tid = threadIdx.x;
     const int n4 = nchunks * 16;                           // float4 per padded row
+    const int per = (n4 + (int)gridDim.y - 1) / (int)gridDim.y, f0 = (int)blockIdx.y * per, f1 = min(n4, f0 + per);
     const size_t tile = (size_t)Mp * 128, chunk_bytes = 2 * tile;
     const size_t row_off = (size_t)(m >> 3) * 1024 + (size_t)(m & 7) * 128;
+    const float4* x4 = reinterpret_cast<const float4*>(X + (size_t)m * (SWIGLU ? 2 * (size_t)K : (size_t)K));
+    auto load = [&](int f) {
+        float4 v = __ldg(x4 + f);
+        if (SWIGLU) v = swiglu_f32x4(v, __ldg(x4 + K / 4 + f));
+        return v;
+    };
     float sc = 1.f;
-    if (m < M) {
+    if (m < M) {                                           // (the CTAs of a cluster share the row)
         uint32_t mx = 0;
-        for (int f = tid; 4 * f < K; f += 256) {
-            const float4 v = __ldg(reinterpret_cast<const float4*>(X + (size_t)m * K + 4 * f));
+        for (int f = f0 + tid; f < f1 && 4 * f < K; f += 256) {
+            const float4 v = load(f);
+            if (cached) s_part[f - f0] = v;                // read back by the same thread
             mx = max(mx, __float_as_uint(v.x) & 0x7FFFFFFFu);
             mx = max(mx, __float_as_uint(v.y) & 0x7FFFFFFFu);
             mx = max(mx, __float_as_uint(v.z) & 0x7FFFFFFFu);
@@ -114,6 +129,11 @@ __global__ void __launch_bounds__(256) q4u_xstage_kernel(const float* __restrict
         mx = s_max[0];
 #pragma unroll
         for (int w = 1; w < 8; ++w) mx = max(mx, s_max[w]);
+        if (tid == 0) s_all = mx;
+        cg::cluster_group cluster = cg::this_cluster();
+        cluster.sync();
+        for (unsigned r = 0; r < cluster.num_blocks(); ++r) mx = max(mx, *cluster.map_shared_rank(&s_all, r));
+        cluster.sync();                                    // nobody leaves before its maximum has been read
         int emax = (int)(mx >> 23);
         float inv = 1.f;
         if (mx != 0 && emax < 255) {                       // the largest |x| of the row goes to [2^14, 2^15)
@@ -123,11 +143,9 @@ __global__ void __launch_bounds__(256) q4u_xstage_kernel(const float* __restrict
         }
         if (tid == 0 && blockIdx.y == 0) inv_sc[m] = inv;
     }
-    // gridDim.y CTAs share a row: each finds the row's largest magnitude (the row is read from L2) and converts its part
-    const int per = (n4 + (int)gridDim.y - 1) / (int)gridDim.y, f0 = (int)blockIdx.y * per, f1 = min(n4, f0 + per);
     for (int f = f0 + tid; f < f1; f += 256) {
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (m < M && 4 * f < K) v = __ldg(reinterpret_cast<const float4*>(X + (size_t)m * K + 4 * f));
+        if (m < M && 4 * f < K) v = cached ? s_part[f - f0] : load(f);
         const float e0 = v.x * sc, e1 = v.y * sc, e2 = v.z * sc, e3 = v.w * sc;
         const __half2 h01 = __floats2half2_rn(e0, e1), h23 = __floats2half2_rn(e2, e3);
         const float2 f01 = __half22float2(h01), f23 = __half22float2(h23);

@@ -434,3 +434,27 @@ def test_capture_above_64_rows_after_a_warm_up_of_64(orc):
         assert c2.lib.mpq_context_poll_status(c2.h) == _lib.OK
         del graph, lin
         c2.close()
+
+
+# parts of a row per cluster: 8 (17 and 32 rows), 6 (48), 4 (64); a last part that is short or empty; a part too long for shared memory
+@pytest.mark.parametrize("N,K,M", [(40, 32, 17), (100, 448, 33), (96, 4096, 48), (64, 11008, 64), (32, 131072, 20)])
+def test_staging_of_a_row_by_a_cluster(ctx, orc, N, K, M):
+    """17..64 rows, one of them zero and one far larger than the others: the oracle's result, and the SwiGLU form equal to the
+    unfused one bit for bit."""
+    import makepad_b200
+    torch = _torch()
+    codes, scales = synth.q4_weight(N, K, seed=41)
+    lin = makepad_b200.QuantLinear(makepad_b200.Q4Weight(ctx, codes, scales))
+    x = synth.activations(M, K, seed=42)
+    x[1] = 0
+    x[2] *= 1e20
+    x[3, K - 1] = 3e4                                                  # the row's largest lies in the last part
+    y = lin(torch.from_numpy(x).cuda()).cpu().numpy()
+    ref = orc.q4_matmul_f64(codes, scales, x)
+    assert (y[1] == 0).all()
+    for m in [0, 2, 3, M - 1]:
+        assert orc.err_report(y[m:m + 1], ref[m:m + 1])["floored_1e-2_rms"] < TOL, m
+    gate_up = torch.from_numpy(synth.activations(M, 2 * K, seed=43)).cuda()
+    assert torch.equal(lin.forward_swiglu(gate_up), lin(makepad_b200.swiglu(ctx, gate_up)))
+    torch.cuda.synchronize()
+    assert ctx.lib.mpq_context_poll_status(ctx.h) == _lib.OK
