@@ -796,17 +796,19 @@ static int32_t q4_umma_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
 
     cudaLaunchAttribute at[2];
     cudaLaunchConfig_t cfg = {};
-    const int parts = std::max(1, std::min(8, 2 * sms / Mp));            // a row is shared by the CTAs of a cluster: about two per SM
+    const int parts = std::max(1, std::min(8, 2 * sms / Mp));            // a row is shared by several CTAs: about two per SM
     const size_t part_bytes = (size_t)((q.nchunks * 16 + parts - 1) / parts) * sizeof(float4);
-    const int cached = part_bytes <= (size_t)47 * 1024;                  // (the shared memory any kernel gets; K up to 96 K with 8 parts)
+    const int cached = swiglu && part_bytes <= (size_t)47 * 1024;                  // (the shared memory any kernel gets; K up to 96 K with 8 parts)
     cfg.gridDim = dim3((unsigned)Mp, (unsigned)parts);
     cfg.blockDim = dim3(256);
     cfg.dynamicSmemBytes = cached ? part_bytes : 0;
     cfg.stream = s;
     launch_pdl(cfg, at, ctx->pdl);
-    at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
-    at[cfg.numAttrs].val.clusterDim.x = 1; at[cfg.numAttrs].val.clusterDim.y = (unsigned)parts; at[cfg.numAttrs].val.clusterDim.z = 1;
-    cfg.numAttrs += 1;
+    if (swiglu) {                                                        // ... which are then a cluster
+        at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        at[cfg.numAttrs].val.clusterDim.x = 1; at[cfg.numAttrs].val.clusterDim.y = (unsigned)parts; at[cfg.numAttrs].val.clusterDim.z = 1;
+        cfg.numAttrs += 1;
+    }
     cudaError_t e = cudaLaunchKernelEx(&cfg, swiglu ? q4u_xstage_kernel<true> : q4u_xstage_kernel<false>, x, M, Mp, (int)q.K, q.nchunks, cached, ctx->q4u_xs, inv_sc);
     ctx->launches += 1;
     if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4u_xstage_kernel launch failed: %s", cudaGetErrorString(e));
@@ -1185,8 +1187,8 @@ extern "C" int32_t mpq_q4_linear_forward_swiglu(mpq_context* ctx, const mpq_weig
         p.swiglu = 1;
         return q4_stream_enqueue(ctx, pl, p, grid, s);
     }
-    if (ctx->q4_umma_min > 0 && M >= ctx->q4_umma_min) return q4_umma_slabs(ctx, q, gate_up_dev, true, M, y_dev, q.N, s);
     if (const int pairs = q4_gemm_route(ctx, q, M, s)) return q4_gemm_slabs(ctx, q, gate_up_dev, true, M, y_dev, q.N, pairs, s);
+    if (ctx->q4_umma_min > 0 && M >= ctx->q4_umma_min) return q4_umma_slabs(ctx, q, gate_up_dev, true, M, y_dev, q.N, s);
     const size_t need = (size_t)M * q.K * sizeof(float);
     if (ctx->swiglu_bytes < need) {
         CU_TRY(ctx, cudaDeviceSynchronize());

@@ -75,23 +75,30 @@ struct Q4ULaunch {
 #endif
 };
 
+// a / b for a >= 0, b > 0 (a 64-bit division costs a hundred-odd instructions; the quotients here nearly always fit 32 bits)
+__host__ __device__ __forceinline__ int q4u_div(long long a, int b)
+{
+    return (a >> 32) ? (int)(a / b) : (int)((uint32_t)a / (uint32_t)b);
+}
+
 // Pieces of batch b when the (batch, chunk) sequence is cut every W: the CTAs first .. last hold one piece each.
 __host__ __device__ __forceinline__ void q4u_pieces(int b, int nchunks, int W, int* first, int* last)
 {
-    *first = (int)(((long long)b * nchunks) / W);
-    *last = (int)((((long long)b + 1) * nchunks - 1) / W);
+    *first = q4u_div((long long)b * nchunks, W);
+    *last = q4u_div(((long long)b + 1) * nchunks - 1, W);
 }
 
 // ---------------------------------------------------------------------------
 // activation staging: fp32 rows -> hi/lo fp16 tiles in the order the MMA's shared-memory descriptor wants
 // ---------------------------------------------------------------------------
-// gridDim.x = staged rows (rows >= M are zeros), gridDim.y = parts of a row = one cluster.  Row m of a chunk's tile lies at
+// gridDim.x = staged rows (rows >= M are zeros), gridDim.y = parts of a row.  Row m of a chunk's tile lies at
 // (m/8)*1024 + (m%8)*128 bytes; inside the row the 16-byte group j (8 halves) is stored at group j ^ (m % 8) (SWIZZLE_128B,
 // K-major).  SWIGLU: X is [M][2K] = [gate | up] and silu(gate) * up is what gets staged.
-// Bound by latency (64 rows are 256 CTAs of a few loads each).  Each CTA finds the largest magnitude of its own part, keeps
-// the part in shared memory (cached) and takes the maximum over the cluster; when every CTA read the whole row for it, the
-// SwiGLU needed a kernel and a pass over memory of its own.  70B feed-forward
-// block at 64 rows: 346 -> 339 us.
+// Bound by latency (64 rows are 256 CTAs of a few loads each).  The CTAs of a row each read all of it (from L2) to find its
+// largest magnitude.  With SWIGLU they are a cluster: each computes its own part once, keeps it in shared memory (cached) and
+// takes the maximum over the cluster, where the SwiGLU was a kernel and a pass over memory in front: 70B feed-forward block at
+// 64 rows 346 -> 339 us.  For plain rows the cluster's launch and barriers cost more than the reads (about 0.8 us of 19 at
+// short K).
 template <bool SWIGLU>
 __global__ void __launch_bounds__(256) q4u_xstage_kernel(const float* __restrict__ X, int M, int Mp, int K, int nchunks, int cached,
                                                           unsigned char* __restrict__ XS, float* __restrict__ inv_sc)
@@ -114,9 +121,9 @@ __global__ void __launch_bounds__(256) q4u_xstage_kernel(const float* __restrict
     float sc = 1.f;
     if (m < M) {                                           // (the CTAs of a cluster share the row)
         uint32_t mx = 0;
-        for (int f = f0 + tid; f < f1 && 4 * f < K; f += 256) {
+        for (int f = (SWIGLU ? f0 : 0) + tid; f < (SWIGLU ? f1 : n4) && 4 * f < K; f += 256) {
             const float4 v = load(f);
-            if (cached) s_part[f - f0] = v;                // read back by the same thread
+            if (SWIGLU && cached) s_part[f - f0] = v;      // read back by the same thread
             mx = max(mx, __float_as_uint(v.x) & 0x7FFFFFFFu);
             mx = max(mx, __float_as_uint(v.y) & 0x7FFFFFFFu);
             mx = max(mx, __float_as_uint(v.z) & 0x7FFFFFFFu);
@@ -129,11 +136,13 @@ __global__ void __launch_bounds__(256) q4u_xstage_kernel(const float* __restrict
         mx = s_max[0];
 #pragma unroll
         for (int w = 1; w < 8; ++w) mx = max(mx, s_max[w]);
-        if (tid == 0) s_all = mx;
-        cg::cluster_group cluster = cg::this_cluster();
-        cluster.sync();
-        for (unsigned r = 0; r < cluster.num_blocks(); ++r) mx = max(mx, *cluster.map_shared_rank(&s_all, r));
-        cluster.sync();                                    // nobody leaves before its maximum has been read
+        if (SWIGLU) {
+            if (tid == 0) s_all = mx;
+            cg::cluster_group cluster = cg::this_cluster();
+            cluster.sync();
+            for (unsigned r = 0; r < cluster.num_blocks(); ++r) mx = max(mx, *cluster.map_shared_rank(&s_all, r));
+            cluster.sync();                                // nobody leaves before its maximum has been read
+        }
         int emax = (int)(mx >> 23);
         float inv = 1.f;
         if (mx != 0 && emax < 255) {                       // the largest |x| of the row goes to [2^14, 2^15)
@@ -145,7 +154,7 @@ __global__ void __launch_bounds__(256) q4u_xstage_kernel(const float* __restrict
     }
     for (int f = f0 + tid; f < f1; f += 256) {
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (m < M && 4 * f < K) v = cached ? s_part[f - f0] : load(f);
+        if (m < M && 4 * f < K) v = SWIGLU && cached ? s_part[f - f0] : load(f);
         const float e0 = v.x * sc, e1 = v.y * sc, e2 = v.z * sc, e3 = v.w * sc;
         const __half2 h01 = __floats2half2_rn(e0, e1), h23 = __floats2half2_rn(e2, e3);
         const float2 f01 = __half22float2(h01), f23 = __half22float2(h23);
