@@ -968,11 +968,11 @@ static int32_t q4_gemm_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
     if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4_gemm_pair_kernel launch failed: %s", cudaGetErrorString(e));
     if (pl.cut) {
         cfg = {};
-        cfg.gridDim = dim3((unsigned)std::min<int64_t>(((int64_t)nb * nt * Mt + 3) / 4, (int64_t)ctx->prop.multiProcessorCount * 16));
+        cfg.gridDim = dim3((unsigned)((int64_t)nb * nt * (Mt / 4)));
         cfg.blockDim = dim3(256);
         cfg.stream = s;
         launch_pdl(cfg, at, ctx->pdl);
-        e = cudaLaunchKernelEx(&cfg, q4g_reduce_kernel, (const float*)ctx->q4_rect_partial, M, Mt, (int)q.N, nt, q.nchunks, W, nb * nt, y, ldy);
+        e = cudaLaunchKernelEx(&cfg, q4g_reduce_kernel, (const float*)ctx->q4_rect_partial, M, Mt, (int)q.N, nt, q.nchunks, W, y, ldy);
         ctx->launches += 1;
         if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4g_reduce_kernel launch failed: %s", cudaGetErrorString(e));
     }
@@ -1081,6 +1081,7 @@ static int q4_slab_rows(const mpq_context* ctx, const Q4Dev& q, int64_t M)
     }
     return 16;
 }
+
 static int32_t q4_umma_slabs(mpq_context* ctx, const Q4Dev& q, const float* x, bool swiglu, int64_t M, float* y, int64_t ldy, cudaStream_t s)
 {
     for (int64_t m0 = 0; m0 < M; m0 += 64) {
@@ -1089,7 +1090,6 @@ static int32_t q4_umma_slabs(mpq_context* ctx, const Q4Dev& q, const float* x, b
     }
     return MPQ_OK;
 }
-
 
 static int32_t q4_forward_checked(mpq_context* ctx, const mpq_weight* w, const float* x_dev, int64_t M, float* y_dev,
                                   int64_t ldy, cudaStream_t s)
