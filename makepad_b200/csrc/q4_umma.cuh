@@ -121,7 +121,8 @@ __global__ void __launch_bounds__(256) q4u_xstage_kernel(const float* __restrict
     float sc = 1.f;
     if (m < M) {                                           // (the CTAs of a cluster share the row)
         uint32_t mx = 0;
-        for (int f = (SWIGLU ? f0 : 0) + tid; f < (SWIGLU ? f1 : n4) && 4 * f < K; f += 256) {
+        const int end = SWIGLU ? min(f1, K / 4) : K / 4;   // one bound: the loads of several rounds go out together
+        for (int f = (SWIGLU ? f0 : 0) + tid; f < end; f += 256) {
             const float4 v = load(f);
             if (SWIGLU && cached) s_part[f - f0] = v;      // read back by the same thread
             mx = max(mx, __float_as_uint(v.x) & 0x7FFFFFFFu);
