@@ -24,6 +24,7 @@
 #include "q4_gemm.cuh"
 #include "q4_rect.cuh"
 #include "q4_umma.cuh"
+#include "scratch.h"
 #include "upload.h"
 
 using namespace mpq;
@@ -41,13 +42,10 @@ struct mpq_context {
     size_t hx_bytes, hy_bytes;
     // scratch of the streaming Q4 kernel: tagged partial tiles of row pair-tiles cut by a boundary
     // between two CTAs' runs (two slots per CTA; write-once / read-once per launch), one status word
-    unsigned char* q4u_xs;    // staged activations of the tcgen05 kernel (grown on demand), then 64 floats of row scales
-    size_t q4u_xs_bytes;
-    float* swiglu_buf;        // SwiGLU output for the Q4 kernels that do not fuse it (grown on demand)
-    size_t swiglu_bytes;
+    Scratch q4u_xs;           // staged activations of the tcgen05 kernels, then the row scales
+    Scratch swiglu_buf;       // SwiGLU output for the Q4 kernels that do not fuse it
     int q4_umma_min;          // fewest activation rows routed to the tcgen05 kernel (0 = never)
-    float* q4_rect_partial;   // [K slices][M][N] partial outputs of the rectangle kernel (grown on demand)
-    size_t q4_rect_partial_bytes;
+    Scratch q4_partial;       // partial outputs: [K slices][M][N] of the rectangle kernel, the pieces of the tcgen05 kernels
     int q4_gemm_min;          // fewest activation rows routed to the CTA-pair kernel (0 = never: slabs of 64 through the tcgen05 kernel)
     bool q4_rect;             // use the rectangle kernel for 5..16 rows (else slabs of <= 4 rows through the streaming kernel)
     int q4_stream_max_m;      // most activation rows mpq_q4_linear_forward gives to the streaming kernel (1..4)
@@ -150,12 +148,6 @@ extern "C" int32_t mpq_context_create(int32_t device, mpq_context** out)
     c->hx = c->hy = nullptr;
     c->hx_bytes = c->hy_bytes = 0;
     c->q4_partials = nullptr;
-    c->q4u_xs = nullptr;
-    c->q4u_xs_bytes = 0;
-    c->swiglu_buf = nullptr;
-    c->swiglu_bytes = 0;
-    c->q4_rect_partial = nullptr;
-    c->q4_rect_partial_bytes = 0;
     c->q4_partials_ctas = 0;
     c->q4_status = nullptr;
     c->upload_stream = nullptr;
@@ -210,9 +202,9 @@ extern "C" int32_t mpq_context_destroy(mpq_context* ctx)
     cudaFree(ctx->hx);
     cudaFree(ctx->hy);
     cudaFree(ctx->q4_partials);
-    cudaFree(ctx->q4u_xs);
-    cudaFree(ctx->swiglu_buf);
-    cudaFree(ctx->q4_rect_partial);
+    ctx->q4u_xs.release();
+    ctx->swiglu_buf.release();
+    ctx->q4_partial.release();
     cudaFree(ctx->q4_status);
     ctx->fp4.release();
     ctx->upload.release();
@@ -692,19 +684,9 @@ static int32_t q4_rect_forward(mpq_context* ctx, const Q4Dev& q, const Q4RectPla
 {
     int32_t st = q4_status_word(ctx);
     if (st) return st;
-    if (pl.nks > 1) {
-        const size_t need = (size_t)pl.nks * M * q.N * sizeof(float);
-        if (ctx->q4_rect_partial_bytes < need) {
-            CU_TRY(ctx, cudaDeviceSynchronize());          // nobody may still be using the old array
-            cudaFree(ctx->q4_rect_partial);
-            ctx->q4_rect_partial = nullptr;
-            ctx->q4_rect_partial_bytes = 0;
-            CU_TRY(ctx, cudaMalloc(&ctx->q4_rect_partial, need));
-            ctx->q4_rect_partial_bytes = need;
-        }
-    }
+    if (pl.nks > 1) CU_TRY(ctx, ctx->q4_partial.reserve((size_t)pl.nks * M * q.N * sizeof(float)));
     Q4RectLaunch p;
-    p.stream = q.stream; p.X = x; p.Y = y; p.partial = ctx->q4_rect_partial;
+    p.stream = q.stream; p.X = x; p.Y = y; p.partial = ctx->q4_partial.as<float>();
     p.M = M; p.N = (int)q.N; p.K = (int)q.K; p.ldy = ldy;
     p.nchunks = q.nchunks; p.nrp = q.nrp; p.ntg = pl.ntg; p.nks = pl.nks; p.slice_chunks = pl.slice_chunks; p.depth = pl.depth;
     p.status = ctx->q4_status;
@@ -729,7 +711,7 @@ static int32_t q4_rect_forward(mpq_context* ctx, const Q4Dev& q, const Q4RectPla
         at[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = at;
         cfg.numAttrs = ctx->pdl ? 1u : 0u;
-        e = cudaLaunchKernelEx(&cfg, q4_rect_reduce_kernel, (const float*)ctx->q4_rect_partial, pl.nks, M, (int)q.N, y, ldy);
+        e = cudaLaunchKernelEx(&cfg, q4_rect_reduce_kernel, (const float*)ctx->q4_partial.as<float>(), pl.nks, M, (int)q.N, y, ldy);
         ctx->launches += 1;
         if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4_rect_reduce_kernel launch failed: %s", cudaGetErrorString(e));
     }
@@ -739,19 +721,6 @@ static int32_t q4_rect_forward(mpq_context* ctx, const Q4Dev& q, const Q4RectPla
 // ---------------------------------------------------------------------------
 // the tcgen05 kernel: 5..64 rows per pass, weights read once
 // ---------------------------------------------------------------------------
-static int32_t q4_partial_scratch(mpq_context* ctx, size_t need)
-{
-    if (ctx->q4_rect_partial_bytes < need) {
-        CU_TRY(ctx, cudaDeviceSynchronize());          // nobody may still be using the old array
-        cudaFree(ctx->q4_rect_partial);
-        ctx->q4_rect_partial = nullptr;
-        ctx->q4_rect_partial_bytes = 0;
-        CU_TRY(ctx, cudaMalloc(&ctx->q4_rect_partial, need));
-        ctx->q4_rect_partial_bytes = need;
-    }
-    return MPQ_OK;
-}
-
 static cudaError_t launch_pdl(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, bool pdl)
 {
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -770,15 +739,9 @@ static int32_t q4_umma_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
     if (st) return st;
     // staged activations: per chunk a hi and a lo tile of Mp rows x 128 bytes, then the row scales
     const size_t xs_bytes = (size_t)q.nchunks * 2 * Mp * 128, need = xs_bytes + 64 * sizeof(float);
-    if (ctx->q4u_xs_bytes < need) {
-        CU_TRY(ctx, cudaDeviceSynchronize());
-        cudaFree(ctx->q4u_xs);
-        ctx->q4u_xs = nullptr;
-        ctx->q4u_xs_bytes = 0;
-        CU_TRY(ctx, cudaMalloc(&ctx->q4u_xs, need));
-        ctx->q4u_xs_bytes = need;
-    }
-    float* inv_sc = reinterpret_cast<float*>(ctx->q4u_xs + (ctx->q4u_xs_bytes - 64 * sizeof(float)));
+    CU_TRY(ctx, ctx->q4u_xs.reserve(need));
+    unsigned char* xs = ctx->q4u_xs.as<unsigned char>();
+    float* inv_sc = reinterpret_cast<float*>(xs + xs_bytes);
     // equal ranges of the (batch, chunk) sequence, one per SM; at least four chunks each (a piece costs a partial slice)
     const int ng = (q.nrp + 3) / 4;
     const int nbatches = (ng + Q4U_TEAMS - 1) / Q4U_TEAMS;
@@ -792,7 +755,8 @@ static int32_t q4_umma_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
         q4u_pieces(bb, q.nchunks, W, &pf, &pl);
         maxp = std::max(maxp, pl - pf + 1);
     }
-    if (maxp > 1 && (st = q4_partial_scratch(ctx, (size_t)maxp * M * q.N * sizeof(float)))) return st;
+    if (maxp > 1) CU_TRY(ctx, ctx->q4_partial.reserve((size_t)maxp * M * q.N * sizeof(float)));
+    float* partial = ctx->q4_partial.as<float>();
 
     cudaLaunchAttribute at[2];
     cudaLaunchConfig_t cfg = {};
@@ -809,12 +773,12 @@ static int32_t q4_umma_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
         at[cfg.numAttrs].val.clusterDim.x = 1; at[cfg.numAttrs].val.clusterDim.y = (unsigned)parts; at[cfg.numAttrs].val.clusterDim.z = 1;
         cfg.numAttrs += 1;
     }
-    cudaError_t e = cudaLaunchKernelEx(&cfg, swiglu ? q4u_xstage_kernel<true> : q4u_xstage_kernel<false>, x, M, Mp, (int)q.K, q.nchunks, cached, ctx->q4u_xs, inv_sc);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, swiglu ? q4u_xstage_kernel<true> : q4u_xstage_kernel<false>, x, M, Mp, (int)q.K, q.nchunks, cached, xs, inv_sc);
     ctx->launches += 1;
     if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4u_xstage_kernel launch failed: %s", cudaGetErrorString(e));
 
     Q4ULaunch p;
-    p.stream = q.stream; p.XS = ctx->q4u_xs; p.inv_sc = inv_sc; p.Y = y; p.partial = ctx->q4_rect_partial;
+    p.stream = q.stream; p.XS = xs; p.inv_sc = inv_sc; p.Y = y; p.partial = partial;
     p.M = M; p.Mp = Mp; p.N = (int)q.N; p.ldy = ldy; p.nchunks = q.nchunks; p.nrp = q.nrp; p.ngroups = ng;
     p.nbatches = nbatches; p.W = W; p.stack = stack; p.status = ctx->q4_status;
     // shared memory: activation ring, the teams' weight rings as deep as the rest allows, barriers (+ 1 KiB for the alignment)
@@ -846,7 +810,7 @@ static int32_t q4_umma_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
         cfg.blockDim = dim3(256);
         cfg.stream = s;
         launch_pdl(cfg, at, ctx->pdl);
-        e = cudaLaunchKernelEx(&cfg, q4u_reduce_kernel, (const float*)ctx->q4_rect_partial, M, (int)q.N, q.nchunks, W, y, ldy);
+        e = cudaLaunchKernelEx(&cfg, q4u_reduce_kernel, (const float*)partial, M, (int)q.N, q.nchunks, W, y, ldy);
         ctx->launches += 1;
         if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4u_reduce_kernel launch failed: %s", cudaGetErrorString(e));
     }
@@ -928,18 +892,12 @@ static int32_t q4_gemm_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
     if (st) return st;
     const Q4GemmPlan pl = q4_gemm_plan(q, M, pairs_max);
     const int nt = pl.nt, Mt = pl.Mt, W = pl.W, nb = (q.nrp + 7) / 8;
-    if (ctx->q4u_xs_bytes < pl.need_xs) {
-        CU_TRY(ctx, cudaDeviceSynchronize());
-        cudaFree(ctx->q4u_xs);
-        ctx->q4u_xs = nullptr;
-        ctx->q4u_xs_bytes = 0;
-        CU_TRY(ctx, cudaMalloc(&ctx->q4u_xs, pl.need_xs));
-        ctx->q4u_xs_bytes = pl.need_xs;
-    }
-    float* inv_sc = reinterpret_cast<float*>(ctx->q4u_xs + pl.xs_bytes);
-    if (pl.cut && (st = q4_partial_scratch(ctx, pl.need_partial))) return st;
+    CU_TRY(ctx, ctx->q4u_xs.reserve(pl.need_xs));
+    CU_TRY(ctx, ctx->q4_partial.reserve(pl.need_partial));
+    unsigned char* xs = ctx->q4u_xs.as<unsigned char>();
+    float *inv_sc = reinterpret_cast<float*>(xs + pl.xs_bytes), *partial = ctx->q4_partial.as<float>();
     CUtensorMap map_x;
-    if (!make_rows128_map(&map_x, ctx->q4u_xs, (int64_t)nt * q.nchunks * 2 * Mt, Mt / 2)) return fail(ctx, MPQ_ERR_CUDA, "cuTensorMapEncodeTiled failed for the staged activations");
+    if (!make_rows128_map(&map_x, xs, (int64_t)nt * q.nchunks * 2 * Mt, Mt / 2)) return fail(ctx, MPQ_ERR_CUDA, "cuTensorMapEncodeTiled failed for the staged activations");
 
     cudaLaunchAttribute at[1];
     cudaLaunchConfig_t cfg = {};
@@ -949,12 +907,12 @@ static int32_t q4_gemm_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
     cfg.dynamicSmemBytes = cached ? (size_t)q.K * 4 : 0;
     cfg.stream = s;
     launch_pdl(cfg, at, ctx->pdl);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, swiglu ? q4g_xstage_kernel<true> : q4g_xstage_kernel<false>, x, M, Mt, (int)q.K, q.nchunks, cached, ctx->q4u_xs, inv_sc);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, swiglu ? q4g_xstage_kernel<true> : q4g_xstage_kernel<false>, x, M, Mt, (int)q.K, q.nchunks, cached, xs, inv_sc);
     ctx->launches += 1;
     if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4g_xstage_kernel launch failed: %s", cudaGetErrorString(e));
 
     Q4GemmLaunch p;
-    p.stream = q.stream; p.inv_sc = inv_sc; p.Y = y; p.partial = ctx->q4_rect_partial;
+    p.stream = q.stream; p.inv_sc = inv_sc; p.Y = y; p.partial = partial;
     p.M = M; p.Mt = Mt; p.N = (int)q.N; p.nt = nt; p.ldy = ldy; p.nchunks = q.nchunks; p.nrp = q.nrp; p.W = W; p.total = pl.total;
     p.status = ctx->q4_status;
     cfg = {};
@@ -972,7 +930,7 @@ static int32_t q4_gemm_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
         cfg.blockDim = dim3(256);
         cfg.stream = s;
         launch_pdl(cfg, at, ctx->pdl);
-        e = cudaLaunchKernelEx(&cfg, q4g_reduce_kernel, (const float*)ctx->q4_rect_partial, M, Mt, (int)q.N, nt, q.nchunks, W, y, ldy);
+        e = cudaLaunchKernelEx(&cfg, q4g_reduce_kernel, (const float*)partial, M, Mt, (int)q.N, nt, q.nchunks, W, y, ldy);
         ctx->launches += 1;
         if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4g_reduce_kernel launch failed: %s", cudaGetErrorString(e));
     }
@@ -1013,7 +971,7 @@ static int q4_gemm_route(const mpq_context* ctx, const Q4Dev& q, int64_t M, cuda
         need_xs = std::max(need_xs, pl.need_xs);
         need_partial = std::max(need_partial, pl.need_partial);
     }
-    if ((ctx->q4u_xs_bytes < need_xs || ctx->q4_rect_partial_bytes < need_partial) && stream_captures(s)) return 0;
+    if ((ctx->q4u_xs.bytes() < need_xs || ctx->q4_partial.bytes() < need_partial) && stream_captures(s)) return 0;
     return pairs;
 }
 
@@ -1189,17 +1147,10 @@ extern "C" int32_t mpq_q4_linear_forward_swiglu(mpq_context* ctx, const mpq_weig
     }
     if (const int pairs = q4_gemm_route(ctx, q, M, s)) return q4_gemm_slabs(ctx, q, gate_up_dev, true, M, y_dev, q.N, pairs, s);
     if (ctx->q4_umma_min > 0 && M >= ctx->q4_umma_min) return q4_umma_slabs(ctx, q, gate_up_dev, true, M, y_dev, q.N, s);
-    const size_t need = (size_t)M * q.K * sizeof(float);
-    if (ctx->swiglu_bytes < need) {
-        CU_TRY(ctx, cudaDeviceSynchronize());
-        cudaFree(ctx->swiglu_buf);
-        ctx->swiglu_buf = nullptr;
-        ctx->swiglu_bytes = 0;
-        CU_TRY(ctx, cudaMalloc(&ctx->swiglu_buf, need));
-        ctx->swiglu_bytes = need;
-    }
-    if ((st = swiglu_launch(ctx, gate_up_dev, M, q.K, ctx->swiglu_buf, s))) return st;
-    return q4_forward_checked(ctx, w, ctx->swiglu_buf, M, y_dev, q.N, s);
+    CU_TRY(ctx, ctx->swiglu_buf.reserve((size_t)M * q.K * sizeof(float)));
+    float* hidden = ctx->swiglu_buf.as<float>();
+    if ((st = swiglu_launch(ctx, gate_up_dev, M, q.K, hidden, s))) return st;
+    return q4_forward_checked(ctx, w, hidden, M, y_dev, q.N, s);
 }
 
 static int32_t grow(mpq_context* ctx, float** buf, size_t* have, size_t need)

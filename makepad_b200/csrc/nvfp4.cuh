@@ -10,6 +10,8 @@
 
 #include <string>
 
+#include "scratch.h"
+
 #include "../../include/mpq.h"
 
 namespace mpq {
@@ -29,12 +31,10 @@ struct Nvfp4Dev {
 };
 
 struct Nvfp4Scratch {
-    uint8_t* sfa_tiled = nullptr;      // activation scale factors re-tiled per call
-    size_t sfa_bytes = 0;
-    float* partial = nullptr;          // fp32 sums of tiles cut along K (at most one wave of tiles: 17 MB)
-    size_t partial_bytes = 0;
+    Scratch sfa_tiled;                 // activation scale factors re-tiled per call
+    Scratch partial;                   // fp32 sums of tiles cut along K (at most one wave of tiles: 17 MB)
     int* status = nullptr;             // set non-zero when a bounded wait in the GEMM kernel ran out
-    void release() { cudaFree(sfa_tiled); cudaFree(status); cudaFree(partial); sfa_tiled = nullptr; status = nullptr; partial = nullptr; sfa_bytes = partial_bytes = 0; }
+    void release() { sfa_tiled.release(); partial.release(); cudaFree(status); status = nullptr; }
 };
 
 void nvfp4_dequant_launch(const uint8_t* codes, const uint8_t* sf, float ts, int64_t R, int64_t K, float* out, cudaStream_t s);

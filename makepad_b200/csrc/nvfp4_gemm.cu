@@ -1275,17 +1275,9 @@ int32_t nvfp4_gemm_launch(Nvfp4Scratch& scratch, const Nvfp4Dev& w, const uint8_
     const bool direct = K % 256 == 0 && (reinterpret_cast<uintptr_t>(a_sf) & 15u) == 0;
     cudaError_t e = cudaSuccess;
     if (!direct) {
-        size_t need = sf_tiled_bytes(M, K, BM, 2);
-        if (scratch.sfa_bytes < need) {
-            cudaDeviceSynchronize();
-            cudaFree(scratch.sfa_tiled);
-            scratch.sfa_tiled = nullptr;
-            scratch.sfa_bytes = 0;
-            e = cudaMalloc(&scratch.sfa_tiled, need);
-            if (e != cudaSuccess) { err = std::string("scratch allocation failed: ") + cudaGetErrorString(e); return MPQ_ERR_CUDA; }
-            scratch.sfa_bytes = need;
-        }
-        e = sf_tile_launch(a_sf, M, K, BM, scratch.sfa_tiled, s, 2);
+        e = scratch.sfa_tiled.reserve(sf_tiled_bytes(M, K, BM, 2));
+        if (e != cudaSuccess) { err = std::string("scratch allocation failed: ") + cudaGetErrorString(e); return MPQ_ERR_CUDA; }
+        e = sf_tile_launch(a_sf, M, K, BM, scratch.sfa_tiled.as<uint8_t>(), s, 2);
         *launches += 1;
         if (e != cudaSuccess) { err = std::string("scale-factor tiling failed: ") + cudaGetErrorString(e); return MPQ_ERR_CUDA; }
     }
@@ -1323,7 +1315,7 @@ int32_t nvfp4_gemm_launch(Nvfp4Scratch& scratch, const Nvfp4Dev& w, const uint8_
             const double cost = 0.42 * ((pp.k_blocks + c - 1) / c) + 5.0 + 0.08 * rows * last * c;
             if (cost < best) { best = cost; splits = c; }
         }
-        if (splits > 1 && scratch.partial_bytes < (size_t)last * splits * 256 * BN * sizeof(float)) {
+        if (splits > 1 && scratch.partial.bytes() < (size_t)last * splits * 256 * BN * sizeof(float)) {
             cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;      // nothing can be allocated while a stream captures
             if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
                 cudaGetLastError();
@@ -1334,18 +1326,10 @@ int32_t nvfp4_gemm_launch(Nvfp4Scratch& scratch, const Nvfp4Dev& w, const uint8_
         pp.whole = splits > 1 ? tiles - last : tiles;
         pp.items = pp.whole + (tiles - pp.whole) * splits;
         if (splits > 1) {
-            const size_t need = (size_t)(pp.items - pp.whole) * 256 * BN * sizeof(float);
-            if (scratch.partial_bytes < need) {
-                cudaDeviceSynchronize();                           // nobody may still be using the old array
-                cudaFree(scratch.partial);
-                scratch.partial = nullptr;
-                scratch.partial_bytes = 0;
-                e = cudaMalloc(&scratch.partial, need);
-                if (e != cudaSuccess) { err = std::string("scratch allocation failed: ") + cudaGetErrorString(e); return MPQ_ERR_CUDA; }
-                scratch.partial_bytes = need;
-            }
+            e = scratch.partial.reserve((size_t)(pp.items - pp.whole) * 256 * BN * sizeof(float));
+            if (e != cudaSuccess) { err = std::string("scratch allocation failed: ") + cudaGetErrorString(e); return MPQ_ERR_CUDA; }
         }
-        pp.partial = scratch.partial;
+        pp.partial = scratch.partial.as<float>();
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)(2 * std::min(nclusters, pp.items)));
         cfg.blockDim = dim3(V2_THREADS);
@@ -1356,7 +1340,7 @@ int32_t nvfp4_gemm_launch(Nvfp4Scratch& scratch, const Nvfp4Dev& w, const uint8_
         at[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = at;
         cfg.numAttrs = pdl ? 1u : 0u;
-        e = cudaLaunchKernelEx(&cfg, nvfp4_gemm_pair_kernel_v2, map_a, map_bh, map_sfa, map_c, pp, (const uint8_t*)scratch.sfa_tiled, (const uint8_t*)w.sf_tiled);
+        e = cudaLaunchKernelEx(&cfg, nvfp4_gemm_pair_kernel_v2, map_a, map_bh, map_sfa, map_c, pp, (const uint8_t*)scratch.sfa_tiled.as<uint8_t>(), (const uint8_t*)w.sf_tiled);
         *launches += 1;
         if (e == cudaSuccess && splits > 1) {
             cfg.gridDim = dim3((unsigned)std::min(sm_count * 8, last * 64));
@@ -1371,7 +1355,7 @@ int32_t nvfp4_gemm_launch(Nvfp4Scratch& scratch, const Nvfp4Dev& w, const uint8_
     CUtensorMap map_b, map_c1;
     if (!make_map(&map_b, w.codes, N, K, BN) || !make_c_map(&map_c1, c, M, N, OUT_COLS)) { err = "cuTensorMapEncodeTiled failed"; return MPQ_ERR_CUDA; }
     GemmParams p;
-    p.sfa = scratch.sfa_tiled; p.sfb = w.sf_tiled; p.C = reinterpret_cast<__nv_bfloat16*>(c);
+    p.sfa = scratch.sfa_tiled.as<uint8_t>(); p.sfb = w.sf_tiled; p.C = reinterpret_cast<__nv_bfloat16*>(c);
     p.M = (int)M; p.N = (int)N; p.K = (int)K;
     p.m_tiles = (int)((M + BM - 1) / BM); p.n_tiles = (int)((N + BN - 1) / BN);
     p.k_blocks = (int)((K + BK - 1) / BK); p.ksteps_pad = ksteps_padded(K);

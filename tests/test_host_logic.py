@@ -1,6 +1,7 @@
 """Host-side logic of the library that needs no GPU: the per-device bookkeeping that guards settings CUDA
 keeps per device (kernel attributes, symbol addresses), compiled with g++ from the header the library uses."""
 import os
+import re
 import subprocess
 import sys
 import tempfile
@@ -55,3 +56,75 @@ def test_no_per_process_flag_guards_a_per_device_setting():
         if f.endswith((".cu", ".cuh")):
             text = open(os.path.join(csrc, f)).read()
             assert "static bool configured" not in text, f
+
+
+SCRATCH = r"""
+#include "scratch.h"
+#include <cstdio>
+#include <cstdlib>
+#include <map>
+static std::map<void*, size_t> live;            // the fake device's blocks
+static size_t most = 0;                         // the largest request that it grants
+static cudaError_t last = cudaSuccess;
+extern "C" cudaError_t cudaMalloc(void** p, size_t n)
+{
+    if (n > most) return last = cudaErrorMemoryAllocation;
+    live[*p = malloc(1)] = n;
+    return cudaSuccess;
+}
+extern "C" cudaError_t cudaFree(void* p)
+{
+    if (p) { live.erase(p); free(p); }
+    return cudaSuccess;
+}
+extern "C" cudaError_t cudaGetLastError() { const cudaError_t e = last; last = cudaSuccess; return e; }
+int main()
+{
+    int bad = 0;
+    mpq::Scratch s;
+    most = 1000000;
+    bad += s.reserve(100) != cudaSuccess || s.bytes() != 100;
+    void* first = s.as<void>();
+    bad += s.reserve(60) != cudaSuccess || s.as<void>() != first;           // enough: nothing changes
+    bad += s.reserve(150) != cudaSuccess || s.bytes() != 200;               // replaced by one of twice the size
+    bad += !live.count(first) || !live.count(s.as<void>());                 // and the replaced block still exists
+    // many small steps: the blocks that were replaced are together smaller than the one in use
+    for (size_t n = 200; n < 20000; n += 7) bad += s.reserve(n) != cudaSuccess || s.bytes() < n;
+    size_t all = 0;
+    for (auto& b : live) all += b.second;
+    bad += all - s.bytes() >= s.bytes();
+    // no room for twice the size: as much as needed; no room for that either: an error, nothing changed, no error left behind
+    const size_t had = s.bytes();
+    most = had + 1;
+    bad += s.reserve(had + 1) != cudaSuccess || s.bytes() != had + 1;
+    void* now = s.as<void>();
+    const size_t blocks = live.size();
+    bad += s.reserve(had + 2) == cudaSuccess || s.bytes() != had + 1 || s.as<void>() != now || live.size() != blocks;
+    bad += cudaGetLastError() != cudaSuccess;
+    s.release();
+    bad += !live.empty() || s.bytes() != 0 || s.as<void>() != nullptr;
+    most = 1000000;
+    bad += s.reserve(10) != cudaSuccess || live.size() != 1;                // and it can be used again
+    s.release();
+    std::printf("%d\n", bad);
+    return bad;
+}
+"""
+
+
+def _run(program, *flags):
+    with tempfile.TemporaryDirectory() as tmp:
+        src, exe = os.path.join(tmp, "t.cpp"), os.path.join(tmp, "t")
+        open(src, "w").write(program)
+        cuda = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+        subprocess.check_call(["g++", "-std=c++17", "-O1", "-I", os.path.join(ROOT, "makepad_b200", "csrc"), "-I", cuda, *flags, src, "-o", exe])
+        out = subprocess.run([exe], capture_output=True, text=True)
+        assert out.returncode == 0 and out.stdout.strip() == "0", out.stdout + out.stderr
+
+
+def test_a_replaced_scratch_block_lives_until_the_context_is_destroyed():
+    """A captured graph holds the addresses of the blocks that its launches were given."""
+    _run(SCRATCH)
+    for f in ("mpq.cu", "nvfp4_gemm.cu", "nvfp4.cuh"):         # and no growing buffer is freed anywhere else
+        text = open(os.path.join(ROOT, "makepad_b200", "csrc", f)).read()
+        assert not re.search(r"cudaFree\([^;]*\b(q4u_xs|swiglu_buf|q4_partial|q4_rect_partial|sfa_tiled|partial)\b", text), f

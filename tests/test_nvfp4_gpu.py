@@ -341,3 +341,42 @@ def test_tiles_split_along_k(ctx, orc, M, N, K):
     rows = sorted({0, M - 1} | set(np.random.default_rng(3).integers(0, M, 6).tolist()))
     c32, _ = orc.nvfp4_gemm(a[rows], sfa[rows], 0.5, b, sfb, 2.0)
     _check(orc, y[rows].view(torch.int16).cpu().numpy().view(np.uint16), c32)
+
+
+def test_a_graph_of_cut_tiles_replays_after_calls_that_need_more_scratch():
+    """4096 x 14336: 1000 rows need 28 partial tiles, 16 rows 57.  A graph of 1000 rows gives the same bits after eager calls of
+    16 rows and calls with another K (whose scale factors are re-tiled into scratch)."""
+    import torch
+    import makepad_b200
+    N, K = 4096, 14336
+    c2 = makepad_b200.Context(0)
+    lin = makepad_b200.QuantLinear(makepad_b200.Nvfp4Weight(c2, *synth.nvfp4_tensor(N, K, seed=61, stream=1), 1.0))
+    odd = makepad_b200.QuantLinear(makepad_b200.Nvfp4Weight(c2, *synth.nvfp4_tensor(512, 6176, seed=62, stream=1), 1.0))
+    g = torch.Generator(device="cuda")
+    g.manual_seed(63)
+
+    def rows(m, k):
+        return (torch.randint(0, 256, (m, k // 2), dtype=torch.uint8, device="cuda", generator=g),
+                (torch.randn((m, k // 16), device="cuda", generator=g).abs() * 0.1).to(torch.float8_e4m3fn).view(torch.uint8), 1.0)
+
+    graphs = []
+    for layer, a in ((lin, rows(1000, K)), (odd, rows(64, 6176))):
+        want = layer(a)
+        torch.cuda.synchronize()
+        y = torch.empty_like(want)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            layer.forward(a, out=y)
+        graphs.append((graph, y, want, a))
+    lin(rows(16, K)), odd(rows(3000, 6176))
+    torch.cuda.synchronize()
+    guard = [torch.full((1 << 18,), 5.0, device="cuda") for _ in range(64)]        # memory that a freed block would have become
+    for graph, y, want, _ in graphs:
+        y.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, want)
+    assert all((t == 5.0).all() for t in guard)
+    assert c2.lib.mpq_context_poll_status(c2.h) == _lib.OK
+    graphs.clear()
+    c2.close()

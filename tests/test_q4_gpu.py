@@ -458,3 +458,44 @@ def test_staging_of_a_row_by_a_cluster(ctx, orc, N, K, M):
     assert torch.equal(lin.forward_swiglu(gate_up), lin(makepad_b200.swiglu(ctx, gate_up)))
     torch.cuda.synchronize()
     assert ctx.lib.mpq_context_poll_status(ctx.h) == _lib.OK
+
+
+def test_a_graph_replays_after_the_scratch_has_grown(orc):
+    """Graphs of 8, 40 and 128 rows, then eager calls that need far more scratch (a prompt, a longer K): the graphs still give what
+    they gave, and write nothing but their own memory."""
+    import makepad_b200
+    torch = _torch()
+    N, K = 1000, 2112
+    c2 = makepad_b200.Context(0)
+    codes, scales = synth.q4_weight(N, K, seed=51)
+    lin = makepad_b200.QuantLinear(makepad_b200.Q4Weight(c2, codes, scales))
+    big = makepad_b200.QuantLinear(makepad_b200.Q4Weight(c2, *synth.q4_weight(3000, 8192, seed=52)))
+    graphs = []
+    for M in (8, 40, 128):
+        x = synth.activations(M, K, seed=53 + M)
+        xd, gud = torch.from_numpy(x).cuda(), torch.from_numpy(synth.activations(M, 2 * K, seed=54)).cuda()
+        lin(xd), lin.forward_swiglu(gud)                               # warm-up
+        torch.cuda.synchronize()
+        y, z = torch.empty((M, N), device="cuda"), torch.empty((M, N), device="cuda")
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            lin.forward(xd, out=y)
+            lin.forward_swiglu(gud, out=z)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert orc.err_report(y.cpu().numpy(), orc.q4_matmul_f64(codes, scales, x))["max_abs_over_rms"] < 2e-5
+        graphs.append((graph, y, z, y.clone(), z.clone(), xd, gud))
+    for M in (40, 600, 2100):
+        big(torch.randn((M, 8192), device="cuda"))
+        big.forward_swiglu(torch.randn((M, 2 * 8192), device="cuda"))
+    torch.cuda.synchronize()
+    guard = [torch.full((1 << 18,), 5.0, device="cuda") for _ in range(64)]        # memory that a freed block would have become
+    for graph, y, z, y0, z0, *_ in graphs:
+        y.fill_(float("nan")), z.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, y0) and torch.equal(z, z0)
+    assert all((g == 5.0).all() for g in guard)
+    assert c2.lib.mpq_context_poll_status(c2.h) == _lib.OK
+    graphs.clear()
+    c2.close()
