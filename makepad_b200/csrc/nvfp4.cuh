@@ -32,7 +32,7 @@ struct Nvfp4Dev {
 
 struct Nvfp4Scratch {
     Scratch sfa_tiled;                 // activation scale factors re-tiled per call
-    Scratch partial;                   // fp32 sums of tiles cut along K (at most one wave of tiles: 17 MB)
+    Scratch partial;                   // fp32 sums of tiles cut along K (one wave of tiles: 17 MB)
     int* status = nullptr;             // set non-zero when a bounded wait in the GEMM kernel ran out
     void release() { sfa_tiled.release(); partial.release(); cudaFree(status); status = nullptr; }
 };

@@ -1315,20 +1315,18 @@ int32_t nvfp4_gemm_launch(Nvfp4Scratch& scratch, const Nvfp4Dev& w, const uint8_
             const double cost = 0.42 * ((pp.k_blocks + c - 1) / c) + 5.0 + 0.08 * rows * last * c;
             if (cost < best) { best = cost; splits = c; }
         }
-        if (splits > 1 && scratch.partial.bytes() < (size_t)last * splits * 256 * BN * sizeof(float)) {
-            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;      // nothing can be allocated while a stream captures
-            if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
-                cudaGetLastError();
-                splits = 1;
-            }
+        // Room for the sums of one wave of tiles (17 MB on 74 pairs), which no cut passes (last * splits <= nclusters): reserved
+        // by the first call outside a capture, so that a later capture of any other call finds it.  Without it tiles stay whole.
+        if (!scratch.partial.bytes()) {
+            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+            const cudaError_t known = cudaStreamIsCapturing(s, &cs);
+            if (known == cudaSuccess && cs == cudaStreamCaptureStatusNone) scratch.partial.reserve((size_t)nclusters * 256 * BN * sizeof(float));
+            else if (known != cudaSuccess) cudaGetLastError();
         }
+        if (!scratch.partial.bytes()) splits = 1;
         pp.splits = splits;
         pp.whole = splits > 1 ? tiles - last : tiles;
         pp.items = pp.whole + (tiles - pp.whole) * splits;
-        if (splits > 1) {
-            e = scratch.partial.reserve((size_t)(pp.items - pp.whole) * 256 * BN * sizeof(float));
-            if (e != cudaSuccess) { err = std::string("scratch allocation failed: ") + cudaGetErrorString(e); return MPQ_ERR_CUDA; }
-        }
         pp.partial = scratch.partial.as<float>();
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)(2 * std::min(nclusters, pp.items)));

@@ -380,3 +380,43 @@ def test_a_graph_of_cut_tiles_replays_after_calls_that_need_more_scratch():
     assert c2.lib.mpq_context_poll_status(c2.h) == _lib.OK
     graphs.clear()
     c2.close()
+
+
+@pytest.mark.parametrize("warm", ["larger", "other kernel"])
+def test_a_captured_gemm_cuts_its_tiles_like_an_eager_one(orc, monkeypatch, warm):
+    """16 rows of 4096 x 14336 want more room for partial tiles than 1000 rows do: captured after a warm-up with the larger M the
+    call still has two launches (GEMM, sum of the cut tiles) and the eager call's bits.  With no room reserved (the warm-up went
+    to the one-CTA kernel) the captured call keeps its tiles whole and agrees with the oracle."""
+    import torch
+    import makepad_b200
+    N, K, M = 4096, 14336, 16
+    b, sfb = synth.nvfp4_tensor(N, K, seed=71, stream=1)
+    a, sfa = synth.nvfp4_tensor(M, K, seed=71, stream=0)
+    big = synth.nvfp4_tensor(1000, K, seed=72, stream=0)
+    c2 = makepad_b200.Context(0)
+    lin = makepad_b200.QuantLinear(makepad_b200.Nvfp4Weight(c2, b, sfb, 1.0))
+    at = (torch.from_numpy(a).cuda(), torch.from_numpy(sfa).cuda(), 0.5)
+    if warm == "other kernel":
+        monkeypatch.setenv("MPQ_FP4_KERNEL", "single")
+    lin((torch.from_numpy(big[0]).cuda(), torch.from_numpy(big[1]).cuda(), 1.0))
+    torch.cuda.synchronize()
+    monkeypatch.delenv("MPQ_FP4_KERNEL", raising=False)
+    y = torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    before = c2.launches
+    with torch.cuda.graph(graph):
+        lin.forward(at, out=y)
+    captured = c2.launches - before
+    graph.replay()
+    torch.cuda.synchronize()
+    before = c2.launches
+    eager = lin(at)
+    assert c2.launches - before == 2
+    assert captured == (2 if warm == "larger" else 1)
+    if warm == "larger":
+        assert torch.equal(y, eager)
+    c32, _ = orc.nvfp4_gemm(a, sfa, 0.5, b, sfb, 1.0)
+    _check(orc, y.view(torch.int16).cpu().numpy().view(np.uint16), c32)
+    assert c2.lib.mpq_context_poll_status(c2.h) == _lib.OK
+    del graph
+    c2.close()
