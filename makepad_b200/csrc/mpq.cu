@@ -22,6 +22,7 @@
 #include "per_device.h"
 #include "q4.cuh"
 #include "q4_gemm.cuh"
+#include "q4_plan.h"
 #include "q4_rect.cuh"
 #include "q4_umma.cuh"
 #include "scratch.h"
@@ -70,6 +71,8 @@ struct mpq_weight {
     int fmt;
     int device;
     Q4Dev q4;
+    size_t q4_rect_partial;   // most partial sums that 2..16 rows of this weight want (the rectangle kernel)
+    int q4_umma_pieces;       // pieces that q4_umma_kernel cuts a batch of this weight into
     Nvfp4Dev fp4;
 };
 
@@ -237,6 +240,9 @@ extern "C" int64_t mpq_context_launch_count(const mpq_context* ctx) { return ctx
 // ---------------------------------------------------------------------------
 // Q4 weights
 // ---------------------------------------------------------------------------
+// what q4_reserve wants to know of a weight
+static void q4_note_needs(const mpq_context* ctx, mpq_weight* w);
+
 // the weight with its device memory, not yet filled
 static int32_t q4_alloc(mpq_context* ctx, int64_t N, int64_t K, mpq_weight** out)
 {
@@ -256,6 +262,7 @@ static int32_t q4_alloc(mpq_context* ctx, int64_t N, int64_t K, mpq_weight** out
         delete w;
         return fail(ctx, MPQ_ERR_CUDA, "cudaMalloc of %zu weight bytes failed: %s", q.bytes(), cudaGetErrorString(e));
     }
+    q4_note_needs(ctx, w);
     *out = w;
     return MPQ_OK;
 }
@@ -646,6 +653,16 @@ static bool q4_rect_plan(const mpq_context* ctx, const Q4Dev& q, int M, Q4RectPl
     return found;
 }
 
+static void q4_note_needs(const mpq_context* ctx, mpq_weight* w)
+{
+    w->q4_umma_pieces = q4_umma_plan(w->q4.nrp, w->q4.nchunks, ctx->prop.multiProcessorCount).pieces;
+    w->q4_rect_partial = 0;
+    Q4RectPlan pl;
+    for (int M = 2; M <= 16 && ctx->q4_rect; ++M)
+        if (q4_rect_plan(ctx, w->q4, M, &pl) && pl.nks > 1)
+            w->q4_rect_partial = std::max(w->q4_rect_partial, (size_t)pl.nks * M * w->q4.N * sizeof(float));
+}
+
 template <int MT>
 static cudaError_t q4_rect_launch_t(int device, const Q4RectLaunch& p, int grid, size_t smem, bool pdl, cudaStream_t s)
 {
@@ -734,28 +751,16 @@ static cudaError_t launch_pdl(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, 
 static int32_t q4_umma_forward(mpq_context* ctx, const Q4Dev& q, const float* x, bool swiglu, int M, float* y, int64_t ldy, cudaStream_t s)
 {
     const int sms = ctx->prop.multiProcessorCount;
-    const int Mp = (M + 15) / 16 * 16;
+    const int Mp = q4_umma_rows(M);
     int32_t st = q4_status_word(ctx);
     if (st) return st;
-    // staged activations: per chunk a hi and a lo tile of Mp rows x 128 bytes, then the row scales
-    const size_t xs_bytes = (size_t)q.nchunks * 2 * Mp * 128, need = xs_bytes + 64 * sizeof(float);
-    CU_TRY(ctx, ctx->q4u_xs.reserve(need));
+    CU_TRY(ctx, ctx->q4u_xs.reserve(q4_umma_need_xs(q.nchunks, M)));
     unsigned char* xs = ctx->q4u_xs.as<unsigned char>();
-    float* inv_sc = reinterpret_cast<float*>(xs + xs_bytes);
-    // equal ranges of the (batch, chunk) sequence, one per SM; at least four chunks each (a piece costs a partial slice)
-    const int ng = (q.nrp + 3) / 4;
-    const int nbatches = (ng + Q4U_TEAMS - 1) / Q4U_TEAMS;
+    float* inv_sc = reinterpret_cast<float*>(xs + q4_umma_xs_bytes(q.nchunks, M));
     const int stack = Mp <= 32 ? 1 : 0;                // accumulators of 2 Mp columns where they fit in a team's 64
-    const long long total = (long long)nbatches * q.nchunks;
-    int W = (int)std::max<long long>((total + sms - 1) / sms, std::min<long long>(4, total));
-    const int grid = (int)((total + W - 1) / W);
-    int maxp = 1;
-    for (int bb = 0; bb < nbatches; ++bb) {
-        int pf, pl;
-        q4u_pieces(bb, q.nchunks, W, &pf, &pl);
-        maxp = std::max(maxp, pl - pf + 1);
-    }
-    if (maxp > 1) CU_TRY(ctx, ctx->q4_partial.reserve((size_t)maxp * M * q.N * sizeof(float)));
+    const Q4UmmaPlan pl = q4_umma_plan(q.nrp, q.nchunks, sms);
+    const int W = pl.W;
+    CU_TRY(ctx, ctx->q4_partial.reserve(q4_umma_need_partial(pl.pieces, M, q.N)));
     float* partial = ctx->q4_partial.as<float>();
 
     cudaLaunchAttribute at[2];
@@ -779,8 +784,8 @@ static int32_t q4_umma_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
 
     Q4ULaunch p;
     p.stream = q.stream; p.XS = xs; p.inv_sc = inv_sc; p.Y = y; p.partial = partial;
-    p.M = M; p.Mp = Mp; p.N = (int)q.N; p.ldy = ldy; p.nchunks = q.nchunks; p.nrp = q.nrp; p.ngroups = ng;
-    p.nbatches = nbatches; p.W = W; p.stack = stack; p.status = ctx->q4_status;
+    p.M = M; p.Mp = Mp; p.N = (int)q.N; p.ldy = ldy; p.nchunks = q.nchunks; p.nrp = q.nrp; p.ngroups = pl.ngroups;
+    p.nbatches = pl.nbatches; p.W = W; p.stack = stack; p.status = ctx->q4_status;
     // shared memory: activation ring, the teams' weight rings as deep as the rest allows, barriers (+ 1 KiB for the alignment)
     const size_t smem_max = (size_t)ctx->prop.sharedMemPerBlockOptin - 256, xring_bytes = (size_t)Q4U_XSTAGES * 2 * Mp * 128;
     p.wstages = (int)std::min<size_t>(Q4U_MAX_WSTAGES, (smem_max - xring_bytes - 2048) / ((size_t)Q4U_TEAMS * Q4U_WSTAGE_BYTES));
@@ -795,7 +800,7 @@ static int32_t q4_umma_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
         configured.mark(ctx->device);
     }
     cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
+    cfg.gridDim = dim3((unsigned)pl.grid);
     cfg.blockDim = dim3(Q4U_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
@@ -803,7 +808,7 @@ static int32_t q4_umma_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
     e = cudaLaunchKernelEx(&cfg, q4_umma_kernel, p);
     ctx->launches += 1;
     if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4_umma_kernel launch failed: %s", cudaGetErrorString(e));
-    if (maxp > 1) {
+    if (pl.pieces > 1) {
         cfg = {};
         const int64_t tot = (int64_t)M * ((q.N + 3) / 4);
         cfg.gridDim = dim3((unsigned)std::min<int64_t>((tot + 255) / 256, (int64_t)sms * 8));
@@ -855,42 +860,12 @@ static int q4_gemm_pairs(const mpq_context* ctx)
     return n;
 }
 
-// How one slab of M rows is cut, and the scratch that takes.
-struct Q4GemmPlan { int nt, Mt, W, pairs; int64_t total; bool cut; size_t xs_bytes, need_xs, need_partial; };
-static Q4GemmPlan q4_gemm_plan(const Q4Dev& q, int M, int pairs_max)
-{
-    Q4GemmPlan pl;
-    // as few activation tiles as possible (each expands the weights again), as equal as possible, in steps of 32 rows (a
-    // quarter of the rows, eight or more, is what a team drains)
-    pl.nt = (M + Q4G_MT_MAX - 1) / Q4G_MT_MAX;
-    pl.Mt = ((M + pl.nt - 1) / pl.nt + 31) / 32 * 32;
-    pl.total = (int64_t)((q.nrp + 7) / 8) * pl.nt * q.nchunks;
-    pl.W = (int)std::max<int64_t>((pl.total + pairs_max - 1) / pairs_max, std::min<int64_t>(Q4G_MIN_W, pl.total));
-    pl.pairs = (int)((pl.total + pl.W - 1) / pl.W);
-    pl.cut = pl.W % q.nchunks != 0;                        // some tile lies in more than one range
-    pl.xs_bytes = (size_t)pl.nt * q.nchunks * 2 * pl.Mt * 128;
-    pl.need_xs = pl.xs_bytes + (size_t)M * sizeof(float);
-    pl.need_partial = pl.cut ? (size_t)pl.pairs * 2 * Q4G_SLOT * sizeof(float) : 0;
-    return pl;
-}
-
-// true when the stream must not see an allocation now
-static bool stream_captures(cudaStream_t s)
-{
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
-        cudaGetLastError();
-        return true;
-    }
-    return cs != cudaStreamCaptureStatusNone;
-}
-
 // y = x . W^T for M > 64 rows; with swiglu x is [M][2K] = [gate | up].  One slab's staged rows take M * K * 4 bytes of scratch.
 static int32_t q4_gemm_forward(mpq_context* ctx, const Q4Dev& q, const float* x, bool swiglu, int M, float* y, int64_t ldy, int pairs_max, cudaStream_t s)
 {
     int32_t st = q4_status_word(ctx);
     if (st) return st;
-    const Q4GemmPlan pl = q4_gemm_plan(q, M, pairs_max);
+    const Q4GemmPlan pl = q4_gemm_plan(q.nrp, q.nchunks, M, pairs_max);
     const int nt = pl.nt, Mt = pl.Mt, W = pl.W, nb = (q.nrp + 7) / 8;
     CU_TRY(ctx, ctx->q4u_xs.reserve(pl.need_xs));
     CU_TRY(ctx, ctx->q4_partial.reserve(pl.need_partial));
@@ -937,15 +912,9 @@ static int32_t q4_gemm_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
     return MPQ_OK;
 }
 
-// Rows per launch of the pair kernel: at most 2048, fewer where K is so long that the staged rows would pass 256 MB.
-static int64_t q4_gemm_slab(const Q4Dev& q)
-{
-    return std::max<int64_t>(Q4G_MT_MAX, std::min<int64_t>(2048, ((int64_t)1 << 26) / q.K / Q4G_MT_MAX * Q4G_MT_MAX));
-}
-
 static int32_t q4_gemm_slabs(mpq_context* ctx, const Q4Dev& q, const float* x, bool swiglu, int64_t M, float* y, int64_t ldy, int pairs_max, cudaStream_t s)
 {
-    const int64_t slab = q4_gemm_slab(q);
+    const int64_t slab = q4_gemm_slab(q.K);
     for (int64_t m0 = 0; m0 < M; m0 += slab) {
         const int32_t st = q4_gemm_forward(ctx, q, x + (size_t)m0 * q.K * (swiglu ? 2 : 1), swiglu, (int)std::min<int64_t>(slab, M - m0),
                                            y + (size_t)m0 * ldy, ldy, pairs_max, s);
@@ -954,24 +923,55 @@ static int32_t q4_gemm_slabs(mpq_context* ctx, const Q4Dev& q, const float* x, b
     return MPQ_OK;
 }
 
-// Pairs to run a call on, or 0 for the kernels of 64 rows and fewer: all calls above 64 rows go to the pair kernel (measured:
-// equal to two slabs of 64 on 57344 x 8192 at 65..96 rows, faster everywhere else) where the tcgen05 path is on and clusters of
-// two can be scheduled.  Slabs of 64 rows want no more scratch than a call of 64 rows; so a capture after such a warm-up,
-// in which nothing can be allocated, keeps to them.
-static int q4_gemm_route(const mpq_context* ctx, const Q4Dev& q, int64_t M, cudaStream_t s)
+// CTA pairs for a call of M rows, or 0 where it is one for the kernels of 64 rows and fewer: all calls above 64 rows go to the
+// pair kernel (measured: equal to two slabs of 64 on 57344 x 8192 at 65..96 rows, faster everywhere else) where the tcgen05
+// path is on and clusters of two can be scheduled.
+static int q4_gemm_wanted(const mpq_context* ctx, int64_t M)
 {
     if (ctx->q4_gemm_min <= 0 || M < ctx->q4_gemm_min || ctx->q4_umma_min <= 0 || M < ctx->q4_umma_min) return 0;
-    const int pairs = q4_gemm_pairs(ctx);
+    return q4_gemm_pairs(ctx);
+}
+
+// true when the stream must not see an allocation now
+static bool stream_captures(cudaStream_t s)
+{
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return cs != cudaStreamCaptureStatusNone;
+}
+
+// Scratch for this call and for every smaller one of the weight, so that a warm-up with the largest M is enough for graphs of
+// them all; with swiglu also the buffer of the rows that the rectangle kernel takes.  Nothing is allocated in a capture, and
+// an allocation that fails is no error here: what the call cannot do without it asks for itself.
+static void q4_reserve(mpq_context* ctx, const mpq_weight* w, int64_t M, bool swiglu, cudaStream_t s)
+{
+    const Q4Dev& q = w->q4;
+    const Q4Needs need = q4_needs(q.N, q.K, q.nrp, q.nchunks, M, w->q4_rect_partial, w->q4_umma_pieces, ctx->q4_umma_min, ctx->q4_gemm_min,
+                                  q4_gemm_wanted(ctx, M));
+    const size_t hidden = swiglu ? (size_t)(ctx->q4_umma_min > 0 ? std::min<int64_t>(M, ctx->q4_umma_min - 1) : M) * q.K * sizeof(float) : 0;
+    if (ctx->q4u_xs.bytes() >= need.xs && ctx->q4_partial.bytes() >= need.partial && ctx->swiglu_buf.bytes() >= hidden && ctx->q4_partials_ctas) return;
+    if (stream_captures(s)) return;
+    ctx->q4u_xs.reserve(need.xs);
+    ctx->q4_partial.reserve(need.partial);
+    ctx->swiglu_buf.reserve(hidden);
+    q4_stream_scratch(ctx, ctx->prop.multiProcessorCount);               // (one row streams)
+}
+
+// Pairs to run a call on, or 0.  Slabs of 64 rows want less scratch than the pair kernel: a capture without a warm-up of its
+// size, in which nothing can be allocated, keeps to them.
+static int q4_gemm_route(const mpq_context* ctx, const Q4Dev& q, int64_t M, cudaStream_t s)
+{
+    const int pairs = q4_gemm_wanted(ctx, M);
     if (!pairs) return 0;
-    const int64_t slab = q4_gemm_slab(q);
-    size_t need_xs = 0, need_partial = 0;
+    const int64_t slab = q4_gemm_slab(q.K);
     for (const int64_t rows : {std::min(M, slab), M % slab}) {
         if (!rows) continue;
-        const Q4GemmPlan pl = q4_gemm_plan(q, (int)rows, pairs);
-        need_xs = std::max(need_xs, pl.need_xs);
-        need_partial = std::max(need_partial, pl.need_partial);
+        const Q4GemmPlan pl = q4_gemm_plan(q.nrp, q.nchunks, (int)rows, pairs);
+        if ((ctx->q4u_xs.bytes() < pl.need_xs || ctx->q4_partial.bytes() < pl.need_partial) && stream_captures(s)) return 0;
     }
-    if ((ctx->q4u_xs.bytes() < need_xs || ctx->q4_partial.bytes() < need_partial) && stream_captures(s)) return 0;
     return pairs;
 }
 
@@ -1052,6 +1052,7 @@ static int32_t q4_umma_slabs(mpq_context* ctx, const Q4Dev& q, const float* x, b
 static int32_t q4_forward_checked(mpq_context* ctx, const mpq_weight* w, const float* x_dev, int64_t M, float* y_dev,
                                   int64_t ldy, cudaStream_t s)
 {
+    if (M > 4 || !q4_prefers_stream(ctx, w->q4, M)) q4_reserve(ctx, w, M, false, s);
     if (const int pairs = q4_gemm_route(ctx, w->q4, M, s)) return q4_gemm_slabs(ctx, w->q4, x_dev, false, M, y_dev, ldy, pairs, s);
     if (ctx->q4_umma_min > 0 && M >= ctx->q4_umma_min) {       // slabs of up to 64 rows on the tcgen05 path
         return q4_umma_slabs(ctx, w->q4, x_dev, false, M, y_dev, ldy, s);
@@ -1145,6 +1146,7 @@ extern "C" int32_t mpq_q4_linear_forward_swiglu(mpq_context* ctx, const mpq_weig
         p.swiglu = 1;
         return q4_stream_enqueue(ctx, pl, p, grid, s);
     }
+    q4_reserve(ctx, w, M, true, s);
     if (const int pairs = q4_gemm_route(ctx, q, M, s)) return q4_gemm_slabs(ctx, q, gate_up_dev, true, M, y_dev, q.N, pairs, s);
     if (ctx->q4_umma_min > 0 && M >= ctx->q4_umma_min) return q4_umma_slabs(ctx, q, gate_up_dev, true, M, y_dev, q.N, s);
     CU_TRY(ctx, ctx->swiglu_buf.reserve((size_t)M * q.K * sizeof(float)));
@@ -1722,6 +1724,7 @@ extern "C" int32_t mpq_weight_load(mpq_context* ctx, const char* path, mpq_weigh
         if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "upload of %s failed: %s", path, cudaGetErrorString(e));
         return fail(ctx, st, "%s: %s", path, st == MPQ_ERR_IO ? "read failed" : "checksum mismatch");
     }
+    if (h.fmt == MPQ_FMT_Q4) q4_note_needs(ctx, w);
     *out = w;
     return MPQ_OK;
 }

@@ -32,9 +32,6 @@ namespace mpq {
 
 constexpr int Q4G_THREADS = 32 * 18;       // (five warps on a scheduler: 96 registers a thread, 64 of them running sums)
 constexpr int Q4G_WSTAGES = 8, Q4G_XSTAGES = 5, Q4G_ASTAGES = 4;
-constexpr int Q4G_MT_MAX = 256;               // activation rows per tile: the accumulator's columns
-constexpr int Q4G_SLOT = 256 * Q4G_MT_MAX;    // floats of one partial slot: [row of x][256 weight rows]
-constexpr int Q4G_MIN_W = 4;                  // fewest chunks per pair
 
 struct Q4GemmLaunch {
     const uint4* stream;

@@ -1,0 +1,111 @@
+// How the tcgen05 Q4 kernels cut a call, and the scratch that it takes.  Host arithmetic, no device code.
+#pragma once
+#include <cuda_runtime.h>
+#include <stddef.h>
+#include <stdint.h>
+
+#include <algorithm>
+
+namespace mpq {
+
+constexpr int Q4U_TEAMS = 4;                  // pipelines per CTA of q4_umma_kernel (a power of two), one group of 128 rows each
+
+// a / b for a >= 0, b > 0 (a 64-bit division costs a hundred-odd instructions; the quotients here nearly always fit 32 bits)
+__host__ __device__ __forceinline__ int q4u_div(long long a, int b)
+{
+    return (a >> 32) ? (int)(a / b) : (int)((uint32_t)a / (uint32_t)b);
+}
+
+// Pieces of batch b when the (batch, chunk) sequence is cut every W: the CTAs first .. last hold one piece each.
+__host__ __device__ __forceinline__ void q4u_pieces(int b, int nchunks, int W, int* first, int* last)
+{
+    *first = q4u_div((long long)b * nchunks, W);
+    *last = q4u_div(((long long)b + 1) * nchunks - 1, W);
+}
+
+// ---------------------------------------------------------------------------
+// q4_umma_kernel: up to 64 rows
+// ---------------------------------------------------------------------------
+// equal ranges of W of the (batch, chunk) sequence, one per SM; at least four chunks each (a piece costs a partial slice)
+struct Q4UmmaPlan { int ngroups, nbatches, W, grid, pieces; };      // pieces: the most that a batch is cut into
+inline Q4UmmaPlan q4_umma_plan(int nrp, int nchunks, int sms)
+{
+    Q4UmmaPlan pl;
+    pl.ngroups = (nrp + 3) / 4;
+    pl.nbatches = (pl.ngroups + Q4U_TEAMS - 1) / Q4U_TEAMS;
+    const int64_t total = (int64_t)pl.nbatches * nchunks;
+    pl.W = (int)std::max<int64_t>((total + sms - 1) / sms, std::min<int64_t>(4, total));
+    pl.grid = (int)((total + pl.W - 1) / pl.W);
+    pl.pieces = 1;
+    for (int b = 0; b < pl.nbatches; ++b) {
+        int first, last;
+        q4u_pieces(b, nchunks, pl.W, &first, &last);
+        pl.pieces = std::max(pl.pieces, last - first + 1);
+    }
+    return pl;
+}
+inline int q4_umma_rows(int M) { return (M + 15) / 16 * 16; }
+// staged activations: per chunk a hi and a lo tile of the padded rows x 128 bytes; behind them the row scales
+inline size_t q4_umma_xs_bytes(int nchunks, int M) { return (size_t)nchunks * 2 * q4_umma_rows(M) * 128; }
+inline size_t q4_umma_need_xs(int nchunks, int M) { return q4_umma_xs_bytes(nchunks, M) + 64 * sizeof(float); }
+inline size_t q4_umma_need_partial(int pieces, int M, int64_t N) { return pieces > 1 ? (size_t)pieces * M * N * sizeof(float) : 0; }
+
+// ---------------------------------------------------------------------------
+// q4_gemm_pair_kernel: more than 64 rows
+// ---------------------------------------------------------------------------
+constexpr int Q4G_MT_MAX = 256;               // activation rows per tile: the accumulator's columns
+constexpr int Q4G_SLOT = 256 * Q4G_MT_MAX;    // floats of one partial slot: [row of x][256 weight rows]
+constexpr int Q4G_MIN_W = 4;                  // fewest chunks per pair
+
+// How one slab of M rows is cut, and the scratch that takes.
+struct Q4GemmPlan { int nt, Mt, W, pairs; int64_t total; bool cut; size_t xs_bytes, need_xs, need_partial; };
+inline Q4GemmPlan q4_gemm_plan(int nrp, int nchunks, int M, int pairs_max)
+{
+    Q4GemmPlan pl;
+    // as few activation tiles as possible (each expands the weights again), as equal as possible, in steps of 32 rows (a
+    // quarter of the rows, eight or more, is what a team drains)
+    pl.nt = (M + Q4G_MT_MAX - 1) / Q4G_MT_MAX;
+    pl.Mt = ((M + pl.nt - 1) / pl.nt + 31) / 32 * 32;
+    pl.total = (int64_t)((nrp + 7) / 8) * pl.nt * nchunks;
+    pl.W = (int)std::max<int64_t>((pl.total + pairs_max - 1) / pairs_max, std::min<int64_t>(Q4G_MIN_W, pl.total));
+    pl.pairs = (int)((pl.total + pl.W - 1) / pl.W);
+    pl.cut = pl.W % nchunks != 0;                          // some tile lies in more than one range
+    pl.xs_bytes = (size_t)pl.nt * nchunks * 2 * pl.Mt * 128;
+    pl.need_xs = pl.xs_bytes + (size_t)M * sizeof(float);
+    pl.need_partial = pl.cut ? (size_t)pl.pairs * 2 * Q4G_SLOT * sizeof(float) : 0;
+    return pl;
+}
+
+// Rows per launch of the pair kernel: at most 2048, fewer where K is so long that the staged rows would pass 256 MB.
+inline int64_t q4_gemm_slab(int64_t K)
+{
+    return std::max<int64_t>(Q4G_MT_MAX, std::min<int64_t>(2048, ((int64_t)1 << 26) / K / Q4G_MT_MAX * Q4G_MT_MAX));
+}
+
+// ---------------------------------------------------------------------------
+// scratch for every call of 2 .. M rows
+// ---------------------------------------------------------------------------
+// Less rows can want more: 512 rows of 57344 x 8192 take 38.8 MB of partial sums, 64 rows 44.0 MB.  A program warms up with its
+// largest call before it captures graphs, so that call reserves what the smaller ones want.  rect_partial: the most that
+// 2 .. 16 rows want; umma_pieces: Q4UmmaPlan::pieces; umma_min, gemm_min: fewest rows of the two kernels (0: never);
+// pairs_max: CTA pairs of the device.
+struct Q4Needs { size_t xs, partial; };
+inline Q4Needs q4_needs(int64_t N, int64_t K, int nrp, int nchunks, int64_t M, size_t rect_partial, int umma_pieces, int umma_min, int gemm_min,
+                        int pairs_max)
+{
+    Q4Needs n = {0, rect_partial};
+    if (umma_min <= 0 || M < umma_min) return n;
+    const int rows = (int)std::min<int64_t>(M, 64);
+    n.xs = q4_umma_need_xs(nchunks, rows);
+    n.partial = std::max(n.partial, q4_umma_need_partial(umma_pieces, rows, N));
+    if (gemm_min <= 0 || M < gemm_min || pairs_max <= 0) return n;
+    // The staged rows grow with M.  The number of ranges does not, but it is at most the device's pairs, and each holds at
+    // least Q4G_MIN_W chunks of the largest call.
+    const Q4GemmPlan pl = q4_gemm_plan(nrp, nchunks, (int)std::min<int64_t>(M, q4_gemm_slab(K)), pairs_max);
+    const int64_t most = std::min<int64_t>(pairs_max, (pl.total + Q4G_MIN_W - 1) / Q4G_MIN_W);
+    n.xs = std::max(n.xs, pl.need_xs);
+    n.partial = std::max(n.partial, (size_t)most * 2 * Q4G_SLOT * sizeof(float));
+    return n;
+}
+
+}  // namespace mpq

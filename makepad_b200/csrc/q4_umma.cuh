@@ -41,11 +41,11 @@
 #include <cuda_fp16.h>
 
 #include "q4.cuh"
+#include "q4_plan.h"
 
 namespace mpq {
 
-constexpr int Q4U_TEAMS = 4;                  // pipelines per CTA (a power of two): issuer warp + four expansion warps each
-constexpr int Q4U_THREADS = 32 * (2 + Q4U_TEAMS + 4 * Q4U_TEAMS);   // weight producer, issuers, expansion warps, activation producer
+constexpr int Q4U_THREADS = 32 * (2 + Q4U_TEAMS + 4 * Q4U_TEAMS);   // weight producer, activation producer; per team an issuer and four expansion warps
 constexpr int Q4U_MAX_WSTAGES = 8;            // weight ring PER TEAM: at most so many stages of one (group, chunk) = 4 units
 constexpr int Q4U_WSTAGE_BYTES = 4 * Q4_UNIT_BYTES;
 constexpr int Q4U_XSTAGES = 4;                // activation ring: stages of one chunk (hi tile + lo tile)
@@ -74,19 +74,6 @@ struct Q4ULaunch {
     unsigned long long* trace;    // diagnostic build: per CTA 16 counters (see the kernel)
 #endif
 };
-
-// a / b for a >= 0, b > 0 (a 64-bit division costs a hundred-odd instructions; the quotients here nearly always fit 32 bits)
-__host__ __device__ __forceinline__ int q4u_div(long long a, int b)
-{
-    return (a >> 32) ? (int)(a / b) : (int)((uint32_t)a / (uint32_t)b);
-}
-
-// Pieces of batch b when the (batch, chunk) sequence is cut every W: the CTAs first .. last hold one piece each.
-__host__ __device__ __forceinline__ void q4u_pieces(int b, int nchunks, int W, int* first, int* last)
-{
-    *first = q4u_div((long long)b * nchunks, W);
-    *last = q4u_div(((long long)b + 1) * nchunks - 1, W);
-}
 
 // ---------------------------------------------------------------------------
 // activation staging: fp32 rows -> hi/lo fp16 tiles in the order the MMA's shared-memory descriptor wants

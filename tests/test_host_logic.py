@@ -128,3 +128,49 @@ def test_a_replaced_scratch_block_lives_until_the_context_is_destroyed():
     for f in ("mpq.cu", "nvfp4_gemm.cu", "nvfp4.cuh"):         # and no growing buffer is freed anywhere else
         text = open(os.path.join(ROOT, "makepad_b200", "csrc", f)).read()
         assert not re.search(r"cudaFree\([^;]*\b(q4u_xs|swiglu_buf|q4_partial|q4_rect_partial|sfa_tiled|partial)\b", text), f
+
+
+NEEDS = r"""
+#include "q4_plan.h"
+#include <cstdio>
+using namespace mpq;
+int main()
+{
+    int bad = 0;
+    const int64_t shapes[][2] = {{57344, 8192}, {128256, 4096}, {22016, 4096}, {4096, 11008}, {8192, 28672}, {500, 1056}, {1, 32}, {33, 288}, {96, 28672}, {20000, 64}};
+    for (auto& nk : shapes)
+        for (int sms : {148, 132})
+            for (int pairs : {74, 66, 0}) {
+                const int64_t N = nk[0], K = nk[1];
+                const int nrp = (int)((N + 31) / 32), nchunks = (int)((K + 63) / 64 + 3) / 4 * 4;
+                const int pieces = q4_umma_plan(nrp, nchunks, sms).pieces;
+                for (int64_t M : {17, 64, 65, 100, 257, 512, 700, 2100}) {
+                    const Q4Needs n = q4_needs(N, K, nrp, nchunks, M, 1000, pieces, 17, 65, pairs);
+                    bad += n.partial < 1000;                                    // what 2..16 rows want
+                    for (int64_t m = 17; m <= M; ++m) {                         // no smaller call, by either kernel, wants more
+                        const int u = (int)(m < 64 ? m : 64);
+                        bad += q4_umma_need_xs(nchunks, u) > n.xs || q4_umma_need_partial(pieces, u, N) > n.partial;
+                        if (m < 65 || !pairs) continue;
+                        const Q4GemmPlan pl = q4_gemm_plan(nrp, nchunks, (int)std::min<int64_t>(m, q4_gemm_slab(K)), pairs);
+                        bad += pl.need_xs > n.xs || pl.need_partial > n.partial;
+                    }
+                }
+            }
+    // the shapes whose 64 rows want more partial sums than 512 rows
+    const int64_t wide[][3] = {{57344, 8192, 44040192}, {128256, 4096, 65667072}};
+    for (auto& s : wide) {
+        const int nrp = (int)(s[0] / 32), nchunks = (int)(s[1] / 64), pieces = q4_umma_plan(nrp, nchunks, 148).pieces;
+        bad += q4_umma_need_partial(pieces, 64, s[0]) != (size_t)s[2] || q4_gemm_plan(nrp, nchunks, 512, 74).need_partial >= (size_t)s[2];
+        bad += q4_needs(s[0], s[1], nrp, nchunks, 512, 0, pieces, 17, 65, 74).partial < (size_t)s[2];
+    }
+    // few rows of x go to kernels with needs of their own
+    bad += q4_needs(4096, 4096, 128, 64, 16, 77, 2, 17, 65, 74).xs != 0 || q4_needs(4096, 4096, 128, 64, 16, 77, 2, 17, 65, 74).partial != 77;
+    bad += q4_needs(4096, 4096, 128, 64, 300, 77, 2, 0, 65, 74).xs != 0;
+    std::printf("%d\n", bad);
+    return bad;
+}
+"""
+
+
+def test_scratch_reserved_for_a_call_is_enough_for_every_smaller_one():
+    _run(NEEDS)

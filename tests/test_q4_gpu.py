@@ -499,3 +499,39 @@ def test_a_graph_replays_after_the_scratch_has_grown(orc):
     assert c2.lib.mpq_context_poll_status(c2.h) == _lib.OK
     graphs.clear()
     c2.close()
+
+
+@pytest.mark.parametrize("N,K,warm", [(500, 1056, 300), (57344, 8192, 512), (4096, 11008, 40)])
+def test_a_warm_up_with_the_largest_call_is_enough_to_capture_smaller_ones(N, K, warm):
+    """After one eager call, captures of every smaller kind of call (streaming, rectangle, both tcgen05 kernels, with and without
+    SwiGLU) allocate nothing, take the kernels that an eager call takes, and give its bits."""
+    import makepad_b200
+    torch = _torch()
+    c2 = makepad_b200.Context(0)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(6)
+    codes = torch.randint(0, 256, (N, K // 2), dtype=torch.uint8, device="cuda", generator=g).cpu().numpy()
+    scales = (torch.rand((N, K // 32), device="cuda", generator=g) * 0.02).to(torch.float16).cpu().numpy().view(np.uint16)
+    lin = makepad_b200.QuantLinear(makepad_b200.Q4Weight(c2, codes, scales))
+    x, gate_up = torch.randn((warm, K), device="cuda", generator=g), torch.randn((warm, 2 * K), device="cuda", generator=g)
+    lin.forward_swiglu(gate_up)
+    torch.cuda.synchronize()
+    done = []
+    for M in [m for m in (1, 3, 5, 16, 17, 64, 100, 257, warm) if m <= warm]:
+        y, z = torch.full((M, N), float("nan"), device="cuda"), torch.full((M, N), float("nan"), device="cuda")
+        graph = torch.cuda.CUDAGraph()
+        before = c2.launches
+        with torch.cuda.graph(graph):
+            lin.forward(x[:M], out=y)
+            lin.forward_swiglu(gate_up[:M], out=z)
+        done.append((M, graph, y, z, c2.launches - before))
+    for M, graph, y, z, launches in done:
+        graph.replay()
+        before = c2.launches
+        want = lin(x[:M]), lin.forward_swiglu(gate_up[:M])
+        assert c2.launches - before == launches, M
+        assert torch.equal(y, want[0]) and torch.equal(z, want[1]), M
+    torch.cuda.synchronize()
+    assert c2.lib.mpq_context_poll_status(c2.h) == _lib.OK
+    done.clear()
+    c2.close()
