@@ -960,9 +960,9 @@ static void q4_reserve(mpq_context* ctx, const mpq_weight* w, int64_t M, bool sw
     q4_stream_scratch(ctx, ctx->prop.multiProcessorCount);               // (one row streams)
 }
 
-// Pairs to run a call on, or 0.  Slabs of 64 rows want less scratch than the pair kernel: a capture without a warm-up of its
-// size, in which nothing can be allocated, keeps to them.
-static int q4_gemm_route(const mpq_context* ctx, const Q4Dev& q, int64_t M, cudaStream_t s)
+// Pairs to run a call on, or 0.  Slabs of 64 rows want less scratch than the pair kernel: a call whose scratch could not be had
+// (in a capture without a warm-up of its size, or for want of memory) keeps to them.
+static int q4_gemm_route(const mpq_context* ctx, const Q4Dev& q, int64_t M)
 {
     const int pairs = q4_gemm_wanted(ctx, M);
     if (!pairs) return 0;
@@ -970,7 +970,7 @@ static int q4_gemm_route(const mpq_context* ctx, const Q4Dev& q, int64_t M, cuda
     for (const int64_t rows : {std::min(M, slab), M % slab}) {
         if (!rows) continue;
         const Q4GemmPlan pl = q4_gemm_plan(q.nrp, q.nchunks, (int)rows, pairs);
-        if ((ctx->q4u_xs.bytes() < pl.need_xs || ctx->q4_partial.bytes() < pl.need_partial) && stream_captures(s)) return 0;
+        if (ctx->q4u_xs.bytes() < pl.need_xs || ctx->q4_partial.bytes() < pl.need_partial) return 0;
     }
     return pairs;
 }
@@ -1053,7 +1053,7 @@ static int32_t q4_forward_checked(mpq_context* ctx, const mpq_weight* w, const f
                                   int64_t ldy, cudaStream_t s)
 {
     if (M > 4 || !q4_prefers_stream(ctx, w->q4, M)) q4_reserve(ctx, w, M, false, s);
-    if (const int pairs = q4_gemm_route(ctx, w->q4, M, s)) return q4_gemm_slabs(ctx, w->q4, x_dev, false, M, y_dev, ldy, pairs, s);
+    if (const int pairs = q4_gemm_route(ctx, w->q4, M)) return q4_gemm_slabs(ctx, w->q4, x_dev, false, M, y_dev, ldy, pairs, s);
     if (ctx->q4_umma_min > 0 && M >= ctx->q4_umma_min) {       // slabs of up to 64 rows on the tcgen05 path
         return q4_umma_slabs(ctx, w->q4, x_dev, false, M, y_dev, ldy, s);
     }
@@ -1147,7 +1147,7 @@ extern "C" int32_t mpq_q4_linear_forward_swiglu(mpq_context* ctx, const mpq_weig
         return q4_stream_enqueue(ctx, pl, p, grid, s);
     }
     q4_reserve(ctx, w, M, true, s);
-    if (const int pairs = q4_gemm_route(ctx, q, M, s)) return q4_gemm_slabs(ctx, q, gate_up_dev, true, M, y_dev, q.N, pairs, s);
+    if (const int pairs = q4_gemm_route(ctx, q, M)) return q4_gemm_slabs(ctx, q, gate_up_dev, true, M, y_dev, q.N, pairs, s);
     if (ctx->q4_umma_min > 0 && M >= ctx->q4_umma_min) return q4_umma_slabs(ctx, q, gate_up_dev, true, M, y_dev, q.N, s);
     CU_TRY(ctx, ctx->swiglu_buf.reserve((size_t)M * q.K * sizeof(float)));
     float* hidden = ctx->swiglu_buf.as<float>();

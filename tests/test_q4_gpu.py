@@ -535,3 +535,38 @@ def test_a_warm_up_with_the_largest_call_is_enough_to_capture_smaller_ones(N, K,
     assert c2.lib.mpq_context_poll_status(c2.h) == _lib.OK
     done.clear()
     c2.close()
+
+
+def test_a_prompt_without_room_for_the_pair_kernel(orc):
+    """With almost all device memory taken, a call whose staged rows do not fit runs as slabs of 64 rows: slower, not refused."""
+    import makepad_b200
+    torch = _torch()
+    N, K, M = 96, 8192, 2048
+    c2 = makepad_b200.Context(0)
+    codes, scales = synth.q4_weight(N, K, seed=81)
+    lin = makepad_b200.QuantLinear(makepad_b200.Q4Weight(c2, codes, scales))
+    x = synth.activations(M, K, seed=82)
+    xd = torch.from_numpy(x).cuda()
+    lin(xd[:64])
+    y = torch.empty((M, N), device="cuda")
+    before = c2.launches
+    lin.forward(xd[:300], out=y[:300])
+    pair_launches = c2.launches - before
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    held = [torch.empty(torch.cuda.mem_get_info()[0] - (40 << 20), dtype=torch.uint8, device="cuda")]    # 2048 staged rows take 64 MB
+    before = c2.launches
+    lin.forward(xd, out=y)
+    slab_launches = c2.launches - before
+    torch.cuda.synchronize()
+    held.clear()
+    torch.cuda.empty_cache()
+    assert pair_launches <= 3 and slab_launches >= 2 * M // 64
+    rows = [0, 63, 64, 1000, M - 1]
+    assert orc.err_report(y[rows].cpu().numpy(), orc.q4_matmul_f64(codes, scales, x[rows]))["max_abs_over_rms"] < 2e-5
+    before = c2.launches
+    lin.forward(xd, out=y)                                             # with room again: the pair kernel
+    assert c2.launches - before <= 3
+    torch.cuda.synchronize()
+    assert c2.lib.mpq_context_poll_status(c2.h) == _lib.OK
+    c2.close()
