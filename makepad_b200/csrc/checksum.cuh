@@ -17,6 +17,8 @@
 #include <stdint.h>
 #include <stdlib.h>
 
+#include "launch.h"
+
 namespace mpq {
 
 constexpr int FNV_CHUNK = 4096;               // bytes per warp of the map kernel: 7000 warps for 28 MB, three quarters of what the SMs hold
@@ -155,11 +157,10 @@ inline cudaError_t fnv1a64_device(const void* buf, int64_t bytes, uint64_t* h, u
     const uint8_t* b = static_cast<const uint8_t*>(buf);
     uint64_t* sum = reinterpret_cast<uint64_t*>(scratch);
     uint32_t* map = reinterpret_cast<uint32_t*>(scratch + off_map);
-    fnv_map_kernel<<<(unsigned)((chunks + 7) / 8), 256, 0, s>>>(b, bytes, chunks, map);
-    fnv_group_kernel<<<(unsigned)groups, 128, 0, s>>>(map, chunks, scratch + off_gmap);
-    fnv_walk_kernel<<<1, 256, 0, s>>>(reinterpret_cast<const uint32_t*>(scratch + off_gmap), groups, (uint32_t)(*h & 0xFFu), scratch + off_start);
-    fnv_sum_kernel<<<(unsigned)groups, FNV_GROUP, 0, s>>>(b, bytes, map, chunks, scratch + off_start, sum);
-    e = cudaGetLastError();
+    e = launch(fnv_map_kernel, (unsigned)((chunks + 7) / 8), 256, s, b, bytes, chunks, map);
+    if (e == cudaSuccess) e = launch(fnv_group_kernel, (unsigned)groups, 128, s, map, chunks, scratch + off_gmap);
+    if (e == cudaSuccess) e = launch(fnv_walk_kernel, 1, 256, s, reinterpret_cast<const uint32_t*>(scratch + off_gmap), groups, (uint32_t)(*h & 0xFFu), scratch + off_start);
+    if (e == cudaSuccess) e = launch(fnv_sum_kernel, (unsigned)groups, FNV_GROUP, s, b, bytes, map, chunks, scratch + off_start, sum);
     uint64_t* host = static_cast<uint64_t*>(malloc((size_t)groups * 9));
     uint8_t* host_l = host ? reinterpret_cast<uint8_t*>(host + groups) : nullptr;
     if (!host && e == cudaSuccess) e = cudaErrorMemoryAllocation;

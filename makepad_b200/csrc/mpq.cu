@@ -98,6 +98,7 @@ static int32_t exchange_note_call(mpq_context* ctx, mpq_exchange* ex, cudaStream
 
 static int32_t fail(mpq_context* ctx, int32_t code, const char* fmt, ...)
 {
+    if (code == MPQ_ERR_CUDA) cudaGetLastError();          // reported here: not left behind for a later call to find
     if (ctx) {
         char buf[512];
         va_list ap;
@@ -142,7 +143,7 @@ extern "C" int32_t mpq_context_create(int32_t device, mpq_context** out)
     if (!out) return MPQ_ERR_INVALID_ARG;
     *out = nullptr;
     int count = 0;
-    if (cudaGetDeviceCount(&count) != cudaSuccess || device < 0 || device >= count) return MPQ_ERR_CUDA;
+    if (cudaGetDeviceCount(&count) != cudaSuccess || device < 0 || device >= count) return fail(nullptr, MPQ_ERR_CUDA, "");
     mpq_context* c = new (std::nothrow) mpq_context();
     if (!c) return MPQ_ERR_CUDA;
     c->magic = CTX_MAGIC;
@@ -156,7 +157,7 @@ extern "C" int32_t mpq_context_create(int32_t device, mpq_context** out)
     c->upload_stream = nullptr;
     if (cudaSetDevice(device) != cudaSuccess || cudaGetDeviceProperties(&c->prop, device) != cudaSuccess) {
         delete c;
-        return MPQ_ERR_CUDA;
+        return fail(nullptr, MPQ_ERR_CUDA, "");
     }
     if (c->prop.major != 10) {   // sm_100a code only; no other path exists
         delete c;
@@ -164,7 +165,7 @@ extern "C" int32_t mpq_context_create(int32_t device, mpq_context** out)
     }
     if (cudaStreamCreateWithFlags(&c->upload_stream, cudaStreamNonBlocking) != cudaSuccess) {
         delete c;
-        return MPQ_ERR_CUDA;
+        return fail(nullptr, MPQ_ERR_CUDA, "");
     }
     const char* e = getenv("MPQ_PDL");
     c->pdl = !(e && e[0] == '0');
@@ -274,12 +275,13 @@ static cudaError_t q4_repack(mpq_context* ctx, const Q4Dev& q, int rp0, int64_t 
     const int nrp = (int)((rows + 31) / 32);
     const int64_t words = (int64_t)nrp * q.nchunks * 256, halves = (int64_t)nrp * q.nchunks * 64;
     unsigned char* to = reinterpret_cast<unsigned char*>(q.stream) + (size_t)rp0 * q.nchunks * Q4_UNIT_BYTES;
-    q4_repack_codes_kernel<<<(unsigned)((words + 255) / 256), 256, 0, s>>>(codes_dev, Kfull, 0, k0, rows, q.K, nrp, q.nchunks,
-                                                                           reinterpret_cast<uint32_t*>(to));
-    q4_repack_scales_kernel<<<(unsigned)((halves + 255) / 256), 256, 0, s>>>(scales_dev, Kfull / 32, 0, k0 / 32, rows, q.K / 32, nrp,
-                                                                             q.nchunks, reinterpret_cast<uint16_t*>(to));
+    cudaError_t e = launch(q4_repack_codes_kernel, (unsigned)((words + 255) / 256), 256, s, codes_dev, Kfull, 0, k0, rows, q.K, nrp, q.nchunks,
+                           reinterpret_cast<uint32_t*>(to));
+    if (e == cudaSuccess)
+        e = launch(q4_repack_scales_kernel, (unsigned)((halves + 255) / 256), 256, s, scales_dev, Kfull / 32, 0, k0 / 32, rows, q.K / 32, nrp, q.nchunks,
+                   reinterpret_cast<uint16_t*>(to));
     ctx->launches += 2;
-    return cudaGetLastError();
+    return e;
 }
 
 static int32_t q4_shard(mpq_context* ctx, int64_t N, int64_t K, int32_t tp_mode, int32_t rank, int32_t world,

@@ -139,3 +139,27 @@ def test_device_checksum_is_the_host_loop(ctx, tmp_path, N, K):
         with pytest.raises(makepad_b200.MpqError) as err:
             makepad_b200.load_weight(ctx, path)
         assert err.value.status == _lib.ERR_FORMAT
+
+
+@pytest.mark.gpu
+def test_a_weight_that_did_not_fit_does_not_fail_the_next_one(ctx, tmp_path):
+    """A creation that finds no device memory reports it once: the error is not left behind for the next creation, load or export."""
+    import makepad_b200
+    codes, scales = synth.q4_weight(96, 1216, seed=5)
+    path = str(tmp_path / "w.q4d")
+    makepad_b200.Q4Weight(ctx, codes, scales).save(path)
+    h = C.c_void_p()
+
+    def too_large():                                                   # 2^40 weights: 618 GB, refused before an array is read
+        assert ctx.lib.mpq_q4_weight_create(ctx.h, 1 << 20, 1 << 20, codes.ctypes.data, scales.ctypes.data, _lib.TP_NONE, 0, 1, C.byref(h)) == _lib.ERR_CUDA
+        assert not h.value
+
+    too_large()
+    w = makepad_b200.Q4Weight(ctx, codes, scales)
+    want = w.dequantize().cpu().numpy()
+    too_large()
+    assert np.array_equal(makepad_b200.load_weight(ctx, path).dequantize().cpu().numpy(), want)
+    too_large()
+    assert np.array_equal(w.dequantize().cpu().numpy(), want)
+    too_large()
+    w.save(path)
