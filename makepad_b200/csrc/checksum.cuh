@@ -138,26 +138,23 @@ __global__ void __launch_bounds__(FNV_GROUP) fnv_sum_kernel(const uint8_t* __res
 // device memory fnv1a64_device wants: 1/32 of the buffer
 inline size_t fnv1a64_scratch_bytes(int64_t bytes)
 {
+    if (bytes <= 0) return 0;
     const int64_t chunks = (bytes + FNV_CHUNK - 1) / FNV_CHUNK, groups = (chunks + FNV_GROUP - 1) / FNV_GROUP;
     return ((size_t)groups * 8 + 127) / 128 * 128 + (size_t)groups * 129 + (size_t)chunks * 128;
 }
 
-// *h = FNV-1a 64 of buf[0, bytes) continued from *h.  buf: 16-byte aligned device memory; scratch: fnv1a64_scratch_bytes, or
-// null to allocate it here.  Waits for the stream.
+// *h = FNV-1a 64 of buf[0, bytes) continued from *h.  buf: 16-byte aligned device memory; scratch: fnv1a64_scratch_bytes of
+// device memory.  Waits for the stream; *h is unchanged on an error.
 inline cudaError_t fnv1a64_device(const void* buf, int64_t bytes, uint64_t* h, uint8_t* scratch, cudaStream_t s)
 {
     if (bytes <= 0) return cudaSuccess;
     const int64_t chunks = (bytes + FNV_CHUNK - 1) / FNV_CHUNK, groups = (chunks + FNV_GROUP - 1) / FNV_GROUP;
     // sums (8 B per group) | group maps (128 B) | chunk maps (128 B) | group starts (1 B)
     const size_t off_gmap = ((size_t)groups * 8 + 127) / 128 * 128, off_map = off_gmap + (size_t)groups * 128, off_start = off_map + (size_t)chunks * 128;
-    uint8_t* own = nullptr;
-    cudaError_t e = scratch ? cudaSuccess : cudaMalloc(&own, off_start + (size_t)groups);
-    if (e != cudaSuccess) return e;
-    if (!scratch) scratch = own;
     const uint8_t* b = static_cast<const uint8_t*>(buf);
     uint64_t* sum = reinterpret_cast<uint64_t*>(scratch);
     uint32_t* map = reinterpret_cast<uint32_t*>(scratch + off_map);
-    e = launch(fnv_map_kernel, (unsigned)((chunks + 7) / 8), 256, s, b, bytes, chunks, map);
+    cudaError_t e = launch(fnv_map_kernel, (unsigned)((chunks + 7) / 8), 256, s, b, bytes, chunks, map);
     if (e == cudaSuccess) e = launch(fnv_group_kernel, (unsigned)groups, 128, s, map, chunks, scratch + off_gmap);
     if (e == cudaSuccess) e = launch(fnv_walk_kernel, 1, 256, s, reinterpret_cast<const uint32_t*>(scratch + off_gmap), groups, (uint32_t)(*h & 0xFFu), scratch + off_start);
     if (e == cudaSuccess) e = launch(fnv_sum_kernel, (unsigned)groups, FNV_GROUP, s, b, bytes, map, chunks, scratch + off_start, sum);
@@ -166,7 +163,8 @@ inline cudaError_t fnv1a64_device(const void* buf, int64_t bytes, uint64_t* h, u
     if (!host && e == cudaSuccess) e = cudaErrorMemoryAllocation;
     if (e == cudaSuccess) e = cudaMemcpyAsync(host, sum, (size_t)groups * 8, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(host_l, scratch + off_start, (size_t)groups, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    const cudaError_t done = cudaStreamSynchronize(s);                  // (on an error too: nobody still uses the scratch)
+    if (e == cudaSuccess) e = done;
     for (int64_t g = 0; e == cudaSuccess && g < groups; ++g) {
         uint64_t pn = 1, sq = FNV_PRIME;
         for (int64_t n = bytes - g * FNV_CHUNK * FNV_GROUP < FNV_CHUNK * FNV_GROUP ? bytes - g * FNV_CHUNK * FNV_GROUP : FNV_CHUNK * FNV_GROUP; n; n >>= 1, sq *= sq)
@@ -174,7 +172,6 @@ inline cudaError_t fnv1a64_device(const void* buf, int64_t bytes, uint64_t* h, u
         *h = (*h - host_l[g]) * pn + host[g];
     }
     free(host);
-    if (own) cudaFree(own);
     return e;
 }
 

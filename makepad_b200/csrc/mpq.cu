@@ -1603,6 +1603,37 @@ extern "C" int32_t mpq_file_info(const char* path, mpq_file_info_t* out)
     return MPQ_OK;
 }
 
+// the checksum of `bytes` of a file from `at` on, continued from *h (false: it cannot be read)
+static bool fnv1a64_file(FILE* f, int64_t at, int64_t bytes, uint64_t* h)
+{
+    uint8_t piece[4096];
+    if (fseek(f, (long)at, SEEK_SET) != 0) return false;
+    for (int64_t left = bytes; left > 0;) {
+        const size_t n = (size_t)std::min<int64_t>(left, (int64_t)sizeof piece);
+        if (fread(piece, n, 1, f) != 1) return false;
+        *h = fnv1a64(piece, n, *h);
+        left -= (int64_t)n;
+    }
+    return true;
+}
+
+// Device memory for the checksum of `bytes`: the context's upload staging where it is large enough (held meanwhile), else
+// memory of its own.  mem is null when there is none: the checksum is then taken on the host.
+struct ChecksumScratch {
+    std::lock_guard<std::mutex> held;
+    uint8_t *mem, *own = nullptr;
+    ChecksumScratch(mpq_context* ctx, int64_t bytes) : held(ctx->upload.staging_lock()), mem(ctx->upload.staging(fnv1a64_scratch_bytes(bytes)))
+    {
+        if (mem) return;
+        if (cudaMalloc(&own, fnv1a64_scratch_bytes(bytes)) != cudaSuccess) {
+            cudaGetLastError();
+            own = nullptr;
+        }
+        mem = own;
+    }
+    ~ChecksumScratch() { cudaFree(own); }
+};
+
 extern "C" int32_t mpq_canonical_save(const char* path, int32_t fmt, int64_t N, int64_t K, const uint8_t* codes_host,
                                       const void* scales_host, float tensor_scale)
 {
@@ -1658,8 +1689,15 @@ extern "C" int32_t mpq_weight_save(mpq_context* ctx, const mpq_weight* w, const 
     if (e == cudaSuccess && h.bytes_b) e = cudaMemcpy(host + h.bytes_a, db, (size_t)h.bytes_b, cudaMemcpyDeviceToHost);
     // the checksum is taken where the bytes lie: the legacy stream runs after the copies above
     h.checksum = FNV_START;
-    if (e == cudaSuccess) e = fnv1a64_device(da, h.bytes_a, &h.checksum, nullptr, 0);
-    if (e == cudaSuccess) e = fnv1a64_device(db, h.bytes_b, &h.checksum, nullptr, 0);
+    if (e == cudaSuccess) {
+        ChecksumScratch scratch(ctx, std::max(h.bytes_a, h.bytes_b));
+        if (scratch.mem) {
+            e = fnv1a64_device(da, h.bytes_a, &h.checksum, scratch.mem, 0);
+            if (e == cudaSuccess) e = fnv1a64_device(db, h.bytes_b, &h.checksum, scratch.mem, 0);
+        } else {
+            h.checksum = fnv1a64(host, (size_t)(h.bytes_a + h.bytes_b));
+        }
+    }
     int32_t st = e == cudaSuccess ? file_write(path, h, host, host + h.bytes_a) : MPQ_ERR_CUDA;
     free(host);
     if (st == MPQ_ERR_CUDA) return fail(ctx, st, "device-to-host copy failed: %s", cudaGetErrorString(e));
@@ -1709,13 +1747,15 @@ extern "C" int32_t mpq_weight_load(mpq_context* ctx, const char* path, mpq_weigh
     // handed out before it agrees.
     void* part[2] = {h.fmt == MPQ_FMT_Q4 ? static_cast<void*>(w->q4.stream) : w->fp4.codes, w->fp4.sf_tiled};
     const int64_t bytes[2] = {h.bytes_a, h.bytes_b};
-    std::lock_guard<std::mutex> staging_held(ctx->upload.staging_lock());
     uint64_t sum = FNV_START;
     int64_t at = (int64_t)sizeof h;
     for (int i = 0; i < 2 && e == cudaSuccess && st == MPQ_OK; at += bytes[i], ++i) {
         if (!bytes[i]) continue;
         if (ctx->upload.run(part[i], nullptr, fileno(f), at, (size_t)bytes[i], ctx->upload_stream, &e) == StagedUpload::READ_FAILED) st = MPQ_ERR_IO;
-        if (st == MPQ_OK && e == cudaSuccess) e = fnv1a64_device(part[i], bytes[i], &sum, ctx->upload.staging(fnv1a64_scratch_bytes(bytes[i])), ctx->upload_stream);
+        if (st != MPQ_OK || e != cudaSuccess) break;
+        ChecksumScratch scratch(ctx, bytes[i]);
+        if (scratch.mem) e = fnv1a64_device(part[i], bytes[i], &sum, scratch.mem, ctx->upload_stream);
+        else if (!fnv1a64_file(f, at, bytes[i], &sum)) st = MPQ_ERR_IO;
     }
     fclose(f);
     if (st == MPQ_OK && e == cudaSuccess && sum != h.checksum) st = MPQ_ERR_FORMAT;

@@ -163,3 +163,45 @@ def test_a_weight_that_did_not_fit_does_not_fail_the_next_one(ctx, tmp_path):
     assert np.array_equal(w.dequantize().cpu().numpy(), want)
     too_large()
     w.save(path)
+
+
+@pytest.mark.gpu
+def test_save_and_load_need_no_device_memory_beside_the_weight(ctx, tmp_path):
+    """The checksum wants 1/32 of the weight's bytes on the device; without them it is taken on the host."""
+    import torch
+    import makepad_b200
+    N, K = 32768, 16384                                                # 302 MB, 9.4 MB for the checksum
+    codes = np.random.default_rng(7).integers(0, 256, (N, K // 2), dtype=np.uint8)
+    scales = np.full((N, K // 32), 0x2C00, dtype=np.uint16)
+    path, full = str(tmp_path / "w.q4d"), str(tmp_path / "full.q4d")
+    c2 = makepad_b200.Context(0)                                       # (its upload has kept no memory that would do)
+    w = makepad_b200.Q4Weight(ctx, codes, scales)
+    w.save(path)
+
+    def hold(left):
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        return torch.empty(torch.cuda.mem_get_info()[0] - left, dtype=torch.uint8, device="cuda")
+
+    held = hold(4 << 20)
+    assert c2.lib.mpq_weight_save(c2.h, w.h, full.encode()) == _lib.OK
+    assert open(full, "rb").read() == open(path, "rb").read()
+    w.destroy()
+    del held
+    held = hold((N * K * 9 // 16) + (6 << 20))
+    back = makepad_b200.load_weight(c2, full)
+    h = C.c_void_p()
+    back.destroy()
+    with open(full, "r+b") as f:                                       # and a damaged file is still found out
+        f.seek(128 + 12345678)
+        byte = f.read(1)[0]
+        f.seek(128 + 12345678)
+        f.write(bytes([byte ^ 1]))
+    assert c2.lib.mpq_weight_load(c2.h, full.encode(), C.byref(h)) == _lib.ERR_FORMAT and not h.value
+    del held
+    torch.cuda.empty_cache()
+    back = makepad_b200.load_weight(c2, path)
+    back.save(full)
+    assert open(full, "rb").read() == open(path, "rb").read()
+    back.destroy()
+    c2.close()
