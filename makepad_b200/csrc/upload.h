@@ -5,6 +5,10 @@
 // host's copy rate (16 GB/s: 1.8 ms for 28 MB) is what is left.  Two to eight filling threads were measured too: 20% faster on
 // a quiet host (2.2 against 2.8 ms), but several times slower on a busy one.  The slots belong to a context: made by its
 // first upload, 4 x 1 MiB, freed with it.
+//
+// Building a Q4 weight, median of 30 creations on three boxes, cudaMemcpy / slots (ms): from pageable arrays 1000 x 2112
+// 1.0..1.1 / 0.50, 12288 x 4096 3.2..3.4 / 2.3..2.6, 28672 x 8192 13.7..14.8 / 12.4..14.3.  Page-locked arrays the copy engine
+// reads by itself at the rate of PCIe (28672 x 8192: 4.5 against 11.5..15 through the slots), so they are handed to it directly.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -29,6 +33,14 @@ public:
         std::lock_guard<std::mutex> hold(lock_);
         Result result = OK;
         cudaError_t e = cudaSuccess;
+        if (src && known(src) && known(static_cast<const char*>(src) + (bytes - 1))) {
+            e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+            *err = e;
+            if (e == cudaSuccess) return OK;
+            cudaGetLastError();                            // (parts in between may be unknown to the driver: through the slots then)
+            e = cudaSuccess;
+        }
         for (size_t at = 0, k = 0; at < bytes && e == cudaSuccess && result == OK; at += PIECE, ++k) {
             Slot& slot = slots_[k % SLOTS];
             if (!slot.done) e = cudaEventCreateWithFlags(&slot.done, cudaEventDisableTiming);
@@ -86,6 +98,15 @@ public:
     }
 
 private:
+    // memory that the driver can copy from by itself: page-locked, managed, or (given for host memory) device memory
+    static bool known(const void* p)
+    {
+        cudaPointerAttributes a = {};
+        if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type != cudaMemoryTypeUnregistered;
+        cudaGetLastError();
+        return false;
+    }
+
     struct Slot { void* mem = nullptr; cudaEvent_t done = nullptr; };
     std::mutex lock_, staging_lock_;
     uint8_t* staging_ = nullptr;

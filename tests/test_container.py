@@ -205,3 +205,33 @@ def test_save_and_load_need_no_device_memory_beside_the_weight(ctx, tmp_path):
     assert open(full, "rb").read() == open(path, "rb").read()
     back.destroy()
     c2.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["page-locked", "half page-locked", "pageable", "device"])
+def test_weights_from_every_kind_of_memory(ctx, kind):
+    """Arrays that the driver reads by itself and arrays that go through the pinned slots give the same weight."""
+    import torch
+    import makepad_b200
+    N, K = 3000, 2112                                                  # 3.2 MB of codes: several slots
+    codes, scales = synth.q4_weight(N, K, seed=91)
+    want = makepad_b200.Q4Weight(ctx, codes, scales).dequantize()
+    c, s = torch.from_numpy(codes), torch.from_numpy(scales.view(np.int16))
+    registered = 0
+    if kind == "page-locked":
+        c, s = c.pin_memory(), s.pin_memory()
+    elif kind == "half page-locked":                                   # the first of the array's pages
+        c = c.clone()
+        registered = (c.data_ptr() + 4095) // 4096 * 4096
+        assert int(torch.cuda.cudart().cudaHostRegister(registered, 1 << 20, 0)) == 0
+    elif kind == "device":
+        c, s = c.cuda(), s.cuda()
+    h = C.c_void_p()
+    ctx.check(ctx.lib.mpq_q4_weight_create(ctx.h, N, K, c.data_ptr(), s.data_ptr(), _lib.TP_NONE, 0, 1, C.byref(h)))
+    if registered:
+        assert int(torch.cuda.cudart().cudaHostUnregister(registered)) == 0
+    out = torch.empty_like(want)
+    ctx.check(ctx.lib.mpq_weight_dequantize(ctx.h, h, out.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    assert torch.equal(out.view(torch.int32), want.view(torch.int32))
+    ctx.lib.mpq_weight_destroy(h)

@@ -174,3 +174,80 @@ int main()
 
 def test_scratch_reserved_for_a_call_is_enough_for_every_smaller_one():
     _run(NEEDS)
+
+
+UPLOAD = r"""
+#include "upload.h"
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <vector>
+static const char *locked_lo = nullptr, *locked_hi = nullptr;              // what the fake driver has page-locked
+static bool refuse_direct = false, refuse_pinned = false;
+static int direct = 0, staged = 0, left_behind = 0;
+static const char *src_lo, *src_hi;
+extern "C" {
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p)
+{
+    a->type = p >= locked_lo && p < locked_hi ? cudaMemoryTypeHost : cudaMemoryTypeUnregistered;
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t)
+{
+    const bool from_source = s >= src_lo && s < src_hi;
+    if (from_source && refuse_direct) { left_behind = 1; return cudaErrorInvalidValue; }
+    memcpy(d, s, n);
+    ++(from_source ? direct : staged);
+    return cudaSuccess;
+}
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned)
+{
+    if (refuse_pinned) { left_behind = 1; return cudaErrorMemoryAllocation; }
+    *p = malloc(n);
+    return cudaSuccess;
+}
+cudaError_t cudaFreeHost(void* p) { free(p); return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { *e = (cudaEvent_t)1; return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaGetLastError() { left_behind = 0; return cudaSuccess; }
+cudaError_t cudaMalloc(void** p, size_t n) { *p = malloc(n); return cudaSuccess; }
+cudaError_t cudaFree(void* p) { free(p); return cudaSuccess; }
+}
+static int upload(mpq::StagedUpload& u, const std::vector<char>& from, size_t off, size_t n)
+{
+    std::vector<char> to(n + 1, 7);
+    cudaError_t e = cudaErrorUnknown;
+    direct = staged = 0;
+    const bool ok = u.run(to.data(), from.data() + off, -1, 0, n, nullptr, &e) == mpq::StagedUpload::OK && e == cudaSuccess;
+    return !ok || memcmp(to.data(), from.data() + off, n) || to[n] != 7 || left_behind;
+}
+int main()
+{
+    int bad = 0;
+    std::vector<char> from(5 * mpq::StagedUpload::PIECE + 123);
+    for (size_t i = 0; i < from.size(); ++i) from[i] = (char)(i * 2654435761u >> 13);
+    src_lo = from.data(), src_hi = src_lo + from.size();
+    const size_t n = from.size();
+    mpq::StagedUpload u;
+    bad += upload(u, from, 0, n) || direct != 0 || staged != 6;            // pageable: piece by piece through the slots
+    bad += upload(u, from, 5, 1) || staged != 1;
+    locked_lo = src_lo, locked_hi = src_hi;
+    bad += upload(u, from, 0, n) || direct != 1 || staged != 0;            // page-locked: one copy of it all
+    bad += upload(u, from, 777, n - 777) || direct != 1;                   // and a part of it
+    locked_hi = src_lo + n / 2;
+    bad += upload(u, from, 0, n) || direct != 0 || staged != 6;            // page-locked in part: through the slots
+    locked_hi = src_hi, refuse_direct = true;
+    bad += upload(u, from, 0, n) || direct != 0 || staged != 6;            // a copy that the driver refuses: through the slots
+    u.release();
+EXTRA
+    std::printf("%d\n", bad);
+    return bad;
+}
+"""
+
+
+def test_page_locked_arrays_are_uploaded_without_a_copy_on_the_host():
+    _run(UPLOAD.replace("EXTRA", ""))
