@@ -12,6 +12,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <stdlib.h>
 #include <string.h>
 #include <unistd.h>
 
@@ -44,7 +45,7 @@ public:
         for (size_t at = 0, k = 0; at < bytes && e == cudaSuccess && result == OK; at += PIECE, ++k) {
             Slot& slot = slots_[k % SLOTS];
             if (!slot.done) e = cudaEventCreateWithFlags(&slot.done, cudaEventDisableTiming);
-            if (e == cudaSuccess && !slot.mem && (e = cudaHostAlloc(&slot.mem, PIECE, cudaHostAllocPortable)) != cudaSuccess) slot.mem = nullptr;
+            if (e == cudaSuccess && !slot.mem) e = slot.make();
             if (e == cudaSuccess) e = cudaEventSynchronize(slot.done);          // the slot's last piece has left it
             if (e != cudaSuccess) break;
             const size_t n = std::min(PIECE, bytes - at);
@@ -91,7 +92,8 @@ public:
         staging_ = nullptr;
         staging_bytes_ = 0;
         for (Slot& s : slots_) {
-            if (s.mem) cudaFreeHost(s.mem);
+            if (s.mem && s.locked) cudaFreeHost(s.mem);
+            else free(s.mem);
             if (s.done) cudaEventDestroy(s.done);
             s = Slot();
         }
@@ -107,7 +109,21 @@ private:
         return false;
     }
 
-    struct Slot { void* mem = nullptr; cudaEvent_t done = nullptr; };
+    struct Slot {
+        void* mem = nullptr;
+        bool locked = false;
+        cudaEvent_t done = nullptr;
+        // Where the system locks no more pages, ordinary memory: the driver then stages the copy, and is done with the slot
+        // when cudaMemcpyAsync returns.
+        cudaError_t make()
+        {
+            locked = cudaHostAlloc(&mem, PIECE, cudaHostAllocPortable) == cudaSuccess;
+            if (locked) return cudaSuccess;
+            cudaGetLastError();
+            mem = malloc(PIECE);
+            return mem ? cudaSuccess : cudaErrorMemoryAllocation;
+        }
+    };
     std::mutex lock_, staging_lock_;
     uint8_t* staging_ = nullptr;
     size_t staging_bytes_ = 0;

@@ -251,3 +251,16 @@ EXTRA
 
 def test_page_locked_arrays_are_uploaded_without_a_copy_on_the_host():
     _run(UPLOAD.replace("EXTRA", ""))
+
+
+def test_uploads_work_where_no_pages_can_be_locked():
+    _run(UPLOAD.replace("EXTRA", """
+    locked_lo = locked_hi = nullptr, refuse_direct = false, refuse_pinned = true;
+    mpq::StagedUpload v;
+    bad += upload(v, from, 0, n) || staged != 6;
+    refuse_pinned = false;
+    bad += upload(v, from, 3, n - 3) || staged != 6;
+    v.release();
+    bad += upload(v, from, 0, n) || staged != 6;
+    v.release();
+"""))
