@@ -917,6 +917,7 @@ nvfp4_gemm_pair_kernel_v2(const __grid_constant__ CUtensorMap map_a, const __gri
             const uint64_t adesc0 = smem_desc_sw128(smem0), bdesc0 = smem_desc_sw128(smem0 + A_BYTES);
             const uint32_t sfc0 = tmem + V2_SF_COL;
             uint32_t soff = 0, sfoff = 0;              // stage * (Q_STAGE_BYTES >> 4), stage * V2_SF_COLS
+            asm volatile("griddepcontrol.wait;" ::: "memory");     // the polls below are for this kernel's own copies, not for the kernels before
             for (int local = 0; local < my_items && ok && !s_abort; ++local) {
                 int kb0, kb1;
                 pair_item(p, pair + local * npairs, &kb0, &kb1);
@@ -967,6 +968,7 @@ nvfp4_gemm_pair_kernel_v2(const __grid_constant__ CUtensorMap map_a, const __gri
         int stage = 0;
         uint32_t phase = 0;
         bool live = true;
+        asm volatile("griddepcontrol.wait;" ::: "memory");         // (as in the issuer)
         for (int item = pair; item < p.items && live && !s_abort; item += npairs) {
             int kb0, kb1;
             pair_item(p, item, &kb0, &kb1);

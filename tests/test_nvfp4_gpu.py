@@ -420,3 +420,43 @@ def test_a_captured_gemm_cuts_its_tiles_like_an_eager_one(orc, monkeypatch, warm
     assert c2.lib.mpq_context_poll_status(c2.h) == _lib.OK
     del graph
     c2.close()
+
+
+# Lets the next kernel in the stream start at once, then takes `ms` milliseconds (and ends in any case after 2^26 looks at the clock).
+SLOW_KERNEL = r"""
+extern "C" __global__ void slow_kernel(long long ms)
+{
+    asm volatile("griddepcontrol.launch_dependents;");
+    unsigned long long t0, t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+    for (int i = 0; i < (1 << 26); ++i) {
+        __nanosleep(1000);
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+        if (t - t0 > (unsigned long long)ms * 1000000ull) break;
+    }
+}
+"""
+
+
+@pytest.mark.parametrize("K", [512, 544])
+def test_waits_do_not_run_out_while_earlier_kernels_are_slow(ctx, orc, K):
+    """Quantisation and GEMM start beside a kernel that triggers its dependents at once and then takes a second: the GEMM's bounded
+    polls begin when that has ended (K = 544: the scale factors are re-tiled by a kernel in between)."""
+    import torch
+    import makepad_b200
+    M, N = 300, 232
+    slow = torch.cuda._compile_kernel(SLOW_KERNEL, "slow_kernel")
+    b, sfb = synth.nvfp4_tensor(N, K, seed=41, stream=1)
+    lin = makepad_b200.QuantLinear(makepad_b200.Nvfp4Weight(ctx, b, sfb, 1.0))
+    x = torch.from_numpy(synth.activations(M, K, seed=42)).cuda()
+    codes, sf = makepad_b200.nvfp4_quantize(ctx, x)
+    want = lin((codes, sf, 1.0))
+    torch.cuda.synchronize()
+    x2 = torch.zeros_like(x)
+    x2.copy_(x)
+    slow(grid=(1, 1, 1), block=(32, 1, 1), args=(1000,))
+    codes, sf = makepad_b200.nvfp4_quantize(ctx, x2)
+    y = lin((codes, sf, 1.0))
+    torch.cuda.synchronize()
+    assert ctx.lib.mpq_context_poll_status(ctx.h) == _lib.OK
+    assert torch.equal(y, want)
