@@ -925,12 +925,12 @@ static int32_t q4_gemm_slabs(mpq_context* ctx, const Q4Dev& q, const float* x, b
     return MPQ_OK;
 }
 
-// CTA pairs for a call of M rows, or 0 where it is one for the kernels of 64 rows and fewer: all calls above 64 rows go to the
-// pair kernel (measured: equal to two slabs of 64 on 57344 x 8192 at 65..96 rows, faster everywhere else) where the tcgen05
-// path is on and clusters of two can be scheduled.
-static int q4_gemm_wanted(const mpq_context* ctx, int64_t M)
+// CTA pairs for a call of M rows, or 0 where it is one for the kernels of 64 rows and fewer: calls above 64 rows go to the pair
+// kernel where the tcgen05 path is on, clusters of two can be scheduled, and two slabs of 64 rows are not the faster form.
+static int q4_gemm_wanted(const mpq_context* ctx, const Q4Dev& q, int64_t M)
 {
     if (ctx->q4_gemm_min <= 0 || M < ctx->q4_gemm_min || ctx->q4_umma_min <= 0 || M < ctx->q4_umma_min) return 0;
+    if (M > 64 && q4_slabs_of_64(q.units(), M)) return 0;
     return q4_gemm_pairs(ctx);
 }
 
@@ -952,7 +952,7 @@ static void q4_reserve(mpq_context* ctx, const mpq_weight* w, int64_t M, bool sw
 {
     const Q4Dev& q = w->q4;
     const Q4Needs need = q4_needs(q.N, q.K, q.nrp, q.nchunks, M, w->q4_rect_partial, w->q4_umma_pieces, ctx->q4_umma_min, ctx->q4_gemm_min,
-                                  q4_gemm_wanted(ctx, M));
+                                  q4_gemm_wanted(ctx, q, M));
     const size_t hidden = swiglu ? (size_t)(ctx->q4_umma_min > 0 ? std::min<int64_t>(M, ctx->q4_umma_min - 1) : M) * q.K * sizeof(float) : 0;
     if (ctx->q4u_xs.bytes() >= need.xs && ctx->q4_partial.bytes() >= need.partial && ctx->swiglu_buf.bytes() >= hidden && ctx->q4_partials_ctas) return;
     if (stream_captures(s)) return;
@@ -966,7 +966,7 @@ static void q4_reserve(mpq_context* ctx, const mpq_weight* w, int64_t M, bool sw
 // (in a capture without a warm-up of its size, or for want of memory) keeps to them.
 static int q4_gemm_route(const mpq_context* ctx, const Q4Dev& q, int64_t M)
 {
-    const int pairs = q4_gemm_wanted(ctx, M);
+    const int pairs = q4_gemm_wanted(ctx, q, M);
     if (!pairs) return 0;
     const int64_t slab = q4_gemm_slab(q.K);
     for (const int64_t rows : {std::min(M, slab), M % slab}) {

@@ -11,8 +11,9 @@
 // pair (tcgen05 cta_group::2, M = 256) fetches half the tile per SM.
 // Measured, 22016 x 4096, slabs of 64 rows / this kernel: 112 / 86 us at 96 rows, 118 / 88 at 128, 236 / 119 at 256,
 // 475 / 217 at 512 (1280 TFLOP/s of fp16 products, 92% of what a plain bf16 GEMM sustains under the power limit); 4096 x 11008:
-// 94 / 58 at 128, 380 / 116 at 512; 57344 x 8192 at 96 / 128 / 256 rows: 343 / 353, 367 / 358, 757 / 501.  Below 65 rows one pass
-// of the other kernel is the faster one (60 / 83 us at 64 rows): here the MMAs of a chunk cost the same for any Mt up to 128.
+// 94 / 58 at 128, 380 / 116 at 512; 57344 x 8192 at 256 rows 757 / 501.  Below 65 rows one pass of the other kernel is the faster
+// one (60 / 83 us at 64 rows): here the MMAs of a chunk cost the same for any Mt up to 128.  Up to 128 rows of a large weight two
+// passes of it are (q4_slabs_of_64).
 //
 // WORK.  Tile = 256 weight rows x Mt activation rows, numbered activation tile fastest; the (tile, chunk) sequence is cut
 // into equal ranges of W chunks, one per pair, so that any shape fills the SMs.  A tile inside one range is stored to y; the
