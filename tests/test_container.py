@@ -116,7 +116,7 @@ def test_stale_or_damaged_cache_files_are_refused(ctx, tmp_path):
 @pytest.mark.gpu
 @pytest.mark.parametrize("N, K", [(1, 32), (33, 288), (96, 1216), (1000, 2112), (4097, 4096), (12320, 4096)])
 def test_device_checksum_is_the_host_loop(ctx, tmp_path, N, K):
-    """The checksum taken on the GPU against the host's byte loop over the same payload (below one chunk of 4096 bytes, across
+    """The checksum taken on the GPU against the host's byte loop over the same payload (just above one chunk of 4096 bytes, across
     chunks, across groups of 64 chunks, and across 64 groups), and a payload byte flipped anywhere is refused."""
     import makepad_b200
     w = makepad_b200.Q4Weight(ctx, *synth.q4_weight(N, K, seed=N))
@@ -235,3 +235,33 @@ def test_weights_from_every_kind_of_memory(ctx, kind):
     torch.cuda.synchronize()
     assert torch.equal(out.view(torch.int32), want.view(torch.int32))
     ctx.lib.mpq_weight_destroy(h)
+
+
+def _fnv1a64(data):
+    h = 0xCBF29CE484222325
+    for b in data:
+        h = (h ^ b) * 0x100000001B3 & 0xFFFFFFFFFFFFFFFF
+    return h
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N, K", [(8, 32), (8, 96), (24, 4096), (232, 544), (248, 4128)])
+def test_device_checksum_continues_from_the_codes_to_the_scale_factors(ctx, tmp_path, N, K):
+    """NVFP4 files have two parts: the stored checksum is that of a plain loop over both.  The codes are less than one chunk of 4096
+    bytes, whole chunks, and more than a group of 64 chunks with a ragged end; a flipped byte in either part is refused."""
+    import makepad_b200
+    w = makepad_b200.Nvfp4Weight(ctx, *synth.nvfp4_tensor(N, K, seed=N + K), 0.5)
+    path = str(tmp_path / "w.fp4d")
+    w.save(path)
+    raw = bytearray(open(path, "rb").read())
+    assert len(raw) > 128 + N * K // 2
+    assert int.from_bytes(raw[56:64], "little") == _fnv1a64(raw[128:])
+    want = w.dequantize()
+    assert np.array_equal(makepad_b200.load_weight(ctx, path).dequantize().cpu().numpy(), want.cpu().numpy())
+    for at in (128, 128 + N * K // 2 - 1, 128 + N * K // 2, len(raw) - 1):
+        bad = bytearray(raw)
+        bad[at] ^= 1
+        open(path, "wb").write(bad)
+        with pytest.raises(makepad_b200.MpqError) as err:
+            makepad_b200.load_weight(ctx, path)
+        assert err.value.status == _lib.ERR_FORMAT
