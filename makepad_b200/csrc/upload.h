@@ -8,7 +8,8 @@
 //
 // Building a Q4 weight, median of 30 creations on three boxes, cudaMemcpy / slots (ms): from pageable arrays 1000 x 2112
 // 1.0..1.1 / 0.50, 12288 x 4096 3.2..3.4 / 2.3..2.6, 28672 x 8192 13.7..14.8 / 12.4..14.3.  Page-locked arrays the copy engine
-// reads by itself at the rate of PCIe (28672 x 8192: 4.5 against 11.5..15 through the slots), so they are handed to it directly.
+// reads by itself at the rate of PCIe (28672 x 8192: 4.5 against 11.5..15 through the slots; with the kept staging memory 3.4), so
+// they are handed to it directly.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -34,13 +35,19 @@ public:
         std::lock_guard<std::mutex> hold(lock_);
         Result result = OK;
         cudaError_t e = cudaSuccess;
-        if (src && known(src) && known(static_cast<const char*>(src) + (bytes - 1))) {
-            e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-            *err = e;
-            if (e == cudaSuccess) return OK;
-            cudaGetLastError();                            // (parts in between may be unknown to the driver: through the slots then)
-            e = cudaSuccess;
+        if (src) {
+            const bool first = known(src), last = known(static_cast<const char*>(src) + (bytes - 1));
+            if (first && last) {
+                // By the legacy stream, as any cudaMemcpy: behind the copies that may still be filling the array.
+                e = cudaStreamSynchronize(stream);
+                if (e == cudaSuccess) e = cudaMemcpy(dst, src, bytes, cudaMemcpyDefault);
+                if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+                *err = e;
+                if (e == cudaSuccess) return OK;
+                cudaGetLastError();                        // (parts in between may be unknown to the driver: through the slots then)
+            }
+            // (a core copies into the slots without waiting for anyone)
+            e = first || last ? cudaDeviceSynchronize() : cudaSuccess;
         }
         for (size_t at = 0, k = 0; at < bytes && e == cudaSuccess && result == OK; at += PIECE, ++k) {
             Slot& slot = slots_[k % SLOTS];

@@ -265,3 +265,21 @@ def test_device_checksum_continues_from_the_codes_to_the_scale_factors(ctx, tmp_
         with pytest.raises(makepad_b200.MpqError) as err:
             makepad_b200.load_weight(ctx, path)
         assert err.value.status == _lib.ERR_FORMAT
+
+
+@pytest.mark.gpu
+def test_page_locked_arrays_that_are_still_being_written(ctx):
+    """Arrays that an asynchronous copy on the default stream fills: the upload follows that copy, as cudaMemcpy does."""
+    import torch
+    import makepad_b200
+    N, K = 1000, 2112
+    codes, scales = synth.q4_weight(N, K, seed=92)
+    want = makepad_b200.Q4Weight(ctx, codes, scales).dequantize()
+    cd, sd = torch.from_numpy(codes).cuda(), torch.from_numpy(scales.view(np.int16)).cuda()
+    c, s = torch.zeros_like(cd, device="cpu").pin_memory(), torch.zeros_like(sd, device="cpu").pin_memory()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(200_000_000)                                     # a tenth of a second
+    c.copy_(cd, non_blocking=True)
+    s.copy_(sd, non_blocking=True)
+    w = makepad_b200.Q4Weight(ctx, c.numpy(), s.numpy().view(np.uint16))
+    assert torch.equal(w.dequantize().view(torch.int32), want.view(torch.int32))

@@ -189,7 +189,7 @@ UPLOAD = r"""
 static const char *locked_lo = nullptr, *locked_hi = nullptr;              // what the fake driver has page-locked
 static bool refuse_direct = false, refuse_pinned = false;
 static int direct = 0, staged = 0, left_behind = 0;
-static const char *src_lo, *src_hi;
+static bool writer_done = true;                                            // a copy that fills the array may still be on its way
 extern "C" {
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p)
 {
@@ -198,12 +198,20 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p)
 }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t)
 {
-    const bool from_source = s >= src_lo && s < src_hi;
-    if (from_source && refuse_direct) { left_behind = 1; return cudaErrorInvalidValue; }
+    if (!writer_done) return cudaErrorUnknown;                             // too early
     memcpy(d, s, n);
-    ++(from_source ? direct : staged);
+    ++staged;
     return cudaSuccess;
 }
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind)
+{
+    if (refuse_direct) { left_behind = 1; return cudaErrorInvalidValue; }
+    writer_done = true;                                                    // it waits for what precedes it
+    memcpy(d, s, n);
+    ++direct;
+    return cudaSuccess;
+}
+cudaError_t cudaDeviceSynchronize() { writer_done = true; return cudaSuccess; }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned)
 {
     if (refuse_pinned) { left_behind = 1; return cudaErrorMemoryAllocation; }
@@ -233,17 +241,17 @@ int main()
     int bad = 0;
     std::vector<char> from(5 * mpq::StagedUpload::PIECE + 123);
     for (size_t i = 0; i < from.size(); ++i) from[i] = (char)(i * 2654435761u >> 13);
-    src_lo = from.data(), src_hi = src_lo + from.size();
+    const char *src_lo = from.data(), *src_hi = src_lo + from.size();
     const size_t n = from.size();
     mpq::StagedUpload u;
     bad += upload(u, from, 0, n) || direct != 0 || staged != 6;            // pageable: piece by piece through the slots
     bad += upload(u, from, 5, 1) || staged != 1;
-    locked_lo = src_lo, locked_hi = src_hi;
+    locked_lo = src_lo, locked_hi = src_hi, writer_done = false;
     bad += upload(u, from, 0, n) || direct != 1 || staged != 0;            // page-locked: one copy of it all
     bad += upload(u, from, 777, n - 777) || direct != 1;                   // and a part of it
-    locked_hi = src_lo + n / 2;
+    locked_hi = src_lo + n / 2, writer_done = false;
     bad += upload(u, from, 0, n) || direct != 0 || staged != 6;            // page-locked in part: through the slots
-    locked_hi = src_hi, refuse_direct = true;
+    locked_hi = src_hi, refuse_direct = true, writer_done = false;
     bad += upload(u, from, 0, n) || direct != 0 || staged != 6;            // a copy that the driver refuses: through the slots
     u.release();
 EXTRA
