@@ -472,6 +472,7 @@ static int32_t q4_stream_scratch(mpq_context* ctx, int ctas)
         size_t bytes = (size_t)n * Q4S_SLOT_BYTES_PER_CTA;
         CU_TRY(ctx, cudaMalloc(&ctx->q4_partials, bytes));
         CU_TRY(ctx, cudaMemset(ctx->q4_partials, 0, bytes));      // tag 0 = empty slot
+        CU_TRY(ctx, cudaStreamSynchronize(cudaStreamLegacy));     // (the launch may be on a stream that does not wait for the default one)
         ctx->q4_partials_ctas = n;
     }
     return MPQ_OK;

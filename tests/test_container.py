@@ -283,3 +283,32 @@ def test_page_locked_arrays_that_are_still_being_written(ctx):
     s.copy_(sd, non_blocking=True)
     w = makepad_b200.Q4Weight(ctx, c.numpy(), s.numpy().view(np.uint16))
     assert torch.equal(w.dequantize().view(torch.int32), want.view(torch.int32))
+
+
+@pytest.mark.gpu
+def test_first_call_on_a_side_stream_finds_its_slots_empty(orc):
+    """The streaming kernel's slots are cleared when they are made; the first launch, on a stream that does not wait for the default
+    one, must find them cleared although their memory held something else before."""
+    import torch
+    import makepad_b200
+    N, K = 1000, 11008                                                 # row tiles that several CTAs share
+    codes, scales = synth.q4_weight(N, K, seed=93)
+    x = synth.activations(1, K, seed=94)
+    ref = orc.q4_matmul_f64(codes, scales, x)
+    side = torch.cuda.Stream()
+    xd = torch.from_numpy(x).cuda()
+    torch.cuda.synchronize()
+    for _ in range(8):
+        dirt = [torch.full((1 << 18,), 1.0, device="cuda") for _ in range(16)]
+        torch.cuda.synchronize()
+        del dirt
+        torch.cuda.empty_cache()                                       # back to the driver: the next slots may lie there
+        c2 = makepad_b200.Context(0)
+        lin = makepad_b200.QuantLinear(makepad_b200.Q4Weight(c2, codes, scales))
+        with torch.cuda.stream(side):
+            y = lin(xd)
+        side.synchronize()
+        assert orc.err_report(y.cpu().numpy(), ref)["max_abs_over_rms"] < 2e-5
+        assert c2.lib.mpq_context_poll_status(c2.h) == _lib.OK
+        del lin
+        c2.close()
