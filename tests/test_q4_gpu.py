@@ -572,3 +572,30 @@ def test_a_prompt_without_room_for_the_pair_kernel(orc):
     torch.cuda.synchronize()
     assert c2.lib.mpq_context_poll_status(c2.h) == _lib.OK
     c2.close()
+
+
+# several slabs of the staging memory with a ragged last one; a K slice of each row; rows of one shard; 32 rows longer than the staging memory
+@pytest.mark.parametrize("N,K,mode,rank,world", [(16500, 4096, "none", 0, 1), (16500, 4096, "row", 1, 2), (33000, 4096, "column", 1, 2), (33, 2097152, "none", 0, 1)])
+def test_weights_larger_than_the_upload_staging(ctx, N, K, mode, rank, world):
+    """A weight that is uploaded and repacked slab by slab holds the bits of one that is repacked from device arrays in one piece."""
+    import makepad_b200
+    torch = _torch()
+    g = torch.Generator(device="cuda")
+    g.manual_seed(7)
+    codes = torch.randint(0, 256, (N, K // 2), dtype=torch.uint8, device="cuda", generator=g)
+    scales = (torch.rand((N, K // 32), device="cuda", generator=g) * 0.02).to(torch.float16)
+    tp = {"none": _lib.TP_NONE, "row": _lib.TP_ROW, "column": _lib.TP_COLUMN}[mode]
+    w = makepad_b200.Q4Weight(ctx, codes.cpu().numpy(), scales.cpu().numpy().view(np.uint16), tp_mode=tp, rank=rank, world=world)
+    if mode == "column":
+        codes, scales = codes[N // 2:].contiguous(), scales[N // 2:].contiguous()
+    if mode == "row":
+        codes, scales = codes[:, K // 4:].contiguous(), scales[:, K // 64:].contiguous()
+    h = C.c_void_p()
+    n, k = codes.shape[0], codes.shape[1] * 2
+    ctx.check(ctx.lib.mpq_q4_weight_create_dev(ctx.h, n, k, codes.data_ptr(), scales.data_ptr(), C.byref(h)))
+    want = torch.empty((n, k), device="cuda")
+    ctx.check(ctx.lib.mpq_weight_dequantize(ctx.h, h, want.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    got = w.dequantize()
+    assert got.shape == want.shape and torch.equal(got.view(torch.int32), want.view(torch.int32))
+    ctx.lib.mpq_weight_destroy(h)
+    w.destroy()
