@@ -81,7 +81,8 @@ const char* mpq_last_error(const mpq_context* ctx);
  * MPQ_ERR_PEER_TIMEOUT if a bounded wait inside a kernel ran out since the
  * last poll; the word is then cleared. */
 int32_t mpq_context_poll_status(mpq_context* ctx);
-/* Number of kernels this context has launched since creation. */
+/* Number of kernels this context has launched since creation (those that take
+ * the checksum of a weight file are not counted). */
 int64_t mpq_context_launch_count(const mpq_context* ctx);
 
 /* ---- Q4 weights ---------------------------------------------------------- */
@@ -89,7 +90,9 @@ int64_t mpq_context_launch_count(const mpq_context* ctx);
  * kernels stream (16x64 tiles, one 16-byte word group per lane).  With
  * tp_mode COLUMN the handle keeps rows [rank*N/world, (rank+1)*N/world); with
  * ROW it keeps K-slice [rank*K/world, (rank+1)*K/world) (K/world must be a
- * multiple of 32).  Pass tp_mode NONE, rank 0, world 1 for the whole matrix. */
+ * multiple of 32).  Pass tp_mode NONE, rank 0, world 1 for the whole matrix.
+ * Page-locked arrays are read behind the work of the default stream, as by
+ * cudaMemcpy, and travel without a copy on the host. */
 int32_t mpq_q4_weight_create(mpq_context* ctx, int64_t N, int64_t K,
                              const uint8_t* codes_host, const uint16_t* scales_host,
                              int32_t tp_mode, int32_t rank, int32_t world, mpq_weight** out);
@@ -122,10 +125,18 @@ int32_t mpq_weight_destroy(mpq_weight* w);
  * four rows while M * K < 16384, is one launch of the streaming kernel; up to
  * 16 rows otherwise one pass of the rectangle kernel (weights read once,
  * only a K slice of x staged per CTA) plus a small reduction; 17..64 rows
- * the tcgen05 kernel, above that the tcgen05 kernel of CTA pairs (activation
- * staging, main kernel, reduction of the pieces).  The first call that needs a scratch buffer (or a larger
- * one) allocates it: make a warm-up call with the largest M before capturing
- * a CUDA graph.  Finite inputs with |x| < 3e38 are handled at any magnitude
+ * the tcgen05 kernel; above that the tcgen05 kernel of CTA pairs, or, up to
+ * 128 rows of a large weight, two slabs of 64 rows (each: activation staging,
+ * main kernel, reduction of the pieces).
+ * Scratch is allocated by the first call that needs it (or more of it).  A
+ * call of more than four rows reserves what every smaller call of the weight
+ * needs as well: make a warm-up call with the largest M of each weight before
+ * capturing CUDA graphs.  A buffer that is replaced by a larger one stays
+ * valid until the context is destroyed, so a captured graph may be replayed
+ * after any later call.  Above 64 rows, a call whose scratch cannot be had (in
+ * a capture after a smaller warm-up, or for want of memory) runs as slabs of
+ * 64 rows: slower, and with other last bits than the call that has it.
+ * Finite inputs with |x| < 3e38 are handled at any magnitude
  * (rows are renormalised by a power of two); a non-finite x yields non-finite
  * outputs in its row. */
 int32_t mpq_q4_linear_forward(mpq_context* ctx, const mpq_weight* w, const float* x_dev, int64_t M,
@@ -211,6 +222,10 @@ int32_t mpq_q4_linear_forward_swiglu(mpq_context* ctx, const mpq_weight* w, cons
  * M >= 1.  When K is a multiple of 256 the kernel reads the activation scale
  * factors straight from that array; otherwise they are first re-tiled on the
  * GPU inside this call (counted in its time) into scratch the context owns.
+ * Where the last wave of output tiles would leave SMs idle, its tiles may be
+ * cut along K; their fp32 sums lie in scratch (17 MB on 148 SMs) that the
+ * context's first call outside a capture reserves.  Without it (no such call,
+ * or no memory) tiles stay whole: slower, and with other last bits.
  * C must not overlap A (it is written with TMA tile stores while other tiles
  * are still being read). */
 int32_t mpq_nvfp4_gemm_forward(mpq_context* ctx, const mpq_weight* w,

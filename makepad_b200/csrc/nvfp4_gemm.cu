@@ -1306,9 +1306,9 @@ int32_t nvfp4_gemm_launch(Nvfp4Scratch& scratch, const Nvfp4Dev& w, const uint8_
         pp.sfa_direct = direct ? 1 : 0;
         // Full waves of tiles go whole; a last wave that leaves pairs idle may be cut along K.  The cut that costs least, by
         // rates measured on 74 pairs (microseconds: a K block of a pair; the launch that adds the items and the fp32 epilogue;
-        // writing and adding the rows of one item); uncut unless it gains a microsecond.  1000 x 4096 x 14336 (2 tiles of 76 in
-        // the second wave): 48.6 -> 40.5 us; 16 x 1024 x 8192 (5 tiles): 17.2 -> 9.6; but 700 x 11008 x 4096 (2 of 150) cut into
-        // eighths of 16 K blocks: 24.9 -> 28.7, left whole.
+        // writing and adding the rows of one item); uncut unless it gains a microsecond.  GEMM and sum in a graph, 1000 x 4096 x 14336
+        // (2 tiles of 76 in the second wave): 47.6 -> 38.8 us; 16 x 1024 x 8192 (5 tiles): 17.2 -> 8.8; but 700 x 11008 x 4096 (2 of
+        // 150) cut into eighths of 16 K blocks: 24.9 -> 28.7, left whole.
         const int tiles = pp.m_pairs * pp.n_tiles, last = tiles % nclusters;
         const double rows = (double)M / (256.0 * pp.m_pairs);
         int splits = 1;

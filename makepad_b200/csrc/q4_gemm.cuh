@@ -6,11 +6,13 @@
 //
 // WHY ANOTHER KERNEL.  q4_umma_kernel takes 64 rows a pass and expands every weight again in every pass: 512 rows were eight
 // passes, each bound by the expansion (1100 cycles per 128 rows x 64 of K, of which the MMAs use 384).  With 256 rows per
-// tile one expansion feeds 12 MMAs of N = 256 = 1536 cycles of tensor pipe, and the kernel is bound by the tensor pipe.
+// tile one expansion feeds 12 MMAs of N = 256 = 1536 cycles of tensor pipe.  That pipe is then active for 69% of the cycles
+// (22016 x 4096 at 512 rows, 1.61 GHz; 62% on 4096 x 11008).  What the other cycles go to has not been taken apart: it idles
+// while a segment of 16 chunks is drained, at the first copies of a range, and while the last pieces are stored.
 // One SM would have to fetch 64 KB of staged activations per 1536 cycles, about what L2 delivers when every SM asks; the
 // pair (tcgen05 cta_group::2, M = 256) fetches half the tile per SM.
 // Measured, 22016 x 4096, slabs of 64 rows / this kernel: 112 / 86 us at 96 rows, 118 / 88 at 128, 236 / 119 at 256,
-// 475 / 217 at 512 (1280 TFLOP/s of fp16 products, 92% of what a plain bf16 GEMM sustains under the power limit); 4096 x 11008:
+// 475 / 217 at 512 (1280 TFLOP/s of fp16 products by event time; a plain bf16 GEMM sustains 1422 under the power limit); 4096 x 11008:
 // 94 / 58 at 128, 380 / 116 at 512; 57344 x 8192 at 256 rows 757 / 501.  Below 65 rows one pass of the other kernel is the faster
 // one (60 / 83 us at 64 rows): here the MMAs of a chunk cost the same for any Mt up to 128.  Up to 128 rows of a large weight two
 // passes of it are (q4_slabs_of_64).
@@ -31,7 +33,7 @@
 
 namespace mpq {
 
-constexpr int Q4G_THREADS = 32 * 18;       // (five warps on a scheduler: 96 registers a thread, 64 of them running sums)
+constexpr int Q4G_THREADS = 32 * 18;       // (five warps on a scheduler: 96 registers a thread, 64 of them running sums; 392 bytes spill)
 constexpr int Q4G_WSTAGES = 8, Q4G_XSTAGES = 5, Q4G_ASTAGES = 4;
 
 struct Q4GemmLaunch {
@@ -416,7 +418,7 @@ q4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 
 // y of the tiles that were cut: their pieces' slots added in order.  64 threads x float4 per (tile, row), four rows of a
 // tile per block.  Bound by latency: with 64-bit divisions, a strided loop and one load on its way at a time it took 26.8 us
-// for 512 x 22016 (7B feed-forward block at 512 rows 394 -> 392 us).
+// for 512 x 22016, now 21.7 (7B feed-forward block at 512 rows 394 -> 392 us).
 __global__ void __launch_bounds__(256) q4g_reduce_kernel(const float* __restrict__ partial, int M, int Mt, int N, int nt, int nchunks, int W,
                                                           float* __restrict__ Y, int64_t ldy)
 {

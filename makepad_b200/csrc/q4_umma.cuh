@@ -84,7 +84,7 @@ struct Q4ULaunch {
 // Bound by latency (64 rows are 256 CTAs of a few loads each).  The CTAs of a row each read all of it (from L2) to find its
 // largest magnitude.  With SWIGLU they are a cluster: each computes its own part once, keeps it in shared memory (cached) and
 // takes the maximum over the cluster, where the SwiGLU was a kernel and a pass over memory in front: 70B feed-forward block at
-// 64 rows 346 -> 339 us.  For plain rows the cluster's launch and barriers cost more than the reads (about 0.8 us of 19 at
+// 64 rows 346 -> 339 us (another day 337 -> 334).  For plain rows the cluster's launch and barriers cost more than the reads (about 0.8 us of 19 at
 // short K).
 template <bool SWIGLU>
 __global__ void __launch_bounds__(256) q4u_xstage_kernel(const float* __restrict__ X, int M, int Mp, int K, int nchunks, int cached,
