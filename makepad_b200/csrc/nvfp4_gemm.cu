@@ -34,6 +34,7 @@
 #include "nvfp4.cuh"
 #include "swiglu.cuh"
 #include "per_device.h"
+#include "settle.cuh"
 
 namespace mpq {
 
@@ -731,6 +732,7 @@ nvfp4_gemm_kernel_v2(const __grid_constant__ CUtensorMap map_a, const __grid_con
     }
     tc_fence_before();
     __syncthreads();
+    settle_after_timeout(s_abort);
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
@@ -1055,6 +1057,7 @@ nvfp4_gemm_pair_kernel_v2(const __grid_constant__ CUtensorMap map_a, const __gri
     }
     tc_fence_before();
     __syncthreads();
+    settle_after_timeout(s_abort);
     cluster_sync_all();                                      // the peer's shared memory and barriers stay valid until both are done
     if (warp == 1) {
         tc_fence_after();

@@ -409,6 +409,7 @@ q4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     }
     q4u_fence_before();
     __syncthreads();
+    settle_after_timeout(s_abort);
     q4g_cluster_sync();                                                          // the peer's shared memory and barriers stay valid until both are done
     if (warp == 17) {
         q4u_fence_after();

@@ -42,6 +42,7 @@
 
 #include "q4.cuh"
 #include "q4_plan.h"
+#include "settle.cuh"
 
 namespace mpq {
 
@@ -616,6 +617,7 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_umma_kernel(const __grid_co
     }
     q4u_fence_before();
     __syncthreads();
+    settle_after_timeout(s_abort);
     if (warp == 1) {
         q4u_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");

@@ -276,3 +276,15 @@ def test_uploads_work_where_no_pages_can_be_locked():
     bad += upload(v, from, 0, n) || staged != 6;
     v.release();
 """))
+
+
+def test_every_kernel_that_can_give_up_a_wait_settles_before_it_ends():
+    """A kernel whose roles share an abort flag waits for what was in flight behind its last CTA barrier, before tensor memory is freed."""
+    kernels = 0
+    for f in ("q4_umma.cuh", "q4_gemm.cuh", "nvfp4_gemm.cu"):
+        text = open(os.path.join(ROOT, "makepad_b200", "csrc", f)).read()
+        for body in text.split("volatile int s_abort;")[1:]:
+            kernels += 1
+            end = body[:body.index("tcgen05.dealloc")]
+            assert "settle_after_timeout(s_abort);" in end[end.rindex("__syncthreads();"):], f
+    assert kernels == 4
