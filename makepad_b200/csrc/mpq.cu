@@ -658,6 +658,7 @@ static bool q4_rect_plan(const mpq_context* ctx, const Q4Dev& q, int M, Q4RectPl
 
 static void q4_note_needs(const mpq_context* ctx, mpq_weight* w)
 {
+    w->q4.mapped = make_q4_stream_map(&w->q4.map, w->q4.stream, w->q4.nrp, w->q4.nchunks);
     w->q4_umma_pieces = q4_umma_plan(w->q4.nrp, w->q4.nchunks, ctx->prop.multiProcessorCount).pieces;
     w->q4_rect_partial = 0;
     Q4RectPlan pl;
@@ -760,7 +761,9 @@ static int32_t q4_umma_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
     CU_TRY(ctx, ctx->q4u_xs.reserve(q4_umma_need_xs(q.nchunks, M)));
     unsigned char* xs = ctx->q4u_xs.as<unsigned char>();
     float* inv_sc = reinterpret_cast<float*>(xs + q4_umma_xs_bytes(q.nchunks, M));
-    const int stack = Mp <= 32 ? 1 : 0;                // accumulators of 2 Mp columns where they fit in a team's 64
+    // by the number of 16-row slices; accumulators of 2 Mp columns where they fit in 64
+    static void (*const kernels[4])(const CUtensorMap, const Q4ULaunch) = {q4_umma_kernel<1, true>, q4_umma_kernel<2, true>, q4_umma_kernel<3, false>, q4_umma_kernel<4, false>};
+    if (!q.mapped) return fail(ctx, MPQ_ERR_CUDA, "cuTensorMapEncodeTiled failed for the weight");
     const Q4UmmaPlan pl = q4_umma_plan(q.nrp, q.nchunks, sms);
     const int W = pl.W;
     CU_TRY(ctx, ctx->q4_partial.reserve(q4_umma_need_partial(pl.pieces, M, q.N)));
@@ -786,20 +789,17 @@ static int32_t q4_umma_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
     if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4u_xstage_kernel launch failed: %s", cudaGetErrorString(e));
 
     Q4ULaunch p;
-    p.stream = q.stream; p.XS = xs; p.inv_sc = inv_sc; p.Y = y; p.partial = partial;
-    p.M = M; p.Mp = Mp; p.N = (int)q.N; p.ldy = ldy; p.nchunks = q.nchunks; p.nrp = q.nrp; p.ngroups = pl.ngroups;
-    p.nbatches = pl.nbatches; p.W = W; p.stack = stack; p.status = ctx->q4_status;
+    p.XS = xs; p.inv_sc = inv_sc; p.Y = y; p.partial = partial;
+    p.M = M; p.Mp = Mp; p.N = (int)q.N; p.ldy = ldy; p.nchunks = q.nchunks;
+    p.nbatches = pl.nbatches; p.W = W; p.status = ctx->q4_status;
     // shared memory: activation ring, the teams' weight rings as deep as the rest allows, barriers (+ 1 KiB for the alignment)
     const size_t smem_max = (size_t)ctx->prop.sharedMemPerBlockOptin - 256, xring_bytes = (size_t)Q4U_XSTAGES * 2 * Mp * 128;
     p.wstages = (int)std::min<size_t>(Q4U_MAX_WSTAGES, (smem_max - xring_bytes - 2048) / ((size_t)Q4U_TEAMS * Q4U_WSTAGE_BYTES));
-#ifdef MPQ_TRACE
-    p.trace = trace_buffer() ? g_trace + (size_t)(g_trace_n++ % 64) * 1024 * 16 : nullptr;
-#endif
     // at least 116 KiB, so that two CTAs never share an SM (each allocates all of its tensor memory)
     const size_t smem = std::max<size_t>(xring_bytes + (size_t)Q4U_TEAMS * p.wstages * Q4U_WSTAGE_BYTES + 1024 + 1024, (size_t)116 * 1024);
     static PerDeviceOnce configured;
     if (configured.needs(ctx->device)) {
-        CU_TRY(ctx, cudaFuncSetAttribute(q4_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max));
+        for (auto kern : kernels) CU_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max));
         configured.mark(ctx->device);
     }
     cfg = {};
@@ -808,7 +808,7 @@ static int32_t q4_umma_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     launch_pdl(cfg, at, ctx->pdl);
-    e = cudaLaunchKernelEx(&cfg, q4_umma_kernel, p);
+    e = cudaLaunchKernelEx(&cfg, kernels[Mp / 16 - 1], q.map, p);
     ctx->launches += 1;
     if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4_umma_kernel launch failed: %s", cudaGetErrorString(e));
     if (pl.pieces > 1) {
@@ -831,37 +831,11 @@ static int32_t q4_umma_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
 static size_t q4_gemm_smem(int Mt)
 {
     // rings, barriers, alignment; at least 116 KiB, so that two CTAs never share an SM (each allocates all of its tensor memory)
-    return std::max<size_t>((size_t)Q4G_XSTAGES * Mt * 128 + (size_t)Q4G_WSTAGES * Q4U_WSTAGE_BYTES + 512 + 1024, (size_t)116 * 1024);
+    return std::max<size_t>((size_t)Q4G_XSTAGES * 2 * Mt * 128 + (size_t)Q4G_GROUPS * Q4G_WSTAGES * Q4U_WSTAGE_BYTES + 512 + 1024, (size_t)116 * 1024);
 }
 
-// CTA pairs the device keeps resident (0: clusters of two cannot be scheduled)
-static int q4_gemm_pairs(const mpq_context* ctx)
-{
-    static int cached[PerDeviceOnce::MAX_DEVICES];
-    static PerDeviceOnce known;
-    if (ctx->device < 0 || ctx->device >= PerDeviceOnce::MAX_DEVICES) return 0;
-    if (!known.needs(ctx->device)) return cached[ctx->device];
-    int n = 0;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(ctx->prop.multiProcessorCount & ~1));
-    cfg.blockDim = dim3(Q4G_THREADS);
-    cfg.dynamicSmemBytes = q4_gemm_smem(Q4G_MT_MAX);
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    if (cudaFuncSetAttribute(q4_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) != cudaSuccess ||
-        cudaFuncSetAttribute(q4g_xstage_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess ||
-        cudaFuncSetAttribute(q4g_xstage_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, q4_gemm_pair_kernel, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        n = 0;
-    }
-    cached[ctx->device] = n;
-    known.mark(ctx->device);
-    return n;
-}
+// half of the CTAs that the device keeps resident
+static int q4_gemm_pairs(const mpq_context* ctx) { return ctx->prop.multiProcessorCount / 2; }
 
 // y = x . W^T for M > 64 rows; with swiglu x is [M][2K] = [gate | up].  One slab's staged rows take M * K * 4 bytes of scratch.
 static int32_t q4_gemm_forward(mpq_context* ctx, const Q4Dev& q, const float* x, bool swiglu, int M, float* y, int64_t ldy, int pairs_max, cudaStream_t s)
@@ -869,13 +843,20 @@ static int32_t q4_gemm_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
     int32_t st = q4_status_word(ctx);
     if (st) return st;
     const Q4GemmPlan pl = q4_gemm_plan(q.nrp, q.nchunks, M, pairs_max);
-    const int nt = pl.nt, Mt = pl.Mt, W = pl.W, nb = (q.nrp + 7) / 8;
+    const int nt = pl.nt, Mt = pl.Mt;
+    if (!q.mapped) return fail(ctx, MPQ_ERR_CUDA, "cuTensorMapEncodeTiled failed for the weight");
     CU_TRY(ctx, ctx->q4u_xs.reserve(pl.need_xs));
     CU_TRY(ctx, ctx->q4_partial.reserve(pl.need_partial));
     unsigned char* xs = ctx->q4u_xs.as<unsigned char>();
     float *inv_sc = reinterpret_cast<float*>(xs + pl.xs_bytes), *partial = ctx->q4_partial.as<float>();
-    CUtensorMap map_x;
-    if (!make_rows128_map(&map_x, xs, (int64_t)nt * q.nchunks * 2 * Mt, Mt / 2)) return fail(ctx, MPQ_ERR_CUDA, "cuTensorMapEncodeTiled failed for the staged activations");
+    static PerDeviceOnce configured;
+    if (configured.needs(ctx->device)) {
+        for (auto kern : {q4_gemm_kernel<3>, q4_gemm_kernel<4>})
+            CU_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)q4_gemm_smem(Q4G_MT_MAX)));
+        CU_TRY(ctx, cudaFuncSetAttribute(q4g_xstage_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        CU_TRY(ctx, cudaFuncSetAttribute(q4g_xstage_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        configured.mark(ctx->device);
+    }
 
     cudaLaunchAttribute at[1];
     cudaLaunchConfig_t cfg = {};
@@ -890,25 +871,25 @@ static int32_t q4_gemm_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
     if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4g_xstage_kernel launch failed: %s", cudaGetErrorString(e));
 
     Q4GemmLaunch p;
-    p.stream = q.stream; p.inv_sc = inv_sc; p.Y = y; p.partial = partial;
-    p.M = M; p.Mt = Mt; p.N = (int)q.N; p.nt = nt; p.ldy = ldy; p.nchunks = q.nchunks; p.nrp = q.nrp; p.W = W; p.total = pl.total;
+    p.XS = xs; p.inv_sc = inv_sc; p.Y = y; p.partial = partial;
+    p.M = M; p.Mt = Mt; p.N = (int)q.N; p.nt = nt; p.ldy = ldy; p.nchunks = q.nchunks; p.full = pl.full; p.rest = pl.rest; p.W = pl.W;
     p.status = ctx->q4_status;
     cfg = {};
-    cfg.gridDim = dim3((unsigned)(2 * pl.pairs));
-    cfg.blockDim = dim3(Q4G_THREADS);
+    cfg.gridDim = dim3((unsigned)pl.grid);
+    cfg.blockDim = dim3(Q4U_THREADS);
     cfg.dynamicSmemBytes = q4_gemm_smem(Mt);
     cfg.stream = s;
     launch_pdl(cfg, at, ctx->pdl);
-    e = cudaLaunchKernelEx(&cfg, q4_gemm_pair_kernel, map_x, p);
+    e = cudaLaunchKernelEx(&cfg, Mt <= 96 ? q4_gemm_kernel<3> : q4_gemm_kernel<4>, q.map, p);
     ctx->launches += 1;
-    if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4_gemm_pair_kernel launch failed: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4_gemm_kernel launch failed: %s", cudaGetErrorString(e));
     if (pl.cut) {
         cfg = {};
-        cfg.gridDim = dim3((unsigned)((int64_t)nb * nt * (Mt / 4)));
+        cfg.gridDim = dim3((unsigned)((int64_t)pl.rest * (Mt / 4)));
         cfg.blockDim = dim3(256);
         cfg.stream = s;
         launch_pdl(cfg, at, ctx->pdl);
-        e = cudaLaunchKernelEx(&cfg, q4g_reduce_kernel, (const float*)partial, M, Mt, (int)q.N, nt, q.nchunks, W, y, ldy);
+        e = cudaLaunchKernelEx(&cfg, q4g_reduce_kernel, (const float*)partial, M, Mt, (int)q.N, nt, q.nchunks, pl.W, pl.full * pl.grid, y, ldy);
         ctx->launches += 1;
         if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4g_reduce_kernel launch failed: %s", cudaGetErrorString(e));
     }

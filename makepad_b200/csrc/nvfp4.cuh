@@ -51,6 +51,8 @@ int32_t nvfp4_gemm_launch(Nvfp4Scratch& scratch, const Nvfp4Dev& w, const uint8_
 
 // TMA map of an array of 128-byte rows, box = box_rows of them, dense (false: the driver's encoder is missing or refuses)
 bool make_rows128_map(CUtensorMap* map, const void* base, int64_t rows, int box_rows);
+// TMA map of a Q4 tile stream (see Q4Dev::map)
+bool make_q4_stream_map(CUtensorMap* map, const void* stream, int nrp, int nchunks);
 
 // launches the tensor-pipe ceiling probe (see nvfp4_mma_probe_kernel); *flop = the flop it executes
 int32_t nvfp4_mma_probe_launch(Nvfp4Scratch& scratch, int device, int sm_count, int mmas, cudaStream_t s, double* flop, std::string& err);

@@ -1240,6 +1240,18 @@ bool make_rows128_map(CUtensorMap* map, const void* base, int64_t rows, int box_
               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+bool make_q4_stream_map(CUtensorMap* map, const void* stream, int nrp, int nchunks)
+{
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return false;
+    cuuint64_t dims[3] = {128u, (cuuint64_t)nchunks * 9, (cuuint64_t)nrp};
+    cuuint64_t strides[2] = {128u, (cuuint64_t)nchunks * 9 * 128};
+    cuuint32_t box[3] = {128u, 9u, 4u};
+    cuuint32_t estr[3] = {1u, 1u, 1u};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(stream), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // CTA pairs the device can keep resident at once (0: the pair kernel cannot be used)
 static int pair_v2_clusters(int device, int sm_count)
 {

@@ -34,6 +34,7 @@
 #include "swiglu.cuh"
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -45,6 +46,8 @@ struct Q4Dev {
     int nrp = 0;               // row pair-tiles  = ceil(N/32)
     int nchunks = 0;           // 64-wide K chunks = ceil(K/64)
     uint4* stream = nullptr;   // nrp*nchunks units of Q4_UNIT_BYTES
+    CUtensorMap map = {};      // the stream as [pair-tile][9 rows per chunk][128 bytes], box = one chunk of four pair-tiles, 128-byte swizzle
+    bool mapped = false;
     int64_t units() const { return (int64_t)nrp * nchunks; }
     size_t bytes() const { return (size_t)nrp * nchunks * 1152; }
 };

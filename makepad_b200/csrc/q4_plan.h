@@ -51,28 +51,34 @@ inline size_t q4_umma_need_xs(int nchunks, int M) { return q4_umma_xs_bytes(nchu
 inline size_t q4_umma_need_partial(int pieces, int M, int64_t N) { return pieces > 1 ? (size_t)pieces * M * N * sizeof(float) : 0; }
 
 // ---------------------------------------------------------------------------
-// q4_gemm_pair_kernel: more than 64 rows
+// q4_gemm_kernel: more than 64 rows
 // ---------------------------------------------------------------------------
-constexpr int Q4G_MT_MAX = 256;               // activation rows per tile: the accumulator's columns
-constexpr int Q4G_SLOT = 256 * Q4G_MT_MAX;    // floats of one partial slot: [row of x][256 weight rows]
-constexpr int Q4G_MIN_W = 4;                  // fewest chunks per pair
+constexpr int Q4G_MT_MAX = 128;               // activation rows per tile: the columns of an accumulator slot
+constexpr int Q4G_ROWS = 256;                 // weight rows per tile
+constexpr int Q4G_SLOT = Q4G_ROWS * Q4G_MT_MAX;      // floats of one partial slot: [row of x][256 weight rows]
+constexpr int Q4G_MIN_W = 4;                  // fewest chunks per range of a cut tile
 
-// How one slab of M rows is cut, and the scratch that takes.
-struct Q4GemmPlan { int nt, Mt, W, pairs; int64_t total; bool cut; size_t xs_bytes, need_xs, need_partial; };
+// How one slab of M rows is cut, and the scratch that takes.  Every CTA (two per `pair`) gets `full` whole tiles; the `rest` tiles
+// that are left over are cut into equal ranges of W chunks, one per CTA (a range touches at most two tiles).
+struct Q4GemmPlan { int nt, Mt, full, rest, W, ranges, grid; bool cut; size_t xs_bytes, need_xs, need_partial; };
 inline Q4GemmPlan q4_gemm_plan(int nrp, int nchunks, int M, int pairs_max)
 {
     Q4GemmPlan pl;
-    // as few activation tiles as possible (each expands the weights again), as equal as possible, in steps of 32 rows (a
-    // quarter of the rows, eight or more, is what a team drains)
+    const int ctas = 2 * pairs_max;
+    // as few activation tiles as possible (each expands the weights again), as equal as possible, in steps of 16 rows
     pl.nt = (M + Q4G_MT_MAX - 1) / Q4G_MT_MAX;
-    pl.Mt = ((M + pl.nt - 1) / pl.nt + 31) / 32 * 32;
-    pl.total = (int64_t)((nrp + 7) / 8) * pl.nt * nchunks;
-    pl.W = (int)std::max<int64_t>((pl.total + pairs_max - 1) / pairs_max, std::min<int64_t>(Q4G_MIN_W, pl.total));
-    pl.pairs = (int)((pl.total + pl.W - 1) / pl.W);
+    pl.Mt = std::max(32, ((M + pl.nt - 1) / pl.nt + 15) / 16 * 16);
+    const int tiles = (nrp + 7) / 8 * pl.nt;
+    pl.full = tiles / ctas;
+    pl.rest = tiles - pl.full * ctas;
+    const int64_t chunks = (int64_t)pl.rest * nchunks;
+    pl.W = (int)std::max<int64_t>((chunks + ctas - 1) / ctas, std::min<int64_t>(Q4G_MIN_W, chunks));
+    pl.ranges = pl.W ? (int)((chunks + pl.W - 1) / pl.W) : 0;
+    pl.grid = pl.full ? ctas : pl.ranges;
     pl.cut = pl.W % nchunks != 0;                          // some tile lies in more than one range
     pl.xs_bytes = (size_t)pl.nt * nchunks * 2 * pl.Mt * 128;
     pl.need_xs = pl.xs_bytes + (size_t)M * sizeof(float);
-    pl.need_partial = pl.cut ? (size_t)pl.pairs * 2 * Q4G_SLOT * sizeof(float) : 0;
+    pl.need_partial = pl.cut ? (size_t)pl.ranges * 2 * Q4G_SLOT * sizeof(float) : 0;
     return pl;
 }
 
@@ -110,7 +116,7 @@ inline Q4Needs q4_needs(int64_t N, int64_t K, int nrp, int nchunks, int64_t M, s
     // The staged rows grow with M.  The number of ranges does not, but it is at most the device's pairs, and each holds at
     // least Q4G_MIN_W chunks of the largest call.
     const Q4GemmPlan pl = q4_gemm_plan(nrp, nchunks, (int)std::min<int64_t>(M, q4_gemm_slab(K)), pairs_max);
-    const int64_t most = std::min<int64_t>(pairs_max, (pl.total + Q4G_MIN_W - 1) / Q4G_MIN_W);
+    const int64_t total = (int64_t)((nrp + 7) / 8) * pl.nt * nchunks, most = std::min<int64_t>(2 * pairs_max, (total + Q4G_MIN_W - 1) / Q4G_MIN_W);
     n.xs = std::max(n.xs, pl.need_xs);
     n.partial = std::max(n.partial, (size_t)most * 2 * Q4G_SLOT * sizeof(float));
     return n;

@@ -1,19 +1,17 @@
 // Q4 linear for up to 64 activation rows on the fifth-generation tensor cores (tcgen05), weights read ONCE.
 //
-//   y[m][n] = sum_k (scale[n][k/32] * code[n][k]) * x[m][k]
+//   y[m][n] = sum over the 32-blocks b of K:  scale[n][b] * sum_{k in b} code[n][k] * x[m][k]
 //
 // The legacy mma.sync path (q4.cuh, q4_rect.cuh) spends tensor-pipe and FMA time per activation row: it is at
-// its arithmetic limit from about eight rows.  Here the products run as tcgen05.mma.kind::f16 with the WEIGHTS as
-// the M = 128 operand, read from TENSOR MEMORY, and the activation rows as the N dimension (16..64), read from
-// shared memory; accumulators (fp32) live in tensor memory.  Nothing but the weight expansion is left on the
-// ordinary pipes, and it does not depend on the number of activation rows.
+// its arithmetic limit from about eight rows.  Here the inner sums run as tcgen05.mma.kind::f16 with the weight CODES as
+// the M = 128 operand, read from TENSOR MEMORY, and the activation rows as the N dimension, read from shared memory; the
+// sums of one 32-block (fp32, in tensor memory) are scaled and added to fp32 registers with FFMAs.
 //
-// EXACTNESS.  A weight s*c (fp16 scale times 4-bit code) needs 15 significant bits, an activation 22+: both
-// are split.  Per 8-byte pair of codes the expansion warps form c as exact fp16 integers, hi = fp16(s*c) and
-// lo = s*c - hi (one HFMA2, exact: the remainder of an fp16 product is representable), and x arrives split as
-// hi + lo fp16 after a per-row power-of-two normalisation (q4u_xstage_kernel).  Per K step of 16 the products
-// hi*xhi, hi*xlo (one MMA against both activation tiles where the accumulator has room) and lo*xhi; lo*xlo is
-// below 2^-22 of the product.  fp32 accumulation in the tensor core, in segments (see Q4U_SEG).
+// EXACTNESS.  A code is an exact fp16 integer; x arrives split as hi + lo fp16 after a per-row power-of-two normalisation
+// (q4u_xstage_kernel): two products per weight and activation.  The tensor core adds four K steps and no more (its own
+// accumulation truncates: over 1024 of K it was a bias of 1e-5 of the output rms), small products first; everything
+// behind that is fp32 fused multiply-add with round to nearest.  (Expanding scale * code, 15 significant bits, to hi + lo fp16
+// instead takes three products.)
 //
 // WORK.  A batch = four consecutive weight groups of 128 rows (they share the activation tiles); the sequence of
 // (batch, chunk) pairs, batch-major, is cut into equal ranges of W chunks, one per CTA, so every SM gets the same
@@ -21,23 +19,27 @@
 // stored to y directly, a batch cut into pieces goes through one partial slice per piece, which q4u_reduce_kernel
 // adds in piece order (deterministic).
 //
-// DATA FLOW per CTA (one per SM).  The CTA is four independent pipelines ("teams") fed by two producer warps; team t owns a
-// weight ring, an A-operand stage and an accumulator in tensor memory, and handles group t of the batch:
-//   warp 0          weight producer: cp.async.bulk of the weight units into the teams' rings (the same tile stream
-//                   every other Q4 kernel reads: no second copy of the weights), as far ahead as the rings allow:
-//                   the bytes in flight per SM are what hides the HBM latency
-//   warp 21         activation producer: cp.async.bulk of the staged activation tiles (a ring of four chunks)
-//   warps 1..4      one MMA issuer per team.  A single thread issues an MMA of N <= 64 only every 45..110 cycles
-//                   (measured; the instruction itself needs 8..32 cycles of tensor pipe), four issuers together
-//                   reach the pipe's rate (36 cycles per MMA of N = 64)
-//   warps 5..20     expansion, four warps per team: thread = one weight row = one tensor-memory lane; shared memory
-//                   -> registers -> hi/lo fp16 -> tcgen05.st into the team's A stage (two halves with their own
-//                   hand-offs: one is filled while the MMAs of the other run); every Q4U_SEG chunks the
-//                   same warps add the team's accumulator (tcgen05.ld) to running fp32 sums (thread-local memory,
-//                   touched once per segment), and after the piece's last chunk store them
+// DATA FLOW per CTA (one per SM):
+//   warps 0..15     four teams of four; team t owns group t of the batch: a weight ring and an A operand of one chunk.  A
+//                   thread is one weight row = one tensor-memory lane.  It turns the codes of a chunk into fp16 (shared
+//                   memory -> registers -> tcgen05.st) and, when the MMAs of a 32-block are done, adds scale * sums to its
+//                   registers (tcgen05.ld); after a piece's last chunk it stores them.
+//   warp 16         MMA issue for all teams, a chunk of one team at a time, into three accumulator slots used in turn
+//   warp 17         copies: the weight units by TMA with the 128-byte swizzle (the same tile stream that every other Q4 kernel
+//                   reads; in its plain order the rows of a quarter warp are 64 bytes apart, a four-way bank conflict), the
+//                   staged activations by cp.async.bulk; as far ahead as the rings allow: the bytes in flight hide the latency
 // Hand-offs are mbarriers; every wait is bounded (a wait that runs out sets the status word and every role
 // leaves its loop; tensor memory is freed on every path).  No TMA load uses multicast.
+//
+// WHAT IT COSTS (measured parts).  An MMA of N = 64 takes 32 cycles of pipe, one of N = 128 64, whoever issues it; the issue of four
+// with operands in ordinary registers 264, so the role of a warp, the waits' outcomes and with them all that the loops count are
+// kept uniform for the compiler.  One look at an mbarrier is a round trip of 90 cycles and two in a row are 170, so the issuing
+// warp looks at all barriers of its next step at once, one per lane.
+// Measured, staging and sum of the pieces included, three products with sums kept in tensor memory / this form (us): 22016 x 4096 at
+// 17 rows 39.8 / 29.7, 32 41.3 / 31.2, 64 59.5 / 49.6; 57344 x 8192 at 64 223 / 147; 8192 x 28672 at 64 140 / 89; 1000 x 2112 at 64
+// 19.7 / 15.0.  The same with pairs of tests per 32-block in one issuing warp: 264 at 57344 x 8192; with run-time operands 175.
 #pragma once
+#include <cuda.h>
 #include <cuda_fp16.h>
 
 #include "q4.cuh"
@@ -46,34 +48,30 @@
 
 namespace mpq {
 
-constexpr int Q4U_THREADS = 32 * (2 + Q4U_TEAMS + 4 * Q4U_TEAMS);   // weight producer, activation producer; per team an issuer and four expansion warps
+constexpr int Q4U_WARP_ISSUE = 4 * Q4U_TEAMS, Q4U_WARP_COPY = Q4U_WARP_ISSUE + 1;     // behind four warps per team
+constexpr int Q4U_THREADS = 32 * 20;          // five warpgroups launched with 96 registers a thread: four go on with 104, one with 64
+constexpr int Q4U_REGS_WORK = 104, Q4U_REGS_REST = 64;
 constexpr int Q4U_MAX_WSTAGES = 8;            // weight ring PER TEAM: at most so many stages of one (group, chunk) = 4 units
-constexpr int Q4U_WSTAGE_BYTES = 4 * Q4_UNIT_BYTES;
+constexpr int Q4U_W_BYTES = 4 * Q4_UNIT_BYTES;
+constexpr int Q4U_WSTAGE_BYTES = 5 * 1024;    // (the swizzle wants stages of whole kilobytes)
 constexpr int Q4U_XSTAGES = 4;                // activation ring: stages of one chunk (hi tile + lo tile)
-constexpr int Q4U_SEG = 16;                   // chunks (1024 of K) a team accumulates inside the tensor core before its sums are drained
-                                              // (measured on 8192 x 28672 at 64 rows: max error 1.4e-5 of the output rms with 16,
-                                              //  2.3e-5 with 32, 3.9e-5 with 64 and more: the bound the tests hold is 2e-5)
-constexpr int Q4U_A_COL = 256;                // accumulators: columns [0, 256), 64 per team; A stages: [256, 512), 64 per team
+constexpr int Q4U_DSLOTS = 3;                 // accumulators: columns [0, 384), slots of two 32-blocks that are used in turn
+constexpr int Q4U_D_COLS = 128;
+constexpr int Q4U_A_COL = 384;                // A operand: [384, 512)
 constexpr uint32_t Q4U_SPIN = 1u << 22;       // tries of one mbarrier before giving up
 
 struct Q4ULaunch {
-    const uint4* stream;          // the Q4 tile stream
     const unsigned char* XS;      // staged activations: per chunk [hi: Mp rows x 128 B | lo: Mp rows x 128 B], 128-byte swizzle
     const float* inv_sc;          // [M] what undoes the per-row normalisation
     float* Y;                     // [M][ldy]: batches that lie in one CTA's range
     float* partial;               // [pieces][M][N]: batches cut into pieces
     int M, Mp, N;                 // Mp = M rounded up to 16
     int64_t ldy;
-    int nchunks, nrp;             // chunks per pair-tile in the stream, pair-tiles
-    int ngroups;                  // 128-row groups = ceil(nrp / 4)
+    int nchunks;                  // chunks per pair-tile in the stream
     int nbatches;                 // batches of four groups
     int W;                        // (batch, chunk) pairs per CTA
     int wstages;                  // stages of each team's weight ring (what shared memory allows, up to Q4U_MAX_WSTAGES)
-    int stack;                    // 1: one MMA multiplies the hi part with both activation tiles (accumulator of 2 Mp columns)
     int* status;
-#ifdef MPQ_TRACE
-    unsigned long long* trace;    // diagnostic build: per CTA 16 counters (see the kernel)
-#endif
 };
 
 // ---------------------------------------------------------------------------
@@ -162,11 +160,7 @@ __device__ __forceinline__ void q4u_bar_init(uint32_t bar, uint32_t count)
 {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
 }
-__device__ __forceinline__ void q4u_bar_arrive(uint32_t bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-// one non-suspending test of a phase parity (its round trip is about 200 cycles: tests of several barriers are issued together)
+// one non-suspending test of a phase parity
 __device__ __forceinline__ uint32_t q4u_bar_test(uint32_t bar, uint32_t parity)
 {
     uint32_t ok;
@@ -174,20 +168,36 @@ __device__ __forceinline__ uint32_t q4u_bar_test(uint32_t bar, uint32_t parity)
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok;
 }
-// bounded wait on a phase parity: false when the limit ran out.  One non-suspending test first (most waits find their
-// phase complete), then try_wait, which suspends the thread for a hardware-chosen time per try.  (A suspend-time hint made
-// the compiler emit a nanosleep polling loop with more instructions; spinning on test_wait issues more still; none of
-// the three forms changed the kernel's time.)
+// Bounded wait of a converged warp on a phase parity: false when the limit ran out.  try_wait suspends the threads for a
+// hardware-chosen time per try.  The vote makes the outcome uniform for the compiler: what the loops around it count stays in uniform registers.
 __device__ __forceinline__ bool q4u_bar_wait(uint32_t bar, uint32_t parity)
 {
-    if (q4u_bar_test(bar, parity)) return true;
-    for (uint32_t n = 0; n < Q4U_SPIN; ++n) {
-        uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (ok) return true;
-    }
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p, q;\n\t.reg .b32 n;\n\tmov.b32 n, 0;\n"
+                 "TRY:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tvote.sync.all.pred p, p, 0xffffffff;\n\t@p bra.uni DONE;\n\t"
+                 "add.u32 n, n, 1;\n\tsetp.lt.u32 q, n, %3;\n\t@q bra.uni TRY;\n"
+                 "DONE:\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity), "n"(Q4U_SPIN) : "memory");
+    return __all_sync(0xFFFFFFFFu, ok);
+}
+// ... by a thread for itself (the ones above and below are for whole warps: a lane alone would wait in the vote for good)
+__device__ __forceinline__ bool q4u_bar_wait_lane(uint32_t bar, uint32_t parity)
+{
+    for (uint32_t n = 0; n < Q4U_SPIN; ++n)
+        if (q4u_bar_test(bar, parity)) return true;
     return false;
+}
+// ... on the barriers of all lanes at once (those of lanes without `mine` are not looked at)
+__device__ __forceinline__ bool q4u_bar_wait_all(uint32_t bar, uint32_t parity, bool mine = true)
+{
+    for (uint32_t n = 0; n < Q4U_SPIN; ++n)
+        if (__all_sync(0xFFFFFFFFu, !mine || q4u_bar_test(bar, parity))) return true;
+    return false;
+}
+// lane 0 of a converged warp arrives (predicated: a branch would bring its own reconvergence)
+__device__ __forceinline__ void q4u_warp_arrive(uint32_t bar, int lane)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar), "r"(lane) : "memory");
 }
 __device__ __forceinline__ void q4u_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void q4u_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -206,17 +216,58 @@ __device__ __forceinline__ void q4u_mma(uint32_t d, uint32_t a, uint64_t bdesc, 
         "}"
         ::"r"(d), "r"(a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
+// one 32-block against the hi and the lo tile: K steps of 16 are 8 columns of A and +32 bytes = +2 in the descriptor.  The small
+// products first.  (Operands that the compiler knows to be uniform: else each goes from a register to a uniform one in front of the
+// instruction, which made the issue of four MMAs take 264 cycles where their pipe time is 128.)
+__device__ __forceinline__ void q4u_mma_block(uint32_t d, uint32_t a, uint64_t bhi, uint64_t blo, uint32_t idesc)
+{
+    q4u_mma(d, a, blo, idesc, 0u);
+    q4u_mma(d, a + 8, blo + 2, idesc, 1u);
+    q4u_mma(d, a, bhi, idesc, 1u);
+    q4u_mma(d, a + 8, bhi + 2, idesc, 1u);
+}
 // registers -> this warp's 32 tensor-memory lanes: thread l writes lane l, register j goes to column +j
 __device__ __forceinline__ void q4u_st8(uint32_t taddr, const uint32_t (&r)[8])
 {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                  ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
-__device__ __forceinline__ void q4u_ld8(uint32_t taddr, uint32_t (&r)[8])
+// sixteen accumulator columns of this warp's 32 lanes, waited for
+__device__ __forceinline__ void q4u_ld16(uint32_t taddr, uint32_t (&r)[16])
 {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\ttcgen05.wait::ld.sync.aligned;"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(taddr) : "memory");
 }
+// ... and thirty-two, from two places
+__device__ __forceinline__ void q4u_ld16x2(uint32_t taddr, uint32_t taddr2, uint32_t (&r)[16], uint32_t (&s)[16])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n\ttcgen05.wait::ld.sync.aligned;"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+                   "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3]), "=r"(s[4]), "=r"(s[5]), "=r"(s[6]), "=r"(s[7]), "=r"(s[8]), "=r"(s[9]), "=r"(s[10]), "=r"(s[11]), "=r"(s[12]), "=r"(s[13]), "=r"(s[14]), "=r"(s[15])
+                 : "r"(taddr), "r"(taddr2) : "memory");
+}
+// two fp32 sums at a time: acc += s * d
+__device__ __forceinline__ void q4u_fma2(uint64_t& acc, uint32_t d0, uint32_t d1, uint64_t s2)
+{
+    asm("{\n\t.reg .b64 t;\n\tmov.b64 t, {%1, %2};\n\tfma.rn.f32x2 %0, t, %3, %0;\n\t}" : "+l"(acc) : "r"(d0), "r"(d1), "l"(s2));
+}
+// ... and acc += s * (d + e)
+__device__ __forceinline__ void q4u_fma2_sum(uint64_t& acc, uint32_t d0, uint32_t d1, uint32_t e0, uint32_t e1, uint64_t s2)
+{
+    asm("{\n\t.reg .b64 t, u;\n\tmov.b64 t, {%1, %2};\n\tmov.b64 u, {%3, %4};\n\tadd.rn.f32x2 t, t, u;\n\tfma.rn.f32x2 %0, t, %5, %0;\n\t}"
+        : "+l"(acc) : "r"(d0), "r"(d1), "r"(e0), "r"(e1), "l"(s2));
+}
+__device__ __forceinline__ uint64_t q4u_pair(float s)
+{
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(v) : "f"(s));
+    return v;
+}
+template <int R>
+__device__ __forceinline__ void q4u_regs_more() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
+template <int R>
+__device__ __forceinline__ void q4u_regs_fewer() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
 // K-major operand tile, SWIZZLE_128B: rows are 128 bytes, 8-row groups 1024 bytes apart
 __device__ __forceinline__ uint64_t q4u_desc_sw128(uint32_t addr)
 {
@@ -228,23 +279,6 @@ __device__ __forceinline__ uint64_t q4u_desc_sw128(uint32_t addr)
     d |= (uint64_t)2 << 61;                         // SWIZZLE_128B
     return d;
 }
-
-// tcgen05.ld of four accumulator columns of this warp's 32 lanes
-__device__ __forceinline__ void q4u_ld4(uint32_t taddr, uint32_t (&r)[4])
-{
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
-}
-
-// dynamic shared memory (1024-byte aligned): activation ring | weight rings | barriers
-#ifdef MPQ_TRACE
-#define Q4U_CYC(var) long long var = clock64();
-#define Q4U_CYC_ADD(acc, since) acc += clock64() - (since);
-#else
-#define Q4U_CYC(var)
-#define Q4U_CYC_ADD(acc, since)
-#endif
-
 __device__ __forceinline__ uint32_t q4u_elect_one()
 {
     uint32_t pred;
@@ -252,373 +286,260 @@ __device__ __forceinline__ uint32_t q4u_elect_one()
     return pred;
 }
 
-__global__ void __launch_bounds__(Q4U_THREADS, 1) q4_umma_kernel(const __grid_constant__ Q4ULaunch p)
+// How a thread of the expansion finds its weight row (= its lane) in a stage of four units that TMA wrote with the 128-byte
+// swizzle: unit q is rows 9q .. 9q + 8 of 128 bytes, the codes of row pairs first, the scales last.
+struct Q4URow {
+    uint32_t code_off, scale_off;     // 16 bytes of K step t: (stage + code_off) ^ (t << 4); both scales of the chunk
+    uint32_t mask;                    // this row's nibbles of a word
+    uint32_t mul, add;                // fp16 pairs: (1024 + nibble in place) * mul + add = the signed code, exact
+    __device__ __forceinline__ Q4URow(int qd, int lane)
+    {
+        const uint32_t g8 = lane & 7, h = (lane >> 3) & 1, tile = lane >> 4;
+        const uint32_t row = qd * 9 + tile * 4 + (g8 >> 1), srow = qd * 9 + 8;
+        code_off = row * 128 + ((((g8 & 1) * 4) ^ (row & 7)) << 4);
+        scale_off = srow * 128 + ((g8 ^ (srow & 7)) << 4) + tile * 8 + h * 4;
+        mask = h ? 0x00F000F0u : 0x000F000Fu;
+        mul = h ? 0x2C002C00u : 0x3C003C00u;                            // 1/16, 1
+        add = h ? 0xD480D480u : 0xE408E408u;                            // -72, -1032
+    }
+    __device__ __forceinline__ uint32_t code2(uint32_t w) const
+    {
+        uint32_t r;
+        asm("{\n\t.reg .b32 t;\n\tlop3.b32 t, %1, %2, 0x64006400, 0xEA;\n\tfma.rn.f16x2 %0, t, %3, %4;\n\t}" : "=r"(r) : "r"(w), "r"(mask), "r"(mul), "r"(add));
+        return r;
+    }
+    // 32-block hf of this row: shared memory -> exact fp16 codes -> sixteen columns of the A operand
+    __device__ __forceinline__ void block(uint32_t stage, int hf, uint32_t dst) const
+    {
+        uint2 w[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+            asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(w[t].x), "=r"(w[t].y) : "r"(((stage + code_off) ^ (uint32_t)(t << 4)) + hf * 8));
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            uint32_t a[8];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {                               // k = 16j + 2t (+8): column 8j + t (+4)
+                const uint32_t v = j ? w[t].y : w[t].x;
+                a[t] = code2(v);
+                a[t + 4] = code2(v >> 8);
+            }
+            q4u_st8(dst + j * 8, a);
+        }
+    }
+    // both of a chunk, stored and waited for; sw = the chunk's scales
+    __device__ __forceinline__ void expand(uint32_t stage, uint32_t dst, uint32_t& sw) const
+    {
+        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(sw) : "r"(stage + scale_off));
+        block(stage, 0, dst);
+        block(stage, 1, dst + 16);
+        asm volatile("tcgen05.wait::st.sync.aligned;" : "+r"(sw)::"memory");              // (and the scales have arrived)
+    }
+};
+
+// acc += s * (the block's sums): 16 * SL activation rows from column d on; with STACK the products with the lo parts lie `lo` columns
+// behind those with the hi parts
+template <int SL, bool STACK>
+__device__ __forceinline__ void q4u_drain(uint64_t (&acc)[SL * 8], uint32_t d, uint32_t lo, uint32_t scale16)
+{
+    const uint64_t s2 = q4u_pair(__half2float(__ushort_as_half((unsigned short)scale16)));
+#pragma unroll
+    for (int sl = 0; sl < SL; ++sl) {
+        uint32_t r[16], r2[16];
+        if (STACK) q4u_ld16x2(d + 16 * sl, d + lo + 16 * sl, r, r2);
+        else q4u_ld16(d + 16 * sl, r);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            if (STACK) q4u_fma2_sum(acc[sl * 8 + q], r[2 * q], r[2 * q + 1], r2[2 * q], r2[2 * q + 1], s2);
+            else q4u_fma2(acc[sl * 8 + q], r[2 * q], r[2 * q + 1], s2);
+        }
+    }
+}
+// the sums of one piece: row m of them goes to out[m * ld]; rows are scaled back by isc0 (lane m) and isc1 (lane m - 32)
+template <int SL>
+__device__ __forceinline__ void q4u_store(uint64_t (&acc)[SL * 8], float* out, int64_t ld, int rows, bool mine, float isc0, float isc1)
+{
+#pragma unroll
+    for (int m = 0; m < SL * 16; ++m) {
+        const float sc = __shfl_sync(0xFFFFFFFFu, m < 32 ? isc0 : isc1, m & 31);
+        const float v = __uint_as_float((uint32_t)(m & 1 ? acc[m >> 1] >> 32 : acc[m >> 1]));
+        if (m < rows && mine) out[(size_t)m * ld] = v * sc;
+    }
+#pragma unroll
+    for (int q = 0; q < SL * 8; ++q) acc[q] = 0;
+}
+
+// dynamic shared memory (1024-byte aligned): activation ring | weight rings | barriers
+template <int SL, bool STACK>
+__global__ void __launch_bounds__(Q4U_THREADS, 1) q4_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ Q4ULaunch p)
 {
     extern __shared__ unsigned char smem_dyn[];
     __shared__ uint32_t s_tmem_base;
     __shared__ volatile int s_abort;
-#ifdef MPQ_TRACE
-    __shared__ unsigned long long s_tr[16];
-    if (threadIdx.x < 16) s_tr[threadIdx.x] = 0;
-#endif
     const uint32_t smem0 = (smem_u32(smem_dyn) + 1023u) & ~1023u;
     const uint32_t xstage_bytes = 2u * p.Mp * 128u;
-    const uint32_t xring = smem0, wring = xring + Q4U_XSTAGES * xstage_bytes;     // activation tiles need the 1024-byte alignment
+    const uint32_t xring = smem0, wring = xring + Q4U_XSTAGES * xstage_bytes;
     constexpr int NW = Q4U_TEAMS * Q4U_MAX_WSTAGES;
     const int WST = p.wstages;
     const uint32_t bars = wring + Q4U_TEAMS * WST * Q4U_WSTAGE_BYTES;
     const uint32_t w_full = bars, w_empty = w_full + 8 * NW, x_full = w_empty + 8 * NW, x_empty = x_full + 8 * Q4U_XSTAGES,
-                   a_full = x_empty + 8 * Q4U_XSTAGES, a_empty = a_full + 16 * Q4U_TEAMS, d_full = a_empty + 16 * Q4U_TEAMS,
-                   d_empty = d_full + 8 * Q4U_TEAMS;     // a_full / a_empty: [team][half]
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+                   a_full = x_empty + 8 * Q4U_XSTAGES, d_full = a_full + 8 * Q4U_TEAMS, d_empty = d_full + 16 * Q4U_TEAMS;   // a_full: [team]; d_full: [team][half of the chunk]
+    const int warp = __shfl_sync(0xFFFFFFFFu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (warp: uniform for the compiler)
     // this CTA's range of the (batch, chunk) sequence
     const long long total = (long long)p.nbatches * p.nchunks;
-    const long long L_begin = (long long)blockIdx.x * p.W, L_end = min(total, L_begin + p.W);
+    const long long L_begin = (long long)blockIdx.x * p.W;
+    const int range = (int)(min(total, L_begin + p.W) - L_begin);
 
     if (threadIdx.x == 0) {
         s_abort = 0;
-        for (int s = 0; s < NW; ++s) { q4u_bar_init(w_full + 8 * s, 1); q4u_bar_init(w_empty + 8 * s, 128); }      // (only Q4U_TEAMS * WST of them are used)
-        for (int s = 0; s < Q4U_XSTAGES; ++s) { q4u_bar_init(x_full + 8 * s, 1); q4u_bar_init(x_empty + 8 * s, Q4U_TEAMS); }
-        for (int s = 0; s < Q4U_TEAMS; ++s) {
-            for (int hf = 0; hf < 2; ++hf) { q4u_bar_init(a_full + 16 * s + 8 * hf, 128); q4u_bar_init(a_empty + 16 * s + 8 * hf, 1); }
-            q4u_bar_init(d_full + 8 * s, 1); q4u_bar_init(d_empty + 8 * s, 128);
-        }
+        for (int s = 0; s < NW; ++s) { q4u_bar_init(w_full + 8 * s, 1); q4u_bar_init(w_empty + 8 * s, 4); }      // (only Q4U_TEAMS * WST of them are used)
+        for (int s = 0; s < Q4U_XSTAGES; ++s) { q4u_bar_init(x_full + 8 * s, 1); q4u_bar_init(x_empty + 8 * s, 1); }
+        for (int s = 0; s < Q4U_TEAMS; ++s) q4u_bar_init(a_full + 8 * s, 4);
+        for (int s = 0; s < 2 * Q4U_TEAMS; ++s) q4u_bar_init(d_full + 8 * s, 1);
+        for (int s = 0; s < Q4U_DSLOTS; ++s) q4u_bar_init(d_empty + 8 * s, 4);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) {
+    if (warp == Q4U_WARP_ISSUE) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)), "r"(512) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     q4u_fence_before();
     __syncthreads();
     q4u_fence_after();
-    const uint32_t tmem = s_tmem_base;
+    const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, s_tmem_base, 0);
 
     asm volatile("griddepcontrol.launch_dependents;");
 
-    if (warp == 0) {
-        // ---------------- weight producer: lane = (team, pair-tile), sixteen copies per instruction ----------------
-        const int tm = lane >> 2, q = lane & 3;
-        const uint64_t l2pol = l2_evict_first_policy();
-        int wn = 0;                                      // stages loaded so far for this lane's team
-        int b = (int)(L_begin / p.nchunks), c = (int)(L_begin % p.nchunks);
-        for (long long L = L_begin; L < L_end && !s_abort; ++L) {
-            const int g = b * Q4U_TEAMS + tm;
-            const bool active = lane < 4 * Q4U_TEAMS && g < p.ngroups;
-            const int ws = tm * WST + wn % WST;
-            bool ok = true;
-            if (active) {
-                ok = q4u_bar_wait(w_empty + 8 * ws, ((uint32_t)(wn / WST) & 1u) ^ 1u);
-                const int npt = min(4, p.nrp - 4 * g);               // pair-tiles of this group that exist
-                if (ok && q == 0) mbar_expect_tx(w_full + 8 * ws, (uint32_t)npt * Q4_UNIT_BYTES);
-                if (ok && q < npt)
-                    bulk_g2s(wring + ws * Q4U_WSTAGE_BYTES + q * Q4_UNIT_BYTES,
-                             reinterpret_cast<const unsigned char*>(p.stream) + ((size_t)(4 * g + q) * p.nchunks + c) * Q4_UNIT_BYTES,
-                             Q4_UNIT_BYTES, w_full + 8 * ws, l2pol);
-                ++wn;
-            }
-            if (__any_sync(0xFFFFFFFFu, !ok)) { if (lane == 0) { atomicExch(p.status, 31); s_abort = 1; } break; }
-            if (++c == p.nchunks) { c = 0; ++b; }
-        }
-    } else if (warp == 1 + 5 * Q4U_TEAMS) {
-        // ---------------- activation producer ----------------
-        if (lane == 0) {
-            // the staged activation is written by the kernel before this one in the stream
-            asm volatile("griddepcontrol.wait;" ::: "memory");
-            int sc = 0;                                  // chunks so far
-            int c = (int)(L_begin % p.nchunks);
-            for (long long L = L_begin; L < L_end && !s_abort; ++L, ++sc, c = c + 1 == p.nchunks ? 0 : c + 1) {
-                const int xs = sc % Q4U_XSTAGES;
-                if (!q4u_bar_wait(x_empty + 8 * xs, ((uint32_t)(sc / Q4U_XSTAGES) & 1u) ^ 1u)) { atomicExch(p.status, 32); s_abort = 1; break; }
-                mbar_expect_tx(x_full + 8 * xs, xstage_bytes);
-                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                             ::"r"(xring + xs * xstage_bytes), "l"(p.XS + (size_t)c * xstage_bytes), "r"(xstage_bytes), "r"(x_full + 8 * xs) : "memory");
-            }
-        }
-    } else if (warp <= Q4U_TEAMS) {
-        // ---------------- MMA issuer of team tm: the whole warp runs the loop, one elected lane issues ----------------
-        const int tm = warp - 1;
-        // f16 x f16 -> f32, K-major both; N = Mp (against one activation tile) or 2 Mp (the hi tile and the lo tile behind it)
-        const uint32_t idesc1 = (1u << 4) | ((uint32_t)(p.Mp >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-        const uint32_t idesc2 = (1u << 4) | ((uint32_t)(p.Mp >> 2) << 17) | ((uint32_t)(128 >> 4) << 24);
-        const uint32_t d = tmem + (uint32_t)tm * 64;
-        const uint32_t a = tmem + Q4U_A_COL + (uint32_t)tm * 64;
-        int n = 0, drains = 0, seg_n = 0, xs = 0;
-        uint32_t xph = 0;
-#ifdef MPQ_TRACE
-        long long cyc_x = 0, cyc_a = 0, cyc_d = 0, cyc_issue = 0;
-        const long long cyc_t0 = clock64();
-#endif
-        int b = (int)(L_begin / p.nchunks), c = (int)(L_begin % p.nchunks) - 1;
-        bool live = true;
-        for (long long L = L_begin; L < L_end && live; ++L) {
-            if (++c == p.nchunks) { c = 0; ++b; }
-            const int xs_now = xs;
-            const uint32_t xph_now = xph;
-            if (++xs == Q4U_XSTAGES) { xs = 0; xph ^= 1u; }
-            Q4U_CYC(t_x)
-            const uint32_t okx = q4u_bar_test(x_full + 8 * xs_now, xph_now);
-            const uint32_t okf0 = q4u_bar_test(a_full + 16 * tm, (uint32_t)n & 1u);      // (only meaningful when this team's group exists)
-            if (!okx && !q4u_bar_wait(x_full + 8 * xs_now, xph_now)) { if (lane == 0) { atomicExch(p.status, 34); s_abort = 1; } break; }
-            Q4U_CYC_ADD(cyc_x, t_x)
-            if (b * Q4U_TEAMS + tm >= p.ngroups) {           // the last batch may lack groups: only the activation stage's hand-back
-                if (lane == 0) q4u_bar_arrive(x_empty + 8 * xs_now);
-                continue;
-            }
-            // a new segment overwrites the accumulator: the expansion warps must have drained the last one
-            Q4U_CYC(t_d)
-            if (seg_n == 0 && drains > 0 && !q4u_bar_wait(d_empty + 8 * tm, (uint32_t)(drains - 1) & 1u)) { if (lane == 0) { atomicExch(p.status, 33); s_abort = 1; } break; }
-            Q4U_CYC_ADD(cyc_d, t_d)
-            ++seg_n;
-            const bool seg_last = seg_n == Q4U_SEG || c == p.nchunks - 1 || L == L_end - 1;      // the segment, the batch or the range ends
-            const uint64_t bx = q4u_desc_sw128(xring + xs_now * xstage_bytes);     // rows [0, Mp) = xhi, [Mp, 2 Mp) = xlo
-            const uint64_t bxlo = q4u_desc_sw128(xring + xs_now * xstage_bytes + p.Mp * 128);
-            // The A stage has two halves (K steps 0, 1 and 2, 3), each with its own hand-offs: the expansion warps fill
-            // one while the MMAs of the other run.
-#pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {
-                Q4U_CYC(t_a)
-                if (!(hf == 0 && okf0) && !q4u_bar_wait(a_full + 16 * tm + 8 * hf, (uint32_t)n & 1u)) { if (lane == 0) { atomicExch(p.status, 35); s_abort = 1; } live = false; break; }
-                Q4U_CYC_ADD(cyc_a, t_a)
-                q4u_fence_after();
-                Q4U_CYC(t_i)
-                if (q4u_elect_one()) {
-#pragma unroll
-                    for (int jj = 0; jj < 2; ++jj) {              // K steps of 16: +32 bytes along K = +2 in the descriptor
-                        const int j = 2 * hf + jj;
-                        const uint32_t ahi = a + hf * 32 + jj * 8, alo = ahi + 16;
-                        const uint32_t acc = (seg_n > 1 || j > 0) ? 1u : 0u;
-                        if (p.stack) {                            // columns [0, Mp) = hi*xhi + lo*xhi, [Mp, 2 Mp) = hi*xlo
-                            q4u_mma(d, ahi, bx + 2 * j, idesc2, acc);
-                            q4u_mma(d, alo, bx + 2 * j, idesc1, 1u);
-                        } else {
-                            q4u_mma(d, ahi, bx + 2 * j, idesc1, acc);
-                            q4u_mma(d, ahi, bxlo + 2 * j, idesc1, 1u);
-                            q4u_mma(d, alo, bx + 2 * j, idesc1, 1u);
-                        }
-                    }
-                    q4u_commit(a_empty + 16 * tm + 8 * hf);     // this half of the A stage is free when these MMAs are done
-                    if (hf == 1) {
-                        q4u_commit(x_empty + 8 * xs_now);       // ... and this team is done with the activation stage
-                        if (seg_last) q4u_commit(d_full + 8 * tm);   // the segment's sums are complete
-                    }
+    if (warp >= Q4U_WARP_ISSUE) {
+        q4u_regs_fewer<Q4U_REGS_REST>();
+        if (warp == Q4U_WARP_COPY) {
+            // ---------------- copies: lane t = weight ring of team t, lane Q4U_TEAMS = the activations, LAG chunks behind ----------------
+            const int LAG = max(0, WST - Q4U_XSTAGES);   // then both kinds of rings are as full as they can be
+            const uint64_t l2pol = l2_evict_first_policy();
+            const bool wlane = lane < Q4U_TEAMS, xlane = lane == Q4U_TEAMS;
+            int b = (int)(L_begin / p.nchunks), c = (int)(L_begin % p.nchunks), cx = c, ws = 0, xs = 0;
+            uint32_t wph = 1, xph = 1;
+            for (int i = 0; i < range + LAG; ++i) {
+                if (__any_sync(0xFFFFFFFFu, s_abort)) break;
+                if (i == LAG) asm volatile("griddepcontrol.wait;" ::: "memory");    // the activations are staged by the kernel before this one
+                const bool now = wlane ? i < range : xlane && i >= LAG;
+                const uint32_t slot = wlane ? (uint32_t)(lane * WST + ws) : (uint32_t)xs;
+                if (!q4u_bar_wait_all((wlane ? w_empty : x_empty) + 8 * slot, wlane ? wph : xph, now)) { if (lane == 0) { atomicExch(p.status, 31); s_abort = 1; } break; }
+                if (now) {
+                    const uint32_t bar = (wlane ? w_full : x_full) + 8 * slot;
+                    mbar_expect_tx(bar, wlane ? Q4U_W_BYTES : xstage_bytes);
+                    if (wlane)                                             // four units; pair-tiles behind the last are zeros (scale 0)
+                        asm volatile("cp.async.bulk.tensor.3d.shared::cta.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %4}], [%5], %6;"
+                                     ::"r"(wring + slot * Q4U_WSTAGE_BYTES), "l"(&map_w), "r"(0), "r"(9 * c), "r"(4 * (b * Q4U_TEAMS + lane)), "r"(bar), "l"(l2pol) : "memory");
+                    else
+                        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                                     ::"r"(xring + slot * xstage_bytes), "l"(p.XS + (size_t)cx * xstage_bytes), "r"(xstage_bytes), "r"(bar) : "memory");
                 }
-                __syncwarp();
-                Q4U_CYC_ADD(cyc_issue, t_i)
+                if (++ws == WST) { ws = 0; wph ^= 1u; }
+                if (++c == p.nchunks) { c = 0; ++b; }
+                if (i >= LAG) {
+                    if (++xs == Q4U_XSTAGES) { xs = 0; xph ^= 1u; }
+                    if (++cx == p.nchunks) cx = 0;
+                }
             }
-            ++n;
-            if (seg_last) { ++drains; seg_n = 0; }
+        } else if (warp == Q4U_WARP_ISSUE) {
+            // ---------------- MMA issue: the whole warp runs the loop, one elected lane issues ----------------
+            const uint32_t ncols = STACK ? 2 * p.Mp : p.Mp;
+            const uint32_t idesc = (1u << 4) | ((ncols >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);      // f16 x f16 -> f32, K-major both
+            int xs = 0, slot = 0, fail = 0;
+            uint32_t xph = 0, dph = 1, aph = 0;          // (the first round of empty slots passes on the parity before the first)
+            for (int i = 0; i < range && !fail; ++i) {
+                const uint64_t bhi = q4u_desc_sw128(xring + xs * xstage_bytes), blo = bhi + (uint64_t)(p.Mp * 8);     // rows [0, Mp) = xhi, [Mp, 2 Mp) = xlo
+#pragma unroll
+                for (int tm = 0; tm < Q4U_TEAMS; ++tm) {
+                    const int what = lane % 3;
+                    const uint32_t bar = what == 0 ? a_full + 8 * tm : what == 1 ? d_empty + 8 * slot : x_full + 8 * xs;
+                    if (!q4u_bar_wait_all(bar, what == 0 ? aph : what == 1 ? dph : xph)) { fail = 32; break; }
+                    q4u_fence_after();
+                    const uint32_t d = tmem + slot * Q4U_D_COLS, a = tmem + Q4U_A_COL + tm * 32, df = d_full + 16 * tm, xe = x_empty + 8 * xs;
+                    if (q4u_elect_one()) {
+#pragma unroll
+                        for (int hf = 0; hf < 2; ++hf) {
+                            if (STACK) {
+                                q4u_mma(d + hf * 64, a + hf * 16, bhi + 4 * hf, idesc, 0u);
+                                q4u_mma(d + hf * 64, a + hf * 16 + 8, bhi + 4 * hf + 2, idesc, 1u);
+                            } else q4u_mma_block(d + hf * 64, a + hf * 16, bhi + 4 * hf, blo + 4 * hf, idesc);
+                            q4u_commit(df + 8 * hf);                           // the block's sums are complete
+                        }
+                        if (tm == Q4U_TEAMS - 1) q4u_commit(xe);               // ... and the activation stage is free
+                    }
+                    __syncwarp();
+                    if (++slot == Q4U_DSLOTS) { slot = 0; dph ^= 1u; }
+                }
+                aph ^= 1u;
+                if (++xs == Q4U_XSTAGES) { xs = 0; xph ^= 1u; }
+            }
+            if (fail && lane == 0) { atomicExch(p.status, fail); s_abort = 1; }
         }
-#ifdef MPQ_TRACE
-        if (p.trace && lane == 0 && tm == 0) {
-            unsigned long long* tr = p.trace + (size_t)blockIdx.x * 32;
-            tr[0] = (unsigned long long)(clock64() - cyc_t0); tr[1] = (unsigned long long)cyc_x; tr[2] = (unsigned long long)cyc_d;
-            tr[3] = (unsigned long long)cyc_a; tr[4] = (unsigned long long)cyc_issue; tr[5] = (unsigned long long)n;
-        }
-#endif
     } else {
-        // ---------------- expansion + drain: warps 5..20 = 4 teams x 4 lane quarters ----------------
-        // Warp qd of a team covers the rows of pair-tile qd of the team's group (one row per thread = one tensor-memory lane).
-        const int e = warp - 1 - Q4U_TEAMS, qd = e & 3, tm = e >> 2;
+        q4u_regs_more<Q4U_REGS_WORK>();
+        // ---------------- expansion + drain: team = warp / 4, lane quarter = warp % 4; one weight row per thread ----------------
+        const int tm = warp >> 2, qd = warp & 3;
+        const Q4URow row(qd, lane);
         const uint32_t lanes = (uint32_t)(qd * 32) << 16;
-        const int tile = lane >> 4, h = (lane >> 3) & 1, g8 = lane & 7; // this thread's weight row inside the pair-tile = lane
-        const uint32_t code_off = (uint32_t)qd * Q4_UNIT_BYTES + tile * 512 + g8 * 64;
-        const uint32_t scale_off = (uint32_t)qd * Q4_UNIT_BYTES + 1024 + g8 * 16 + tile * 8 + h * 4;
-        const uint32_t shA = 4 * h, shB = 4 * h + 8;
-        const uint32_t k1032 = 0x64086408u;                             // fp16 1032, twice
-        const uint32_t dst = tmem + lanes + Q4U_A_COL + (uint32_t)tm * 64;
-        const uint32_t dacc = tmem + lanes + (uint32_t)tm * 64;
-        float racc[64];                                                 // running fp32 sums of the drained segments, one per activation row (local memory: touched once per segment)
+        const uint32_t dst = tmem + lanes + Q4U_A_COL + (uint32_t)tm * 32, dacc = tmem + lanes;
+        const uint32_t wf = w_full + 8 * tm * WST, af = a_full + 8 * tm, df = d_full + 16 * tm;
+        const uint32_t ring = wring + (uint32_t)(tm * WST) * Q4U_WSTAGE_BYTES;
+        uint64_t acc[SL * 8];                                           // running fp32 sums, two activation rows each
 #pragma unroll
-        for (int i = 0; i < 64; ++i) racc[i] = 0.f;
-        int n = 0, drains = 0, seg_n = 0, wsi = 0;
-        uint32_t wph = 0;
-        bool waited = false, live = true;
-        float isc0 = 0.f, isc1 = 0.f;
-#ifdef MPQ_TRACE
-        long long cyc_w = 0, cyc_ae = 0, cyc_df = 0, cyc_exp = 0, cyc_st = 0, cyc_drain = 0, cyc_store = 0, gap_top = 0, gap_lds = 0, gap_arr = 0, t_prev = 0;
-        const long long cyc_t0 = clock64();
-#endif
-        int b = (int)(L_begin / p.nchunks), c = (int)(L_begin % p.nchunks) - 1;
-        for (long long L = L_begin; L < L_end && live; ++L) {
-            if (++c == p.nchunks) { c = 0; ++b; }
-            const int g = b * Q4U_TEAMS + tm;
-            if (g >= p.ngroups) continue;                               // no such group in the last batch
-            const bool exists = 4 * g + qd < p.nrp;                     // the last group may lack pair-tiles: they expand to zeros
-            const int ws = tm * WST + wsi;
-            const uint32_t wph_now = wph;
-            if (++wsi == WST) { wsi = 0; wph ^= 1u; }
-#ifdef MPQ_TRACE
-            if (t_prev) gap_top += clock64() - t_prev;
-#endif
-            Q4U_CYC(t_w)
-            // the stage's three waits usually find their phases complete: their tests go out together (one round trip)
-            const uint32_t okw = q4u_bar_test(w_full + 8 * ws, wph_now);
-            const uint32_t oka[2] = {q4u_bar_test(a_empty + 16 * tm, ((uint32_t)n & 1u) ^ 1u), q4u_bar_test(a_empty + 16 * tm + 8, ((uint32_t)n & 1u) ^ 1u)};
-            if (!okw && !q4u_bar_wait(w_full + 8 * ws, wph_now)) { if (lane == 0) { atomicExch(p.status, 36); s_abort = 1; } break; }
-            Q4U_CYC_ADD(cyc_w, t_w)
-            Q4U_CYC(t_g1)
-            const uint32_t base = wring + ws * Q4U_WSTAGE_BYTES;
-            uint4 seg[4];
-            uint32_t sw = 0;
-            if (exists) {
-#pragma unroll
-                for (int t = 0; t < 4; ++t) seg[t] = lds128(base + code_off + t * 16);
-                asm volatile("ld.shared.b32 %0, [%1];" : "=r"(sw) : "r"(base + scale_off));
-            } else {
-#pragma unroll
-                for (int t = 0; t < 4; ++t) seg[t] = make_uint4(0x88888888u, 0x88888888u, 0x88888888u, 0x88888888u);   // code 0
-            }
-            Q4U_CYC_ADD(gap_lds, t_g1)
-            // Two halves of the A stage (K steps 0, 1 = the first 32-block; 2, 3 = the second): while the MMAs of one half
-            // run, the other is being filled.
-#pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {
-                Q4U_CYC(t_ae)
-                if (!oka[hf] && !q4u_bar_wait(a_empty + 16 * tm + 8 * hf, ((uint32_t)n & 1u) ^ 1u)) { if (lane == 0) { atomicExch(p.status, 37); s_abort = 1; } live = false; break; }
-                Q4U_CYC_ADD(cyc_ae, t_ae)
-                q4u_fence_after();
-                Q4U_CYC(t_e)
-                const uint32_t s16 = hf == 0 ? (sw & 0xFFFFu) : (sw >> 16);
-                const uint32_t s2u = s16 | (s16 << 16);
-#pragma unroll
-                for (int jj = 0; jj < 2; ++jj) {
-                    const int j = 2 * hf + jj;
-                    uint32_t hi[8], lo[8];
-#pragma unroll
-                    for (int t = 0; t < 4; ++t) {
-                        const uint32_t w = j == 0 ? seg[t].x : j == 1 ? seg[t].y : j == 2 ? seg[t].z : seg[t].w;
-#pragma unroll
-                        for (int u = 0; u < 2; ++u) {            // k = 16j + 2t (+8): tensor-memory column t (+4) of the step
-                            const uint32_t bits = ((w >> (u ? shB : shA)) & 0x000F000Fu) | 0x64006400u;      // halves 1024 + n
-                            uint32_t code, vh, vl;                                                             // fp16 pairs in plain registers
-                            asm("sub.f16x2 %0, %1, %2;" : "=r"(code) : "r"(bits), "r"(k1032));                // n - 8, exact
-                            asm("mul.f16x2 %0, %1, %2;" : "=r"(vh) : "r"(code), "r"(s2u));
-                            asm("{\n\t.reg .b32 t;\n\tneg.f16x2 t, %3;\n\tfma.rn.f16x2 %0, %1, %2, t;\n\t}" : "=r"(vl) : "r"(code), "r"(s2u), "r"(vh));   // exact remainder
-                            hi[t + 4 * u] = vh;
-                            lo[t + 4 * u] = vl;
-                        }
-                    }
-                    q4u_st8(dst + hf * 32 + jj * 8, hi);
-                    q4u_st8(dst + hf * 32 + 16 + jj * 8, lo);
-                }
-                Q4U_CYC_ADD(cyc_exp, t_e)
-                if (hf == 1) {
-                    // The stores took every register the shared-memory loads produced as operands: the loads have
-                    // completed, so the weight stage may be overwritten.  (Releasing it right after issuing the loads
-                    // would let the next copy land under them.)
-                    q4u_bar_arrive(w_empty + 8 * ws);             // every thread, after its own stores took its registers
-                }
-                Q4U_CYC(t_s)
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                q4u_fence_before();
-                q4u_bar_arrive(a_full + 16 * tm + 8 * hf);         // every thread, after its own stores are complete
-                Q4U_CYC_ADD(cyc_st, t_s)
-            }
-            if (!live) break;
-#ifdef MPQ_TRACE
-            t_prev = clock64();
-#endif
-            ++n; ++seg_n;
-            // ---- end of a K segment: add the accumulator to the running sums (the tensor core's own accumulation
-            // loses about 2^-20 of the sum per MMA, so it is kept to Q4U_SEG chunks)
-            const bool piece_last = c == p.nchunks - 1 || L == L_end - 1;
-            if (!(seg_n == Q4U_SEG || piece_last)) continue;
-            seg_n = 0;
-            Q4U_CYC(t_df)
-            if (!q4u_bar_wait(d_full + 8 * tm, (uint32_t)drains & 1u)) { if (lane == 0) { atomicExch(p.status, 38); s_abort = 1; } break; }
-            Q4U_CYC_ADD(cyc_df, t_df)
-            ++drains;
-            q4u_fence_after();
-            Q4U_CYC(t_dr)
-#ifdef MPQ_TRACE
-            if (p.trace && lane == 0 && e == 0 && drains <= 4) s_tr[2 * (drains - 1)] = (unsigned long long)(clock64() - cyc_t0);
-#endif
-            {
-                // 32 accumulator columns per wait.  Columns: [0, Mp) (+ [Mp, 2 Mp) of the stacked form, which add to the same rows).
-                // The block loop is not unrolled, so that racc is addressed dynamically and stays in local memory.
-                const int ncols = p.stack ? 2 * p.Mp : p.Mp;
-#pragma unroll 1
-                for (int blk = 0; 32 * blk < ncols; ++blk) {
-                    uint32_t r[32];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        uint32_t (&rq)[8] = *reinterpret_cast<uint32_t (*)[8]>(&r[8 * q]);
-                        if (32 * blk + 8 * q < ncols) q4u_ld8(dacc + 32 * blk + 8 * q, rq);
-                        else {
-#pragma unroll
-                            for (int i = 0; i < 8; ++i) rq[i] = 0u;
-                        }
-                    }
-#ifdef MPQ_TRACE
-                    if (p.trace && lane == 0 && e == 0 && drains == 1 && blk == 0) s_tr[11] = (unsigned long long)(clock64() - cyc_t0);
-#endif
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#ifdef MPQ_TRACE
-                    if (p.trace && lane == 0 && e == 0 && drains == 1 && blk == 0) s_tr[12] = (unsigned long long)(clock64() - cyc_t0);
-#endif
-                    if (p.stack && p.Mp == 16) {
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) racc[i] += __uint_as_float(r[i]) + __uint_as_float(r[16 + i]);
-                    } else {
-                        float* sums = racc + (p.stack ? 0 : 32 * blk);
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) sums[i] += __uint_as_float(r[i]);
-                    }
-                }
-            }
-#ifdef MPQ_TRACE
-            if (p.trace && lane == 0 && e == 0 && drains == 1) s_tr[13] = (unsigned long long)(clock64() - cyc_t0);
-#endif
+        for (int i = 0; i < SL * 8; ++i) acc[i] = 0;
+        int ws = 0, slot = tm == Q4U_DSLOTS ? 0 : tm, fail = 0, left = range;
+        uint32_t wph = 0, dph = 0, sw = 0;
+        int b = (int)(L_begin / p.nchunks), c = (int)(L_begin % p.nchunks);
+        // the next chunk -> the A operand, which is free: the sums of the chunk that it held have been drained
+        auto expand = [&]() {
+            if (!q4u_bar_wait(wf + 8 * ws, wph)) return false;
+            row.expand(ring + ws * Q4U_WSTAGE_BYTES, dst, sw);
             q4u_fence_before();
-            q4u_bar_arrive(d_empty + 8 * tm);                   // (every thread) the next segment may overwrite the accumulator
-            Q4U_CYC_ADD(cyc_drain, t_dr)
-#ifdef MPQ_TRACE
-            if (p.trace && lane == 0 && e == 0 && drains <= 4) s_tr[1 + 2 * (drains - 1)] = (unsigned long long)(clock64() - cyc_t0);
-#endif
-            if (!piece_last) continue;
-            Q4U_CYC(t_so)
+            __syncwarp();
+            q4u_warp_arrive(af, lane);
+            q4u_warp_arrive(wf + 8 * NW + 8 * ws, lane);                // w_empty: the stores took every register the loads produced
+            if (++ws == WST) { ws = 0; wph ^= 1u; }
+            return true;
+        };
+        if (!expand()) fail = 36;
+        while (left > 0 && !fail) {
+            const int after = max(0, left - (p.nchunks - c));           // chunks left behind this piece
+            do {
+                const uint32_t d = dacc + slot * Q4U_D_COLS, s = sw;
+                if (!q4u_bar_wait(df, dph)) { fail = 35; break; }
+                q4u_fence_after();
+                q4u_drain<SL, STACK>(acc, d, p.Mp, s & 0xFFFFu);
+                if (!q4u_bar_wait(df + 8, dph)) { fail = 35; break; }
+                q4u_fence_after();
+                q4u_drain<SL, STACK>(acc, d + 64, p.Mp, s >> 16);
+                q4u_fence_before();
+                __syncwarp();
+                q4u_warp_arrive(d_empty + 8 * slot, lane);
+                if (++slot == Q4U_DSLOTS) slot = 0;                     // (four items further)
+                dph ^= 1u;
+                if (--left > 0 && !expand()) { fail = 36; break; }
+            } while (left > after);
+            if (fail) break;
             // ---- the piece's sums: to y when this range holds the whole batch, else to the piece's slice
             // inv_sc comes from the kernel before this one.  Lane l keeps rows l and l + 32 of it: read inside the store loop
             // the loads would be ordered behind the stores (they may alias for all the compiler knows), one round trip per row.
-            if (!waited) {
-                asm volatile("griddepcontrol.wait;" ::: "memory");
-                waited = true;
-                isc0 = lane < p.M ? p.inv_sc[lane] : 0.f;
-                isc1 = lane + 32 < p.M ? p.inv_sc[lane + 32] : 0.f;
-            }
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            const float isc0 = lane < p.M ? p.inv_sc[lane] : 0.f, isc1 = lane + 32 < p.M ? p.inv_sc[lane + 32] : 0.f;
             int pf, pl;
             q4u_pieces(b, p.nchunks, p.W, &pf, &pl);
-            const int nrow = g * 128 + qd * 32 + lane;
-            float* out = pf == pl ? p.Y : p.partial + (size_t)((int)blockIdx.x - pf) * p.M * p.N;
-            const int64_t ld = pf == pl ? p.ldy : (int64_t)p.N;
-#pragma unroll
-            for (int m = 0; m < 64; ++m) {
-                const float sc = __shfl_sync(0xFFFFFFFFu, m < 32 ? isc0 : isc1, m & 31);
-                if (m < p.M && nrow < p.N) out[(size_t)m * ld + nrow] = racc[m] * sc;
-                racc[m] = 0.f;
-            }
-            Q4U_CYC_ADD(cyc_store, t_so)
+            const int nrow = (b * Q4U_TEAMS + tm) * 128 + qd * 32 + lane;
+            float* out = (pf == pl ? p.Y : p.partial + (size_t)((int)blockIdx.x - pf) * p.M * p.N) + nrow;
+            q4u_store<SL>(acc, out, pf == pl ? p.ldy : (int64_t)p.N, p.M, nrow < p.N, isc0, isc1);
+            c = 0;
+            ++b;
         }
-#ifdef MPQ_TRACE
-        if (p.trace && lane == 0 && e == 0) {
-            p.trace[(size_t)blockIdx.x * 32 + 6] = (unsigned long long)cyc_store;
-            p.trace[(size_t)blockIdx.x * 32 + 24] = (unsigned long long)gap_top;
-            p.trace[(size_t)blockIdx.x * 32 + 25] = (unsigned long long)gap_lds;
-            p.trace[(size_t)blockIdx.x * 32 + 26] = (unsigned long long)gap_arr;
-            for (int i = 0; i < 8; ++i) p.trace[(size_t)blockIdx.x * 32 + 16 + i] = s_tr[i];
-            for (int i = 11; i < 14; ++i) p.trace[(size_t)blockIdx.x * 32 + 16 + i] = s_tr[i];
-            unsigned long long* tr = p.trace + (size_t)blockIdx.x * 32 + 8;
-            tr[0] = (unsigned long long)(clock64() - cyc_t0); tr[1] = (unsigned long long)cyc_w; tr[2] = (unsigned long long)cyc_ae;
-            tr[3] = (unsigned long long)cyc_exp; tr[4] = (unsigned long long)cyc_st; tr[5] = (unsigned long long)cyc_df;
-            tr[6] = (unsigned long long)cyc_drain; tr[7] = (unsigned long long)n;
-        }
-#endif
+        if (fail && lane == 0) { atomicExch(p.status, fail); s_abort = 1; }
     }
     q4u_fence_before();
     __syncthreads();
     settle_after_timeout(s_abort);
-    if (warp == 1) {
+    if (warp == Q4U_WARP_ISSUE) {
         q4u_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
     }
@@ -686,7 +607,7 @@ __global__ void __launch_bounds__(128, 1) q4u_mma_probe_kernel(int n_cols, int i
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     {
         const uint32_t ones[8] = {0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u};
-        for (int c = 0; c < 128; c += 8) q4u_st8(tmem + ((uint32_t)(warp * 32) << 16) + Q4U_A_COL + c, ones);
+        for (int c = 0; c < 128; c += 8) q4u_st8(tmem + ((uint32_t)(warp * 32) << 16) + 256 + c, ones);
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     }
     q4u_fence_before();
@@ -695,14 +616,14 @@ __global__ void __launch_bounds__(128, 1) q4u_mma_probe_kernel(int n_cols, int i
     if (warp < issuers && lane == 0) {
         const uint32_t idesc = (1u << 4) | ((uint32_t)(n_cols >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
         const uint64_t bd = q4u_desc_sw128(smem0);
-        const uint32_t d = tmem + (uint32_t)warp * 64, a = tmem + Q4U_A_COL + (uint32_t)warp * 32;
+        const uint32_t d = tmem + (uint32_t)warp * 64, a = tmem + 256 + (uint32_t)warp * 32;
         const long long t0 = clock64();
         for (int r = 0; r < reps; ++r) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) q4u_mma(d, a + j * 8, bd + 2 * j, idesc, (r > 0 || j > 0) ? 1u : 0u);
         }
         q4u_commit(bars + 8 * warp);
-        if (!q4u_bar_wait(bars + 8 * warp, 0)) atomicExch(status, 39);
+        if (!q4u_bar_wait_lane(bars + 8 * warp, 0)) atomicExch(status, 39);
         if (warp == 0) cycles[blockIdx.x] = clock64() - t0;
     }
     q4u_fence_before();
