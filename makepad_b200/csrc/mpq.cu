@@ -876,7 +876,7 @@ static int32_t q4_gemm_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
     p.status = ctx->q4_status;
     cfg = {};
     cfg.gridDim = dim3((unsigned)pl.grid);
-    cfg.blockDim = dim3(Q4U_THREADS);
+    cfg.blockDim = dim3(Q4G_THREADS);
     cfg.dynamicSmemBytes = q4_gemm_smem(Mt);
     cfg.stream = s;
     launch_pdl(cfg, at, ctx->pdl);

@@ -1,11 +1,13 @@
 // Q4 linear for more than 64 activation rows (prompts): tiles of 256 weight rows x up to 128 activation rows.
 //
 // The arithmetic and the roles are q4_umma_kernel's: weight codes as exact fp16 integers in tensor memory, activations split hi + lo,
-// two products, the sums of one 32-block scaled and added in fp32 registers.  A tile has two groups of 128 weight rows, and two
-// teams of four warps share a group: one expands the first 32-block of a chunk, the other the second; each drains half of the columns.
+// two products, the sums of one 32-block scaled and added in fp32 registers.  A tile has two groups of 128 weight rows, one per team of
+// four warps; a thread is one weight row and holds its sums with all activation rows of the tile.
 // One expansion of a weight feeds 4 MMAs of N = 128 = 256 cycles of tensor pipe per 32-block.
-// Measured, CTA pairs on 256 x 256 tiles with three products / this form (us): 22016 x 4096 at 96 rows 81.8 / 57.5, 128 83.9 / 62.0, 256
-// 115 / 98.9, 512 215 / 180; 4096 x 11008 at 512 113 / 104; 57344 x 8192 at 128 366 / 235; 1000 x 2112 at 128 16.5 / 15.4.
+// Measured, CTA pairs on 256 x 256 tiles with three products / this form (us): 22016 x 4096 at 96 rows 81.8 / 52.3, 128 83.9 / 59, 256
+// 115 / 93, 512 215 / 168..172; 4096 x 11008 at 512 113 / 95; 57344 x 8192 at 128 366 / 215; 1000 x 2112 at 128 16.5 / 15.6.  With
+// four teams of 104 registers, two per group: 180 at 512 rows.  A chunk's MMAs are 1024 cycles of pipe; a worker warp spends 620 on its
+// drains (FFMA pipe: 528 for the two warps of a scheduler), 210 on the expansion, the rest on waits of 90 cycles and more each.
 //
 // WORK.  Tiles are numbered activation tile fastest.  Every CTA gets the same number of whole tiles, which go straight to y; the
 // tiles that are left over are cut along K into equal ranges, one per CTA, so that any shape fills the SMs.  The pieces of a cut
@@ -15,7 +17,12 @@
 
 namespace mpq {
 
-constexpr int Q4G_GROUPS = 2;              // groups of 128 weight rows per tile, two teams of four warps each
+constexpr int Q4G_GROUPS = 2;              // groups of 128 weight rows per tile, one team of four warps each
+constexpr int Q4G_WARP_ISSUE = 4 * Q4G_GROUPS, Q4G_WARP_COPY = Q4G_WARP_ISSUE + 1;
+constexpr int Q4G_THREADS = 32 * 12;       // three warpgroups launched with 168 registers a thread: two go on with 216, one with 72
+constexpr int Q4G_REGS_WORK = 216, Q4G_REGS_REST = 72;
+constexpr int Q4G_D_SLOTS = 3, Q4G_D_COLS = 128;      // accumulators: columns [0, 384), used in turn
+constexpr int Q4G_A_COL = 384;             // A stages: two of one chunk per group
 constexpr int Q4G_WSTAGES = 8, Q4G_XSTAGES = 4;
 
 struct Q4GemmLaunch {
@@ -101,7 +108,6 @@ struct Q4GWalk {
         tile = rest_left ? p.full * (int)gridDim.x + q4u_div(begin, p.nchunks) : (int)blockIdx.x;
         c = rest_left ? (int)(begin - (int64_t)q4u_div(begin, p.nchunks) * p.nchunks) : 0;
     }
-    __device__ __forceinline__ bool piece_last(int nchunks) const { return c == nchunks - 1 || rest_left == 1; }
     __device__ __forceinline__ void next(int nchunks)
     {
         --left;
@@ -111,10 +117,19 @@ struct Q4GWalk {
             if (--rest_left == 0) { c = 0; tile = (int)blockIdx.x; }
         } else if (c == nchunks) { c = 0; tile += (int)gridDim.x; }
     }
+    // over the n chunks up to the end of a tile or of the range
+    __device__ __forceinline__ void skip(int n, int nchunks)
+    {
+        left -= n - 1;
+        if (rest_left > 0) rest_left -= n - 1;
+        c += n - 1;
+        next(nchunks);
+    }
 };
 
+// SL: half of the tile's 16-row slices, rounded up
 template <int SL>
-__global__ void __launch_bounds__(Q4U_THREADS, 1) q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ Q4GemmLaunch p)
+__global__ void __launch_bounds__(Q4G_THREADS, 1) q4_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ Q4GemmLaunch p)
 {
     extern __shared__ unsigned char smem_dyn[];
     __shared__ uint32_t s_tmem_base;
@@ -124,20 +139,20 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_gemm_kernel(const __grid_co
     const uint32_t xring = smem0, wring = xring + Q4G_XSTAGES * xstage_bytes;
     constexpr int NW = Q4G_GROUPS * Q4G_WSTAGES;
     const uint32_t w_full = wring + NW * Q4U_WSTAGE_BYTES, w_empty = w_full + 8 * NW, x_full = w_empty + 8 * NW, x_empty = x_full + 8 * Q4G_XSTAGES,
-                   a_full = x_empty + 8 * Q4G_XSTAGES, d_full = a_full + 32 * Q4G_GROUPS,
-                   d_empty = d_full + 16 * Q4G_GROUPS;   // a_full: [group][chunk % 2][half]; d_full: [group][half]
+                   a_full = x_empty + 8 * Q4G_XSTAGES, d_full = a_full + 16 * Q4G_GROUPS,
+                   d_empty = d_full + 16 * Q4G_GROUPS;   // a_full: [group][chunk % 2]; d_full: [group][half]
     const int warp = __shfl_sync(0xFFFFFFFFu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
         s_abort = 0;
-        for (int s = 0; s < NW; ++s) { q4u_bar_init(w_full + 8 * s, 1); q4u_bar_init(w_empty + 8 * s, 8); }
+        for (int s = 0; s < NW; ++s) { q4u_bar_init(w_full + 8 * s, 1); q4u_bar_init(w_empty + 8 * s, 4); }
         for (int s = 0; s < Q4G_XSTAGES; ++s) { q4u_bar_init(x_full + 8 * s, 1); q4u_bar_init(x_empty + 8 * s, 1); }
-        for (int s = 0; s < 4 * Q4G_GROUPS; ++s) q4u_bar_init(a_full + 8 * s, 4);
+        for (int s = 0; s < 2 * Q4G_GROUPS; ++s) q4u_bar_init(a_full + 8 * s, 4);
         for (int s = 0; s < 2 * Q4G_GROUPS; ++s) q4u_bar_init(d_full + 8 * s, 1);
-        for (int s = 0; s < Q4U_DSLOTS; ++s) q4u_bar_init(d_empty + 8 * s, 8);
+        for (int s = 0; s < Q4G_D_SLOTS; ++s) q4u_bar_init(d_empty + 8 * s, 4);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == Q4U_WARP_ISSUE) {
+    if (warp == Q4G_WARP_ISSUE) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)), "r"(512) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -147,9 +162,9 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_gemm_kernel(const __grid_co
     const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, s_tmem_base, 0);
     asm volatile("griddepcontrol.launch_dependents;");
 
-    if (warp >= Q4U_WARP_ISSUE) {
-        q4u_regs_fewer<Q4U_REGS_REST>();
-        if (warp == Q4U_WARP_COPY) {
+    if (warp >= Q4G_WARP_ISSUE) {
+        q4u_regs_fewer<Q4G_REGS_REST>();
+        if (warp == Q4G_WARP_COPY) {
             // ---------------- copies: lane g = weight ring of group g, lane Q4G_GROUPS = the activations, LAG chunks behind ----------------
             constexpr int LAG = Q4G_WSTAGES - Q4G_XSTAGES;
             const uint64_t l2pol = l2_evict_first_policy();
@@ -163,7 +178,7 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_gemm_kernel(const __grid_co
                 if (i == LAG) asm volatile("griddepcontrol.wait;" ::: "memory");    // the activations are staged by the kernel before this one
                 const bool now = wlane ? i < count : xlane && i >= LAG;
                 const uint32_t slot = wlane ? (uint32_t)(lane * Q4G_WSTAGES + ws) : (uint32_t)xs;
-                if (!q4u_bar_wait_all((wlane ? w_empty : x_empty) + 8 * slot, wlane ? wph : xph, now)) { if (lane == 0) { atomicExch(p.status, 41); s_abort = 1; } break; }
+                if (!q4u_bar_poll<100>((wlane ? w_empty : x_empty) + 8 * slot, wlane ? wph : xph, now)) { if (lane == 0) { atomicExch(p.status, 41); s_abort = 1; } break; }
                 if (now) {
                     const uint32_t bar = (wlane ? w_full : x_full) + 8 * slot;
                     mbar_expect_tx(bar, wlane ? Q4U_W_BYTES : xstage_bytes);
@@ -181,7 +196,7 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_gemm_kernel(const __grid_co
                     x.next(p.nchunks);
                 }
             }
-        } else if (warp == Q4U_WARP_ISSUE) {
+        } else if (warp == Q4G_WARP_ISSUE) {
             // ---------------- MMA issue: the whole warp runs the loop, one elected lane issues ----------------
             const uint32_t idesc = (1u << 4) | ((uint32_t)(p.Mt >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);      // f16 x f16 -> f32, K-major both
             const int count = Q4GWalk(p).left;
@@ -192,96 +207,116 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_gemm_kernel(const __grid_co
 #pragma unroll
                 for (int k = 0; k < 2 * Q4G_GROUPS; ++k) {                             // 32-block k / 2 of group k % 2
                     const int hf = k >> 1, g = k & 1, what = lane % 3;
-                    const uint32_t bar = what == 0 ? a_full + 32 * g + 16 * (i & 1) + 8 * hf : what == 1 ? d_empty + 8 * slot : x_full + 8 * xs;
-                    if (!q4u_bar_wait_all(bar, what == 0 ? (uint32_t)(i >> 1) & 1u : what == 1 ? dph : xph)) { fail = 42; break; }
+                    const uint32_t bar = what == 0 ? a_full + 16 * g + 8 * (i & 1) : what == 1 ? d_empty + 8 * slot : x_full + 8 * xs;
+                    if (!q4u_bar_poll<0>(bar, what == 0 ? (uint32_t)(i >> 1) & 1u : what == 1 ? dph : xph)) { fail = 42; break; }
                     q4u_fence_after();
-                    const uint32_t d = tmem + slot * Q4U_D_COLS, a = tmem + Q4U_A_COL + g * 64 + (i & 1) * 32 + hf * 16, df = d_full + 16 * g + 8 * hf, xe = x_empty + 8 * xs;
+                    const uint32_t d = tmem + slot * Q4G_D_COLS, a = tmem + Q4G_A_COL + g * 64 + (i & 1) * 32 + hf * 16, df = d_full + 16 * g + 8 * hf, xe = x_empty + 8 * xs;
                     if (q4u_elect_one()) {
                         q4u_mma_block(d, a, bhi + 4 * hf, blo + 4 * hf, idesc);
                         q4u_commit(df);                                                // the block's sums are complete
                         if (k == 2 * Q4G_GROUPS - 1) q4u_commit(xe);                   // ... and the activation stage is free
                     }
                     __syncwarp();
-                    if (++slot == Q4U_DSLOTS) { slot = 0; dph ^= 1u; }
+                    if (++slot == Q4G_D_SLOTS) { slot = 0; dph ^= 1u; }
                 }
                 if (++xs == Q4G_XSTAGES) { xs = 0; xph ^= 1u; }
             }
             if (fail && lane == 0) { atomicExch(p.status, fail); s_abort = 1; }
         }
     } else {
-        q4u_regs_more<Q4U_REGS_WORK>();
-        // ---------------- expansion + drain: team = warp / 4, lane quarter = warp % 4; one weight row per thread ----------------
-        const int g = warp >> 3, half = (warp >> 2) & 1, qd = warp & 3;
+        q4u_regs_more<Q4G_REGS_WORK>();
+        // ---------------- expansion + drain: team = group = warp / 4, lane quarter = warp % 4; one weight row per thread ----------------
+        const int g = warp >> 2, qd = warp & 3;
         const Q4URow row(qd, lane);
         const uint32_t lanes = (uint32_t)(qd * 32) << 16;
-        const int h0 = ((p.Mt >> 4) + 1) / 2 * 16;                      // columns of the first team of a group (SL * 16 of them are read, whatever they hold)
-        const int first = half ? h0 : 0;
-        uint32_t dst = tmem + lanes + Q4U_A_COL + (uint32_t)g * 64 + half * 16, af = a_full + 32 * g + 8 * half;
-        const uint32_t dacc = tmem + lanes + first;
+        uint32_t dst = tmem + lanes + Q4G_A_COL + (uint32_t)g * 64, af = a_full + 16 * g;
+        const uint32_t dacc = tmem + lanes;
         const uint32_t wf = w_full + 8 * g * Q4G_WSTAGES, df = d_full + 16 * g;
         const uint32_t ring = wring + (uint32_t)(g * Q4G_WSTAGES) * Q4U_WSTAGE_BYTES;
-        uint64_t acc[SL * 8];                                           // running fp32 sums, two activation rows each
+        uint64_t acc[2][SL * 8];                                        // running fp32 sums, two activation rows each (past Mt: of whatever the columns hold)
 #pragma unroll
-        for (int i = 0; i < SL * 8; ++i) acc[i] = 0;
+        for (int i = 0; i < SL * 8; ++i) acc[0][i] = acc[1][i] = 0;
         int ws = 0, slot = g, fail = 0;
-        uint32_t wph = 0, dph = 0, sw0, sw1 = 0, sw2 = 0;               // scales of the chunk that is drained, and of the two behind it
+        uint32_t wph = 0, dph = 0, sw0 = 0, sw1 = 0, sw2 = 0;           // scales of the chunk that is drained, and of the two behind it
+        uint2 codes[2][4];
         Q4GWalk w(p);
-        bool from_start = w.c == 0;
-        // this team's half of the chunk in weight stage ws -> its A stage, which is free: the block that it held has been drained
-        auto expand = [&](uint32_t& sw) {
-            if (!q4u_bar_wait(wf + 8 * ws, wph)) return false;
+        // the chunk in weight stage ws -> registers
+        auto load = [&](uint32_t& sw) {
             const uint32_t stage = ring + ws * Q4U_WSTAGE_BYTES;
-            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(sw) : "r"(stage + row.scale_off));
-            row.block(stage, half, dst);
+            sw = row.scales(stage);
+            row.load(codes[0], stage, 0);
+            row.load(codes[1], stage, 1);
+        };
+        // ... -> its A stage, which is free: the blocks that it held have been drained
+        auto expand = [&](uint32_t& sw) {
+            row.expand(codes[0], dst);
+            row.expand(codes[1], dst + 16);
             asm volatile("tcgen05.wait::st.sync.aligned;" : "+r"(sw)::"memory");                // (and the scales have arrived)
             q4u_fence_before();
             __syncwarp();
             q4u_warp_arrive(af, lane);
-            q4u_warp_arrive(wf + 8 * NW + 8 * ws, lane);                // w_empty: the store took every register the loads produced
+            q4u_warp_arrive(wf + 8 * NW + 8 * ws, lane);                // w_empty: the stores took every register the loads produced
             if (++ws == Q4G_WSTAGES) { ws = 0; wph ^= 1u; }
             dst ^= 32;                                                  // the other of the two A stages, and its barrier
-            af ^= 16;
-            return true;
+            af ^= 8;
         };
-        if (!expand(sw0) || (w.left > 1 && !expand(sw1))) fail = 46;
-        while (w.left && !fail) {
-#pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {
-                if (!q4u_bar_wait(df + 8 * hf, dph)) { fail = 45; break; }
-                q4u_fence_after();
-                q4u_drain<SL, false>(acc, dacc + slot * Q4U_D_COLS, 0, hf ? sw0 >> 16 : sw0 & 0xFFFFu);
-                q4u_fence_before();
-                __syncwarp();
-                q4u_warp_arrive(d_empty + 8 * slot, lane);
-                slot += 2;
-                if (slot >= Q4U_DSLOTS) slot -= Q4U_DSLOTS;
+        if (q4u_bar_wait(wf, 0)) {
+            load(sw0);
+            expand(sw0);
+            if (w.left > 1) {
+                if (q4u_bar_wait(wf + 8, 0)) { load(sw1); expand(sw1); }
+                else fail = 46;
             }
+        } else fail = 46;
+        while (w.left && !fail) {
+            int piece = w.rest_left ? min(w.rest_left, p.nchunks - w.c) : p.nchunks;          // chunks of this piece
+            const int behind = w.left - piece;
+            const bool whole = w.c == 0 && piece == p.nchunks;
+            do {
+                --piece;
+                const bool more = piece + behind > 1, look = more && (lane & 1);
+#pragma unroll
+                for (int hf = 0; hf < 2; ++hf) {
+                    // with the first block's sums the weights of the chunk that is expanded next: one round trip
+                    if (!(hf ? q4u_bar_wait(df + 8, dph) : q4u_bar_wait(look ? wf + 8 * ws : df, look ? wph : dph))) { fail = 45; break; }
+                    q4u_fence_after();
+                    if (hf == 0 && more) load(sw2);
+                    const uint32_t d = dacc + slot * Q4G_D_COLS, scale = hf ? sw0 >> 16 : sw0 & 0xFFFFu;
+                    q4u_drain<SL, false, true>(acc[0], d, 0, scale);
+                    q4u_drain<SL, false, true>(acc[1], d + SL * 16, 0, scale);
+                    q4u_fence_before();
+                    __syncwarp();
+                    q4u_warp_arrive(d_empty + 8 * slot, lane);
+                    slot += 2;
+                    if (slot >= Q4G_D_SLOTS) slot -= Q4G_D_SLOTS;
+                }
+                if (fail) break;
+                dph ^= 1u;
+                if (more) expand(sw2);
+                sw0 = sw1;
+                sw1 = sw2;
+            } while (piece);
             if (fail) break;
-            dph ^= 1u;
-            if (w.left > 2 && !expand(sw2)) { fail = 46; break; }
-            sw0 = sw1;
-            sw1 = sw2;
-            if (w.piece_last(p.nchunks)) {
-                // the piece's sums: to y when this range holds the whole tile, else to the range's slot
-                asm volatile("griddepcontrol.wait;" ::: "memory");      // inv_sc, and y and the slots may still be read
-                const int b = w.tile / p.nt, m0 = (w.tile - b * p.nt) * p.Mt + first, rows = min(half ? p.Mt - h0 : h0, p.M - m0);
+            // the piece's sums: to y when this range holds the whole tile, else to the range's slot
+            asm volatile("griddepcontrol.wait;" ::: "memory");          // inv_sc, and y and the slots may still be read
+            const int b = w.tile / p.nt, col = g * 128 + qd * 32 + lane, nrow = b * 256 + col;
+            const int at = w.tile != p.full * (int)gridDim.x + q4u_div((int64_t)blockIdx.x * p.W, p.nchunks);
+            float* slot_out = p.partial + ((size_t)blockIdx.x * 2 + at) * Q4G_SLOT + col;
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int r0 = u * SL * 16, m0 = (w.tile - b * p.nt) * p.Mt + r0, rows = min(min(SL * 16, p.Mt - r0), p.M - m0);
                 // lane l keeps rows l and l + 32: read inside the store loop the loads would be ordered behind the stores
                 const float isc0 = lane < rows ? p.inv_sc[m0 + lane] : 0.f, isc1 = lane + 32 < rows ? p.inv_sc[m0 + lane + 32] : 0.f;
-                const int col = g * 128 + qd * 32 + lane, nrow = b * 256 + col;
-                const bool whole = from_start && w.c == p.nchunks - 1;
-                const int at = w.tile != p.full * (int)gridDim.x + q4u_div((int64_t)blockIdx.x * p.W, p.nchunks);
-                float* out = whole ? p.Y + (size_t)m0 * p.ldy + nrow : p.partial + ((size_t)blockIdx.x * 2 + at) * Q4G_SLOT + (size_t)first * 256 + col;
-                q4u_store<SL>(acc, out, whole ? p.ldy : 256, rows, !whole || nrow < p.N, isc0, isc1);
-                from_start = true;
+                q4u_store<SL>(acc[u], whole ? p.Y + (size_t)m0 * p.ldy + nrow : slot_out + (size_t)r0 * 256, whole ? p.ldy : 256, rows, !whole || nrow < p.N, isc0, isc1);
             }
-            w.next(p.nchunks);
+            w.skip(w.left - behind, p.nchunks);
         }
         if (fail && lane == 0) { atomicExch(p.status, fail); s_abort = 1; }
     }
     q4u_fence_before();
     __syncthreads();
     settle_after_timeout(s_abort);
-    if (warp == Q4U_WARP_ISSUE) {
+    if (warp == Q4G_WARP_ISSUE) {
         q4u_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
     }

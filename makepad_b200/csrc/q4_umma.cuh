@@ -34,10 +34,12 @@
 // WHAT IT COSTS (measured parts).  An MMA of N = 64 takes 32 cycles of pipe, one of N = 128 64, whoever issues it; the issue of four
 // with operands in ordinary registers 264, so the role of a warp, the waits' outcomes and with them all that the loops count are
 // kept uniform for the compiler.  One look at an mbarrier is a round trip of 90 cycles and two in a row are 170, so the issuing
-// warp looks at all barriers of its next step at once, one per lane.
+// warp looks at all barriers of its next step at once, one per lane, and between the two halves of a step's MMAs (57344 x 8192: 16 rows
+// 92 / 85 us, 64 rows 146 / 133).
 // Measured, staging and sum of the pieces included, three products with sums kept in tensor memory / this form (us): 22016 x 4096 at
-// 17 rows 39.8 / 29.7, 32 41.3 / 31.2, 64 59.5 / 49.6; 57344 x 8192 at 64 223 / 147; 8192 x 28672 at 64 140 / 89; 1000 x 2112 at 64
-// 19.7 / 15.0.  The same with pairs of tests per 32-block in one issuing warp: 264 at 57344 x 8192; with run-time operands 175.
+// 32 rows 41.3 / 35, 64 59.5 / 48; 57344 x 8192 at 64 223 / 133; 8192 x 28672 at 64 140 / 85; 1000 x 2112 at 64
+// 19.7 / 15.0.  Tests of one barrier after the other per 32-block: 264 at 57344 x 8192; run-time operands 175; two A stages per team
+// up to 32 rows: 104 / 122.
 #pragma once
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -55,9 +57,8 @@ constexpr int Q4U_MAX_WSTAGES = 8;            // weight ring PER TEAM: at most s
 constexpr int Q4U_W_BYTES = 4 * Q4_UNIT_BYTES;
 constexpr int Q4U_WSTAGE_BYTES = 5 * 1024;    // (the swizzle wants stages of whole kilobytes)
 constexpr int Q4U_XSTAGES = 4;                // activation ring: stages of one chunk (hi tile + lo tile)
-constexpr int Q4U_DSLOTS = 3;                 // accumulators: columns [0, 384), slots of two 32-blocks that are used in turn
-constexpr int Q4U_D_COLS = 128;
-constexpr int Q4U_A_COL = 384;                // A operand: [384, 512)
+constexpr int Q4U_DSLOTS = 3, Q4U_D_COLS = 128;      // accumulators: columns [0, 384), slots of two 32-blocks that are used in turn
+constexpr int Q4U_A_COL = 384;                // A operand: [384, 512), a chunk per team (a second one up to 32 rows, in place of accumulators, was 10% slower)
 constexpr uint32_t Q4U_SPIN = 1u << 22;       // tries of one mbarrier before giving up
 
 struct Q4ULaunch {
@@ -168,17 +169,18 @@ __device__ __forceinline__ uint32_t q4u_bar_test(uint32_t bar, uint32_t parity)
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok;
 }
-// Bounded wait of a converged warp on a phase parity: false when the limit ran out.  try_wait suspends the threads for a
+// Bounded wait of a converged warp on a phase parity, or on one per lane: false when the limit ran out.  try_wait suspends the threads for a
 // hardware-chosen time per try.  The vote makes the outcome uniform for the compiler: what the loops around it count stays in uniform registers.
 __device__ __forceinline__ bool q4u_bar_wait(uint32_t bar, uint32_t parity)
 {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p, q;\n\t.reg .b32 n;\n\tmov.b32 n, 0;\n"
-                 "TRY:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tvote.sync.all.pred p, p, 0xffffffff;\n\t@p bra.uni DONE;\n\t"
-                 "add.u32 n, n, 1;\n\tsetp.lt.u32 q, n, %3;\n\t@q bra.uni TRY;\n"
-                 "DONE:\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(bar), "r"(parity), "n"(Q4U_SPIN) : "memory");
-    return __all_sync(0xFFFFFFFFu, ok);
+    uint32_t all;
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .b32 n;\n\tmov.b32 n, 0;\n"
+                 "TRY:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tvote.sync.ballot.b32 %0, p, 0xffffffff;\n\t"
+                 "setp.eq.u32 p, %0, 0xffffffff;\n\t@p bra.uni DONE;\n\t"
+                 "add.u32 n, n, 1;\n\tsetp.lt.u32 p, n, %3;\n\t@p bra.uni TRY;\n"
+                 "DONE:\n\t}"
+                 : "=r"(all) : "r"(bar), "r"(parity), "n"(Q4U_SPIN) : "memory");
+    return all == 0xFFFFFFFFu;
 }
 // ... by a thread for itself (the ones above and below are for whole warps: a lane alone would wait in the vote for good)
 __device__ __forceinline__ bool q4u_bar_wait_lane(uint32_t bar, uint32_t parity)
@@ -187,11 +189,14 @@ __device__ __forceinline__ bool q4u_bar_wait_lane(uint32_t bar, uint32_t parity)
         if (q4u_bar_test(bar, parity)) return true;
     return false;
 }
-// ... on the barriers of all lanes at once (those of lanes without `mine` are not looked at)
-__device__ __forceinline__ bool q4u_bar_wait_all(uint32_t bar, uint32_t parity, bool mine = true)
+// ... with a look at a time, and SLEEP ns between two of them; the barriers of lanes without `mine` are not looked at
+template <int SLEEP>
+__device__ __forceinline__ bool q4u_bar_poll(uint32_t bar, uint32_t parity, bool mine = true)
 {
-    for (uint32_t n = 0; n < Q4U_SPIN; ++n)
+    for (uint32_t n = 0; n < Q4U_SPIN; ++n) {
         if (__all_sync(0xFFFFFFFFu, !mine || q4u_bar_test(bar, parity))) return true;
+        if (SLEEP) __nanosleep(SLEEP);
+    }
     return false;
 }
 // lane 0 of a converged warp arrives (predicated: a branch would bring its own reconvergence)
@@ -216,15 +221,19 @@ __device__ __forceinline__ void q4u_mma(uint32_t d, uint32_t a, uint64_t bdesc, 
         "}"
         ::"r"(d), "r"(a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
-// one 32-block against the hi and the lo tile: K steps of 16 are 8 columns of A and +32 bytes = +2 in the descriptor.  The small
-// products first.  (Operands that the compiler knows to be uniform: else each goes from a register to a uniform one in front of the
+// one 32-block against the hi or the lo tile: K steps of 16 are 8 columns of A and +32 bytes = +2 in the descriptor.
+// (Operands that the compiler knows to be uniform: else each goes from a register to a uniform one in front of the
 // instruction, which made the issue of four MMAs take 264 cycles where their pipe time is 128.)
+__device__ __forceinline__ void q4u_mma_half(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate)
+{
+    q4u_mma(d, a, b, idesc, accumulate);
+    q4u_mma(d, a + 8, b + 2, idesc, 1u);
+}
+// ... against both, the small products first
 __device__ __forceinline__ void q4u_mma_block(uint32_t d, uint32_t a, uint64_t bhi, uint64_t blo, uint32_t idesc)
 {
-    q4u_mma(d, a, blo, idesc, 0u);
-    q4u_mma(d, a + 8, blo + 2, idesc, 1u);
-    q4u_mma(d, a, bhi, idesc, 1u);
-    q4u_mma(d, a + 8, bhi + 2, idesc, 1u);
+    q4u_mma_half(d, a, blo, idesc, 0u);
+    q4u_mma_half(d, a, bhi, idesc, 1u);
 }
 // registers -> this warp's 32 tensor-memory lanes: thread l writes lane l, register j goes to column +j
 __device__ __forceinline__ void q4u_st8(uint32_t taddr, const uint32_t (&r)[8])
@@ -308,13 +317,16 @@ struct Q4URow {
         asm("{\n\t.reg .b32 t;\n\tlop3.b32 t, %1, %2, 0x64006400, 0xEA;\n\tfma.rn.f16x2 %0, t, %3, %4;\n\t}" : "=r"(r) : "r"(w), "r"(mask), "r"(mul), "r"(add));
         return r;
     }
-    // 32-block hf of this row: shared memory -> exact fp16 codes -> sixteen columns of the A operand
-    __device__ __forceinline__ void block(uint32_t stage, int hf, uint32_t dst) const
+    // 32-block hf of this row in shared memory -> registers
+    __device__ __forceinline__ void load(uint2 (&w)[4], uint32_t stage, int hf) const
     {
-        uint2 w[4];
 #pragma unroll
         for (int t = 0; t < 4; ++t)
             asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(w[t].x), "=r"(w[t].y) : "r"(((stage + code_off) ^ (uint32_t)(t << 4)) + hf * 8));
+    }
+    // ... -> exact fp16 codes -> sixteen columns of the A operand
+    __device__ __forceinline__ void expand(const uint2 (&w)[4], uint32_t dst) const
+    {
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             uint32_t a[8];
@@ -327,31 +339,44 @@ struct Q4URow {
             q4u_st8(dst + j * 8, a);
         }
     }
-    // both of a chunk, stored and waited for; sw = the chunk's scales
-    __device__ __forceinline__ void expand(uint32_t stage, uint32_t dst, uint32_t& sw) const
+    __device__ __forceinline__ uint32_t scales(uint32_t stage) const
     {
-        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(sw) : "r"(stage + scale_off));
-        block(stage, 0, dst);
-        block(stage, 1, dst + 16);
-        asm volatile("tcgen05.wait::st.sync.aligned;" : "+r"(sw)::"memory");              // (and the scales have arrived)
+        uint32_t v;
+        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(stage + scale_off));
+        return v;
     }
 };
 
 // acc += s * (the block's sums): 16 * SL activation rows from column d on; with STACK the products with the lo parts lie `lo` columns
 // behind those with the hi parts
-template <int SL, bool STACK>
+// PAIRS: 32 columns on their way at a time
+template <int SL, bool STACK, bool PAIRS>
 __device__ __forceinline__ void q4u_drain(uint64_t (&acc)[SL * 8], uint32_t d, uint32_t lo, uint32_t scale16)
 {
     const uint64_t s2 = q4u_pair(__half2float(__ushort_as_half((unsigned short)scale16)));
+    uint32_t r[16], r2[16];
+    if (STACK) {
 #pragma unroll
-    for (int sl = 0; sl < SL; ++sl) {
-        uint32_t r[16], r2[16];
-        if (STACK) q4u_ld16x2(d + 16 * sl, d + lo + 16 * sl, r, r2);
-        else q4u_ld16(d + 16 * sl, r);
+        for (int sl = 0; sl < SL; ++sl) {
+            q4u_ld16x2(d + 16 * sl, d + lo + 16 * sl, r, r2);
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            if (STACK) q4u_fma2_sum(acc[sl * 8 + q], r[2 * q], r[2 * q + 1], r2[2 * q], r2[2 * q + 1], s2);
-            else q4u_fma2(acc[sl * 8 + q], r[2 * q], r[2 * q + 1], s2);
+            for (int q = 0; q < 8; ++q) q4u_fma2_sum(acc[sl * 8 + q], r[2 * q], r[2 * q + 1], r2[2 * q], r2[2 * q + 1], s2);
+        }
+    } else {
+#pragma unroll
+        for (int sl = 0; sl + 1 < SL; sl += 2) {
+            if (PAIRS) q4u_ld16x2(d + 16 * sl, d + 16 * sl + 16, r, r2);
+            else q4u_ld16(d + 16 * sl, r);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) q4u_fma2(acc[sl * 8 + q], r[2 * q], r[2 * q + 1], s2);
+            if (!PAIRS) q4u_ld16(d + 16 * sl + 16, r2);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) q4u_fma2(acc[sl * 8 + 8 + q], r2[2 * q], r2[2 * q + 1], s2);
+        }
+        if (SL & 1) {
+            q4u_ld16(d + 16 * (SL - 1), r);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) q4u_fma2(acc[(SL - 1) * 8 + q], r[2 * q], r[2 * q + 1], s2);
         }
     }
 }
@@ -424,7 +449,7 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_umma_kernel(const __grid_co
                 if (i == LAG) asm volatile("griddepcontrol.wait;" ::: "memory");    // the activations are staged by the kernel before this one
                 const bool now = wlane ? i < range : xlane && i >= LAG;
                 const uint32_t slot = wlane ? (uint32_t)(lane * WST + ws) : (uint32_t)xs;
-                if (!q4u_bar_wait_all((wlane ? w_empty : x_empty) + 8 * slot, wlane ? wph : xph, now)) { if (lane == 0) { atomicExch(p.status, 31); s_abort = 1; } break; }
+                if (!q4u_bar_poll<100>((wlane ? w_empty : x_empty) + 8 * slot, wlane ? wph : xph, now)) { if (lane == 0) { atomicExch(p.status, 31); s_abort = 1; } break; }
                 if (now) {
                     const uint32_t bar = (wlane ? w_full : x_full) + 8 * slot;
                     mbar_expect_tx(bar, wlane ? Q4U_W_BYTES : xstage_bytes);
@@ -446,33 +471,42 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_umma_kernel(const __grid_co
             // ---------------- MMA issue: the whole warp runs the loop, one elected lane issues ----------------
             const uint32_t ncols = STACK ? 2 * p.Mp : p.Mp;
             const uint32_t idesc = (1u << 4) | ((ncols >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);      // f16 x f16 -> f32, K-major both
+            const int what = lane % 3;
             int xs = 0, slot = 0, fail = 0;
             uint32_t xph = 0, dph = 1, aph = 0;          // (the first round of empty slots passes on the parity before the first)
+            bool ready = false;                          // the barriers of the next step have been seen
+            // what this lane looks at before a step: the team's A operand, the accumulator slot, the activations
+            auto bar = [&](int tm) { return what == 0 ? a_full + 8 * tm : what == 1 ? d_empty + 8 * slot : x_full + 8 * xs; };
+            auto parity = [&]() { return what == 0 ? aph : what == 1 ? dph : xph; };
             for (int i = 0; i < range && !fail; ++i) {
                 const uint64_t bhi = q4u_desc_sw128(xring + xs * xstage_bytes), blo = bhi + (uint64_t)(p.Mp * 8);     // rows [0, Mp) = xhi, [Mp, 2 Mp) = xlo
 #pragma unroll
                 for (int tm = 0; tm < Q4U_TEAMS; ++tm) {
-                    const int what = lane % 3;
-                    const uint32_t bar = what == 0 ? a_full + 8 * tm : what == 1 ? d_empty + 8 * slot : x_full + 8 * xs;
-                    if (!q4u_bar_wait_all(bar, what == 0 ? aph : what == 1 ? dph : xph)) { fail = 32; break; }
+                    if (!ready && !q4u_bar_poll<0>(bar(tm), parity())) { fail = 32; break; }
                     q4u_fence_after();
                     const uint32_t d = tmem + slot * Q4U_D_COLS, a = tmem + Q4U_A_COL + tm * 32, df = d_full + 16 * tm, xe = x_empty + 8 * xs;
+                    auto issue = [&](int hf) {
+                        if (STACK) {
+                            q4u_mma(d + hf * 64, a + hf * 16, bhi + 4 * hf, idesc, 0u);
+                            q4u_mma(d + hf * 64, a + hf * 16 + 8, bhi + 4 * hf + 2, idesc, 1u);
+                        } else q4u_mma_block(d + hf * 64, a + hf * 16, bhi + 4 * hf, blo + 4 * hf, idesc);
+                        q4u_commit(df + 8 * hf);                               // the block's sums are complete
+                    };
+                    if (q4u_elect_one()) issue(0);
+                    __syncwarp();
+                    // the look at the next step's barriers takes as long as these MMAs: the pipe would be idle behind the others
+                    if (++slot == Q4U_DSLOTS) { slot = 0; dph ^= 1u; }
+                    if (tm == Q4U_TEAMS - 1) {
+                        aph ^= 1u;
+                        if (++xs == Q4U_XSTAGES) { xs = 0; xph ^= 1u; }
+                    }
+                    ready = __all_sync(0xFFFFFFFFu, q4u_bar_test(bar((tm + 1) % Q4U_TEAMS), parity()));
                     if (q4u_elect_one()) {
-#pragma unroll
-                        for (int hf = 0; hf < 2; ++hf) {
-                            if (STACK) {
-                                q4u_mma(d + hf * 64, a + hf * 16, bhi + 4 * hf, idesc, 0u);
-                                q4u_mma(d + hf * 64, a + hf * 16 + 8, bhi + 4 * hf + 2, idesc, 1u);
-                            } else q4u_mma_block(d + hf * 64, a + hf * 16, bhi + 4 * hf, blo + 4 * hf, idesc);
-                            q4u_commit(df + 8 * hf);                           // the block's sums are complete
-                        }
+                        issue(1);
                         if (tm == Q4U_TEAMS - 1) q4u_commit(xe);               // ... and the activation stage is free
                     }
                     __syncwarp();
-                    if (++slot == Q4U_DSLOTS) { slot = 0; dph ^= 1u; }
                 }
-                aph ^= 1u;
-                if (++xs == Q4U_XSTAGES) { xs = 0; xph ^= 1u; }
             }
             if (fail && lane == 0) { atomicExch(p.status, fail); s_abort = 1; }
         }
@@ -494,7 +528,15 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_umma_kernel(const __grid_co
         // the next chunk -> the A operand, which is free: the sums of the chunk that it held have been drained
         auto expand = [&]() {
             if (!q4u_bar_wait(wf + 8 * ws, wph)) return false;
-            row.expand(ring + ws * Q4U_WSTAGE_BYTES, dst, sw);
+            const uint32_t stage = ring + ws * Q4U_WSTAGE_BYTES;
+            sw = row.scales(stage);
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+                uint2 w[4];
+                row.load(w, stage, hf);
+                row.expand(w, dst + hf * 16);
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" : "+r"(sw)::"memory");                // (and the scales have arrived)
             q4u_fence_before();
             __syncwarp();
             q4u_warp_arrive(af, lane);
@@ -509,14 +551,14 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_umma_kernel(const __grid_co
                 const uint32_t d = dacc + slot * Q4U_D_COLS, s = sw;
                 if (!q4u_bar_wait(df, dph)) { fail = 35; break; }
                 q4u_fence_after();
-                q4u_drain<SL, STACK>(acc, d, p.Mp, s & 0xFFFFu);
+                q4u_drain<SL, STACK, SL != 4>(acc, d, p.Mp, s & 0xFFFFu);
                 if (!q4u_bar_wait(df + 8, dph)) { fail = 35; break; }
                 q4u_fence_after();
-                q4u_drain<SL, STACK>(acc, d + 64, p.Mp, s >> 16);
+                q4u_drain<SL, STACK, SL != 4>(acc, d + 64, p.Mp, s >> 16);
                 q4u_fence_before();
                 __syncwarp();
                 q4u_warp_arrive(d_empty + 8 * slot, lane);
-                if (++slot == Q4U_DSLOTS) slot = 0;                     // (four items further)
+                if (++slot == Q4U_DSLOTS) slot = 0;              // (four items further)
                 dph ^= 1u;
                 if (--left > 0 && !expand()) { fail = 36; break; }
             } while (left > after);
