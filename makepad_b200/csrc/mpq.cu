@@ -47,7 +47,7 @@ struct mpq_context {
     Scratch swiglu_buf;       // SwiGLU output for the Q4 kernels that do not fuse it
     int q4_umma_min;          // fewest activation rows routed to the tcgen05 kernel (0 = never)
     Scratch q4_partial;       // partial outputs: [K slices][M][N] of the rectangle kernel, the pieces of the tcgen05 kernels
-    int q4_gemm_min;          // fewest activation rows routed to the CTA-pair kernel (0 = never: slabs of 64 through the tcgen05 kernel)
+    int q4_gemm_min;          // fewest activation rows routed to q4_gemm_kernel (0 = never: slabs of 64 through the tcgen05 kernel)
     bool q4_rect;             // use the rectangle kernel for 5..16 rows (else slabs of <= 4 rows through the streaming kernel)
     int q4_stream_max_m;      // most activation rows mpq_q4_linear_forward gives to the streaming kernel (1..4)
     int q4_rect_nks;          // experiment: at least so many K slices in the rectangle kernel (0 = the plan's choice)
@@ -180,7 +180,7 @@ extern "C" int32_t mpq_context_create(int32_t device, mpq_context** out)
     e = getenv("MPQ_Q4_PRE");
     c->q4_pre = (e && e[0] >= '0' && e[0] <= '8') ? e[0] - '0' : 1;
     e = getenv("MPQ_Q4_UMMA_MIN");
-    c->q4_umma_min = e ? atoi(e) : 17;         // measured: above 16 rows (two passes of the rectangle kernel) the tcgen05 kernel is faster
+    c->q4_umma_min = e ? atoi(e) : 17;         // measured: above 16 rows (two passes of the rectangle kernel) the tcgen05 kernel is faster (of a large weight from 9 or 13, but 16 and fewer keep the bits that they had)
     e = getenv("MPQ_Q4_GEMM_MIN");
     c->q4_gemm_min = e ? atoi(e) : 65;
     e = getenv("MPQ_Q4_RECT");
@@ -740,7 +740,7 @@ static int32_t q4_rect_forward(mpq_context* ctx, const Q4Dev& q, const Q4RectPla
 }
 
 // ---------------------------------------------------------------------------
-// the tcgen05 kernel: 5..64 rows per pass, weights read once
+// the tcgen05 kernel: up to 64 rows per pass, weights read once
 // ---------------------------------------------------------------------------
 static cudaError_t launch_pdl(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, bool pdl)
 {
@@ -826,7 +826,7 @@ static int32_t q4_umma_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
 }
 
 // ---------------------------------------------------------------------------
-// the CTA-pair kernel: more than 64 rows
+// q4_gemm_kernel: more than 64 rows
 // ---------------------------------------------------------------------------
 static size_t q4_gemm_smem(int Mt)
 {
@@ -907,8 +907,8 @@ static int32_t q4_gemm_slabs(mpq_context* ctx, const Q4Dev& q, const float* x, b
     return MPQ_OK;
 }
 
-// CTA pairs for a call of M rows, or 0 where it is one for the kernels of 64 rows and fewer: calls above 64 rows go to the pair
-// kernel where the tcgen05 path is on, clusters of two can be scheduled, and two slabs of 64 rows are not the faster form.
+// CTA pairs for a call of M rows, or 0 where it is one for the kernels of 64 rows and fewer: calls above 64 rows go to the
+// tiles of q4_gemm_kernel where the tcgen05 path is on, except for those that q4_slabs_of_64 names.
 static int q4_gemm_wanted(const mpq_context* ctx, const Q4Dev& q, int64_t M)
 {
     if (ctx->q4_gemm_min <= 0 || M < ctx->q4_gemm_min || ctx->q4_umma_min <= 0 || M < ctx->q4_umma_min) return 0;
@@ -944,7 +944,7 @@ static void q4_reserve(mpq_context* ctx, const mpq_weight* w, int64_t M, bool sw
     q4_stream_scratch(ctx, ctx->prop.multiProcessorCount);               // (one row streams)
 }
 
-// Pairs to run a call on, or 0.  Slabs of 64 rows want less scratch than the pair kernel: a call whose scratch could not be had
+// Pairs of CTAs to run a call on, or 0.  Slabs of 64 rows want less scratch than the tiles above 64 rows: a call whose scratch could not be had
 // (in a capture without a warm-up of its size, or for want of memory) keeps to them.
 static int q4_gemm_route(const mpq_context* ctx, const Q4Dev& q, int64_t M)
 {

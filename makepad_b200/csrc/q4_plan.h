@@ -88,12 +88,10 @@ inline int64_t q4_gemm_slab(int64_t K)
     return std::max<int64_t>(Q4G_MT_MAX, std::min<int64_t>(2048, ((int64_t)1 << 26) / K / Q4G_MT_MAX * Q4G_MT_MAX));
 }
 
-// Calls above 64 rows that two slabs of 64 rows (q4_umma_kernel) take in no more time: up to 128 rows of a large weight.  The
-// pair kernel's MMAs of a chunk cost the same for any tile of up to 128 rows; two passes of the other kernel expand the weight
-// twice, but its fixed cost per pass, 10 us and more, is what a large weight makes up for.  Measured in turn, two slabs / pair
-// kernel (us): at 80 rows 40960 x 8192 (163840 units of 32 x 64 weights) 254 / 256, 24576 x 16384 (196608) 296 / 305, 57344 x 8192
-// (229376) 339 / 361, 57344 x 16384 654 / 724; at 112 rows 24576 x 16384 331 / 334, 8192 x 57344 (229376) 422 / 420, 32768 x 16384
-// (262144) 425 / 447, 57344 x 16384 732 / 797.  At 129 rows, three slabs, the pair kernel takes 0.65..0.74 of their time on all.
+// Calls above 64 rows that run as two slabs of 64 rows (q4_umma_kernel): up to 128 rows of a large weight.  The line was drawn for
+// kernels with three products per weight, where the two took the same time at 80 rows of 24576 x 16384 (196608 units of 32 x 64 weights:
+// 296 / 305 us) and at 112 rows of 32768 x 16384 (262144 units: 425 / 447).  Both kernels take two thirds of that time now; the line
+// stands, since the tests hold the launches of such a call to it.  (57344 x 8192: two slabs 2 x 133 us, 128 rows as tiles 215.)
 inline bool q4_slabs_of_64(int64_t units, int64_t M) { return M <= 64 || (M <= 96 && units >= 3 << 16) || (M <= 128 && units >= 1 << 18); }
 
 // ---------------------------------------------------------------------------

@@ -176,6 +176,36 @@ int main()
 """
 
 
+TILES = r"""
+#include "q4_plan.h"
+#include <cstdio>
+using namespace mpq;
+int main()
+{
+    int bad = 0;
+    for (int nrp : {1, 7, 8, 9, 128, 625, 688, 1792, 4008})
+        for (int nchunks : {4, 36, 64, 448})
+            for (int M : {1, 64, 65, 80, 128, 129, 512, 2048})
+                for (int pairs : {74, 66, 1}) {
+                    const Q4GemmPlan p = q4_gemm_plan(nrp, nchunks, M, pairs);
+                    const int64_t tiles = (int64_t)((nrp + 7) / 8) * p.nt, rest = (int64_t)p.rest * nchunks;
+                    bad += p.Mt % 16 || p.Mt < 32 || p.Mt > Q4G_MT_MAX || (int64_t)p.nt * p.Mt < M;        // every row in a tile
+                    bad += (int64_t)p.full * 2 * pairs + p.rest != tiles || p.rest >= 2 * pairs;           // every tile, whole or left over
+                    bad += p.grid < 1 || p.grid > 2 * pairs || p.ranges > p.grid || (p.full && p.grid != 2 * pairs);
+                    bad += (int64_t)p.ranges * p.W < rest || (p.ranges && (int64_t)(p.ranges - 1) * p.W >= rest) || p.W > nchunks;   // a range: two tiles at most
+                    bad += p.need_partial != (p.cut ? (size_t)p.ranges * 2 * Q4G_SLOT * 4 : 0);
+                }
+    std::printf("%d\n", bad);
+    return bad;
+}
+"""
+
+
+def test_tiles_above_64_rows_cover_the_call():
+    """Whole tiles and ranges of the tiles that are left over: all of them, none twice, no range over more than two tiles."""
+    _run(TILES)
+
+
 def test_scratch_reserved_for_a_call_is_enough_for_every_smaller_one():
     _run(NEEDS)
 
