@@ -28,6 +28,12 @@ def _np_ptr(a: np.ndarray):
     return C.c_void_p(a.ctypes.data)
 
 
+def _raw(h):
+    """The address in a handle, or None of one that was given up: ctypes converts an integer in a fraction of the time that a
+    c_void_p takes (and Tensor.new_empty allocates in a fraction of torch.empty's with dtype and device)."""
+    return None if h is None else h.value
+
+
 def _stream() -> int:
     """The current stream of the current device.  (The stream object that torch.cuda.current_stream() builds costs more host
     time than the launch itself.)"""
@@ -201,15 +207,18 @@ class QuantLinear:
                 return y
             if x.dtype != torch.float32 or not x.is_cuda or not x.is_contiguous():
                 raise MpqError(_lib.ERR_INVALID_ARG, "x must be a contiguous fp32 CUDA tensor")
-            x2 = x if x.dim() == 2 and x.shape[1] == w.K else x.reshape(-1, w.K)
-            y = torch.empty((x2.shape[0], w.N), dtype=torch.float32, device=x.device) if out is None else out
-            ctx.check(ctx.lib.mpq_q4_linear_forward(ctx.h, w.h, x2.data_ptr(), x2.shape[0], y.data_ptr(), _stream()))
+            shape = x.shape
+            if len(shape) != 2 or shape[1] != w.K:
+                x = x.reshape(-1, w.K)
+                shape = x.shape
+            M = shape[0]
+            y = x.new_empty(M, w.N) if out is None else out
+            ctx.check(ctx.lib.mpq_q4_linear_forward(_raw(ctx.h), _raw(w.h), x.data_ptr(), M, y.data_ptr(), _stream()))
             return y
         codes, sf, ts = x
         M = codes.shape[0]
-        y = torch.empty((M, w.N), dtype=torch.bfloat16, device=codes.device) if out is None else out
-        ctx.check(ctx.lib.mpq_nvfp4_gemm_forward(ctx.h, w.h, codes.data_ptr(), sf.data_ptr(),
-                                                 C.c_float(ts), M, y.data_ptr(), _stream()))
+        y = codes.new_empty((M, w.N), dtype=torch.bfloat16) if out is None else out
+        ctx.check(ctx.lib.mpq_nvfp4_gemm_forward(_raw(ctx.h), _raw(w.h), codes.data_ptr(), sf.data_ptr(), ts, M, y.data_ptr(), _stream()))
         return y
 
     __call__ = forward
@@ -224,8 +233,8 @@ class QuantLinear:
         if gate_up.dtype != torch.float32 or not gate_up.is_cuda or not gate_up.is_contiguous():
             raise MpqError(_lib.ERR_INVALID_ARG, "gate_up must be a contiguous fp32 CUDA tensor")
         g2 = gate_up if gate_up.dim() == 2 and gate_up.shape[1] == 2 * w.K else gate_up.reshape(-1, 2 * w.K)
-        y = torch.empty((g2.shape[0], w.N), dtype=torch.float32, device=gate_up.device) if out is None else out
-        ctx.check(ctx.lib.mpq_q4_linear_forward_swiglu(ctx.h, w.h, g2.data_ptr(), g2.shape[0], y.data_ptr(), _stream()))
+        y = g2.new_empty(g2.shape[0], w.N) if out is None else out
+        ctx.check(ctx.lib.mpq_q4_linear_forward_swiglu(_raw(ctx.h), _raw(w.h), g2.data_ptr(), g2.shape[0], y.data_ptr(), _stream()))
         return y
 
 
@@ -242,11 +251,12 @@ def nvfp4_quantize(ctx: Context, x, tensor_scale: float = 1.0, swiglu_fused: boo
     """fp32 or bf16 [M][K] on the GPU -> (codes u8 [M][K/2], sf u8 [M][K/16]) ready to be the GEMM's A.  With swiglu_fused
     the input is [M][2K] = [gate | up] and silu(gate) * up is what gets quantised."""
     import torch
-    M = x.shape[0]
-    K = x.shape[1] // 2 if swiglu_fused else x.shape[1]
-    codes = torch.empty((M, K // 2), dtype=torch.uint8, device=x.device)
-    sf = torch.empty((M, K // 16), dtype=torch.uint8, device=x.device)
+    M, K = x.shape[0], x.shape[1]
+    if swiglu_fused:
+        K //= 2
+    codes = x.new_empty((M, K // 2), dtype=torch.uint8)
+    sf = x.new_empty((M, K // 16), dtype=torch.uint8)
     fn = ctx.lib.mpq_nvfp4_quantize_swiglu if swiglu_fused else ctx.lib.mpq_nvfp4_quantize_activations
-    ctx.check(fn(ctx.h, x.data_ptr(), 1 if x.dtype == torch.bfloat16 else 0, M, K, C.c_float(tensor_scale),
+    ctx.check(fn(_raw(ctx.h), x.data_ptr(), 1 if x.dtype == torch.bfloat16 else 0, M, K, tensor_scale,
                  codes.data_ptr(), sf.data_ptr(), _stream()))
     return codes, sf
