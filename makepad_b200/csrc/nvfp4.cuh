@@ -49,8 +49,6 @@ void nvfp4_weight_dequant_launch(const Nvfp4Dev& w, float* out, cudaStream_t s);
 int32_t nvfp4_gemm_launch(Nvfp4Scratch& scratch, const Nvfp4Dev& w, const uint8_t* a_codes, const uint8_t* a_sf, float ta,
                           int64_t M, uint16_t* c, int device, int sm_count, bool pdl, cudaStream_t s, int* launches, std::string& err);
 
-// TMA map of an array of 128-byte rows, box = box_rows of them, dense (false: the driver's encoder is missing or refuses)
-bool make_rows128_map(CUtensorMap* map, const void* base, int64_t rows, int box_rows);
 // TMA map of a Q4 tile stream (see Q4Dev::map)
 bool make_q4_stream_map(CUtensorMap* map, const void* stream, int nrp, int nchunks);
 

@@ -1228,18 +1228,6 @@ static bool make_c_map(CUtensorMap* map, void* base, int64_t M, int64_t N, int b
               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-bool make_rows128_map(CUtensorMap* map, const void* base, int64_t rows, int box_rows)
-{
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return false;
-    cuuint64_t dims[2] = {128u, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {128u};
-    cuuint32_t box[2] = {128u, (cuuint32_t)box_rows};
-    cuuint32_t estr[2] = {1u, 1u};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 bool make_q4_stream_map(CUtensorMap* map, const void* stream, int nrp, int nchunks)
 {
     EncodeTiledFn fn = encode_fn();
