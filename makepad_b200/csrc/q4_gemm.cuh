@@ -202,6 +202,7 @@ __global__ void __launch_bounds__(Q4G_THREADS, 1) q4_gemm_kernel(const __grid_co
             const int count = Q4GWalk(p).left;
             int xs = 0, slot = 0, fail = 0;
             uint32_t xph = 0, dph = 1;                   // (the first round of empty slots passes on the parity before the first)
+            asm volatile("griddepcontrol.wait;" ::: "memory");     // the polls below are for this kernel's own copies, not for the kernels before
             for (int i = 0; i < count && !fail; ++i) {
                 const uint64_t bhi = q4u_desc_sw128(xring + xs * xstage_bytes), blo = bhi + (uint64_t)(p.Mt * 8);
 #pragma unroll
@@ -268,6 +269,7 @@ __global__ void __launch_bounds__(Q4G_THREADS, 1) q4_gemm_kernel(const __grid_co
                 else fail = 46;
             }
         } else fail = 46;
+        asm volatile("griddepcontrol.wait;" ::: "memory");              // (as in q4_umma_kernel)
         while (w.left && !fail) {
             int piece = w.rest_left ? min(w.rest_left, p.nchunks - w.c) : p.nchunks;          // chunks of this piece
             const int behind = w.left - piece;
@@ -298,7 +300,6 @@ __global__ void __launch_bounds__(Q4G_THREADS, 1) q4_gemm_kernel(const __grid_co
             } while (piece);
             if (fail) break;
             // the piece's sums: to y when this range holds the whole tile, else to the range's slot
-            asm volatile("griddepcontrol.wait;" ::: "memory");          // inv_sc, and y and the slots may still be read
             const int b = w.tile / p.nt, col = g * 128 + qd * 32 + lane, nrow = b * 256 + col;
             const int at = w.tile != p.full * (int)gridDim.x + q4u_div((int64_t)blockIdx.x * p.W, p.nchunks);
             float* slot_out = p.partial + ((size_t)blockIdx.x * 2 + at) * Q4G_SLOT + col;

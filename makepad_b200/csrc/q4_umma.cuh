@@ -478,6 +478,7 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_umma_kernel(const __grid_co
             // what this lane looks at before a step: the team's A operand, the accumulator slot, the activations
             auto bar = [&](int tm) { return what == 0 ? a_full + 8 * tm : what == 1 ? d_empty + 8 * slot : x_full + 8 * xs; };
             auto parity = [&]() { return what == 0 ? aph : what == 1 ? dph : xph; };
+            asm volatile("griddepcontrol.wait;" ::: "memory");     // the polls below are for this kernel's own copies, not for the kernels before
             for (int i = 0; i < range && !fail; ++i) {
                 const uint64_t bhi = q4u_desc_sw128(xring + xs * xstage_bytes), blo = bhi + (uint64_t)(p.Mp * 8);     // rows [0, Mp) = xhi, [Mp, 2 Mp) = xlo
 #pragma unroll
@@ -544,7 +545,10 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_umma_kernel(const __grid_co
             if (++ws == WST) { ws = 0; wph ^= 1u; }
             return true;
         };
-        if (!expand()) fail = 36;
+        if (!expand()) fail = 36;                                       // (needs nothing of the kernels before)
+        // Here, and in the issuing warp, so that a slow kernel in front is not counted against the bounds of the waits for sums; inv_sc
+        // comes from it too, and y and the slices may still be read.
+        asm volatile("griddepcontrol.wait;" ::: "memory");
         while (left > 0 && !fail) {
             const int after = max(0, left - (p.nchunks - c));           // chunks left behind this piece
             do {
@@ -564,9 +568,8 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_umma_kernel(const __grid_co
             } while (left > after);
             if (fail) break;
             // ---- the piece's sums: to y when this range holds the whole batch, else to the piece's slice
-            // inv_sc comes from the kernel before this one.  Lane l keeps rows l and l + 32 of it: read inside the store loop
-            // the loads would be ordered behind the stores (they may alias for all the compiler knows), one round trip per row.
-            asm volatile("griddepcontrol.wait;" ::: "memory");
+            // Lane l keeps rows l and l + 32 of inv_sc: read inside the store loop the loads would be ordered behind the stores
+            // (they may alias for all the compiler knows), one round trip per row.
             const float isc0 = lane < p.M ? p.inv_sc[lane] : 0.f, isc1 = lane + 32 < p.M ? p.inv_sc[lane + 32] : 0.f;
             int pf, pl;
             q4u_pieces(b, p.nchunks, p.W, &pf, &pl);

@@ -318,3 +318,15 @@ def test_every_kernel_that_can_give_up_a_wait_settles_before_it_ends():
             end = body[:body.index("tcgen05.dealloc")]
             assert "settle_after_timeout(s_abort);" in end[end.rindex("__syncthreads();"):], f
     assert kernels == 4
+
+
+def test_waits_for_staged_rows_begin_behind_the_kernels_before():
+    """In the Q4 tcgen05 kernels the issuing warp and the workers wait for the kernels before (griddepcontrol.wait) ahead of their first
+    bounded wait for what depends on the staged activations."""
+    for f in ("q4_umma.cuh", "q4_gemm.cuh"):
+        text = open(os.path.join(ROOT, "makepad_b200", "csrc", f)).read()
+        issue = text[text.index("// ---------------- MMA issue"):]
+        assert "griddepcontrol.wait" in issue[:issue.index("q4u_bar_poll<0>(")], f
+        work = text[text.index("// ---------------- expansion + drain"):]
+        first = work.index("df, dph)" if f == "q4_umma.cuh" else "q4u_bar_wait(df + 8, dph)")
+        assert "griddepcontrol.wait" in work[:first], f

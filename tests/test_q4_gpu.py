@@ -599,3 +599,46 @@ def test_weights_larger_than_the_upload_staging(ctx, N, K, mode, rank, world):
     assert got.shape == want.shape and torch.equal(got.view(torch.int32), want.view(torch.int32))
     ctx.lib.mpq_weight_destroy(h)
     w.destroy()
+
+
+# Lets the next kernel in the stream start at once, then takes `ms` milliseconds (and ends in any case after 2^26 looks at the clock).
+SLOW_KERNEL = r"""
+extern "C" __global__ void slow_kernel(long long ms)
+{
+    asm volatile("griddepcontrol.launch_dependents;");
+    unsigned long long t0, t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+    for (int i = 0; i < (1 << 26); ++i) {
+        __nanosleep(1000);
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+        if (t - t0 > (unsigned long long)ms * 1000000ull) break;
+    }
+}
+"""
+
+
+# rows, fewest rows of the tcgen05 path: staging of fewer CTAs than SMs (16, 80, 128: the kernel behind it starts on the others), and of more
+@pytest.mark.parametrize("M,umma_min", [(16, 9), (40, 17), (80, 17), (128, 17), (300, 17)])
+def test_waits_do_not_run_out_while_earlier_kernels_are_slow(orc, monkeypatch, M, umma_min):
+    """Staging and tcgen05 kernel start beside a kernel that triggers its dependents at once and then takes a second: their bounded
+    waits for what the staging writes begin when that has ended, and the call gives the bits of an undisturbed one."""
+    import makepad_b200
+    torch = _torch()
+    monkeypatch.setenv("MPQ_Q4_UMMA_MIN", str(umma_min))
+    c2 = makepad_b200.Context(0)
+    N, K = 520, 1120
+    codes, scales = synth.q4_weight(N, K, seed=91)
+    lin = makepad_b200.QuantLinear(makepad_b200.Q4Weight(c2, codes, scales))
+    x = synth.activations(M, K, seed=92)
+    xd = torch.from_numpy(x).cuda()
+    slow = torch.cuda._compile_kernel(SLOW_KERNEL, "slow_kernel")
+    want = lin(xd)
+    torch.cuda.synchronize()
+    assert orc.err_report(want.cpu().numpy(), orc.q4_matmul_f64(codes, scales, x))["max_abs_over_rms"] < 2e-5
+    y = torch.full_like(want, float("nan"))
+    slow(grid=(1, 1, 1), block=(32, 1, 1), args=(1000,))
+    lin.forward(xd, out=y)
+    torch.cuda.synchronize()
+    assert c2.lib.mpq_context_poll_status(c2.h) == _lib.OK
+    assert torch.equal(y, want)
+    c2.close()
