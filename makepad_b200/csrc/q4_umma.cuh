@@ -171,6 +171,8 @@ __device__ __forceinline__ uint32_t q4u_bar_test(uint32_t bar, uint32_t parity)
 }
 // Bounded wait of a converged warp on a phase parity, or on one per lane: false when the limit ran out.  try_wait suspends the threads for a
 // hardware-chosen time per try.  The vote makes the outcome uniform for the compiler: what the loops around it count stays in uniform registers.
+// A vote orders no memory: behind it only the lane that looked at a barrier may read what that barrier hands over.  __syncwarp does order
+// it, so that after this wait, and after the look below, every lane may read what any of them waited for.
 __device__ __forceinline__ bool q4u_bar_wait(uint32_t bar, uint32_t parity)
 {
     uint32_t all;
@@ -180,6 +182,7 @@ __device__ __forceinline__ bool q4u_bar_wait(uint32_t bar, uint32_t parity)
                  "add.u32 n, n, 1;\n\tsetp.lt.u32 p, n, %3;\n\t@p bra.uni TRY;\n"
                  "DONE:\n\t}"
                  : "=r"(all) : "r"(bar), "r"(parity), "n"(Q4U_SPIN) : "memory");
+    __syncwarp();
     return all == 0xFFFFFFFFu;
 }
 // ... by a thread for itself (the ones above and below are for whole warps: a lane alone would wait in the vote for good)
@@ -189,12 +192,19 @@ __device__ __forceinline__ bool q4u_bar_wait_lane(uint32_t bar, uint32_t parity)
         if (q4u_bar_test(bar, parity)) return true;
     return false;
 }
+// one look of a converged warp, a barrier per lane
+__device__ __forceinline__ bool q4u_bar_look(uint32_t bar, uint32_t parity, bool mine = true)
+{
+    const bool all = __all_sync(0xFFFFFFFFu, !mine || q4u_bar_test(bar, parity));
+    __syncwarp();
+    return all;
+}
 // ... with a look at a time, and SLEEP ns between two of them; the barriers of lanes without `mine` are not looked at
 template <int SLEEP>
 __device__ __forceinline__ bool q4u_bar_poll(uint32_t bar, uint32_t parity, bool mine = true)
 {
     for (uint32_t n = 0; n < Q4U_SPIN; ++n) {
-        if (__all_sync(0xFFFFFFFFu, !mine || q4u_bar_test(bar, parity))) return true;
+        if (q4u_bar_look(bar, parity, mine)) return true;
         if (SLEEP) __nanosleep(SLEEP);
     }
     return false;
@@ -501,7 +511,7 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_umma_kernel(const __grid_co
                         aph ^= 1u;
                         if (++xs == Q4U_XSTAGES) { xs = 0; xph ^= 1u; }
                     }
-                    ready = __all_sync(0xFFFFFFFFu, q4u_bar_test(bar((tm + 1) % Q4U_TEAMS), parity()));
+                    ready = q4u_bar_look(bar((tm + 1) % Q4U_TEAMS), parity());
                     if (q4u_elect_one()) {
                         issue(1);
                         if (tm == Q4U_TEAMS - 1) q4u_commit(xe);               // ... and the activation stage is free

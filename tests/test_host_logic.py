@@ -330,3 +330,19 @@ def test_waits_for_staged_rows_begin_behind_the_kernels_before():
         work = text[text.index("// ---------------- expansion + drain"):]
         first = work.index("df, dph)" if f == "q4_umma.cuh" else "q4u_bar_wait(df + 8, dph)")
         assert "griddepcontrol.wait" in work[:first], f
+
+
+def test_waits_of_a_warp_on_several_barriers_order_memory():
+    """A vote over the lanes' barriers orders no memory: where lanes look at different ones, a __syncwarp stands between the vote and
+    whatever reads what was waited for, and no kernel votes on barriers in any other way."""
+    csrc = os.path.join(ROOT, "makepad_b200", "csrc")
+    text = open(os.path.join(csrc, "q4_umma.cuh")).read()
+    for name in ("bool q4u_bar_wait(", "bool q4u_bar_look("):
+        body = text[text.index(name):]
+        body = body[:body.index("\n}")]
+        vote = max(body.rfind("vote.sync"), body.rfind("_sync("))
+        assert "__syncwarp();" in body[vote:] and "return" not in body[vote:body.index("__syncwarp();")], name
+    poll = text[text.index("bool q4u_bar_poll("):]
+    assert "q4u_bar_look(" in poll[:poll.index("\n}")]
+    votes = [m for f in ("q4_umma.cuh", "q4_gemm.cuh") for m in re.findall(r"_sync\([^;]*q4u_bar_test", open(os.path.join(csrc, f)).read())]
+    assert len(votes) == 1, votes                                      # the one of q4u_bar_look
