@@ -59,7 +59,9 @@ constexpr int Q4U_WSTAGE_BYTES = 5 * 1024;    // (the swizzle wants stages of wh
 constexpr int Q4U_XSTAGES = 4;                // activation ring: stages of one chunk (hi tile + lo tile)
 constexpr int Q4U_DSLOTS = 3, Q4U_D_COLS = 128;      // accumulators: columns [0, 384), slots of two 32-blocks that are used in turn
 constexpr int Q4U_A_COL = 384;                // A operand: [384, 512), a chunk per team (a second one up to 32 rows, in place of accumulators, was 10% slower)
-constexpr uint32_t Q4U_SPIN = 1u << 22;       // tries of one mbarrier before giving up
+// Looks at one mbarrier before giving up: 2^22 of 90 cycles, and 2^17 tries of 4 us (measured, of one that fails), 0.2..0.5 s either way: when a
+// role has given up, the others follow soon.  All that is waited for is this kernel's own work of microseconds.
+constexpr uint32_t Q4U_SPIN = 1u << 22, Q4U_TRIES = 1u << 17;
 
 struct Q4ULaunch {
     const unsigned char* XS;      // staged activations: per chunk [hi: Mp rows x 128 B | lo: Mp rows x 128 B], 128-byte swizzle
@@ -169,8 +171,8 @@ __device__ __forceinline__ uint32_t q4u_bar_test(uint32_t bar, uint32_t parity)
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok;
 }
-// Bounded wait of a converged warp on a phase parity, or on one per lane: false when the limit ran out.  try_wait suspends the threads for a
-// hardware-chosen time per try.  The vote makes the outcome uniform for the compiler: what the loops around it count stays in uniform registers.
+// Bounded wait of a converged warp on a phase parity, or on one per lane: false when the limit ran out.  try_wait suspends the threads, for
+// 4 us if it fails.  The vote makes the outcome uniform for the compiler: what the loops around it count stays in uniform registers.
 // A vote orders no memory: behind it only the lane that looked at a barrier may read what that barrier hands over.  __syncwarp does order
 // it, so that after this wait, and after the look below, every lane may read what any of them waited for.
 __device__ __forceinline__ bool q4u_bar_wait(uint32_t bar, uint32_t parity)
@@ -181,7 +183,7 @@ __device__ __forceinline__ bool q4u_bar_wait(uint32_t bar, uint32_t parity)
                  "setp.eq.u32 p, %0, 0xffffffff;\n\t@p bra.uni DONE;\n\t"
                  "add.u32 n, n, 1;\n\tsetp.lt.u32 p, n, %3;\n\t@p bra.uni TRY;\n"
                  "DONE:\n\t}"
-                 : "=r"(all) : "r"(bar), "r"(parity), "n"(Q4U_SPIN) : "memory");
+                 : "=r"(all) : "r"(bar), "r"(parity), "n"(Q4U_TRIES) : "memory");
     __syncwarp();
     return all == 0xFFFFFFFFu;
 }

@@ -642,3 +642,35 @@ def test_waits_do_not_run_out_while_earlier_kernels_are_slow(orc, monkeypatch, M
     assert c2.lib.mpq_context_poll_status(c2.h) == _lib.OK
     assert torch.equal(y, want)
     c2.close()
+
+
+def test_a_wait_that_runs_out_takes_less_than_a_second():
+    """The bounded wait of the tcgen05 kernels' workers: on a barrier that nothing completes it gives up, soon enough that a kernel one of
+    whose roles gave up does not hold the GPU; on a completed one it succeeds."""
+    torch = _torch()
+    text = open(os.path.join(os.path.dirname(_lib.__file__), "csrc", "q4_umma.cuh")).read()
+    helpers = text[text.index("__device__ __forceinline__ void q4u_bar_init("):text.index("// lane 0 of a converged warp arrives")]
+    limits = text[text.index("constexpr uint32_t Q4U_SPIN"):].split("\n")[0]
+    kernel = torch.cuda._compile_kernel("typedef unsigned int uint32_t;\n" + limits + "\n" + helpers + r"""
+extern "C" __global__ void run_out_kernel(long long* out)
+{
+    __shared__ __align__(8) unsigned long long bars[2];
+    const uint32_t bar = (uint32_t)__cvta_generic_to_shared(bars);
+    if (threadIdx.x == 0) {
+        q4u_bar_init(bar, 1);
+        q4u_bar_init(bar + 8, 1);
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar + 8) : "memory");
+    }
+    __syncthreads();
+    unsigned long long t0, t1;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+    const bool done = q4u_bar_wait(bar + 8, 0), never = q4u_bar_wait(bar, 0);
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
+    if (threadIdx.x == 0) { out[0] = done; out[1] = never; out[2] = (long long)(t1 - t0); }
+}
+""", "run_out_kernel")
+    out = torch.full((3,), -1, dtype=torch.int64, device="cuda")
+    kernel(grid=(1, 1, 1), block=(32, 1, 1), args=(out,))
+    done, never, ns = out.tolist()
+    assert done == 1 and never == 0
+    assert 1e7 < ns < 1e9, ns
