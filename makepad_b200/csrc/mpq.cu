@@ -763,7 +763,6 @@ static int32_t q4_umma_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
     float* inv_sc = reinterpret_cast<float*>(xs + q4_umma_xs_bytes(q.nchunks, M));
     // by the number of 16-row slices; accumulators of 2 Mp columns where they fit in 64
     static void (*const kernels[4])(const CUtensorMap, const Q4ULaunch) = {q4_umma_kernel<1, true>, q4_umma_kernel<2, true>, q4_umma_kernel<3, false>, q4_umma_kernel<4, false>};
-    if (!q.mapped) return fail(ctx, MPQ_ERR_CUDA, "cuTensorMapEncodeTiled failed for the weight");
     const Q4UmmaPlan pl = q4_umma_plan(q.nrp, q.nchunks, sms);
     const int W = pl.W;
     CU_TRY(ctx, ctx->q4_partial.reserve(q4_umma_need_partial(pl.pieces, M, q.N)));
@@ -844,7 +843,6 @@ static int32_t q4_gemm_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
     if (st) return st;
     const Q4GemmPlan pl = q4_gemm_plan(q.nrp, q.nchunks, M, pairs_max);
     const int nt = pl.nt, Mt = pl.Mt;
-    if (!q.mapped) return fail(ctx, MPQ_ERR_CUDA, "cuTensorMapEncodeTiled failed for the weight");
     CU_TRY(ctx, ctx->q4u_xs.reserve(pl.need_xs));
     CU_TRY(ctx, ctx->q4_partial.reserve(pl.need_partial));
     unsigned char* xs = ctx->q4u_xs.as<unsigned char>();
@@ -907,13 +905,12 @@ static int32_t q4_gemm_slabs(mpq_context* ctx, const Q4Dev& q, const float* x, b
     return MPQ_OK;
 }
 
-// CTA pairs for a call of M rows, or 0 where it is one for the kernels of 64 rows and fewer: calls above 64 rows go to the
-// tiles of q4_gemm_kernel where the tcgen05 path is on, except for those that q4_slabs_of_64 names.
+static Q4Route q4_route(const mpq_context* ctx, const Q4Dev& q, int64_t M) { return q4_route(q.units(), M, ctx->q4_umma_min, ctx->q4_gemm_min, q.mapped); }
+
+// CTA pairs for a call of M rows, or 0 where it is one for the kernels of 64 rows and fewer
 static int q4_gemm_wanted(const mpq_context* ctx, const Q4Dev& q, int64_t M)
 {
-    if (ctx->q4_gemm_min <= 0 || M < ctx->q4_gemm_min || ctx->q4_umma_min <= 0 || M < ctx->q4_umma_min) return 0;
-    if (M > 64 && q4_slabs_of_64(q.units(), M)) return 0;
-    return q4_gemm_pairs(ctx);
+    return q4_route(ctx, q, M) == Q4Route::Tiles ? q4_gemm_pairs(ctx) : 0;
 }
 
 // true when the stream must not see an allocation now
@@ -933,9 +930,10 @@ static bool stream_captures(cudaStream_t s)
 static void q4_reserve(mpq_context* ctx, const mpq_weight* w, int64_t M, bool swiglu, cudaStream_t s)
 {
     const Q4Dev& q = w->q4;
-    const Q4Needs need = q4_needs(q.N, q.K, q.nrp, q.nchunks, M, w->q4_rect_partial, w->q4_umma_pieces, ctx->q4_umma_min, ctx->q4_gemm_min,
+    const int umma_min = q4_umma_from(ctx->q4_umma_min, q.mapped);
+    const Q4Needs need = q4_needs(q.N, q.K, q.nrp, q.nchunks, M, w->q4_rect_partial, w->q4_umma_pieces, umma_min, ctx->q4_gemm_min,
                                   q4_gemm_wanted(ctx, q, M));
-    const size_t hidden = swiglu ? (size_t)(ctx->q4_umma_min > 0 ? std::min<int64_t>(M, ctx->q4_umma_min - 1) : M) * q.K * sizeof(float) : 0;
+    const size_t hidden = swiglu ? (size_t)(umma_min > 0 ? std::min<int64_t>(M, umma_min - 1) : M) * q.K * sizeof(float) : 0;
     if (ctx->q4u_xs.bytes() >= need.xs && ctx->q4_partial.bytes() >= need.partial && ctx->swiglu_buf.bytes() >= hidden && ctx->q4_partials_ctas) return;
     if (stream_captures(s)) return;
     ctx->q4u_xs.reserve(need.xs);
@@ -1038,9 +1036,7 @@ static int32_t q4_forward_checked(mpq_context* ctx, const mpq_weight* w, const f
 {
     if (M > 4 || !q4_prefers_stream(ctx, w->q4, M)) q4_reserve(ctx, w, M, false, s);
     if (const int pairs = q4_gemm_route(ctx, w->q4, M)) return q4_gemm_slabs(ctx, w->q4, x_dev, false, M, y_dev, ldy, pairs, s);
-    if (ctx->q4_umma_min > 0 && M >= ctx->q4_umma_min) {       // slabs of up to 64 rows on the tcgen05 path
-        return q4_umma_slabs(ctx, w->q4, x_dev, false, M, y_dev, ldy, s);
-    }
+    if (q4_route(ctx, w->q4, M) != Q4Route::Slabs16) return q4_umma_slabs(ctx, w->q4, x_dev, false, M, y_dev, ldy, s);
     const int slab = q4_slab_rows(ctx, w->q4, M);
     for (int64_t m0 = 0; m0 < M; m0 += slab) {
         int m = (int)std::min<int64_t>(slab, M - m0);
@@ -1132,7 +1128,7 @@ extern "C" int32_t mpq_q4_linear_forward_swiglu(mpq_context* ctx, const mpq_weig
     }
     q4_reserve(ctx, w, M, true, s);
     if (const int pairs = q4_gemm_route(ctx, q, M)) return q4_gemm_slabs(ctx, q, gate_up_dev, true, M, y_dev, q.N, pairs, s);
-    if (ctx->q4_umma_min > 0 && M >= ctx->q4_umma_min) return q4_umma_slabs(ctx, q, gate_up_dev, true, M, y_dev, q.N, s);
+    if (q4_route(ctx, q, M) != Q4Route::Slabs16) return q4_umma_slabs(ctx, q, gate_up_dev, true, M, y_dev, q.N, s);
     CU_TRY(ctx, ctx->swiglu_buf.reserve((size_t)M * q.K * sizeof(float)));
     float* hidden = ctx->swiglu_buf.as<float>();
     if ((st = swiglu_launch(ctx, gate_up_dev, M, q.K, hidden, s))) return st;

@@ -94,6 +94,19 @@ inline int64_t q4_gemm_slab(int64_t K)
 // stands, since the tests hold the launches of such a call to it.  (57344 x 8192: two slabs 2 x 133 us, 128 rows as tiles 215.)
 inline bool q4_slabs_of_64(int64_t units, int64_t M) { return M <= 64 || (M <= 96 && units >= 3 << 16) || (M <= 128 && units >= 1 << 18); }
 
+// Where a call of M rows goes: slabs of 16 rows and fewer through the other kernels, or the tcgen05 kernels in slabs of 64 rows or as tiles.
+// umma_min, gemm_min: fewest rows of q4_umma_kernel and of q4_gemm_kernel (0: never).  Both fetch the weights through a tensor map; a
+// weight for which the driver has made none (mapped = false) stays with the kernels that need none.
+enum class Q4Route { Slabs16, Slabs64, Tiles };
+inline int q4_umma_from(int umma_min, bool mapped) { return mapped ? umma_min : 0; }
+inline Q4Route q4_route(int64_t units, int64_t M, int umma_min, int gemm_min, bool mapped)
+{
+    const int from = q4_umma_from(umma_min, mapped);
+    if (from <= 0 || M < from) return Q4Route::Slabs16;
+    if (gemm_min <= 0 || M < gemm_min || (M > 64 && q4_slabs_of_64(units, M))) return Q4Route::Slabs64;
+    return Q4Route::Tiles;
+}
+
 // ---------------------------------------------------------------------------
 // scratch for every call of 2 .. M rows
 // ---------------------------------------------------------------------------

@@ -346,3 +346,34 @@ def test_waits_of_a_warp_on_several_barriers_order_memory():
     assert "q4u_bar_look(" in poll[:poll.index("\n}")]
     votes = [m for f in ("q4_umma.cuh", "q4_gemm.cuh") for m in re.findall(r"_sync\([^;]*q4u_bar_test", open(os.path.join(csrc, f)).read())]
     assert len(votes) == 1, votes                                      # the one of q4u_bar_look
+
+
+ROUTES = r"""
+#include "q4_plan.h"
+#include <cstdio>
+using namespace mpq;
+int main()
+{
+    int bad = 0;
+    for (int64_t units : {1, 196608, 262144})
+        for (int64_t M = 1; M <= 2100; ++M) {
+            bad += q4_route(units, M, 17, 65, false) != Q4Route::Slabs16;                              // no tensor map: every call still has a kernel
+            bad += q4_route(units, M, 0, 65, true) != Q4Route::Slabs16;
+            bad += q4_route(units, M, 17, 65, true) != (M < 17 ? Q4Route::Slabs16 : q4_slabs_of_64(units, M) ? Q4Route::Slabs64 : Q4Route::Tiles);
+            bad += q4_route(units, M, 17, 0, true) != (M < 17 ? Q4Route::Slabs16 : Q4Route::Slabs64);
+        }
+    // ... and no scratch of kernels that it does not reach
+    bad += q4_needs(4096, 4096, 128, 64, 300, 77, 2, q4_umma_from(17, false), 65, 0).xs != 0;
+    std::printf("%d\n", bad);
+    return bad;
+}
+"""
+
+
+def test_a_weight_without_a_tensor_map_is_not_refused():
+    """The tcgen05 kernels read weights through a tensor map of the driver's; where it made none, calls of 17 rows and more run as slabs of
+    16 rows (as with MPQ_Q4_UMMA_MIN=0), and no call returns an error for the map's sake."""
+    _run(ROUTES)
+    text = open(os.path.join(ROOT, "makepad_b200", "csrc", "mpq.cu")).read()
+    assert not re.search(r"!q\.mapped\) return fail", text)
+    assert not re.search(r"ctx->q4_umma_min (>|<|>=|<=) ", text)          # routes go through q4_route, which knows of the map

@@ -674,3 +674,23 @@ extern "C" __global__ void run_out_kernel(long long* out)
     done, never, ns = out.tolist()
     assert done == 1 and never == 0
     assert 1e7 < ns < 1e9, ns
+
+
+@pytest.mark.parametrize("M", [17, 150])
+def test_rows_above_16_without_the_tcgen05_kernels(orc, monkeypatch, M):
+    """The form that a call takes where the tcgen05 kernels are off, or their tensor map could not be made: slabs of 16 rows."""
+    import makepad_b200
+    torch = _torch()
+    monkeypatch.setenv("MPQ_Q4_UMMA_MIN", "0")
+    c2 = makepad_b200.Context(0)
+    N, K = 257, 1120
+    codes, scales = synth.q4_weight(N, K, seed=95)
+    lin = makepad_b200.QuantLinear(makepad_b200.Q4Weight(c2, codes, scales))
+    x = synth.activations(M, K, seed=96)
+    rep = orc.err_report(lin(torch.from_numpy(x).cuda()).cpu().numpy(), orc.q4_matmul_f64(codes, scales, x))
+    assert rep["floored_1e-2_rms"] < TOL and rep["max_abs_over_rms"] < 2e-5, rep
+    gate_up = torch.from_numpy(synth.activations(M, 2 * K, seed=97)).cuda()
+    assert torch.equal(lin.forward_swiglu(gate_up), lin(makepad_b200.swiglu(c2, gate_up)))
+    torch.cuda.synchronize()
+    assert c2.lib.mpq_context_poll_status(c2.h) == _lib.OK
+    c2.close()
