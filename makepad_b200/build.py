@@ -1,7 +1,7 @@
 """Builds libmpq.so in-tree with nvcc for sm_100a (cross-compiles without a GPU).
 
 `python -m makepad_b200.build [-v] [--trace]`; --trace builds the diagnostic variant libmpq_trace.so
-(-DMPQ_TRACE: the Q4 streaming kernel stamps its phases, see makepad_b200/timeline.py).
+(-DMPQ_TRACE: the Q4 streaming and tcgen05 kernels stamp their phases, see makepad_b200/timeline.py).
 """
 from __future__ import annotations
 

@@ -562,6 +562,8 @@ static unsigned long long* trace_buffer()
     }
     return g_trace;
 }
+// the next launch's slot, for grids that fit one
+static unsigned long long* trace_slot(int grid) { return trace_buffer() && grid <= 1024 ? g_trace + (size_t)(g_trace_n++ % 64) * 1024 * 16 : nullptr; }
 // Waits for the device and returns a host copy of the array (valid until the next call).
 extern "C" unsigned long long* mpq_debug_trace(int32_t* launches)
 {
@@ -579,7 +581,7 @@ static int32_t q4_stream_enqueue(mpq_context* ctx, const Q4StreamPlan& pl, const
 {
 #ifdef MPQ_TRACE
     Q4StreamLaunch p = p_in;
-    p.trace = (trace_buffer() && grid <= 1024) ? g_trace + (size_t)(g_trace_n++ % 64) * 1024 * 16 : nullptr;
+    p.trace = trace_slot(grid);
 #else
     const Q4StreamLaunch& p = p_in;
 #endif
@@ -791,6 +793,9 @@ static int32_t q4_umma_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
     p.XS = xs; p.inv_sc = inv_sc; p.Y = y; p.partial = partial;
     p.M = M; p.Mp = Mp; p.N = (int)q.N; p.ldy = ldy; p.nchunks = q.nchunks;
     p.nbatches = pl.nbatches; p.W = W; p.status = ctx->q4_status;
+#ifdef MPQ_TRACE
+    p.trace = trace_slot(pl.grid);
+#endif
     // shared memory: activation ring, the teams' weight rings as deep as the rest allows, barriers (+ 1 KiB for the alignment)
     const size_t smem_max = (size_t)ctx->prop.sharedMemPerBlockOptin - 256, xring_bytes = (size_t)Q4U_XSTAGES * 2 * Mp * 128;
     p.wstages = (int)std::min<size_t>(Q4U_MAX_WSTAGES, (smem_max - xring_bytes - 2048) / ((size_t)Q4U_TEAMS * Q4U_WSTAGE_BYTES));
@@ -872,6 +877,9 @@ static int32_t q4_gemm_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
     p.XS = xs; p.inv_sc = inv_sc; p.Y = y; p.partial = partial;
     p.M = M; p.Mt = Mt; p.N = (int)q.N; p.nt = nt; p.ldy = ldy; p.nchunks = q.nchunks; p.full = pl.full; p.rest = pl.rest; p.W = pl.W;
     p.status = ctx->q4_status;
+#ifdef MPQ_TRACE
+    p.trace = trace_slot(pl.grid);
+#endif
     cfg = {};
     cfg.gridDim = dim3((unsigned)pl.grid);
     cfg.blockDim = dim3(Q4G_THREADS);

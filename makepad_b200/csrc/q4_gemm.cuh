@@ -35,6 +35,9 @@ struct Q4GemmLaunch {
     int nchunks;
     int full, rest, W;            // whole tiles per CTA; tiles that are left over, cut into ranges of W chunks, one per CTA
     int* status;
+#ifdef MPQ_TRACE
+    unsigned long long* trace;    // as in Q4ULaunch
+#endif
 };
 
 // Rows -> hi/lo tiles of Mt rows x 128 bytes, [tile][chunk][hi | lo], swizzled as the MMA's descriptor wants; one row per
@@ -142,6 +145,7 @@ __global__ void __launch_bounds__(Q4G_THREADS, 1) q4_gemm_kernel(const __grid_co
                    a_full = x_empty + 8 * Q4G_XSTAGES, d_full = a_full + 16 * Q4G_GROUPS,
                    d_empty = d_full + 16 * Q4G_GROUPS;   // a_full: [group][chunk % 2]; d_full: [group][half]
     const int warp = __shfl_sync(0xFFFFFFFFu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    Q4U_TRACE(0, threadIdx.x == 0)
 
     if (threadIdx.x == 0) {
         s_abort = 0;
@@ -160,6 +164,7 @@ __global__ void __launch_bounds__(Q4G_THREADS, 1) q4_gemm_kernel(const __grid_co
     __syncthreads();
     q4u_fence_after();
     const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, s_tmem_base, 0);
+    Q4U_TRACE(1, threadIdx.x == 0)
     asm volatile("griddepcontrol.launch_dependents;");
 
     if (warp >= Q4G_WARP_ISSUE) {
@@ -189,6 +194,7 @@ __global__ void __launch_bounds__(Q4G_THREADS, 1) q4_gemm_kernel(const __grid_co
                         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                                      ::"r"(xring + slot * xstage_bytes), "l"(p.XS + ((size_t)(x.tile % p.nt) * p.nchunks + x.c) * xstage_bytes), "r"(xstage_bytes), "r"(bar) : "memory");
                 }
+                Q4U_TRACE(2, i == 0 && lane == 0)
                 if (++ws == Q4G_WSTAGES) { ws = 0; wph ^= 1u; }
                 if (i < count) w.next(p.nchunks);
                 if (i >= LAG) {
@@ -270,6 +276,7 @@ __global__ void __launch_bounds__(Q4G_THREADS, 1) q4_gemm_kernel(const __grid_co
             }
         } else fail = 46;
         asm volatile("griddepcontrol.wait;" ::: "memory");              // (as in q4_umma_kernel)
+        Q4U_TRACE(3, threadIdx.x == 0)
         while (w.left && !fail) {
             int piece = w.rest_left ? min(w.rest_left, p.nchunks - w.c) : p.nchunks;          // chunks of this piece
             const int behind = w.left - piece;
@@ -281,6 +288,7 @@ __global__ void __launch_bounds__(Q4G_THREADS, 1) q4_gemm_kernel(const __grid_co
                 for (int hf = 0; hf < 2; ++hf) {
                     // with the first block's sums the weights of the chunk that is expanded next: one round trip
                     if (!(hf ? q4u_bar_wait(df + 8, dph) : q4u_bar_wait(look ? wf + 8 * ws : df, look ? wph : dph))) { fail = 45; break; }
+                    Q4U_TRACE(4, threadIdx.x == 0 && hf == 0 && piece + behind + 1 == Q4GWalk(p).left)
                     q4u_fence_after();
                     if (hf == 0 && more) load(sw2);
                     const uint32_t d = dacc + slot * Q4G_D_COLS, scale = hf ? sw0 >> 16 : sw0 & 0xFFFFu;
@@ -299,6 +307,7 @@ __global__ void __launch_bounds__(Q4G_THREADS, 1) q4_gemm_kernel(const __grid_co
                 sw1 = sw2;
             } while (piece);
             if (fail) break;
+            Q4U_TRACE(5, threadIdx.x == 0)
             // the piece's sums: to y when this range holds the whole tile, else to the range's slot
             const int b = w.tile / p.nt, col = g * 128 + qd * 32 + lane, nrow = b * 256 + col;
             const int at = w.tile != p.full * (int)gridDim.x + q4u_div((int64_t)blockIdx.x * p.W, p.nchunks);
@@ -310,12 +319,14 @@ __global__ void __launch_bounds__(Q4G_THREADS, 1) q4_gemm_kernel(const __grid_co
                 const float isc0 = lane < rows ? p.inv_sc[m0 + lane] : 0.f, isc1 = lane + 32 < rows ? p.inv_sc[m0 + lane + 32] : 0.f;
                 q4u_store<SL>(acc[u], whole ? p.Y + (size_t)m0 * p.ldy + nrow : slot_out + (size_t)r0 * 256, whole ? p.ldy : 256, rows, !whole || nrow < p.N, isc0, isc1);
             }
+            Q4U_TRACE(6, threadIdx.x == 0)
             w.skip(w.left - behind, p.nchunks);
         }
         if (fail && lane == 0) { atomicExch(p.status, fail); s_abort = 1; }
     }
     q4u_fence_before();
     __syncthreads();
+    Q4U_TRACE(7, threadIdx.x == 0)
     settle_after_timeout(s_abort);
     if (warp == Q4G_WARP_ISSUE) {
         q4u_fence_after();

@@ -75,7 +75,23 @@ struct Q4ULaunch {
     int W;                        // (batch, chunk) pairs per CTA
     int wstages;                  // stages of each team's weight ring (what shared memory allows, up to Q4U_MAX_WSTAGES)
     int* status;
+#ifdef MPQ_TRACE
+    unsigned long long* trace;    // [CTAs][16]: %globaltimer stamps, entry 15 = 1 (diagnostic build only)
+#endif
 };
+
+// Diagnostic build (-DMPQ_TRACE): one thread of the role concerned records when it passed a phase (the names are in timeline.py).
+#ifdef MPQ_TRACE
+#define Q4U_TRACE(slot, who)                                                       \
+    if (p.trace && (who)) {                                                        \
+        unsigned long long t_;                                                     \
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_));                     \
+        p.trace[(size_t)blockIdx.x * 16 + (slot)] = t_;                            \
+        if ((slot) == 0) p.trace[(size_t)blockIdx.x * 16 + 15] = 1;                \
+    }
+#else
+#define Q4U_TRACE(slot, who)
+#endif
 
 // ---------------------------------------------------------------------------
 // activation staging: fp32 rows -> hi/lo fp16 tiles in the order the MMA's shared-memory descriptor wants
@@ -422,6 +438,7 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_umma_kernel(const __grid_co
     const uint32_t w_full = bars, w_empty = w_full + 8 * NW, x_full = w_empty + 8 * NW, x_empty = x_full + 8 * Q4U_XSTAGES,
                    a_full = x_empty + 8 * Q4U_XSTAGES, d_full = a_full + 8 * Q4U_TEAMS, d_empty = d_full + 16 * Q4U_TEAMS;   // a_full: [team]; d_full: [team][half of the chunk]
     const int warp = __shfl_sync(0xFFFFFFFFu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (warp: uniform for the compiler)
+    Q4U_TRACE(0, threadIdx.x == 0)
     // this CTA's range of the (batch, chunk) sequence
     const long long total = (long long)p.nbatches * p.nchunks;
     const long long L_begin = (long long)blockIdx.x * p.W;
@@ -444,6 +461,7 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_umma_kernel(const __grid_co
     __syncthreads();
     q4u_fence_after();
     const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, s_tmem_base, 0);
+    Q4U_TRACE(1, threadIdx.x == 0)
 
     asm volatile("griddepcontrol.launch_dependents;");
 
@@ -472,6 +490,7 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_umma_kernel(const __grid_co
                         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                                      ::"r"(xring + slot * xstage_bytes), "l"(p.XS + (size_t)cx * xstage_bytes), "r"(xstage_bytes), "r"(bar) : "memory");
                 }
+                Q4U_TRACE(2, i == 0 && lane == 0)
                 if (++ws == WST) { ws = 0; wph ^= 1u; }
                 if (++c == p.nchunks) { c = 0; ++b; }
                 if (i >= LAG) {
@@ -561,11 +580,13 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_umma_kernel(const __grid_co
         // Here, and in the issuing warp, so that a slow kernel in front is not counted against the bounds of the waits for sums; inv_sc
         // comes from it too, and y and the slices may still be read.
         asm volatile("griddepcontrol.wait;" ::: "memory");
+        Q4U_TRACE(3, threadIdx.x == 0)
         while (left > 0 && !fail) {
             const int after = max(0, left - (p.nchunks - c));           // chunks left behind this piece
             do {
                 const uint32_t d = dacc + slot * Q4U_D_COLS, s = sw;
                 if (!q4u_bar_wait(df, dph)) { fail = 35; break; }
+                Q4U_TRACE(4, threadIdx.x == 0 && left == range)
                 q4u_fence_after();
                 q4u_drain<SL, STACK, SL != 4>(acc, d, p.Mp, s & 0xFFFFu);
                 if (!q4u_bar_wait(df + 8, dph)) { fail = 35; break; }
@@ -579,6 +600,7 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_umma_kernel(const __grid_co
                 if (--left > 0 && !expand()) { fail = 36; break; }
             } while (left > after);
             if (fail) break;
+            Q4U_TRACE(5, threadIdx.x == 0)
             // ---- the piece's sums: to y when this range holds the whole batch, else to the piece's slice
             // Lane l keeps rows l and l + 32 of inv_sc: read inside the store loop the loads would be ordered behind the stores
             // (they may alias for all the compiler knows), one round trip per row.
@@ -588,6 +610,7 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_umma_kernel(const __grid_co
             const int nrow = (b * Q4U_TEAMS + tm) * 128 + qd * 32 + lane;
             float* out = (pf == pl ? p.Y : p.partial + (size_t)((int)blockIdx.x - pf) * p.M * p.N) + nrow;
             q4u_store<SL>(acc, out, pf == pl ? p.ldy : (int64_t)p.N, p.M, nrow < p.N, isc0, isc1);
+            Q4U_TRACE(6, threadIdx.x == 0)
             c = 0;
             ++b;
         }
@@ -595,6 +618,7 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_umma_kernel(const __grid_co
     }
     q4u_fence_before();
     __syncthreads();
+    Q4U_TRACE(7, threadIdx.x == 0)
     settle_after_timeout(s_abort);
     if (warp == Q4U_WARP_ISSUE) {
         q4u_fence_after();

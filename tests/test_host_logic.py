@@ -377,3 +377,39 @@ def test_a_weight_without_a_tensor_map_is_not_refused():
     text = open(os.path.join(ROOT, "makepad_b200", "csrc", "mpq.cu")).read()
     assert not re.search(r"!q\.mapped\) return fail", text)
     assert not re.search(r"ctx->q4_umma_min (>|<|>=|<=) ", text)          # routes go through q4_route, which knows of the map
+
+
+def test_a_timeline_of_kernels_that_are_not_stamped_is_refused():
+    """The diagnostic library returns no array when nothing was stamped: a message then, not a read of address zero."""
+    import ctypes as C
+    import numpy as np
+    import pytest
+    from makepad_b200 import timeline
+    stamps = np.arange(64 * 1024 * 16, dtype=np.uint64)
+
+    class Debug:                                                       # stands for the library's mpq_debug_trace
+        def __init__(self, ptr, launches):
+            self.ptr, self.launches = ptr, launches
+
+        def __call__(self, count):
+            C.cast(count, C.POINTER(C.c_int32))[0] = self.launches
+            return self.ptr
+
+    class Lib:
+        def __init__(self, ptr, launches):
+            self.mpq_debug_trace = Debug(ptr, launches)
+
+    with pytest.raises(RuntimeError, match="0 of 24 launches"):
+        timeline.read_trace(Lib(None, 0), 24)
+    with pytest.raises(RuntimeError, match="18 of 24 launches"):       # some projections of a layer stream, others do not
+        timeline.read_trace(Lib(stamps.ctypes.data, 18), 24)
+    assert (timeline.read_trace(Lib(stamps.ctypes.data, 24), 24).ravel() == stamps).all()
+
+
+def test_the_tcgen05_kernels_are_stamped_in_the_diagnostic_build():
+    """What the timeline names, the kernels stamp: phases 0..7 in each, and their launches pass the array."""
+    csrc = os.path.join(ROOT, "makepad_b200", "csrc")
+    for f in ("q4_umma.cuh", "q4_gemm.cuh"):
+        text = open(os.path.join(csrc, f)).read()
+        assert sorted(re.findall(r"Q4U_TRACE\((\d),", text)) == list("01234567"), f
+    assert open(os.path.join(csrc, "mpq.cu")).read().count("p.trace = trace_slot(") == 3
