@@ -99,36 +99,7 @@ __global__ void __launch_bounds__(256) q4g_xstage_kernel(const float* __restrict
     }
 }
 
-// Walks the (tile, chunk) pairs of one CTA; every role runs the same walk.  First the CTA's range of the tiles that are left
-// over, then its whole tiles, one from each wave (so that the activation tiles of a weight tile run side by side).
-struct Q4GWalk {
-    int left, rest_left, tile, c;
-    __device__ __forceinline__ Q4GWalk(const Q4GemmLaunch& p)
-    {
-        const int64_t begin = (int64_t)blockIdx.x * p.W, end = min((int64_t)p.rest * p.nchunks, begin + p.W);
-        rest_left = (int)max((int64_t)0, end - begin);
-        left = rest_left + p.full * p.nchunks;
-        tile = rest_left ? p.full * (int)gridDim.x + q4u_div(begin, p.nchunks) : (int)blockIdx.x;
-        c = rest_left ? (int)(begin - (int64_t)q4u_div(begin, p.nchunks) * p.nchunks) : 0;
-    }
-    __device__ __forceinline__ void next(int nchunks)
-    {
-        --left;
-        ++c;
-        if (rest_left > 0) {
-            if (c == nchunks) { c = 0; ++tile; }
-            if (--rest_left == 0) { c = 0; tile = (int)blockIdx.x; }
-        } else if (c == nchunks) { c = 0; tile += (int)gridDim.x; }
-    }
-    // over the n chunks up to the end of a tile or of the range
-    __device__ __forceinline__ void skip(int n, int nchunks)
-    {
-        left -= n - 1;
-        if (rest_left > 0) rest_left -= n - 1;
-        c += n - 1;
-        next(nchunks);
-    }
-};
+__device__ __forceinline__ Q4GWalk q4g_walk(const Q4GemmLaunch& p) { return Q4GWalk((int)blockIdx.x, (int)gridDim.x, p.full, p.rest, p.W, p.nchunks); }
 
 // SL: half of the tile's 16-row slices, rounded up
 template <int SL>
@@ -176,7 +147,7 @@ __global__ void __launch_bounds__(Q4G_THREADS, 1) q4_gemm_kernel(const __grid_co
             const bool wlane = lane < Q4G_GROUPS, xlane = lane == Q4G_GROUPS;
             int ws = 0, xs = 0;
             uint32_t wph = 1, xph = 1;
-            Q4GWalk w(p), x = w;
+            Q4GWalk w = q4g_walk(p), x = w;
             const int count = w.left;
             for (int i = 0; i < count + LAG; ++i) {
                 if (__any_sync(0xFFFFFFFFu, s_abort)) break;
@@ -196,16 +167,16 @@ __global__ void __launch_bounds__(Q4G_THREADS, 1) q4_gemm_kernel(const __grid_co
                 }
                 Q4U_TRACE(2, i == 0 && lane == 0)
                 if (++ws == Q4G_WSTAGES) { ws = 0; wph ^= 1u; }
-                if (i < count) w.next(p.nchunks);
+                if (i < count) w.next(p.nchunks, (int)blockIdx.x, (int)gridDim.x);
                 if (i >= LAG) {
                     if (++xs == Q4G_XSTAGES) { xs = 0; xph ^= 1u; }
-                    x.next(p.nchunks);
+                    x.next(p.nchunks, (int)blockIdx.x, (int)gridDim.x);
                 }
             }
         } else if (warp == Q4G_WARP_ISSUE) {
             // ---------------- MMA issue: the whole warp runs the loop, one elected lane issues ----------------
             const uint32_t idesc = (1u << 4) | ((uint32_t)(p.Mt >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);      // f16 x f16 -> f32, K-major both
-            const int count = Q4GWalk(p).left;
+            const int count = q4g_walk(p).left;
             int xs = 0, slot = 0, fail = 0;
             uint32_t xph = 0, dph = 1;                   // (the first round of empty slots passes on the parity before the first)
             asm volatile("griddepcontrol.wait;" ::: "memory");     // the polls below are for this kernel's own copies, not for the kernels before
@@ -246,7 +217,7 @@ __global__ void __launch_bounds__(Q4G_THREADS, 1) q4_gemm_kernel(const __grid_co
         int ws = 0, slot = g, fail = 0;
         uint32_t wph = 0, dph = 0, sw0 = 0, sw1 = 0, sw2 = 0;           // scales of the chunk that is drained, and of the two behind it
         uint2 codes[2][4];
-        Q4GWalk w(p);
+        Q4GWalk w = q4g_walk(p);
         // the chunk in weight stage ws -> registers
         auto load = [&](uint32_t& sw) {
             const uint32_t stage = ring + ws * Q4U_WSTAGE_BYTES;
@@ -288,7 +259,7 @@ __global__ void __launch_bounds__(Q4G_THREADS, 1) q4_gemm_kernel(const __grid_co
                 for (int hf = 0; hf < 2; ++hf) {
                     // with the first block's sums the weights of the chunk that is expanded next: one round trip
                     if (!(hf ? q4u_bar_wait(df + 8, dph) : q4u_bar_wait(look ? wf + 8 * ws : df, look ? wph : dph))) { fail = 45; break; }
-                    Q4U_TRACE(4, threadIdx.x == 0 && hf == 0 && piece + behind + 1 == Q4GWalk(p).left)
+                    Q4U_TRACE(4, threadIdx.x == 0 && hf == 0 && piece + behind + 1 == q4g_walk(p).left)
                     q4u_fence_after();
                     if (hf == 0 && more) load(sw2);
                     const uint32_t d = dacc + slot * Q4G_D_COLS, scale = hf ? sw0 >> 16 : sw0 & 0xFFFFu;
@@ -310,7 +281,7 @@ __global__ void __launch_bounds__(Q4G_THREADS, 1) q4_gemm_kernel(const __grid_co
             Q4U_TRACE(5, threadIdx.x == 0)
             // the piece's sums: to y when this range holds the whole tile, else to the range's slot
             const int b = w.tile / p.nt, col = g * 128 + qd * 32 + lane, nrow = b * 256 + col;
-            const int at = w.tile != p.full * (int)gridDim.x + q4u_div((int64_t)blockIdx.x * p.W, p.nchunks);
+            const int at = w.tile != p.full * (int)gridDim.x + q4g_first_tile((int)blockIdx.x, p.W, p.nchunks);
             float* slot_out = p.partial + ((size_t)blockIdx.x * 2 + at) * Q4G_SLOT + col;
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
@@ -320,7 +291,7 @@ __global__ void __launch_bounds__(Q4G_THREADS, 1) q4_gemm_kernel(const __grid_co
                 q4u_store<SL>(acc[u], whole ? p.Y + (size_t)m0 * p.ldy + nrow : slot_out + (size_t)r0 * 256, whole ? p.ldy : 256, rows, !whole || nrow < p.N, isc0, isc1);
             }
             Q4U_TRACE(6, threadIdx.x == 0)
-            w.skip(w.left - behind, p.nchunks);
+            w.skip(w.left - behind, p.nchunks, (int)blockIdx.x, (int)gridDim.x);
         }
         if (fail && lane == 0) { atomicExch(p.status, fail); s_abort = 1; }
     }
@@ -349,7 +320,7 @@ __global__ void __launch_bounds__(256) q4g_reduce_kernel(const float* __restrict
     if (pf == pl || m >= M || n >= N) return;
     // the range's first tile uses its first slot; a piece that starts with the tile and is not the range's first uses the second
     const float4* src = reinterpret_cast<const float4*>(partial + (size_t)r * 256) + q;
-    const bool second = cut != q4u_div((int64_t)pf * W, nchunks);               // (ranges behind the first begin inside the tile)
+    const bool second = cut != q4g_first_tile(pf, W, nchunks);                  // (ranges behind the first begin inside the tile)
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int s = pf; s <= pl; s += 4) {                                          // four slots on their way at a time, added in order
         float4 u[4];

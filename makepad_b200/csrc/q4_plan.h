@@ -82,6 +82,40 @@ inline Q4GemmPlan q4_gemm_plan(int nrp, int nchunks, int M, int pairs_max)
     return pl;
 }
 
+// The tile, counted among those that are left over, in which a range of W chunks begins.
+__host__ __device__ __forceinline__ int q4g_first_tile(int range, int W, int nchunks) { return q4u_div((int64_t)range * W, nchunks); }
+
+// Walks the (tile, chunk) pairs of one CTA (`block` of `grid`); every role runs the same walk.  First the CTA's range of the tiles that
+// are left over, then its whole tiles, one from each wave (so that the activation tiles of a weight tile run side by side).
+struct Q4GWalk {
+    int left, rest_left, tile, c;
+    __host__ __device__ __forceinline__ Q4GWalk(int block, int grid, int full, int rest, int W, int nchunks)
+    {
+        const int64_t begin = (int64_t)block * W, chunks = (int64_t)rest * nchunks, end = begin + W < chunks ? begin + W : chunks;
+        rest_left = end > begin ? (int)(end - begin) : 0;
+        left = rest_left + full * nchunks;
+        tile = rest_left ? full * grid + q4g_first_tile(block, W, nchunks) : block;
+        c = rest_left ? (int)(begin - (int64_t)q4g_first_tile(block, W, nchunks) * nchunks) : 0;
+    }
+    __host__ __device__ __forceinline__ void next(int nchunks, int block, int grid)
+    {
+        --left;
+        ++c;
+        if (rest_left > 0) {
+            if (c == nchunks) { c = 0; ++tile; }
+            if (--rest_left == 0) { c = 0; tile = block; }
+        } else if (c == nchunks) { c = 0; tile += grid; }
+    }
+    // over the n chunks up to the end of a tile or of the range
+    __host__ __device__ __forceinline__ void skip(int n, int nchunks, int block, int grid)
+    {
+        left -= n - 1;
+        if (rest_left > 0) rest_left -= n - 1;
+        c += n - 1;
+        next(nchunks, block, grid);
+    }
+};
+
 // Rows per launch of the pair kernel: at most 2048, fewer where K is so long that the staged rows would pass 256 MB.
 inline int64_t q4_gemm_slab(int64_t K)
 {

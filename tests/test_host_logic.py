@@ -206,6 +206,73 @@ def test_tiles_above_64_rows_cover_the_call():
     _run(TILES)
 
 
+WALK = r"""
+#include "q4_plan.h"
+#include <cstdio>
+#include <cstdlib>
+#include <vector>
+using namespace mpq;
+struct Piece { int tile, c0, n, slot; };               // slot: -1 = straight to y, else the slot that the kernel writes
+int main()
+{
+    int bad = 0, both = 0;
+    for (int nrp : {1, 9, 128, 625, 938, 1792})
+        for (int nchunks : {4, 8, 20, 36})
+            for (int M : {65, 129, 300, 512})
+                for (int pairs : {74, 66, 1}) {
+                    const Q4GemmPlan p = q4_gemm_plan(nrp, nchunks, M, pairs);
+                    const int tiles = p.full * p.grid + p.rest;
+                    both += p.full && p.cut;
+                    std::vector<int> seen((size_t)tiles * nchunks, 0);
+                    std::vector<std::vector<Piece>> pieces(tiles);
+                    for (int block = 0; block < p.grid; ++block) {
+                        Q4GWalk w(block, p.grid, p.full, p.rest, p.W, nchunks), k = w;      // copies and MMAs; workers, piece by piece
+                        while (k.left) {
+                            const int n = k.rest_left ? std::min(k.rest_left, nchunks - k.c) : nchunks;
+                            const bool whole = k.c == 0 && n == nchunks;
+                            const int at = k.tile != p.full * p.grid + q4g_first_tile(block, p.W, nchunks);
+                            if (k.tile < 0 || k.tile >= tiles || n < 1) return 1;
+                            pieces[k.tile].push_back({k.tile, k.c, n, whole ? -1 : block * 2 + at});
+                            for (int i = 0; i < n; ++i) {
+                                bad += w.tile != k.tile || w.c != k.c + i || w.left != k.left - i;      // the same walk
+                                ++seen[(size_t)w.tile * nchunks + w.c];
+                                w.next(nchunks, block, p.grid);
+                            }
+                            k.skip(n, nchunks, block, p.grid);
+                        }
+                        bad += w.left != 0;
+                    }
+                    for (int s : seen) bad += s != 1;                                       // every chunk of every tile once
+                    for (int t = 0; t < tiles; ++t) {
+                        if (t < p.full * p.grid) { bad += pieces[t].size() != 1 || pieces[t][0].slot != -1; continue; }
+                        const int cut = t - p.full * p.grid;                                // the sum reads, in order, what was written
+                        int pf, pl;
+                        q4u_pieces(cut, nchunks, p.W, &pf, &pl);
+                        bad += (int)pieces[t].size() != pl - pf + 1;
+                        if (pf == pl) { bad += pieces[t][0].slot != -1; continue; }
+                        const bool second = cut != q4g_first_tile(pf, p.W, nchunks);
+                        int c = 0;
+                        for (int s = pf; s <= pl && s - pf < (int)pieces[t].size(); ++s) {
+                            const Piece& q = pieces[t][s - pf];
+                            bad += q.slot != s * 2 + (s == pf && second) || q.c0 != c;
+                            c += q.n;
+                        }
+                        bad += c != nchunks;
+                    }
+                }
+    bad += both < 20;                                                                       // the form of long prompts is among them
+    std::printf("%d\n", bad);
+    return bad != 0;
+}
+"""
+
+
+def test_the_walk_over_tiles_above_64_rows_visits_every_chunk_once():
+    """Cut ranges first, then whole tiles: copies, MMAs and workers walk alike, no chunk is left out or taken twice, and the sum of a cut
+    tile reads the slots that its pieces were written to."""
+    _run(WALK)
+
+
 def test_scratch_reserved_for_a_call_is_enough_for_every_smaller_one():
     _run(NEEDS)
 

@@ -381,10 +381,12 @@ def test_f16_mma_issue_probe(ctx):
     assert ctx.lib.mpq_context_poll_status(ctx.h) == _lib.OK
 
 
-# one ragged tile; tiles of 32 x 3; a pair-tile short of a group; whole tiles and cut ones; one chunk per segment; long K (many
-# pieces of one tile); several activation tiles with a ragged last one; more rows than one launch stages
+# one ragged tile, two; a pair-tile short of a group; several activation tiles; a K of one padded group with a whole tile for every CTA and
+# none cut; long K (many pieces of one tile); a ragged last activation tile; more rows than one launch stages; and, behind a cut range, one
+# whole tile per CTA: ranges of 13 of 20 chunks that cross tiles, of 12 of 20, of 4 of 8 (148 SMs)
 @pytest.mark.parametrize("N,K,M", [(1, 32, 65), (40, 160, 65), (257, 1120, 96), (1000, 2112, 300), (4096, 4096, 256), (20000, 64, 129),
-                                   (96, 28672, 70), (4096, 11008, 128), (2500, 1056, 513), (33, 288, 2100)])
+                                   (96, 28672, 70), (4096, 11008, 128), (2500, 1056, 513), (33, 288, 2100),
+                                   (20000, 1056, 300), (30000, 1120, 129), (20000, 288, 129)])
 def test_pair_kernel_above_64_rows(ctx, orc, N, K, M):
     """The CTA-pair kernel against the binary64 oracle (the bound of the other tcgen05 kernel: the arithmetic is the same),
     nothing written outside the output, the same bits twice, and the SwiGLU form equal to the unfused one bit for bit."""
