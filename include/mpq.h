@@ -125,9 +125,11 @@ int32_t mpq_weight_destroy(mpq_weight* w);
  * four rows while M * K < 16384, is one launch of the streaming kernel; up to
  * 16 rows otherwise one pass of the rectangle kernel (weights read once,
  * only a K slice of x staged per CTA) plus a small reduction; 17..64 rows
- * the tcgen05 kernel; above that the tcgen05 kernel of CTA pairs, or, up to
- * 128 rows of a large weight, two slabs of 64 rows (each: activation staging,
- * main kernel, reduction of the pieces).
+ * the tcgen05 kernel; above that the tcgen05 kernel on tiles of 256 weight
+ * rows x up to 128 activation rows, or, up to 128 rows of a large weight, two
+ * slabs of 64 rows (each: activation staging, main kernel, reduction of the
+ * pieces).  Where the driver cannot make a tensor map of the weight, 17 rows
+ * and more run as slabs of 16.
  * Scratch is allocated by the first call that needs it (or more of it).  A
  * call of more than four rows reserves what every smaller call of the weight
  * needs as well: make a warm-up call with the largest M of each weight before

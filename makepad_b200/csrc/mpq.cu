@@ -838,7 +838,7 @@ static size_t q4_gemm_smem(int Mt)
     return std::max<size_t>((size_t)Q4G_XSTAGES * 2 * Mt * 128 + (size_t)Q4G_GROUPS * Q4G_WSTAGES * Q4U_WSTAGE_BYTES + 512 + 1024, (size_t)116 * 1024);
 }
 
-// half of the CTAs that the device keeps resident
+// half of the CTAs that the device keeps resident (what q4_gemm_plan counts in; of an odd number of SMs one stays idle)
 static int q4_gemm_pairs(const mpq_context* ctx) { return ctx->prop.multiProcessorCount / 2; }
 
 // y = x . W^T for M > 64 rows; with swiglu x is [M][2K] = [gate | up].  One slab's staged rows take M * K * 4 bytes of scratch.
@@ -915,7 +915,7 @@ static int32_t q4_gemm_slabs(mpq_context* ctx, const Q4Dev& q, const float* x, b
 
 static Q4Route q4_route(const mpq_context* ctx, const Q4Dev& q, int64_t M) { return q4_route(q.units(), M, ctx->q4_umma_min, ctx->q4_gemm_min, q.mapped); }
 
-// CTA pairs for a call of M rows, or 0 where it is one for the kernels of 64 rows and fewer
+// pairs_max for a call of M rows, or 0 where it is one for the kernels of 64 rows and fewer
 static int q4_gemm_wanted(const mpq_context* ctx, const Q4Dev& q, int64_t M)
 {
     return q4_route(ctx, q, M) == Q4Route::Tiles ? q4_gemm_pairs(ctx) : 0;
@@ -950,7 +950,7 @@ static void q4_reserve(mpq_context* ctx, const mpq_weight* w, int64_t M, bool sw
     q4_stream_scratch(ctx, ctx->prop.multiProcessorCount);               // (one row streams)
 }
 
-// Pairs of CTAs to run a call on, or 0.  Slabs of 64 rows want less scratch than the tiles above 64 rows: a call whose scratch could not be had
+// ... to run it with, or 0.  Slabs of 64 rows want less scratch than the tiles above 64 rows: a call whose scratch could not be had
 // (in a capture without a warm-up of its size, or for want of memory) keeps to them.
 static int q4_gemm_route(const mpq_context* ctx, const Q4Dev& q, int64_t M)
 {

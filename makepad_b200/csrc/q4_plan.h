@@ -58,8 +58,9 @@ constexpr int Q4G_ROWS = 256;                 // weight rows per tile
 constexpr int Q4G_SLOT = Q4G_ROWS * Q4G_MT_MAX;      // floats of one partial slot: [row of x][256 weight rows]
 constexpr int Q4G_MIN_W = 4;                  // fewest chunks per range of a cut tile
 
-// How one slab of M rows is cut, and the scratch that takes.  Every CTA (two per `pair`) gets `full` whole tiles; the `rest` tiles
-// that are left over are cut into equal ranges of W chunks, one per CTA (a range touches at most two tiles).
+// How one slab of M rows is cut, and the scratch that takes.  pairs_max: half of the CTAs that the device keeps resident.  Every CTA gets
+// `full` whole tiles; the `rest` tiles that are left over are cut into equal ranges of W chunks, one per CTA (a range touches at most two
+// tiles).
 struct Q4GemmPlan { int nt, Mt, full, rest, W, ranges, grid; bool cut; size_t xs_bytes, need_xs, need_partial; };
 inline Q4GemmPlan q4_gemm_plan(int nrp, int nchunks, int M, int pairs_max)
 {
@@ -116,16 +117,18 @@ struct Q4GWalk {
     }
 };
 
-// Rows per launch of the pair kernel: at most 2048, fewer where K is so long that the staged rows would pass 256 MB.
+// Rows per launch of q4_gemm_kernel: at most 2048, fewer where K is so long that the staged rows would pass 256 MB.
 inline int64_t q4_gemm_slab(int64_t K)
 {
     return std::max<int64_t>(Q4G_MT_MAX, std::min<int64_t>(2048, ((int64_t)1 << 26) / K / Q4G_MT_MAX * Q4G_MT_MAX));
 }
 
 // Calls above 64 rows that run as two slabs of 64 rows (q4_umma_kernel): up to 128 rows of a large weight.  The line was drawn for
-// kernels with three products per weight, where the two took the same time at 80 rows of 24576 x 16384 (196608 units of 32 x 64 weights:
-// 296 / 305 us) and at 112 rows of 32768 x 16384 (262144 units: 425 / 447).  Both kernels take two thirds of that time now; the line
-// stands, since the tests hold the launches of such a call to it.  (57344 x 8192: two slabs 2 x 133 us, 128 rows as tiles 215.)
+// kernels with three products per weight, where the two forms took the same time on it.  It is not where today's kernels meet: tiles are the
+// faster form on all of this side.  Two slabs / tiles, us: 24576 x 16384 (196608 units of 32 x 64 weights) at 65 rows 188 / 157, 80
+// 191 / 157, 96 212..220 / 160; 57344 x 8192 (229376) at 65 250..261 / 213..221, 80 246 / 199..204, 96 264 / 199; 32768 x 16384 (262144) at
+// 65 280..289 / 240..251, 96 293 / 228, 112 308..312 / 247..251, 128 340 / 270..274.  So the line can go: a call then takes half the
+// launches and has the tiles' bits, which is a change of its own.
 inline bool q4_slabs_of_64(int64_t units, int64_t M) { return M <= 64 || (M <= 96 && units >= 3 << 16) || (M <= 128 && units >= 1 << 18); }
 
 // Where a call of M rows goes: slabs of 16 rows and fewer through the other kernels, or the tcgen05 kernels in slabs of 64 rows or as tiles.
@@ -147,7 +150,7 @@ inline Q4Route q4_route(int64_t units, int64_t M, int umma_min, int gemm_min, bo
 // Less rows can want more: 512 rows of 57344 x 8192 take 38.8 MB of partial sums, 64 rows 44.0 MB.  A program warms up with its
 // largest call before it captures graphs, so that call reserves what the smaller ones want.  rect_partial: the most that
 // 2 .. 16 rows want; umma_pieces: Q4UmmaPlan::pieces; umma_min, gemm_min: fewest rows of the two kernels (0: never);
-// pairs_max: CTA pairs of the device.
+// pairs_max: as in q4_gemm_plan, or 0 where no call runs as tiles.
 struct Q4Needs { size_t xs, partial; };
 inline Q4Needs q4_needs(int64_t N, int64_t K, int nrp, int nchunks, int64_t M, size_t rect_partial, int umma_pieces, int umma_min, int gemm_min,
                         int pairs_max)
@@ -158,7 +161,7 @@ inline Q4Needs q4_needs(int64_t N, int64_t K, int nrp, int nchunks, int64_t M, s
     n.xs = q4_umma_need_xs(nchunks, rows);
     n.partial = std::max(n.partial, q4_umma_need_partial(umma_pieces, rows, N));
     if (gemm_min <= 0 || M < gemm_min || pairs_max <= 0) return n;
-    // The staged rows grow with M.  The number of ranges does not, but it is at most the device's pairs, and each holds at
+    // The staged rows grow with M.  The number of ranges does not, but it is at most one per CTA, and each holds at
     // least Q4G_MIN_W chunks of the largest call.
     const Q4GemmPlan pl = q4_gemm_plan(nrp, nchunks, (int)std::min<int64_t>(M, q4_gemm_slab(K)), pairs_max);
     const int64_t total = (int64_t)((nrp + 7) / 8) * pl.nt * nchunks, most = std::min<int64_t>(2 * pairs_max, (total + Q4G_MIN_W - 1) / Q4G_MIN_W);

@@ -29,7 +29,8 @@
 //                   reads; in its plain order the rows of a quarter warp are 64 bytes apart, a four-way bank conflict), the
 //                   staged activations by cp.async.bulk; as far ahead as the rings allow: the bytes in flight hide the latency
 // Hand-offs are mbarriers; every wait is bounded (a wait that runs out sets the status word and every role
-// leaves its loop; tensor memory is freed on every path).  No TMA load uses multicast.
+// leaves its loop; tensor memory is freed on every path).  Waits for what depends on the kernels before begin when those have ended
+// (griddepcontrol.wait), so that a slow one is not counted against the bounds.  No TMA load uses multicast.
 //
 // WHAT IT COSTS (measured parts).  An MMA of N = 64 takes 32 cycles of pipe, one of N = 128 64, whoever issues it; the issue of four
 // with operands in ordinary registers 264, so the role of a warp, the waits' outcomes and with them all that the loops count are

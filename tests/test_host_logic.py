@@ -163,7 +163,7 @@ int main()
         bad += q4_umma_need_partial(pieces, 64, s[0]) != (size_t)s[2] || q4_gemm_plan(nrp, nchunks, 512, 74).need_partial >= (size_t)s[2];
         bad += q4_needs(s[0], s[1], nrp, nchunks, 512, 0, pieces, 17, 65, 74).partial < (size_t)s[2];
     }
-    // two slabs of 64 rows instead of the pair kernel: up to 96 rows of a large weight, up to 128 of a very large one
+    // two slabs of 64 rows instead of tiles: up to 96 rows of a large weight, up to 128 of a very large one
     const int64_t route[][3] = {{196607, 65, 0}, {196608, 65, 1}, {196608, 96, 1}, {196608, 97, 0}, {262143, 97, 0}, {262144, 97, 1}, {262144, 128, 1},
                                 {262144, 129, 0}, {1 << 30, 129, 0}, {1, 64, 1}, {1, 65, 0}, {256512, 96, 1}, {256512, 128, 0}};
     for (auto& r : route) bad += q4_slabs_of_64(r[0], r[1]) != (r[2] != 0);

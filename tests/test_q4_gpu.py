@@ -388,7 +388,7 @@ def test_f16_mma_issue_probe(ctx):
                                    (96, 28672, 70), (4096, 11008, 128), (2500, 1056, 513), (33, 288, 2100),
                                    (20000, 1056, 300), (30000, 1120, 129), (20000, 288, 129)])
 def test_pair_kernel_above_64_rows(ctx, orc, N, K, M):
-    """The CTA-pair kernel against the binary64 oracle (the bound of the other tcgen05 kernel: the arithmetic is the same),
+    """The kernel of 256 x 128 tiles against the binary64 oracle (the bound of the other tcgen05 kernel: the arithmetic is the same),
     nothing written outside the output, the same bits twice, and the SwiGLU form equal to the unfused one bit for bit."""
     import makepad_b200
     torch = _torch()
@@ -412,7 +412,7 @@ def test_pair_kernel_above_64_rows(ctx, orc, N, K, M):
 
 def test_capture_above_64_rows_after_a_warm_up_of_64(orc):
     """A capture cannot allocate: with the scratch of a 64-row warm-up the call keeps to slabs of 64 rows, with that of a full
-    warm-up it takes the pair kernel; both replay to the oracle's result."""
+    warm-up it takes the kernel of tiles; both replay to the oracle's result."""
     import makepad_b200
     torch = _torch()
     N, K, M = 500, 1056, 300
@@ -532,7 +532,7 @@ def test_a_warm_up_with_the_largest_call_is_enough_to_capture_smaller_ones(N, K,
         before = c2.launches
         want = lin(x[:M]), lin.forward_swiglu(gate_up[:M])
         assert c2.launches - before == launches, M
-        if M in (96, 100):                                             # a large weight: two slabs of 64 rows up to 96, then the pair kernel
+        if M in (96, 100):                                             # a large weight: two slabs of 64 rows up to 96, then tiles
             assert launches == (12 if M == 96 and N == 57344 else 6), M
         assert torch.equal(y, want[0]) and torch.equal(z, want[1]), M
     torch.cuda.synchronize()
@@ -569,7 +569,7 @@ def test_a_prompt_without_room_for_the_pair_kernel(orc):
     rows = [0, 63, 64, 1000, M - 1]
     assert orc.err_report(y[rows].cpu().numpy(), orc.q4_matmul_f64(codes, scales, x[rows]))["max_abs_over_rms"] < 2e-5
     before = c2.launches
-    lin.forward(xd, out=y)                                             # with room again: the pair kernel
+    lin.forward(xd, out=y)                                             # with room again: tiles
     assert c2.launches - before <= 3
     torch.cuda.synchronize()
     assert c2.lib.mpq_context_poll_status(c2.h) == _lib.OK
