@@ -725,9 +725,8 @@ static int32_t q4_rect_forward(mpq_context* ctx, const Q4Dev& q, const Q4RectPla
     if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4_rect_kernel launch failed: %s", cudaGetErrorString(e));
     if (pl.nks > 1) {
         cudaLaunchConfig_t cfg = {};
-        const int64_t total = ((int64_t)M * q.N + 3) / 4;              // four columns per thread where the shapes allow
-        cfg.gridDim = dim3((unsigned)std::min<int64_t>((total + 255) / 256, (int64_t)ctx->prop.multiProcessorCount * 8));
-        cfg.blockDim = dim3(256);
+        cfg.gridDim = dim3((unsigned)((q.N + 4 * Q4R_REDUCE_THREADS - 1) / (4 * Q4R_REDUCE_THREADS)), (unsigned)M);
+        cfg.blockDim = dim3(Q4R_REDUCE_THREADS);
         cfg.stream = s;
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -817,9 +816,8 @@ static int32_t q4_umma_forward(mpq_context* ctx, const Q4Dev& q, const float* x,
     if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4_umma_kernel launch failed: %s", cudaGetErrorString(e));
     if (pl.pieces > 1) {
         cfg = {};
-        const int64_t tot = (int64_t)M * ((q.N + 3) / 4);
-        cfg.gridDim = dim3((unsigned)std::min<int64_t>((tot + 255) / 256, (int64_t)sms * 8));
-        cfg.blockDim = dim3(256);
+        cfg.gridDim = dim3((unsigned)pl.nbatches, (unsigned)M);
+        cfg.blockDim = dim3(32 * Q4U_TEAMS);
         cfg.stream = s;
         launch_pdl(cfg, at, ctx->pdl);
         e = cudaLaunchKernelEx(&cfg, q4u_reduce_kernel, (const float*)partial, M, (int)q.N, q.nchunks, W, y, ldy);

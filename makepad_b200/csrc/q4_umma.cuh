@@ -627,36 +627,46 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_umma_kernel(const __grid_co
     }
 }
 
-// y[m][n] = sum of the pieces' partial slices, in piece order, for the batches the main kernel cut into pieces.
-// One thread per four consecutive columns (N is a multiple of 4 or the tail is done one by one); all rows m of them.
-__global__ void __launch_bounds__(256) q4u_reduce_kernel(const float* __restrict__ partial, int M, int N, int nchunks, int W,
-                                                          float* __restrict__ Y, int64_t ldy)
+// y[m][n] = sum of the pieces' partial slices, in piece order, for the batches the main kernel cut into pieces.  One batch of 512
+// columns per blockIdx.x, one row per blockIdx.y, four columns per thread where the shapes allow.  Bound by latency, and at 57344 x 8192 by the
+// slices' way through L2: whole batches leave before any load, the pieces' divisions are made while the kernel before ends, and the loads
+// of up to Q4U_REDUCE_LOADS pieces go out together.  Calls before / now (us, in a graph): 4096 x 4096 (16 pieces) at 17 rows 15.1 / 14.2, 64 rows
+// 18.9 / 18.0; 22016 x 4096 at 64 39.7 / 38.6; 1000 x 2112 at 20 11.3 / 10.7.
+constexpr int Q4U_REDUCE_LOADS = 8;
+__global__ void __launch_bounds__(32 * Q4U_TEAMS) q4u_reduce_kernel(const float* __restrict__ partial, int M, int N, int nchunks, int W,
+                                                                    float* __restrict__ Y, int64_t ldy)
 {
     asm volatile("griddepcontrol.launch_dependents;");
+    int pf, pl;
+    q4u_pieces((int)blockIdx.x, nchunks, W, &pf, &pl);
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int nq = (N + 3) / 4;
-    const bool vec = (N & 3) == 0 && (ldy & 3) == 0 && ((reinterpret_cast<uintptr_t>(Y) | reinterpret_cast<uintptr_t>(partial)) & 15) == 0;
-    const int64_t total = (int64_t)M * nq;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int m = (int)(i / nq), n = (int)(i % nq) * 4;
-        int pf, pl;
-        q4u_pieces(n / (128 * Q4U_TEAMS), nchunks, W, &pf, &pl);      // four columns never straddle a batch of 512
-        if (pf == pl) continue;
-        const int np = pl - pf + 1;
-        if (vec) {
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int s = 0; s < np; ++s) {
-                const float4 t = __ldcs(reinterpret_cast<const float4*>(partial + ((size_t)s * M + m) * N + n));
-                v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
-            }
-            *reinterpret_cast<float4*>(Y + (size_t)m * ldy + n) = v;
-        } else {
-            for (int k = 0; k < 4 && n + k < N; ++k) {
-                float v = 0.f;
-                for (int s = 0; s < np; ++s) v += partial[((size_t)s * M + m) * N + n + k];
-                Y[(size_t)m * ldy + n + k] = v;
-            }
+    if (pf == pl) return;
+    const int np = pl - pf + 1, m = blockIdx.y;
+    const size_t slice = (size_t)M * N;
+    const float* src = partial + (size_t)m * N;
+    float* y = Y + (size_t)m * ldy;
+    if ((N & 3) == 0 && (ldy & 3) == 0 && ((reinterpret_cast<uintptr_t>(Y) | reinterpret_cast<uintptr_t>(partial)) & 15) == 0) {
+        const int n = ((int)blockIdx.x * 32 * Q4U_TEAMS + (int)threadIdx.x) * 4;
+        if (n >= N) return;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int s = 0; s < np; s += Q4U_REDUCE_LOADS) {
+            float4 u[Q4U_REDUCE_LOADS];
+#pragma unroll
+            for (int k = 0; k < Q4U_REDUCE_LOADS; ++k)
+                if (s + k < np) u[k] = __ldcs(reinterpret_cast<const float4*>(src + (s + k) * slice + n));
+#pragma unroll
+            for (int k = 0; k < Q4U_REDUCE_LOADS; ++k)
+                if (s + k < np) { v.x += u[k].x; v.y += u[k].y; v.z += u[k].z; v.w += u[k].w; }
         }
+        *reinterpret_cast<float4*>(y + n) = v;
+        return;
+    }
+    for (int c = threadIdx.x; c < 128 * Q4U_TEAMS; c += 32 * Q4U_TEAMS) {
+        const int n = (int)blockIdx.x * 128 * Q4U_TEAMS + c;
+        if (n >= N) return;
+        float v = 0.f;
+        for (int s = 0; s < np; ++s) v += __ldcs(src + s * slice + n);
+        y[n] = v;
     }
 }
 
