@@ -174,7 +174,7 @@ extern "C" int32_t mpq_context_create(int32_t device, mpq_context** out)
     e = getenv("MPQ_Q4_STREAM");
     c->q4_stream = !(e && e[0] == '0');
     e = getenv("MPQ_Q4_GROUP");
-    c->q4_group = (e && (e[0] == '1' || e[0] == '2')) ? e[0] - '0' : 0;
+    c->q4_group = (e && (e[0] == '1' || e[0] == '2' || e[0] == '4')) ? e[0] - '0' : 0;
     e = getenv("MPQ_Q4_DEPTH");
     c->q4_depth = (e && e[0] >= '1' && e[0] <= '8') ? e[0] - '0' : 2;
     e = getenv("MPQ_Q4_PRE");
@@ -481,6 +481,8 @@ static int32_t q4_stream_scratch(mpq_context* ctx, int ctas)
 // The streaming kernel applies when M <= 4 and the staged activation plus a ring fit in shared memory.
 struct Q4StreamPlan { int depth, G, pre; size_t smem; };
 static const size_t Q4S_STATIC_SMEM = 512;                 // s_max, wrp, zero page, rounded up
+// whole row pair-tiles per CTA when there is about one per SM or more: no tile is then shared between CTAs
+static bool q4_stream_tiles(const mpq_context* ctx, const Q4Dev& q) { return ctx->q4_tile_mode && (int64_t)q.nrp * 10 >= (int64_t)ctx->prop.multiProcessorCount * 6; }
 static bool q4_stream_plan(const mpq_context* ctx, const Q4Dev& q, int M, Q4StreamPlan* pl)
 {
     if (!ctx->q4_stream || M > 4) return false;
@@ -489,12 +491,21 @@ static bool q4_stream_plan(const mpq_context* ctx, const Q4Dev& q, int M, Q4Stre
                          (size_t)Q4S_WARPS * 2 * 4 * 32 * 4;
     // a CTA may use 227 KiB of an SM's shared memory
     const size_t budget = (size_t)227 * 1024 - Q4S_STATIC_SMEM;
-    for (int G = 2; G >= 1; --G) {
+    // Copies of four chunks where one row leaves room for two of them per warp and the longest run of a warp does not get longer: 22016 x 4096
+    // at one row 12.3 us with two chunks, 11.6 with four; at two rows 4096 x 4096 6.6 and 6.8.  longest: units of that run in groups of G.
+    const int sms = ctx->prop.multiProcessorCount;
+    auto longest = [&](int G) {
+        const int64_t gpr = q.nchunks / G, most = q4_stream_tiles(ctx, q) ? ((q.nrp + sms - 1) / sms) * gpr : (q.units() / G + sms - 1) / sms;
+        return (most + Q4S_WARPS - 1) / Q4S_WARPS * G;
+    };
+    for (int G = 4; G >= 1; G /= 2) {
         if (ctx->q4_group && G != ctx->q4_group) continue;
         const size_t stage = (size_t)Q4S_WARPS * G * Q4_UNIT_BYTES;
         if (fixed + stage > budget) continue;
+        const int depth = (int)std::min<size_t>((size_t)std::min(ctx->q4_depth, Q4S_MAX_DEPTH), (budget - fixed) / stage);
+        if (G == 4 && !ctx->q4_group && (M > 1 || depth < 2 || longest(4) > longest(2))) continue;
         pl->G = G;
-        pl->depth = (int)std::min<size_t>((size_t)std::min(ctx->q4_depth, Q4S_MAX_DEPTH), (budget - fixed) / stage);
+        pl->depth = depth;
         pl->smem = fixed + stage * pl->depth;
         pl->pre = std::min(ctx->q4_pre, pl->depth);
         return true;
@@ -502,10 +513,10 @@ static bool q4_stream_plan(const mpq_context* ctx, const Q4Dev& q, int M, Q4Stre
     return false;
 }
 
-template <int G>
+template <int G, bool ONE, bool SWIGLU>
 static cudaError_t q4_stream_launch_t(int device, const Q4StreamLaunch& p, int grid, size_t smem, bool pdl, cudaStream_t s)
 {
-    auto kern = q4_stream_kernel<G>;
+    auto kern = q4_stream_kernel<G, ONE, SWIGLU>;
     static PerDeviceOnce configured;                      // the attribute is per device, not per process
     if (configured.needs(device)) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227 * 1024 - Q4S_STATIC_SMEM));
@@ -524,6 +535,12 @@ static cudaError_t q4_stream_launch_t(int device, const Q4StreamLaunch& p, int g
     cfg.numAttrs = pdl ? 1u : 0u;
     return cudaLaunchKernelEx(&cfg, kern, p);
 }
+template <int G>
+static cudaError_t q4_stream_launch_g(int device, const Q4StreamLaunch& p, bool swiglu, int grid, size_t smem, bool pdl, cudaStream_t s)
+{
+    if (p.M == 1) return swiglu ? q4_stream_launch_t<G, true, true>(device, p, grid, smem, pdl, s) : q4_stream_launch_t<G, true, false>(device, p, grid, smem, pdl, s);
+    return swiglu ? q4_stream_launch_t<G, false, true>(device, p, grid, smem, pdl, s) : q4_stream_launch_t<G, false, false>(device, p, grid, smem, pdl, s);
+}
 
 // Launch parameters of the streaming kernel for one slab of M <= 4 rows, everything but the scratch
 // pointers and the exchange; returns the grid size.  Shared by every entry point that launches it.
@@ -533,17 +550,17 @@ static int q4_stream_params(const mpq_context* ctx, const Q4Dev& q, const Q4Stre
     const int sms = ctx->prop.multiProcessorCount;
     const int groups = (int)(q.units() / pl.G);
     const int W = (int)std::min<int64_t>((int64_t)sms * Q4S_WARPS, groups);
-    // whole row pair-tiles per CTA when there is about one per SM or more: no tile is then shared between CTAs
-    p->tile_mode = (ctx->q4_tile_mode && (int64_t)q.nrp * 10 >= (int64_t)sms * 6) ? 1 : 0;
-    p->nrp = q.nrp;
+    p->tile_mode = q4_stream_tiles(ctx, q) ? 1 : 0;
+    const int grid = p->tile_mode ? std::min(sms, q.nrp) : (W + Q4S_WARPS - 1) / Q4S_WARPS;
+    p->tiles_each = q.nrp / grid; p->tiles_more = q.nrp % grid;
+    p->gpr_magic = q4s_gpr_magic(groups, q.nchunks / pl.G);
     p->stream = q.stream; p->X = x; p->Y = y; p->M = M; p->N = (int)q.N; p->K = (int)q.K; p->ldy = ldy;
-    p->swiglu = 0;
     p->nchunks = q.nchunks; p->groups = groups; p->warps_total = W; p->depth = pl.depth; p->pre = pl.pre;
     p->partials = nullptr; p->status = nullptr;
     p->xworld = 0; p->xrank = 0; p->xslot = 0; p->xlimit = 0;
     for (int r = 0; r < 8; ++r) p->xpeer[r] = nullptr;
     p->xmine = nullptr;
-    return p->tile_mode ? std::min(sms, q.nrp) : (W + Q4S_WARPS - 1) / Q4S_WARPS;
+    return grid;
 }
 
 #ifdef MPQ_TRACE
@@ -577,7 +594,8 @@ extern "C" unsigned long long* mpq_debug_trace(int32_t* launches)
 }
 #endif
 
-static int32_t q4_stream_enqueue(mpq_context* ctx, const Q4StreamPlan& pl, const Q4StreamLaunch& p_in, int grid, cudaStream_t s)
+// swiglu: X is [M][2K] = [gate | up], and the activation is silu(gate) * up
+static int32_t q4_stream_enqueue(mpq_context* ctx, const Q4StreamPlan& pl, const Q4StreamLaunch& p_in, bool swiglu, int grid, cudaStream_t s)
 {
 #ifdef MPQ_TRACE
     Q4StreamLaunch p = p_in;
@@ -585,7 +603,9 @@ static int32_t q4_stream_enqueue(mpq_context* ctx, const Q4StreamPlan& pl, const
 #else
     const Q4StreamLaunch& p = p_in;
 #endif
-    cudaError_t e = pl.G == 2 ? q4_stream_launch_t<2>(ctx->device, p, grid, pl.smem, ctx->pdl, s) : q4_stream_launch_t<1>(ctx->device, p, grid, pl.smem, ctx->pdl, s);
+    cudaError_t e = pl.G == 4 ? q4_stream_launch_g<4>(ctx->device, p, swiglu, grid, pl.smem, ctx->pdl, s)
+                  : pl.G == 2 ? q4_stream_launch_g<2>(ctx->device, p, swiglu, grid, pl.smem, ctx->pdl, s)
+                              : q4_stream_launch_g<1>(ctx->device, p, swiglu, grid, pl.smem, ctx->pdl, s);
     ctx->launches += 1;
     if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4_stream_kernel launch failed: %s", cudaGetErrorString(e));
     return MPQ_OK;
@@ -607,7 +627,7 @@ static int32_t q4_stream_forward(mpq_context* ctx, const Q4Dev& q, const Q4Strea
         for (int r = 0; r < ex->world; ++r) p.xpeer[r] = ex->peer[r] + half;
         p.xmine = p.xpeer[ex->rank];
     }
-    return q4_stream_enqueue(ctx, pl, p, grid, s);
+    return q4_stream_enqueue(ctx, pl, p, false, grid, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -1129,8 +1149,7 @@ extern "C" int32_t mpq_q4_linear_forward_swiglu(mpq_context* ctx, const mpq_weig
         const int grid = q4_stream_params(ctx, q, pl, gate_up_dev, (int)M, y_dev, q.N, &p);
         if ((st = q4_stream_scratch(ctx, grid))) return st;
         p.partials = ctx->q4_partials; p.status = ctx->q4_status;
-        p.swiglu = 1;
-        return q4_stream_enqueue(ctx, pl, p, grid, s);
+        return q4_stream_enqueue(ctx, pl, p, true, grid, s);
     }
     q4_reserve(ctx, w, M, true, s);
     if (const int pairs = q4_gemm_route(ctx, q, M)) return q4_gemm_slabs(ctx, q, gate_up_dev, true, M, y_dev, q.N, pairs, s);
@@ -1229,7 +1248,7 @@ extern "C" int32_t mpq_q4_linear_forward_static(mpq_context* ctx, const mpq_weig
             return fail(ctx, MPQ_ERR_UNSUPPORTED, "this launch needs %d scratch slots, the static array holds %d", grid, Q4_STATIC_MAX_CTAS);
         p.partials = reinterpret_cast<uint2*>(base + 256);
         p.status = status_dev ? status_dev : reinterpret_cast<int*>(base);
-        if ((st = q4_stream_enqueue(ctx, pl, p, grid, s))) return st;
+        if ((st = q4_stream_enqueue(ctx, pl, p, false, grid, s))) return st;
     }
     return MPQ_OK;
 }

@@ -454,6 +454,12 @@ __global__ void __launch_bounds__(Q4_THREADS) q4_linear_kernel(const Q4Launch p)
 // to y.  A tile shared by warps of one CTA is summed through shared memory, in
 // warp order, when the CTA has drained its runs.  A tile cut by the boundary
 // between two CTAs is finished through global scratch (q4s_cross_cta).
+//
+// What bounds it: up to about 10 MB per launch the fixed parts (prologue, staging of x, merge, the next launch's wait), else the run
+// itself, 43 cycles per unit and SM against 47..51 at the HBM rate.  One row takes copies of four chunks (G = 4): one barrier wait and one
+// refill for four units.  Before (two chunks per copy, waits in front of each copy's arithmetic, divisions in the prologue, one warp per shared tile
+// in the merge) / now, us per launch in a graph: 4096 x 4096 5.55 / 4.78, 12288 x 4096 8.6 / 7.85, 22016 x 4096 12.05 / 11.6, 4096 x 11008
+// 9.7 / 8.5, 1000 x 2112 6.4 / 5.3, 57344 x 8192 45.6 / 43.9, 2 rows of 4096 x 4096 7.1 / 6.6 (four chunks per copy: 6.8).
 constexpr int Q4S_WARPS = 16;                    // one CTA of sixteen warps per SM
 constexpr int Q4S_THREADS = Q4S_WARPS * 32;
 constexpr int Q4S_MAX_DEPTH = 8;                 // most ring stages per warp
@@ -463,19 +469,19 @@ constexpr size_t Q4S_SLOT_BYTES_PER_CTA = 2 * 32 * 4 * sizeof(uint2);   // two t
 
 struct Q4StreamLaunch {
     const uint4* stream;
-    const float* X;         // [M][K]; with swiglu: [M][2K] = [gate | up], and the activation is silu(gate) * up
+    const float* X;         // [M][K]; with SWIGLU: [M][2K] = [gate | up], and the activation is silu(gate) * up
     float* Y;               // [M][ldy]
     int M, N, K;
-    int swiglu;             // 1: SwiGLU is applied while the activation is staged
     int64_t ldy;
     int nchunks;            // per row pair-tile, a multiple of G
     int groups;             // nrp * nchunks / G
     int warps_total;        // W: warps that own a run (<= NW*gridDim.x, <= groups); split mode only
-    int tile_mode;          // 1: CTA b owns row pair-tiles [b*nrp/grid, (b+1)*nrp/grid) and its warps split them
-    int nrp;                // row pair-tiles
+    int tile_mode;          // 1: each CTA owns whole row pair-tiles and its warps split them: CTA b has tiles_each, the first tiles_more of them one more
+    int tiles_each, tiles_more;
+    uint32_t gpr_magic;     // ceil(2^32 / groups per row pair-tile), or 0 where a group's tile has to be found by division (q4s_tile_of)
     int depth;              // ring stages per warp (<= Q4S_MAX_DEPTH)
     int pre;                // stages copied before the dependency on the previous kernel resolves (the rest after the activation loads)
-    uint2* partials;        // [CTAs][2][32 lanes][4] (value, tag) pairs
+    uint2* partials;        // [CTAs][2][4][32 lanes] (value, tag) pairs
     int* status;            // set non-zero when a bounded wait ran out
     // row-parallel mode (xworld > 0): finished tiles are not written to Y but pushed, as (value, 1) pairs,
     // into slot [xrank] of every rank's exchange buffer; then every rank adds the xworld slots of its own
@@ -549,6 +555,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
         : "=r"(ok) : "r"(bar), "r"(parity), "r"(limit) : "memory");
     return ok != 0;
 }
+// one look, without waiting
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
 // Weights are read once per call: the copies carry an evict-first L2 policy so that they do not push the
 // (small, re-read) activations and outputs out of L2.
 __device__ __forceinline__ uint64_t l2_evict_first_policy()
@@ -562,6 +576,14 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar), "l"(policy) : "memory");
 }
+// expect the bytes and fetch them, by the thread that has `go` (predicated: a branch would bring its own reconvergence)
+__device__ __forceinline__ void bulk_refill(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar, uint64_t policy, bool go)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %5, 0;\n\t"
+                 "@p mbarrier.arrive.expect_tx.shared::cta.b64 _, [%3], %2;\n\t"
+                 "@p cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;\n\t}"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar), "l"(policy), "r"((int)go) : "memory");
+}
 
 // floor(i * groups / W); 64-bit division costs a hundred-odd instructions, and these run before a CTA's first copy,
 // so the product is divided in 32 bits whenever it fits (it does for every matrix up to a few GB)
@@ -571,6 +593,12 @@ __device__ __forceinline__ int q4s_run_start(int i, int groups, int W)
     if (prod < 0x100000000ull) return (int)((uint32_t)prod / (uint32_t)W);
     return (int)(prod / (uint64_t)W);
 }
+// Row pair-tile of group gidx.  The quotient of the magic multiplication is exact while gidx * gpr < 2^32, which the host checks.
+__host__ __device__ __forceinline__ uint32_t q4s_gpr_magic(int64_t groups, int gpr)
+{
+    return gpr > 1 && groups * gpr < ((int64_t)1 << 32) ? (uint32_t)((((uint64_t)1 << 32) + gpr - 1) / gpr) : 0u;
+}
+__device__ __forceinline__ int q4s_tile_of(int gidx, int gpr, uint32_t magic) { return magic ? (int)__umulhi((uint32_t)gidx, magic) : gidx / gpr; }
 // index of the warp whose run contains group gidx
 __device__ __forceinline__ int q4s_owner(int gidx, int groups, int W)
 {
@@ -605,24 +633,18 @@ __device__ __forceinline__ uint2 ld_tagged_sys(const uint2* p)
     return unpack_tagged(w);
 }
 
-// Write one finished row pair-tile to y.  v[tile*2+h] belongs to row tile*16 + g + 8h, activation row t.
-__device__ __forceinline__ void q4s_store_tile(const Q4StreamLaunch& p, const float (&v)[4], int rp, int lane)
+// Value q = tile*2+h of one lane of a finished row pair-tile -> y: row tile*16 + g + 8h, activation row t.
+__device__ __forceinline__ void q4s_store_value(const Q4StreamLaunch& p, float v, int q, int rp, int lane)
 {
-    const int g = lane >> 2, t = lane & 3;
-    if (t < p.M) {
+    const int g = lane >> 2, t = lane & 3, n = rp * 32 + (q >> 1) * 16 + g + 8 * (q & 1);
+    if (t < p.M && n < p.N) {
+        if (p.xworld > 0) {                      // plain peer stores over NVLink: one 8-byte store per rank
+            const size_t e = (size_t)p.xrank * p.xslot + (size_t)t * p.N + n;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            int n = rp * 32 + (q >> 1) * 16 + g + 8 * (q & 1);
-            if (n < p.N) {
-                if (p.xworld > 0) {                      // plain peer stores over NVLink: one 8-byte store per rank
-                    const size_t e = (size_t)p.xrank * p.xslot + (size_t)t * p.N + n;
-#pragma unroll
-                    for (int r = 0; r < 8; ++r)
-                        if (r < p.xworld) st_tagged_sys(p.xpeer[r] + e, v[q], 1u);
-                } else {
-                    p.Y[(size_t)t * p.ldy + n] = v[q];
-                }
-            }
+            for (int r = 0; r < 8; ++r)
+                if (r < p.xworld) st_tagged_sys(p.xpeer[r] + e, v, 1u);
+        } else {
+            p.Y[(size_t)t * p.ldy + n] = v;
         }
     }
 }
@@ -634,33 +656,28 @@ __device__ __forceinline__ void q4s_store_tile(const Q4StreamLaunch& p, const fl
 // the sum does not depend on timing, writes y, and clears the slots it consumed.  A slot is written
 // once and read once per launch, and the next launch writes only after this one has completed, so the
 // protocol needs no per-launch state (it is safe under CUDA-graph replay).
-__device__ __noinline__ void q4s_cross_cta(const Q4StreamLaunch& p, float v0, float v1, float v2, float v3, int rp, int r0,
-                                           int r1, int cta_first_rp, int lane)
+// Each of four warps does this for one value q of the tile's lanes.
+__device__ __noinline__ void q4s_cross_cta(const Q4StreamLaunch& p, float v, int q, int rp, int r0, int r1, int cta_first_rp, int lane)
 {
-    float v[4] = {v0, v1, v2, v3};
     const int W = p.warps_total;
     const int c0 = q4s_owner(r0, p.groups, W) / Q4S_WARPS;
     if ((int)blockIdx.x != c0) {
-        uint2* mine = p.partials + (((size_t)blockIdx.x * 2 + (rp == cta_first_rp ? 0 : 1)) * 32 + lane) * 4;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) st_tagged(mine + q, v[q], 1u);
+        st_tagged(p.partials + (((size_t)blockIdx.x * 2 + (rp == cta_first_rp ? 0 : 1)) * 4 + q) * 32 + lane, v, 1u);
         return;
     }
     const int c1 = q4s_owner(r1 - 1, p.groups, W) / Q4S_WARPS;
     // every later CTA starts its run inside this tile, so the tile is its first one (slot 0)
-    const uint2* src = p.partials + (((size_t)(c0 + 1) * 2) * 32 + lane) * 4;
-    for (int c = c0 + 1; c <= c1; c += 4) {                // four contributors' loads in flight at a time
-        uint2 r[4][4];
+    uint2* src = p.partials + (((size_t)(c0 + 1) * 2) * 4 + q) * 32 + lane;
+    for (int c = c0 + 1; c <= c1; c += 8) {                // eight contributors' loads in flight at a time
+        uint2 r[8];
         bool ok = false;
         for (uint32_t spin = 0; spin < Q4S_SPIN_LIMIT && !ok; ++spin) {
             ok = true;
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    r[u][q] = (c + u <= c1) ? ld_tagged(src + (size_t)u * 256 + q) : make_uint2(0u, 1u);
-                    ok = ok && (r[u][q].y == 1u);
-                }
+            for (int u = 0; u < 8; ++u) {
+                r[u] = (c + u <= c1) ? ld_tagged(src + (size_t)u * 256) : make_uint2(0u, 1u);
+                ok = ok && (r[u].y == 1u);
+            }
             ok = __all_sync(0xFFFFFFFFu, ok);
         }
         if (!ok) {
@@ -668,15 +685,13 @@ __device__ __noinline__ void q4s_cross_cta(const Q4StreamLaunch& p, float v0, fl
             return;
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                v[q] += __uint_as_float(r[u][q].x);
-                if (c + u <= c1) st_tagged(const_cast<uint2*>(src) + (size_t)u * 256 + q, 0.f, 0u);   // consumed: free the slot
-            }
-        src += 4 * 256;
+        for (int u = 0; u < 8; ++u) {
+            v += __uint_as_float(r[u].x);
+            if (c + u <= c1) st_tagged(src + (size_t)u * 256, 0.f, 0u);   // consumed: free the slot
+        }
+        src += 8 * 256;
     }
-    q4s_store_tile(p, v, rp, lane);
+    q4s_store_value(p, v, q, rp, lane);
 }
 
 // One float4 of x (element index 4f of activation row m) -> normalised hi/lo fp16 fragments in xs, block
@@ -716,50 +731,50 @@ __device__ __forceinline__ void q4s_stage_one(float4 v, bool on, int m, int f, f
     }
 }
 
-// One pass over this thread's share of x (float4 index i = m * pk4 + f over M rows of pk4 float4): returns the largest
-// |x| bit pattern seen and, if CONVERT, stages the fragments with scale sc.
-template <bool CONVERT>
+// One pass over this thread's share of x (float4 index i = m * pk4 + f over M rows of pk4 float4; ONE: M = 1): returns the largest
+// |x| bit pattern seen and, if CONVERT, stages the fragments with scale sc.  The loads of LOADS float4 per thread are on their way at a time.
+// (Four threads per 32-block with four 8-byte loads and two 16-byte stores each, instead of float4 and eight 4-byte stores, take half the
+// instructions but four times the requests to L2: 4096 x 4096 at one row 4.77 / 4.97 us, 4096 x 11008 8.49 / 9.58.)
+template <bool CONVERT, bool ONE, bool SWIGLU>
 __device__ __forceinline__ uint32_t q4s_stage_pass(const Q4StreamLaunch& p, int pk4, int total4, float sc, int ncols, uint4* xs,
-                                                   float4* cs, int tid, int lane, int threads)
+                                                   float4* cs, int tid, int lane)
 {
+    constexpr int LOADS = ONE && !SWIGLU ? 6 : 4;
     uint32_t mx = 0;
-    const int iters = (total4 + threads - 1) / threads;
-    for (int it0 = 0; it0 < iters; it0 += 4) {
-        float4 v[4];
-        int mm[4], ff[4];
-        bool on[4];
+    for (int base = 0; base < total4; base += LOADS * Q4S_THREADS) {
+        float4 v[LOADS];
+        int mm[LOADS], ff[LOADS];
+        bool on[LOADS];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {                      // up to four loads in flight per thread
-            const int i = (it0 + u) * threads + tid;
-            on[u] = it0 + u < iters && i < total4;
+        for (int u = 0; u < LOADS; ++u) {
+            const int i = base + u * Q4S_THREADS + tid;
+            on[u] = i < total4;
             const int ii = on[u] ? i : 0;
-            mm[u] = (ii >= pk4) + (ii >= 2 * pk4) + (ii >= 3 * pk4);       // M <= 4
+            mm[u] = ONE ? 0 : (ii >= pk4) + (ii >= 2 * pk4) + (ii >= 3 * pk4);       // M <= 4
             ff[u] = ii - mm[u] * pk4;
             v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
             if (on[u] && 4 * ff[u] < p.K) {
-                if (p.swiglu) {
-                    const float* row = p.X + (size_t)mm[u] * 2 * p.K + 4 * ff[u];
-                    v[u] = swiglu_f32x4(*reinterpret_cast<const float4*>(row), *reinterpret_cast<const float4*>(row + p.K));
-                } else {
-                    v[u] = *reinterpret_cast<const float4*>(p.X + (size_t)mm[u] * p.K + 4 * ff[u]);
-                }
+                const float* row = p.X + (ONE ? 0 : (size_t)mm[u] * (SWIGLU ? 2 : 1) * p.K) + 4 * ff[u];
+                v[u] = *reinterpret_cast<const float4*>(row);
+                if (SWIGLU) v[u] = swiglu_f32x4(v[u], *reinterpret_cast<const float4*>(row + p.K));
             }
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            if ((it0 + u) * threads >= total4) break;       // the same for the whole CTA: nothing left to stage
+        for (int u = 0; u < LOADS; ++u) {
+            if (base + u * Q4S_THREADS >= total4) break;    // the same for the whole CTA: nothing left to stage
             mx = max(mx, __float_as_uint(v[u].x) & 0x7FFFFFFFu);
             mx = max(mx, __float_as_uint(v[u].y) & 0x7FFFFFFFu);
             mx = max(mx, __float_as_uint(v[u].z) & 0x7FFFFFFFu);
             mx = max(mx, __float_as_uint(v[u].w) & 0x7FFFFFFFu);
-            if (CONVERT) q4s_stage_one(v[u], on[u], mm[u], ff[u], sc, ncols, p.M, xs, cs, lane);
+            if (CONVERT) q4s_stage_one(v[u], on[u], mm[u], ff[u], sc, ncols, ONE ? 1 : p.M, xs, cs, lane);
         }
     }
     return mx;
 }
 
 // dynamic shared memory: ring [16 warps][depth][G units] | xs | cs | mbarriers | wpart (the warps' parked partial tiles)
-template <int G>
+// ONE: a single activation row.  SWIGLU: X is [M][2K] = [gate | up] and silu(gate) * up is what gets staged.
+template <int G, bool ONE, bool SWIGLU>
 __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_constant__ Q4StreamLaunch p)
 {
     constexpr int STAGE_BYTES = G * Q4_UNIT_BYTES;
@@ -770,7 +785,7 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
     __shared__ uint4 zero_pg[2];                  // what lanes outside the 2M real columns read
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    const int M = p.M, ncols = 2 * M, D = p.depth;
+    const int M = ONE ? 1 : p.M, ncols = 2 * M, D = p.depth;
     Q4S_TRACE(0)
     if (lane < 2) wrp[warp][lane] = -1;
     if (tid < 2) zero_pg[tid] = make_uint4(0, 0, 0, 0);
@@ -785,10 +800,12 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
     const int gpr = p.nchunks / G;                            // groups per row pair-tile
     int cta_gb, cta_ge, gb, ge;
     if (p.tile_mode) {
-        cta_gb = q4s_run_start((int)blockIdx.x, p.nrp, (int)gridDim.x) * gpr;
-        cta_ge = q4s_run_start((int)blockIdx.x + 1, p.nrp, (int)gridDim.x) * gpr;
-        gb = cta_gb + q4s_run_start(warp, cta_ge - cta_gb, NW);
-        ge = cta_gb + q4s_run_start(warp + 1, cta_ge - cta_gb, NW);
+        const int b = (int)blockIdx.x, first = b * p.tiles_each + min(b, p.tiles_more);
+        cta_gb = first * gpr;
+        cta_ge = (first + p.tiles_each + (b < p.tiles_more)) * gpr;
+        const int n = cta_ge - cta_gb;                        // (fewer groups than warps: the first n take one each, so that a tile's sharers are consecutive)
+        gb = cta_gb + (n < NW ? min(warp, n) : q4s_run_start(warp, n, NW));
+        ge = cta_gb + (n < NW ? min(warp + 1, n) : q4s_run_start(warp + 1, n, NW));
     } else {
         cta_gb = q4s_run_start(min(W, (int)blockIdx.x * NW), p.groups, W);
         cta_ge = q4s_run_start(min(W, (int)(blockIdx.x + 1) * NW), p.groups, W);
@@ -796,7 +813,8 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
         ge = gw < W ? q4s_run_start(gw + 1, p.groups, W) : 0;
     }
     const int ngroups = ge - gb;
-    const unsigned char* gnext = reinterpret_cast<const unsigned char*>(p.stream) + (size_t)gb * STAGE_BYTES;
+    const unsigned char* run = reinterpret_cast<const unsigned char*>(p.stream) + (size_t)gb * STAGE_BYTES;
+    const unsigned char* gnext = run + (size_t)D * STAGE_BYTES;      // what a drained stage is filled with
     const uint32_t ring_u32 = smem_u32(ring), bars_u32 = smem_u32(bars);
     Q4S_TRACE(1)
 
@@ -805,7 +823,7 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
-    int issued = 0;
+    int issued = 0;                                           // (lane 0's)
     const uint64_t l2pol = l2_evict_first_policy();
     // p.pre stages go out before the dependency on the previous kernel resolves, the rest of the ring right after the
     // activation loads have been issued.
@@ -813,8 +831,7 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
         if (lane == 0) {
             for (; issued < n; ++issued) {
                 mbar_expect_tx(bars_u32 + issued * 8, STAGE_BYTES);
-                bulk_g2s(ring_u32 + issued * STAGE_BYTES, gnext, STAGE_BYTES, bars_u32 + issued * 8, l2pol);
-                gnext += STAGE_BYTES;
+                bulk_g2s(ring_u32 + issued * STAGE_BYTES, run + issued * STAGE_BYTES, STAGE_BYTES, bars_u32 + issued * 8, l2pol);
             }
         }
     };
@@ -831,8 +848,7 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
     // [1, 2^15) (the split is then good to 2^-25 of it); otherwise, and for several rows, a second pass stages with the scale.
     const int pk4 = p.nchunks * 16;                       // float4 per activation row, padding included
     const int total4 = M * pk4;
-    uint32_t mx = M == 1 ? q4s_stage_pass<true>(p, pk4, total4, 1.f, ncols, xs, cs, tid, lane, THREADS)
-                         : q4s_stage_pass<false>(p, pk4, total4, 1.f, ncols, xs, cs, tid, lane, THREADS);
+    uint32_t mx = q4s_stage_pass<ONE, ONE, SWIGLU>(p, pk4, total4, 1.f, ncols, xs, cs, tid, lane);
     issue_upto(min(D, ngroups));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
@@ -842,7 +858,7 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
 #pragma unroll
     for (int w = 1; w < NW; ++w) mx = max(mx, s_max[w]);
     float inv_sc = 1.f;
-    if (M > 1 || (mx != 0 && (mx < 0x3F800000u || mx >= 0x47000000u))) {      // 1.0, 2^15
+    if (!ONE || (mx != 0 && (mx < 0x3F800000u || mx >= 0x47000000u))) {       // 1.0, 2^15
         int emax = (int)(mx >> 23);
         float sc = 1.f;
         if (mx != 0 && emax < 255) {
@@ -850,7 +866,7 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
             sc = __uint_as_float((uint32_t)(268 - emax) << 23);
             inv_sc = __uint_as_float((uint32_t)(emax - 14) << 23);
         }
-        q4s_stage_pass<true>(p, pk4, total4, sc, ncols, xs, cs, tid, lane, THREADS);
+        q4s_stage_pass<true, ONE, SWIGLU>(p, pk4, total4, sc, ncols, xs, cs, tid, lane);
         __syncthreads();
     }
     Q4S_TRACE(4)
@@ -859,7 +875,7 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
     const float fA = 16777216.f * inv_sc;                     // 2^24: undo the subnormal weight encoding
     const float fB = 1048576.f * inv_sc;                      // 2^20: rows g+8 carry an extra factor 16
     float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-    int rp = gb / gpr;
+    int rp = q4s_tile_of(gb, gpr, p.gpr_magic);
     int cg = gb - rp * gpr;                                   // group index inside the tile
     const int first_rp = rp;
     // per-lane shared-memory addresses into the staged activation; lanes outside the real columns sit on a page of zeros
@@ -881,7 +897,8 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
         float v[4] = {acc[0][0] * fA, acc[0][1] * fB, acc[1][0] * fA, acc[1][1] * fB};
         const int r0 = tile_rp * gpr;
         if (gb <= r0 && r0 + gpr <= ge) {
-            q4s_store_tile(p, v, tile_rp, lane);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) q4s_store_value(p, v[q], q, tile_rp, lane);
         } else {
             const int slot = tile_rp == first_rp ? 0 : 1;
 #pragma unroll
@@ -895,20 +912,24 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
     const long long cyc_loop0 = clock64();
 #endif
 
+    // The look at the next stage's barrier is a round trip of about 90 cycles: it is taken while this stage's last unit is multiplied.
+    bool ready = false;
     for (int j = 0; j < ngroups; ++j) {
         Q4S_CYC(c_w)
-        const bool arrived = mbar_wait(bars_u32 + s * 8, parity, Q4S_SPIN_LIMIT);
+        const bool arrived = ready || mbar_wait(bars_u32 + s * 8, parity, Q4S_SPIN_LIMIT);
         Q4S_CYC_ADD(cyc_wait, c_w)
         if (!arrived) {
             // Record it, issue nothing more, and give every copy still in flight the same generous bounded wait, so
             // that none lands in shared memory after this CTA has left (if one still does not arrive, the hazard stays).
             if (lane == 0) {
                 atomicExch(p.status, 1);
-                for (int idx = j + 1; idx < issued; ++idx) mbar_wait(bars_u32 + (idx % D) * 8, (uint32_t)(idx / D) & 1u, Q4S_SPIN_LIMIT);
+                for (int idx = j + 1; idx < min(ngroups, j + D); ++idx) mbar_wait(bars_u32 + (idx % D) * 8, (uint32_t)(idx / D) & 1u, Q4S_SPIN_LIMIT);
             }
             timed_out = true;
             break;
         }
+        const int next_s = s + 1 == D ? 0 : s + 1;
+        const uint32_t next_parity = next_s ? parity : parity ^ 1u;
         const uint32_t st = s * STAGE_BYTES;
 #pragma unroll
         for (int q = 0; q < G; ++q) {
@@ -919,6 +940,7 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
             const float4 cf = make_float4(__uint_as_float(cfu.x), __uint_as_float(cfu.y), __uint_as_float(cfu.z), __uint_as_float(cfu.w));
             xsp += xstep;
             csp += cstep;
+            if (q == G - 1) ready = mbar_test(bars_u32 + next_s * 8, next_parity);
             const uint32_t wt[2][4] = {{w0.x, w0.y, w0.z, w0.w}, {w1.x, w1.y, w1.z, w1.w}};
             const uint32_t sw[2][2] = {{sv.x, sv.y}, {sv.z, sv.w}};
 #pragma unroll
@@ -941,13 +963,8 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
         ++cg;
         Q4S_CYC(c_r)
         __syncwarp();
-        if (lane == 0 && issued < ngroups) {               // refill the stage just drained
-            mbar_expect_tx(bars_u32 + s * 8, STAGE_BYTES);
-            bulk_g2s(ring_u32 + s * STAGE_BYTES, gnext, STAGE_BYTES, bars_u32 + s * 8, l2pol);
-            gnext += STAGE_BYTES;
-            ++issued;
-        }
-        __syncwarp();
+        bulk_refill(ring_u32 + s * STAGE_BYTES, gnext, STAGE_BYTES, bars_u32 + s * 8, l2pol, lane == 0 && j + D < ngroups);    // the stage just drained
+        gnext += STAGE_BYTES;
         Q4S_CYC_ADD(cyc_refill, c_r)
 #ifdef MPQ_TRACE
         if (j == 0) cyc_first = clock64() - cyc_loop0;
@@ -960,7 +977,8 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
             xsp = xs0;
             csp = cs0;
         }
-        if (++s == D) { s = 0; parity ^= 1u; }
+        s = next_s;
+        parity = next_parity;
     }
     if (cg != 0 && !timed_out) flush(rp);  // the run ended inside a row pair-tile
 #ifdef MPQ_TRACE
@@ -974,30 +992,30 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
     __syncthreads();
     Q4S_TRACE(6)
 
-    // ---- tiles shared between warps: add the parked partials in warp order.  Segment (w, slot) opens a
-    // tile if the valid segment before it belongs to another tile; its warp then sums the following ones.
-    const int cta_first_rp = cta_gb / gpr;
+    // ---- tiles shared between warps: add the parked partials in warp order.  Segment (w, slot) opens a tile if no segment before it
+    // belongs to the same one; four warps then add the tile's segments, one of its four values per lane each (one warp for all four, and a
+    // search for each segment, took 0.9..1.8 us).  The sharers are consecutive warps, and all but the first have the tile in slot 0.
     const int entry = wrp[lane >> 1][lane & 1];             // lane i holds segment i = (warp i/2, slot i%2)
+    const uint32_t peers = __match_any_sync(0xFFFFFFFFu, entry);
+    uint32_t openers = __ballot_sync(0xFFFFFFFFu, entry >= 0 && (peers & ((1u << lane) - 1u)) == 0);
+    const int cta_first_rp = q4s_tile_of(cta_gb, gpr, p.gpr_magic), q = warp & 3;
+    for (int skip = warp >> 2; openers; openers &= openers - 1u) {
+        if (skip--) continue;
+        skip = NW / 4 - 1;
+        const int first = __ffs(openers) - 1, my = __shfl_sync(0xFFFFFFFFu, entry, first), count = __popc(__shfl_sync(0xFFFFFFFFu, peers, first));
+        const float* src = wpart + q * 32 + lane;
+        float v = src[first * 128];
+        src += (first & ~1) * 128;
+        for (int k = 1; k < count; k += 8) {
+            float u[8];
 #pragma unroll
-    for (int slot = 0; slot < 2; ++slot) {
-        const int idx0 = warp * 2 + slot;
-        const int my = __shfl_sync(0xFFFFFFFFu, entry, idx0);
-        if (my < 0) continue;
-        uint32_t same = __ballot_sync(0xFFFFFFFFu, entry == my);
-        if (same & ((1u << idx0) - 1u)) continue;           // an earlier warp opened this tile
-        float v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;
-        for (; same; same &= same - 1u) {                   // ascending segment order: a fixed summation order
-            const int idx = __ffs(same) - 1;
-            const float* src = wpart + (size_t)idx * 128 + lane;
-            v0 += src[0]; v1 += src[32]; v2 += src[64]; v3 += src[96];
+            for (int i = 0; i < 8; ++i) u[i] = k + i < count ? src[(k + i) * 256] : 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v += u[i];
         }
         const int r0 = my * gpr, r1 = r0 + gpr;
-        if (cta_gb <= r0 && r1 <= cta_ge) {
-            const float v[4] = {v0, v1, v2, v3};
-            q4s_store_tile(p, v, my, lane);
-        } else {
-            q4s_cross_cta(p, v0, v1, v2, v3, my, r0, r1, cta_first_rp, lane);
-        }
+        if (cta_gb <= r0 && r1 <= cta_ge) q4s_store_value(p, v, q, my, lane);
+        else q4s_cross_cta(p, v, q, my, r0, r1, cta_first_rp, lane);
     }
 
     Q4S_TRACE(7)
