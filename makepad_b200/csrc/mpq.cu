@@ -51,13 +51,14 @@ struct mpq_context {
     bool q4_rect;             // use the rectangle kernel for 5..16 rows (else slabs of <= 4 rows through the streaming kernel)
     int q4_stream_max_m;      // most activation rows mpq_q4_linear_forward gives to the streaming kernel (1..4)
     int q4_rect_nks;          // experiment: at least so many K slices in the rectangle kernel (0 = the plan's choice)
+    bool q4_rect_cluster;     // K slices of the rectangle kernel as clusters where they fit
     int q4_rect_depth;        // ring depth of the rectangle kernel: 0 = choose, else 1..8
     uint2* q4_partials;
     int q4_partials_ctas;
     int* q4_status;
     bool q4_stream;           // use the streaming kernel where the activation fits in shared memory
     bool q4_tile_mode;        // let CTAs own whole row pair-tiles when the matrix has enough of them
-    int q4_group;             // chunks per bulk copy of the streaming kernel: 0 = choose, 1 or 2
+    int q4_group;             // chunks per bulk copy of the streaming kernel: 0 = choose, 1, 2 or 4
     int q4_depth;             // most ring stages per warp
     int q4_pre;               // stages copied before the dependency resolves (the rest right after the activation loads)
     bool q4_slab4;            // M > 4 as slabs of four rows through the streaming kernel
@@ -189,6 +190,8 @@ extern "C" int32_t mpq_context_create(int32_t device, mpq_context** out)
     c->q4_stream_max_m = (e && e[0] >= '1' && e[0] <= '4') ? e[0] - '0' : 4;
     e = getenv("MPQ_Q4_RECT_NKS");
     c->q4_rect_nks = e ? atoi(e) : 0;
+    e = getenv("MPQ_Q4_RECT_CLUSTER");
+    c->q4_rect_cluster = !(e && e[0] == '0');
     e = getenv("MPQ_Q4_RECT_DEPTH");
     c->q4_rect_depth = (e && e[0] >= '1' && e[0] <= '8') ? e[0] - '0' : 0;
     e = getenv("MPQ_Q4_SLAB4");
@@ -633,7 +636,37 @@ static int32_t q4_stream_forward(mpq_context* ctx, const Q4Dev& q, const Q4Strea
 // ---------------------------------------------------------------------------
 // the rectangle kernel: up to 16 rows, any K, weights read once
 // ---------------------------------------------------------------------------
-struct Q4RectPlan { int mt, depth, slice_chunks, nks, ntg; size_t smem; };
+struct Q4RectPlan { int mt, depth, slice_chunks, nks, ntg; bool cluster; size_t smem; };
+
+// Clusters of `size` CTAs of the rectangle kernel (one per SM) that the device keeps resident at once.
+static int q4_rect_clusters(int device, int size)
+{
+    static int most[PerDeviceOnce::MAX_DEVICES][Q4R_MAX_CLUSTER + 1];
+    static PerDeviceOnce known;
+    int* n = most[device >= 0 && device < PerDeviceOnce::MAX_DEVICES ? device : 0];
+    if (known.needs(device)) {
+        auto kern = q4_rect_kernel<4>;
+        const size_t smem = (size_t)120 * 1024;            // more than half of an SM's, as the register file
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227 * 1024 - 1024));
+        for (int c = 2; c <= Q4R_MAX_CLUSTER; ++c) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(1024, (unsigned)c);
+            cfg.blockDim = dim3(Q4R_THREADS);
+            cfg.dynamicSmemBytes = smem;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = (unsigned)c; at[0].val.clusterDim.z = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            int found = 0;
+            if (e != cudaSuccess || cudaOccupancyMaxActiveClusters(&found, kern, &cfg) != cudaSuccess) { cudaGetLastError(); found = 0; }
+            n[c] = found;
+        }
+        known.mark(device);
+    }
+    return n[size];
+}
+
 static bool q4_rect_plan(const mpq_context* ctx, const Q4Dev& q, int M, Q4RectPlan* pl)
 {
     if (M < 1 || M > 16) return false;
@@ -641,41 +674,47 @@ static bool q4_rect_plan(const mpq_context* ctx, const Q4Dev& q, int M, Q4RectPl
     const int sms = ctx->prop.multiProcessorCount;
     const size_t per_chunk = (size_t)2 * mp * 128 + (size_t)2 * mp * 8;          // fragments + corrections
     const size_t wpart = (size_t)Q4R_WARPS * (4 * mt) * 32 * 4, bars = (size_t)Q4R_WARPS * Q4S_MAX_DEPTH * 8;
-    const size_t total = (size_t)227 * 1024 - 512;
+    const size_t total = (size_t)227 * 1024 - 1024;
     // The deeper ring first (measured: two stages per warp with more K slices beat one stage with fewer);
     // MPQ_Q4_RECT_DEPTH pins the ring depth.
-    bool found = false;
     for (int depth = ctx->q4_rect_depth ? std::min(ctx->q4_rect_depth, (int)Q4S_MAX_DEPTH) : 2; depth >= 1; --depth) {
         if (ctx->q4_rect_depth && depth != ctx->q4_rect_depth) continue;
         const size_t ring = (size_t)Q4R_WARPS * depth * Q4R_STAGE_BYTES;
         if (ring + wpart + bars + per_chunk * Q4R_G > total) continue;
         int max_slice = (int)((total - ring - wpart - bars) / per_chunk) / Q4R_G * Q4R_G;
-        // K slices.  More of them shorten what every CTA stages of x and lengthen the reduction of the slices, and the
-        // split has to divide the chunks and the tiles evenly over the SMs: the candidates' cost is estimated from measured
-        // rates (microseconds: main loop per tile and chunk by MMA tile count, staging per row and chunk, reduction per
-        // output element and slice) and the cheapest is taken.
+        // K slices.  More of them shorten what every CTA stages of x and lengthen the sum of the slices, clusters of them leave SMs
+        // idle (74 of two, 45 of three, 33 of four, 26, 22, 15, 15 of eight), and the split has to divide the chunks and the tiles
+        // evenly.  The candidates' cost is estimated and the cheapest is taken: microseconds, fitted to 418 measured calls (2 to 16 rows
+        // of 512 x 1024 to 57344 x 8192 in every split; what it takes is 0.6 % slower than the best of them on average, at most 6 %):
+        // main loop per unit of the longest warp's run by MMA tile count; staging per row and chunk, and once more where a
+        // thread's registers do not hold its part of it; for the slices' sum what a cluster sends, or a second launch and its reads.
         const int nks_min = (q.nchunks + max_slice - 1) / max_slice;
         const int nks_max = std::max(nks_min, std::min(16, q.nchunks / (2 * Q4R_G)));
-        static const double c_main[4] = {0.035, 0.050, 0.070, 0.089};
-        int nks = nks_min, slice = 0;
+        static const double c_main[4] = {0.0285, 0.037, 0.048, 0.058};
         double best_cost = 1e30;
         for (int cand = nks_min; cand <= nks_max; ++cand) {
             if (ctx->q4_rect_nks > 0 && cand != std::min(std::max(ctx->q4_rect_nks, nks_min), nks_max)) continue;
             const int sl = ((q.nchunks + cand - 1) / cand + Q4R_G - 1) / Q4R_G * Q4R_G;
             const int real = (q.nchunks + sl - 1) / sl;
-            const int tg = std::max(1, std::min(q.nrp, sms / real));
-            const int tiles = (q.nrp + tg - 1) / tg;
-            const double cost = c_main[mt - 1] * tiles * sl + 0.012 * mp * sl + (real > 1 ? 5e-6 * real * (double)M * (double)q.N : 0.0);
-            if (cost < best_cost) { best_cost = cost; nks = real; slice = sl; }
+            if (real > sms) continue;                      // (cannot happen for K below a few million)
+            for (int cluster = 0; cluster <= (real > 1 && real <= Q4R_MAX_CLUSTER && ctx->q4_rect_cluster); ++cluster) {
+                const int room = cluster ? q4_rect_clusters(ctx->device, real) : sms / real;
+                if (room < 1) continue;
+                const int tg = std::max(1, std::min(q.nrp, room)), tiles = (q.nrp + tg - 1) / tg;
+                const size_t smem = ring + per_chunk * sl + wpart + bars + (cluster ? 16 + (size_t)(tiles * mt + real - 1) / real * real * 512 : 0);
+                if (smem > total) continue;
+                const int run = (tiles * (sl / Q4R_G) + Q4R_WARPS - 1) / Q4R_WARPS * Q4R_G;
+                const double cost = c_main[mt - 1] * Q4R_WARPS * run + 0.0116 * mp * sl + (mp * sl > Q4R_CACHE * Q4R_THREADS / 16 ? 1.6 : 0.0) +
+                                    (cluster ? 0.95 + 0.012 * tiles * mp : real > 1 ? 3.3 + 2.3e-6 * real * (double)M * (double)q.N : 0.0);
+                if (cost < best_cost) {
+                    best_cost = cost;
+                    pl->mt = mt; pl->depth = depth; pl->slice_chunks = sl; pl->nks = real; pl->ntg = tg; pl->cluster = cluster != 0; pl->smem = smem;
+                }
+            }
         }
-        if (nks > sms) continue;                           // (cannot happen for K below a few million)
-        if (found) continue;
-        found = true;
-        pl->mt = mt; pl->depth = depth; pl->slice_chunks = slice; pl->nks = nks;
-        pl->ntg = std::max(1, std::min(q.nrp, sms / nks));
-        pl->smem = ring + per_chunk * slice + wpart + bars;
+        if (best_cost < 1e30) return true;
     }
-    return found;
+    return false;
 }
 
 static void q4_note_needs(const mpq_context* ctx, mpq_weight* w)
@@ -685,30 +724,36 @@ static void q4_note_needs(const mpq_context* ctx, mpq_weight* w)
     w->q4_rect_partial = 0;
     Q4RectPlan pl;
     for (int M = 2; M <= 16 && ctx->q4_rect; ++M)
-        if (q4_rect_plan(ctx, w->q4, M, &pl) && pl.nks > 1)
+        if (q4_rect_plan(ctx, w->q4, M, &pl) && pl.nks > 1 && !pl.cluster)
             w->q4_rect_partial = std::max(w->q4_rect_partial, (size_t)pl.nks * M * w->q4.N * sizeof(float));
 }
 
 template <int MT>
-static cudaError_t q4_rect_launch_t(int device, const Q4RectLaunch& p, int grid, size_t smem, bool pdl, cudaStream_t s)
+static cudaError_t q4_rect_launch_t(int device, const Q4RectLaunch& p, int groups, size_t smem, bool pdl, cudaStream_t s)
 {
     auto kern = q4_rect_kernel<MT>;
     static PerDeviceOnce configured;
     if (configured.needs(device)) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227 * 1024 - 512));
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227 * 1024 - 1024));
         if (e != cudaSuccess) return e;
         configured.mark(device);
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
+    cfg.gridDim = dim3((unsigned)groups, (unsigned)p.nks);
     cfg.blockDim = dim3(Q4R_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
+    int na = pdl ? 1 : 0;
+    if (p.cluster) {
+        at[na].id = cudaLaunchAttributeClusterDimension;
+        at[na].val.clusterDim.x = 1; at[na].val.clusterDim.y = (unsigned)p.nks; at[na].val.clusterDim.z = 1;
+        ++na;
+    }
     cfg.attrs = at;
-    cfg.numAttrs = pdl ? 1u : 0u;
+    cfg.numAttrs = (unsigned)na;
     return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
@@ -727,23 +772,29 @@ static int32_t q4_rect_forward(mpq_context* ctx, const Q4Dev& q, const Q4RectPla
 {
     int32_t st = q4_status_word(ctx);
     if (st) return st;
-    if (pl.nks > 1) CU_TRY(ctx, ctx->q4_partial.reserve((size_t)pl.nks * M * q.N * sizeof(float)));
+    const bool sum = pl.nks > 1 && !pl.cluster;            // the slices go through memory
+    if (sum) CU_TRY(ctx, ctx->q4_partial.reserve((size_t)pl.nks * M * q.N * sizeof(float)));
     Q4RectLaunch p;
     p.stream = q.stream; p.X = x; p.Y = y; p.partial = ctx->q4_partial.as<float>();
     p.M = M; p.N = (int)q.N; p.K = (int)q.K; p.ldy = ldy;
-    p.nchunks = q.nchunks; p.nrp = q.nrp; p.ntg = pl.ntg; p.nks = pl.nks; p.slice_chunks = pl.slice_chunks; p.depth = pl.depth;
-    p.status = ctx->q4_status;
-    const int grid = pl.ntg * pl.nks;
+    p.nchunks = q.nchunks; p.tiles_each = q.nrp / pl.ntg; p.tiles_more = q.nrp % pl.ntg; p.nks = pl.nks; p.slice_chunks = pl.slice_chunks;
+    const int last = q.nchunks - (pl.nks - 1) * pl.slice_chunks, mp = 4 * pl.mt;
+    const int64_t tiles = p.tiles_each + 1;
+    p.gpr_magic = q4s_gpr_magic(tiles * (pl.slice_chunks / Q4R_G), pl.slice_chunks / Q4R_G); p.gpr_magic_last = q4s_gpr_magic(tiles * (last / Q4R_G), last / Q4R_G);
+    p.pk4_magic = q4s_gpr_magic((int64_t)mp * pl.slice_chunks * 16 + Q4R_THREADS * Q4R_CACHE, pl.slice_chunks * 16);
+    p.pk4_magic_last = q4s_gpr_magic((int64_t)mp * last * 16 + Q4R_THREADS * Q4R_CACHE, last * 16);
+    p.nks_magic = q4s_gpr_magic(tiles * pl.mt, pl.nks);
+    p.cluster = pl.cluster; p.depth = pl.depth; p.status = ctx->q4_status;
     cudaError_t e;
     switch (pl.mt) {
-        case 1: e = q4_rect_launch_t<1>(ctx->device, p, grid, pl.smem, ctx->pdl, s); break;
-        case 2: e = q4_rect_launch_t<2>(ctx->device, p, grid, pl.smem, ctx->pdl, s); break;
-        case 3: e = q4_rect_launch_t<3>(ctx->device, p, grid, pl.smem, ctx->pdl, s); break;
-        default: e = q4_rect_launch_t<4>(ctx->device, p, grid, pl.smem, ctx->pdl, s); break;
+        case 1: e = q4_rect_launch_t<1>(ctx->device, p, pl.ntg, pl.smem, ctx->pdl, s); break;
+        case 2: e = q4_rect_launch_t<2>(ctx->device, p, pl.ntg, pl.smem, ctx->pdl, s); break;
+        case 3: e = q4_rect_launch_t<3>(ctx->device, p, pl.ntg, pl.smem, ctx->pdl, s); break;
+        default: e = q4_rect_launch_t<4>(ctx->device, p, pl.ntg, pl.smem, ctx->pdl, s); break;
     }
     ctx->launches += 1;
     if (e != cudaSuccess) return fail(ctx, MPQ_ERR_CUDA, "q4_rect_kernel launch failed: %s", cudaGetErrorString(e));
-    if (pl.nks > 1) {
+    if (sum) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)((q.N + 4 * Q4R_REDUCE_THREADS - 1) / (4 * Q4R_REDUCE_THREADS)), (unsigned)M);
         cfg.blockDim = dim3(Q4R_REDUCE_THREADS);
