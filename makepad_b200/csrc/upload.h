@@ -22,6 +22,15 @@
 
 namespace mpq {
 
+// memory that the driver can copy from by itself: page-locked, managed, or (given for host memory) device memory
+inline bool driver_knows(const void* p)
+{
+    cudaPointerAttributes a = {};
+    if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type != cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    return false;
+}
+
 class StagedUpload {
 public:
     static constexpr int SLOTS = 4;
@@ -36,7 +45,7 @@ public:
         Result result = OK;
         cudaError_t e = cudaSuccess;
         if (src) {
-            const bool first = known(src), last = known(static_cast<const char*>(src) + (bytes - 1));
+            const bool first = driver_knows(src), last = driver_knows(static_cast<const char*>(src) + (bytes - 1));
             if (first && last) {
                 // By the legacy stream, as any cudaMemcpy: behind the copies that may still be filling the array.
                 e = cudaStreamSynchronize(stream);
@@ -107,15 +116,6 @@ public:
     }
 
 private:
-    // memory that the driver can copy from by itself: page-locked, managed, or (given for host memory) device memory
-    static bool known(const void* p)
-    {
-        cudaPointerAttributes a = {};
-        if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type != cudaMemoryTypeUnregistered;
-        cudaGetLastError();
-        return false;
-    }
-
     struct Slot {
         void* mem = nullptr;
         bool locked = false;
