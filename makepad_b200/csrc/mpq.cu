@@ -1827,6 +1827,7 @@ extern "C" int32_t mpq_weight_load(mpq_context* ctx, const char* path, mpq_weigh
         w->fp4.N = h.N; w->fp4.K = h.K; w->fp4.tensor_scale = h.tensor_scale; w->fp4.sf_tiled_bytes = (size_t)h.bytes_b;
         if (e == cudaSuccess) e = cudaMalloc(&w->fp4.codes, (size_t)h.bytes_a);
         if (e == cudaSuccess) e = cudaMalloc(&w->fp4.sf_tiled, (size_t)h.bytes_b);
+        if (e == cudaSuccess) nvfp4_weight_map(w->fp4);
     }
     // The payload goes straight to where the weight lives; the checksum is taken there, of what arrived, and no weight is
     // handed out before it agrees.

@@ -22,6 +22,8 @@ struct Nvfp4Dev {
     uint8_t* codes = nullptr;          // canonical [N][K/2]: already K-major, which is what the MMA wants
     uint8_t* sf_tiled = nullptr;       // scale factors in the 128x4 tile order the tensor core reads (the only copy)
     size_t sf_tiled_bytes = 0;
+    CUtensorMap map_first = {}, map_second = {};     // the codes as nvfp4_rows_kernel fetches them: K blocks of 128 and of 96 rows
+    bool mapped = false;
     size_t device_bytes() const { return (size_t)N * (K / 2) + sf_tiled_bytes; }
     void release()
     {
@@ -48,6 +50,9 @@ size_t nvfp4_sf_tiled_bytes(int64_t N, int64_t K);
 void nvfp4_weight_dequant_launch(const Nvfp4Dev& w, float* out, cudaStream_t s);
 int32_t nvfp4_gemm_launch(Nvfp4Scratch& scratch, const Nvfp4Dev& w, const uint8_t* a_codes, const uint8_t* a_sf, float ta,
                           int64_t M, uint16_t* c, int device, int sm_count, bool pdl, cudaStream_t s, int* launches, std::string& err);
+
+// the maps of a weight whose codes are in place (none where the driver makes none: its calls then take the other kernels)
+void nvfp4_weight_map(Nvfp4Dev& w);
 
 // TMA map of a Q4 tile stream (see Q4Dev::map)
 bool make_q4_stream_map(CUtensorMap* map, const void* stream, int nrp, int nchunks);
