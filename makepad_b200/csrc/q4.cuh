@@ -459,7 +459,8 @@ __global__ void __launch_bounds__(Q4_THREADS) q4_linear_kernel(const Q4Launch p)
 // itself, 43 cycles per unit and SM against 47..51 at the HBM rate.  One row takes copies of four chunks (G = 4): one barrier wait and one
 // refill for four units.  Before (two chunks per copy, waits in front of each copy's arithmetic, divisions in the prologue, one warp per shared tile
 // in the merge) / now, us per launch in a graph: 4096 x 4096 5.55 / 4.78, 12288 x 4096 8.6 / 7.85, 22016 x 4096 12.05 / 11.6, 4096 x 11008
-// 9.7 / 8.5, 1000 x 2112 6.4 / 5.3, 57344 x 8192 45.6 / 43.9, 2 rows of 4096 x 4096 7.1 / 6.6 (four chunks per copy: 6.8).
+// 9.7 / 8.5, 1000 x 2112 6.4 / 5.3, 57344 x 8192 45.6 / 43.9, 2 rows of 4096 x 4096 7.1 / 6.6 (four chunks per copy: 6.8).  With the staging's
+// slots found once per thread and its maximum by reductions of a warp: 4.57, 7.7, 11.5, 8.3, 5.1, 43.6; 6.4.
 constexpr int Q4S_WARPS = 16;                    // one CTA of sixteen warps per SM
 constexpr int Q4S_THREADS = Q4S_WARPS * 32;
 constexpr int Q4S_MAX_DEPTH = 8;                 // most ring stages per warp
@@ -702,7 +703,19 @@ __device__ __noinline__ void q4s_cross_cta(const Q4StreamLaunch& p, float v, int
 //                                                  the block's scaled x: the hi column's C operand (the lo column's is 0);
 //                                                  hi + lo differs from the scaled x by < 2^-22 of it, which is what the
 //                                                  sum may be off by as well
-__device__ __forceinline__ void q4s_stage_one(float4 v, bool on, int m, int f, float sc, int ncols, int M, uint4* xs, float4* cs,
+// Where a thread's float4 lies inside its chunk is the same for all of them (the threads of a CTA are whole chunks apart): the slots are
+// found once per thread.
+struct Q4StageSlot {
+    int blk, s0, s1, in;                                   // block of the chunk; slots of thread tt0 and tt0 + 1 of the fragment; word inside them
+    __device__ __forceinline__ explicit Q4StageSlot(int r) : blk(r >> 3)
+    {
+        const int jj = (r >> 2) & 1, up = (r >> 1) & 1, tt0 = (r & 1) * 2;
+        s0 = tt0 * 2 + blk;
+        s1 = s0 + 2;
+        in = jj * 2 + up;
+    }
+};
+__device__ __forceinline__ void q4s_stage_one(float4 v, bool on, int m, int chunk, const Q4StageSlot& at, float sc, int ncols, int M, uint4* xs, float4* cs,
                                               int lane)
 {
     const float e0 = v.x * sc, e1 = v.y * sc, e2 = v.z * sc, e3 = v.w * sc;
@@ -710,24 +723,21 @@ __device__ __forceinline__ void q4s_stage_one(float4 v, bool on, int m, int f, f
     const float2 f01 = __half22float2(h01), f23 = __half22float2(h23);
     const __half2 l01 = __floats2half2_rn(e0 - f01.x, e1 - f01.y), l23 = __floats2half2_rn(e2 - f23.x, e3 - f23.y);
     float sum = (e0 + e1) + (e2 + e3);
-    const int chunk = f >> 4, r = f & 15;
-    const int blk = r >> 3, jj = (r >> 2) & 1, up = (r >> 1) & 1, tt0 = (r & 1) * 2;
     if (on) {
         // Column c keeps its eight 16-byte slots (t, block) at slot ^ (c & 7): the eight columns an MMA's lanes read
         // together then fall into different banks.
-        __half2* dst = reinterpret_cast<__half2*>(xs + ((size_t)chunk * ncols + 2 * m) * 8);   // 8 uint4 per column
-        const int s0 = tt0 * 2 + blk, s1 = s0 + 2, in = jj * 2 + up;                           // thread tt0 and tt0 + 1 of the fragment
+        __half2* dst = reinterpret_cast<__half2*>(xs) + (chunk * ncols + 2 * m) * 32 + at.in;   // 32 half2 per column
         const int chi = (2 * m) & 7, clo = (2 * m + 1) & 7;
-        dst[((s0 ^ chi) << 2) + in] = h01;
-        dst[((s1 ^ chi) << 2) + in] = h23;
-        dst[32 + ((s0 ^ clo) << 2) + in] = l01;           // next column (lo): 8 uint4 = 32 half2 further
-        dst[32 + ((s1 ^ clo) << 2) + in] = l23;
+        dst[(at.s0 ^ chi) << 2] = h01;
+        dst[(at.s1 ^ chi) << 2] = h23;
+        dst[32 + ((at.s0 ^ clo) << 2)] = l01;             // next column (lo)
+        dst[32 + ((at.s1 ^ clo) << 2)] = l23;
     }
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);   // 8 consecutive lanes cover one 32-block of one row
     if (on && (lane & 7) == 0) {
         const float c = -8.f * 5.9604644775390625e-8f * sum;                        // -8 * 2^-24
-        reinterpret_cast<float2*>(cs + ((size_t)chunk * M + m))[blk] = make_float2(c, 16.f * c);
+        reinterpret_cast<float2*>(cs + (chunk * M + m))[at.blk] = make_float2(c, 16.f * c);
     }
 }
 
@@ -740,6 +750,7 @@ __device__ __forceinline__ uint32_t q4s_stage_pass(const Q4StreamLaunch& p, int 
                                                    float4* cs, int tid, int lane)
 {
     constexpr int LOADS = ONE && !SWIGLU ? 6 : 4;
+    const Q4StageSlot at(tid & 15);                        // (pk4 and the CTA's threads are multiples of a chunk's 16 float4)
     uint32_t mx = 0;
     for (int base = 0; base < total4; base += LOADS * Q4S_THREADS) {
         float4 v[LOADS];
@@ -766,7 +777,7 @@ __device__ __forceinline__ uint32_t q4s_stage_pass(const Q4StreamLaunch& p, int 
             mx = max(mx, __float_as_uint(v[u].y) & 0x7FFFFFFFu);
             mx = max(mx, __float_as_uint(v[u].z) & 0x7FFFFFFFu);
             mx = max(mx, __float_as_uint(v[u].w) & 0x7FFFFFFFu);
-            if (CONVERT) q4s_stage_one(v[u], on[u], mm[u], ff[u], sc, ncols, ONE ? 1 : p.M, xs, cs, lane);
+            if (CONVERT) q4s_stage_one(v[u], on[u], mm[u], ONE ? ((base + u * Q4S_THREADS) >> 4) + (tid >> 4) : ff[u] >> 4, at, sc, ncols, ONE ? 1 : p.M, xs, cs, lane);
         }
     }
     return mx;
@@ -850,13 +861,10 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
     const int total4 = M * pk4;
     uint32_t mx = q4s_stage_pass<ONE, ONE, SWIGLU>(p, pk4, total4, 1.f, ncols, xs, cs, tid, lane);
     issue_upto(min(D, ngroups));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
+    mx = __reduce_max_sync(0xFFFFFFFFu, mx);
     if (lane == 0) s_max[warp] = mx;
     __syncthreads();
-    mx = s_max[0];
-#pragma unroll
-    for (int w = 1; w < NW; ++w) mx = max(mx, s_max[w]);
+    mx = __reduce_max_sync(0xFFFFFFFFu, s_max[lane & (NW - 1)]);
     float inv_sc = 1.f;
     if (!ONE || (mx != 0 && (mx < 0x3F800000u || mx >= 0x47000000u))) {       // 1.0, 2^15
         int emax = (int)(mx >> 23);

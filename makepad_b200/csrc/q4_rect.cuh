@@ -32,6 +32,7 @@ constexpr int Q4R_MAX_CLUSTER = 8;                        // K slices of a clust
 // Slices always through memory, one warp per shared tile in the last phase, divisions in prologue and staging, a barrier look in front of
 // every copy's arithmetic / this form, us per call in a graph: 4096 x 4096 at 4 rows 8.2 / 6.2, 8 10.15 / 7.7, 16 13.0 / 11.0; 12288 x 4096 at 8
 // 14.8 / 13.1; 22016 x 4096 at 8 20.1 / 18.1, 16 30.9 / 29.4; 4096 x 11008 at 8 14.6 / 13.2; 1000 x 2112 at 13 9.2 / 5.9; 57344 x 8192 at 8 66.6 / 65.2.
+// With the staging's slots found once per thread: 22016 x 4096 at 8 17.8, 4096 x 11008 at 8 12.8, 2000 x 6016 at 8 7.26 / 7.04.
 
 struct Q4RectLaunch {
     const uint4* stream;
@@ -63,28 +64,25 @@ __device__ __forceinline__ void q4r_st_async(uint32_t addr, uint32_t bar, int ra
 // One float4 of x (element 4f of the slice, activation row m of MP staged rows) -> fragments and corrections.
 //   xs: uint4 [chunk][2 MP columns][4 t][2 blocks]  as in the streaming kernel
 //   cs: float2[chunk][2 blocks][MP]                 (c, 16c) per row: the hi column's C operand
-__device__ __forceinline__ void q4r_stage_one(float4 v, int m, int f, float sc, int MP, uint32_t xs_u32, uint32_t cs_u32, int lane)
+__device__ __forceinline__ void q4r_stage_one(float4 v, int m, int chunk, const Q4StageSlot& at, float sc, int MP, uint32_t xs_u32, uint32_t cs_u32, int lane)
 {
     const float e0 = v.x * sc, e1 = v.y * sc, e2 = v.z * sc, e3 = v.w * sc;
     const __half2 h01 = __floats2half2_rn(e0, e1), h23 = __floats2half2_rn(e2, e3);
     const float2 f01 = __half22float2(h01), f23 = __half22float2(h23);
     const __half2 l01 = __floats2half2_rn(e0 - f01.x, e1 - f01.y), l23 = __floats2half2_rn(e2 - f23.x, e3 - f23.y);
     float sum = (e0 + e1) + (e2 + e3);
-    const int chunk = f >> 4, r = f & 15;
-    const int blk = r >> 3, jj = (r >> 2) & 1, up = (r >> 1) & 1, tt0 = (r & 1) * 2;
     // column c (128 bytes) keeps its eight 16-byte slots (t, block) at slot ^ (c & 7): bank-conflict-free fragment loads
-    const uint32_t col = xs_u32 + ((uint32_t)(chunk * 2 * MP + 2 * m) * 8) * 16;
-    const uint32_t s0 = tt0 * 2 + blk, s1 = s0 + 2, in = (uint32_t)(jj * 2 + up) * 4;
+    const uint32_t col = xs_u32 + (uint32_t)(chunk * 2 * MP + 2 * m) * 128 + at.in * 4;
     const uint32_t chi = (2 * m) & 7, clo = (2 * m + 1) & 7;
-    asm volatile("st.shared.b32 [%0], %1;" ::"r"(col + ((s0 ^ chi) << 4) + in), "r"(*reinterpret_cast<const uint32_t*>(&h01)) : "memory");
-    asm volatile("st.shared.b32 [%0], %1;" ::"r"(col + ((s1 ^ chi) << 4) + in), "r"(*reinterpret_cast<const uint32_t*>(&h23)) : "memory");
-    asm volatile("st.shared.b32 [%0], %1;" ::"r"(col + 128 + ((s0 ^ clo) << 4) + in), "r"(*reinterpret_cast<const uint32_t*>(&l01)) : "memory");
-    asm volatile("st.shared.b32 [%0], %1;" ::"r"(col + 128 + ((s1 ^ clo) << 4) + in), "r"(*reinterpret_cast<const uint32_t*>(&l23)) : "memory");
+    asm volatile("st.shared.b32 [%0], %1;" ::"r"(col + ((at.s0 ^ chi) << 4)), "r"(*reinterpret_cast<const uint32_t*>(&h01)) : "memory");
+    asm volatile("st.shared.b32 [%0], %1;" ::"r"(col + ((at.s1 ^ chi) << 4)), "r"(*reinterpret_cast<const uint32_t*>(&h23)) : "memory");
+    asm volatile("st.shared.b32 [%0], %1;" ::"r"(col + 128 + ((at.s0 ^ clo) << 4)), "r"(*reinterpret_cast<const uint32_t*>(&l01)) : "memory");
+    asm volatile("st.shared.b32 [%0], %1;" ::"r"(col + 128 + ((at.s1 ^ clo) << 4)), "r"(*reinterpret_cast<const uint32_t*>(&l23)) : "memory");
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);   // 8 consecutive lanes cover one 32-block of one row
     if ((lane & 7) == 0) {
         const float c = -8.f * 5.9604644775390625e-8f * sum;                        // -8 * 2^-24
-        asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(cs_u32 + (uint32_t)((chunk * 2 + blk) * MP + m) * 8), "f"(c), "f"(16.f * c) : "memory");
+        asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(cs_u32 + (uint32_t)((chunk * 2 + at.blk) * MP + m) * 8), "f"(c), "f"(16.f * c) : "memory");
     }
 }
 
@@ -160,6 +158,7 @@ __global__ void __launch_bounds__(Q4R_THREADS, 1) q4_rect_kernel(const __grid_co
     // One pass over the slice where it fits: each thread keeps its first Q4R_CACHE float4 in registers between the search
     // for the largest magnitude and the conversion, with all of their loads in flight at once (read one by one, each
     // iteration of the conversion waited for its own L2 round trip: 5 to 7 us of a 37 us kernel).
+    const Q4StageSlot at(tid & 15);                        // (pk4 and the CTA's threads are multiples of a chunk's 16 float4)
     float4 cache[Q4R_CACHE];
     uint32_t mx = 0;
 #pragma unroll
@@ -188,13 +187,10 @@ __global__ void __launch_bounds__(Q4R_THREADS, 1) q4_rect_kernel(const __grid_co
             mx = max(mx, __float_as_uint(v.w) & 0x7FFFFFFFu);
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
+    mx = __reduce_max_sync(0xFFFFFFFFu, mx);
     if (lane == 0) s_max[warp] = mx;
     __syncthreads();
-    mx = s_max[0];
-#pragma unroll
-    for (int w = 1; w < Q4R_WARPS; ++w) mx = max(mx, s_max[w]);
+    mx = __reduce_max_sync(0xFFFFFFFFu, s_max[lane & (Q4R_WARPS - 1)]);
     int emax = (int)(mx >> 23);
     float sc = 1.f, inv_sc = 1.f;
     if (mx != 0 && emax < 255) {
@@ -207,7 +203,7 @@ __global__ void __launch_bounds__(Q4R_THREADS, 1) q4_rect_kernel(const __grid_co
         const int i = it * Q4R_THREADS + tid;
         if (it * Q4R_THREADS + (tid & ~31) >= total4) break;
         const int m = q4s_tile_of(i, pk4, pk4_magic), f = i - m * pk4;
-        q4r_stage_one(cache[it], m, f, sc, MP, xs_u32, cs_u32, lane);
+        q4r_stage_one(cache[it], m, f >> 4, at, sc, MP, xs_u32, cs_u32, lane);
     }
     // what did not fit in the registers is read again, again Q4R_CACHE loads in flight per thread
     for (int base = Q4R_CACHE * Q4R_THREADS; base < total4; base += Q4R_CACHE * Q4R_THREADS) {
@@ -224,7 +220,7 @@ __global__ void __launch_bounds__(Q4R_THREADS, 1) q4_rect_kernel(const __grid_co
             const int i = base + it * Q4R_THREADS + tid;
             if (base + it * Q4R_THREADS + (tid & ~31) >= total4) break;
             const int m = q4s_tile_of(i, pk4, pk4_magic), f = i - m * pk4;
-            q4r_stage_one(cache[it], m, f, sc, MP, xs_u32, cs_u32, lane);
+            q4r_stage_one(cache[it], m, f >> 4, at, sc, MP, xs_u32, cs_u32, lane);
         }
     }
     __syncthreads();
