@@ -1005,7 +1005,10 @@ nvfp4_gemm_pair_kernel_v2(const __grid_constant__ CUtensorMap map_a, const __gri
         for (int item = pair; item < p.items && !s_abort; item += npairs, ++local) {
             int kb0, kb1;
             const int tile = pair_item(p, item, &kb0, &kb1), nt = tile / p.m_pairs, mp = tile - nt * p.m_pairs;
-            if (!bar_spin(bar_acc_full, (uint32_t)local & 1u, SPIN_LIMIT)) { if (lane == 0) { atomicExch(p.status, 16); s_abort = 1; } break; }
+            // Suspended meanwhile (up to 2^17 tries of 4 us): eight warps that look all the time take issue slots and power from the others.
+            // Spinning / this, us: 2048 x 14336 x 4096 56.8 / 55.8, 1000 x 28672 x 4096 58.3 / 57.2, 1000 x 4096 x 14336 39.1 / 37.9.  (The producer and
+            // the writers lost with it: their hand-offs are on the MMAs' way.)
+            if (!bar_wait(bar_acc_full, (uint32_t)local & 1u, 1u << 17)) { if (lane == 0) { atomicExch(p.status, 16); s_abort = 1; } break; }
             tc_fence_after();
             const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + half * V2_EPI_COLS;
             uint32_t r[V2_EPI_COLS];
