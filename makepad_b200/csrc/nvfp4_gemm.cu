@@ -30,6 +30,7 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <cstring>
 
 #include "nvfp4.cuh"
 #include "swiglu.cuh"
@@ -1290,7 +1291,7 @@ static bool partial_room(Nvfp4Scratch& scratch, int pairs, cudaStream_t s)
 
 // Up to RW_MAX_ROWS activation rows through nvfp4_rows_kernel.
 static int32_t nvfp4_rows_launch(Nvfp4Scratch& scratch, const Nvfp4Dev& w, const uint8_t* a_codes, const uint8_t* a_sf, float ta, int M, uint16_t* c, int device,
-                                 int sm_count, bool pdl, cudaStream_t s, int* launches, std::string& err)
+                                 int sm_count, bool pdl, int pinned, cudaStream_t s, int* launches, std::string& err)
 {
     RowsParams p;
     p.M = M; p.Mp = (M + 15) / 16 * 16; p.N = (int)w.N; p.K = (int)w.K;
@@ -1302,15 +1303,15 @@ static int32_t nvfp4_rows_launch(Nvfp4Scratch& scratch, const Nvfp4Dev& w, const
     p.stages = std::min(RW_MAX_STAGES, (RW_SMEM_MOST - 1024) / stage);
     // Cuts of K, by estimated cost (us): a K block of a CTA; a second launch (1.5 of device time, and the host's 2.5 where it is the host that is
     // waited for), and what the cuts write for it.  Never more CTAs than are resident at once: 8192 x 8192 at 16 rows, 32 K blocks, uncut 18.0, in four 11.0, in five (370 CTAs) 15.1.
-    const char* env = getenv("MPQ_FP4_ROWS_SPLITS");
-    const int most = env ? atoi(env) : 16;
+    // (pinned: as many cuts as that, as far as K goes)
+    const int most = pinned ? pinned : 16;
     int splits = 1;
     const double per_block = 0.44 + 0.0055 * p.Mp;
-    double best = env ? 1e30 : per_block * p.k_blocks;
-    for (int n = 2; n <= std::min(most, p.k_blocks / SPLIT_MIN_BLOCKS) && (env || tiles * n <= 2 * sm_count); ++n) {
+    double best = pinned ? 1e30 : per_block * p.k_blocks;
+    for (int n = 2; n <= std::min(most, p.k_blocks / SPLIT_MIN_BLOCKS) && (pinned || tiles * n <= 2 * sm_count); ++n) {
         const size_t bytes = (size_t)tiles * n * p.Mp * 128 * sizeof(float);
         const double cost = per_block * ((p.k_blocks + n - 1) / n) + 3.6 + bytes / 3e6;
-        if (env || cost < best) { best = cost; splits = n; }
+        if (pinned || cost < best) { best = cost; splits = n; }
     }
     if (splits > 1 && (!partial_room(scratch, sm_count / 2, s) || scratch.partial.bytes() < (size_t)tiles * splits * p.Mp * 128 * sizeof(float))) splits = 1;
     p.splits = splits;
@@ -1356,10 +1357,12 @@ int32_t nvfp4_gemm_launch(Nvfp4Scratch& scratch, const Nvfp4Dev& w, const uint8_
         if (e == cudaSuccess) e = cudaMemset(scratch.status, 0, sizeof(int));
         if (e != cudaSuccess) { err = std::string("status allocation failed: ") + cudaGetErrorString(e); return MPQ_ERR_CUDA; }
     }
-    // MPQ_FP4_KERNEL=single forces the one-CTA kernel, pair the kernels of CTA pairs, which the parity tests use to cover all
+    // MPQ_FP4_KERNEL=single forces the one-CTA kernel, pair the kernel of CTA pairs, rows=<n> so many cuts of K in the one of few rows, which
+    // the parity tests use to cover all
     const char* env = getenv("MPQ_FP4_KERNEL");
-    const bool single = env && std::string(env) == "single", pair = env && std::string(env) == "pair";
-    if (M <= RW_MAX_ROWS && w.mapped && !single && !pair) return nvfp4_rows_launch(scratch, w, a_codes, a_sf, ta, (int)M, c, device, sm_count, pdl, s, launches, err);
+    const bool single = env && strcmp(env, "single") == 0, pair = env && strcmp(env, "pair") == 0;
+    if (M <= RW_MAX_ROWS && w.mapped && !single && !pair)
+        return nvfp4_rows_launch(scratch, w, a_codes, a_sf, ta, (int)M, c, device, sm_count, pdl, env && strncmp(env, "rows=", 5) == 0 ? atoi(env + 5) : 0, s, launches, err);
     // The activations' scale factors are read straight from the canonical [M][K/16] array when a K block's 16 bytes per
     // row can be a TMA box (row pitch a multiple of 16 bytes); otherwise they are re-tiled first, like the weights'.
     const bool direct = K % 256 == 0 && (reinterpret_cast<uintptr_t>(a_sf) & 15u) == 0;

@@ -21,7 +21,7 @@ def test_few_rows_against_the_oracle(ctx, orc, monkeypatch, N, K, splits):
     import makepad_b200
     import torch
     if splits != "0":
-        monkeypatch.setenv("MPQ_FP4_ROWS_SPLITS", splits)
+        monkeypatch.setenv("MPQ_FP4_KERNEL", "rows=" + splits)
     b, sfb = synth.nvfp4_tensor(N, K, seed=91, stream=1)
     lin = makepad_b200.QuantLinear(makepad_b200.Nvfp4Weight(ctx, b, sfb, 2.0))
     for M in (1, 15, 16, 17, 33, 48, 64):
