@@ -34,10 +34,22 @@ def _raw(h):
     return None if h is None else h.value
 
 
+_torch_module = None
+
+
+def _torch():
+    """torch, imported by the first call that needs it (an import statement in each call is 0.1 us of a host-bound pass of 7)."""
+    global _torch_module
+    if _torch_module is None:
+        import torch
+        _torch_module = torch
+    return _torch_module
+
+
 def _stream() -> int:
     """The current stream of the current device.  (The stream object that torch.cuda.current_stream() builds costs more host
     time than the launch itself.)"""
-    import torch
+    torch = _torch()
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
@@ -197,7 +209,7 @@ class QuantLinear:
         self.ctx = weight.ctx
 
     def forward(self, x, out=None):
-        import torch
+        torch = _torch()
         w, ctx = self.w, self.ctx
         if w.fmt == _lib.FMT_Q4:
             if isinstance(x, np.ndarray):                      # host path: copies inside the library
@@ -226,7 +238,7 @@ class QuantLinear:
     def forward_swiglu(self, gate_up, out=None):
         """Q4 only: y = (silu(gate) * up) . W^T for gate_up fp32 [M][2K] = [gate | up] on the GPU (the down projection of a
         feed-forward block with the SwiGLU fused into the kernel's activation staging)."""
-        import torch
+        torch = _torch()
         w, ctx = self.w, self.ctx
         if w.fmt != _lib.FMT_Q4:
             raise MpqError(_lib.ERR_INVALID_ARG, "forward_swiglu is for Q4 weights")
@@ -250,7 +262,7 @@ def swiglu(ctx: Context, gate_up):
 def nvfp4_quantize(ctx: Context, x, tensor_scale: float = 1.0, swiglu_fused: bool = False):
     """fp32 or bf16 [M][K] on the GPU -> (codes u8 [M][K/2], sf u8 [M][K/16]) ready to be the GEMM's A.  With swiglu_fused
     the input is [M][2K] = [gate | up] and silu(gate) * up is what gets quantised."""
-    import torch
+    torch = _torch()
     M, K = x.shape[0], x.shape[1]
     if swiglu_fused:
         K //= 2
