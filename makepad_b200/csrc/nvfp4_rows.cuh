@@ -22,6 +22,9 @@ namespace mpq {
 constexpr int RW_THREADS = 192, RW_MAX_ROWS = 64, RW_MAX_STAGES = 6, RW_TMEM_COLS = 256;
 constexpr int RW_SF_COLS = 32;                             // tensor-memory columns of a stage: [weights: 4 K steps x 4 | activations: 4 x 4]
 constexpr int RW_SMEM_MOST = 112 * 1024;
+// Tries of a suspended wait (up to 4 us each): the producer and the epilogue wait so, the others look all the time.  Eight shapes of 1 to 64 rows, all
+// spinning / this: 28672 x 4096 at 16 rows 14.0 / 13.85 us, 4096 x 14336 10.2 / 10.0, 4096 x 4096 5.84 / 5.73, the rest within 0.5 %.
+constexpr uint32_t RW_TRIES = 1u << 17;
 static_assert(RW_MAX_ROWS + RW_MAX_STAGES * RW_SF_COLS <= RW_TMEM_COLS, "accumulator and scale factors of two CTAs must fit in tensor memory");
 
 struct RowsParams {
@@ -112,7 +115,7 @@ nvfp4_rows_kernel(const __grid_constant__ CUtensorMap map_first, const __grid_co
             int s = 0;
             uint32_t phase = 0;
             for (int i = ahead; i < count && !s_abort; ++i) {
-                if (!bar_spin(bar_empty + 8 * s, phase, SPIN_LIMIT)) { atomicExch(p.status, 21); s_abort = 1; break; }
+                if (!bar_wait(bar_empty + 8 * s, phase, RW_TRIES)) { atomicExch(p.status, 21); s_abort = 1; break; }
                 load_w(i, s);
                 load_x(i, s);
                 if (++s == p.stages) { s = 0; phase ^= 1u; }
@@ -177,7 +180,7 @@ nvfp4_rows_kernel(const __grid_constant__ CUtensorMap map_first, const __grid_co
         }
         // ---- epilogue: lane = weight row, column = activation row
         if (live && !s_abort) {
-            if (bar_spin(bar_acc, 0, SPIN_LIMIT)) {
+            if (bar_wait(bar_acc, 0, RW_TRIES)) {
                 tc_fence_after();
                 const int row = quarter * 32 + lane, n = n0 + row;
                 const bool mine = row < wrows && n < p.N;
