@@ -1250,7 +1250,8 @@ extern "C" int32_t mpq_q4_linear_forward_host(mpq_context* ctx, const mpq_weight
     const size_t xb = (size_t)M * w->q4.K * 4, yb = (size_t)M * w->q4.N * 4;
     std::lock_guard<std::mutex> hold(ctx->host_lock);
     if ((st = grow(ctx, &ctx->hx, &ctx->hx_bytes, xb))) return st;
-    const bool x_pages = !driver_knows(x_host) && ctx->host_x.reserve(xb), y_pages = !driver_knows(y_host) && ctx->host_y.reserve(yb);
+    const bool x_pages = !driver_knows(x_host) && ctx->host_x.reserve(xb, HostPages::MOST_IN),
+               y_pages = !driver_knows(y_host) && ctx->host_y.reserve(yb, x_pages ? HostPages::MOST_OUT : HostPages::MOST_OUT_BEHIND_COPY);
     if (!y_pages && (st = grow(ctx, &ctx->hy, &ctx->hy_bytes, yb))) return st;
     cudaError_t e;
     if (x_pages) {

@@ -375,6 +375,46 @@ def test_uploads_work_where_no_pages_can_be_locked():
 """))
 
 
+PAGES = r"""
+#include "host_pages.h"
+#include <cstdio>
+#include <cstdlib>
+static int locked = 0, live = 0;
+static bool refuse = false;
+extern "C" {
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned)
+{
+    if (refuse) return cudaErrorMemoryAllocation;
+    ++locked, ++live;
+    *p = malloc(n);
+    return cudaSuccess;
+}
+cudaError_t cudaFreeHost(void* p) { --live; free(p); return cudaSuccess; }
+cudaError_t cudaHostGetDevicePointer(void** d, void* h, unsigned) { *d = h; return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+}
+int main()
+{
+    int bad = 0;
+    mpq::HostPages pages;
+    const size_t most = mpq::HostPages::MOST_OUT;
+    for (size_t n = 16; n <= most; n += 4096) bad += !pages.reserve(n, most) || pages.bytes < n || pages.bytes > most || live != 1;
+    bad += locked > 6;                                                     // rows that grow by a page a call: 64 KB, 128 KB ... 1 MB
+    bad += pages.reserve(most + 16, most) || !pages.reserve(most, most);
+    bad += mpq::HostPages::MOST_IN > 524288 || mpq::HostPages::MOST_OUT_BEHIND_COPY > 786432;
+    pages.release();
+    refuse = true;
+    bad += pages.reserve(16, most) || pages.bytes || live;
+    std::printf("%d\n", bad);
+    return bad;
+}
+"""
+
+
+def test_pages_for_host_rows_grow_in_doubling_steps():
+    _run(PAGES)
+
+
 def test_every_kernel_that_can_give_up_a_wait_settles_before_it_ends():
     """A kernel whose roles share an abort flag waits for what was in flight behind its last CTA barrier, before tensor memory is freed."""
     kernels = 0
