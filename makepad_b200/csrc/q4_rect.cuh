@@ -27,6 +27,7 @@ constexpr int Q4R_STAGE_BYTES = Q4R_G * Q4_UNIT_BYTES;
 constexpr int Q4R_CACHE = 8;                              // float4 of the activation slice a thread keeps in registers while it is staged
 
 constexpr int Q4R_MAX_CLUSTER = 8;                        // K slices of a cluster
+constexpr uint32_t Q4R_SUM_TRIES = 1u << 17;              // tries (up to 4 us each) of the wait for the slices that the other CTAs send: half a second
 
 // What bounds it: up to about 10 MB of weights the fixed parts, above that the legacy tensor path and the FP pipes from about eight rows.
 // Slices always through memory, one warp per shared tile in the last phase, divisions in prologue and staging, a barrier look in front of
@@ -382,8 +383,12 @@ __global__ void __launch_bounds__(Q4R_THREADS, 1) q4_rect_kernel(const __grid_co
     }
 
     // ---- a cluster's slices: this CTA adds its items, in slice order
+    // A CTA of the cluster may still be waiting for its weights when this one gives up.  So no CTA leaves before all have sent what they
+    // have: a store into the shared memory of a CTA that is gone would be a fault.  (Relaxed: what is sent is ordered by the barrier that
+    // counts it.  All the stores of a CTA precede the arrival that the others wait for, and with it nearly all of the wait is over.)
     if (p.cluster) {
-        const bool arrived = mbar_wait(sent_u32, 0, Q4S_SPIN_LIMIT);
+        asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+        const bool arrived = mbar_wait(sent_u32, 0, Q4R_SUM_TRIES);
         if (arrived)
             for (int i = warp; i < own_items; i += Q4R_WARPS) {
                 const uint32_t at = out_u32 + (uint32_t)(i * p.nks * 32 + lane) * 16;
@@ -398,10 +403,9 @@ __global__ void __launch_bounds__(Q4R_THREADS, 1) q4_rect_kernel(const __grid_co
                 const int item = i * p.nks + ks;
                 store(p.Y, p.ldy, item / MT, item % MT, v);
             }
-        else {
-            if (lane == 0) atomicExch(p.status, 12);
-            settle_after_timeout(true);                    // what the others may still send lands first
-        }
+        else if (lane == 0) atomicExch(p.status, 12);
+        asm volatile("barrier.cluster.wait;" ::: "memory");
+        settle_after_timeout(!arrived);                    // what was on its way lands first
     }
 }
 

@@ -427,6 +427,19 @@ def test_every_kernel_that_can_give_up_a_wait_settles_before_it_ends():
     assert kernels == 4
 
 
+def test_no_cta_of_a_cluster_leaves_while_another_may_still_store_into_it():
+    """q4_rect_kernel: every CTA arrives at a cluster barrier behind its last remote store, and waits for the others there before it leaves,
+    whether its own wait for the slices ran out or not; what was on its way then lands before it ends."""
+    text = open(os.path.join(ROOT, "makepad_b200", "csrc", "q4_rect.cuh")).read()
+    kernel = text[text.index("q4_rect_kernel(const __grid_constant__"):]
+    kernel = kernel[:kernel.index("\n}")]
+    last_put = kernel.rindex("put(")
+    end = kernel[last_put:]
+    arrive, sums, wait, settle = (end.index(t) for t in ("barrier.cluster.arrive.relaxed", "mbar_wait(sent_u32, 0,", "barrier.cluster.wait", "settle_after_timeout(!arrived)"))
+    assert arrive < sums < wait < settle
+    assert "return" not in kernel[kernel.index("barrier.cluster.arrive"):].replace("if (m >= p.M) return;", "")
+
+
 def test_waits_for_staged_rows_begin_behind_the_kernels_before():
     """In the Q4 tcgen05 kernels the issuing warp and the workers wait for the kernels before (griddepcontrol.wait) ahead of their first
     bounded wait for what depends on the staged activations."""
