@@ -1313,7 +1313,8 @@ static int32_t nvfp4_rows_launch(Nvfp4Scratch& scratch, const Nvfp4Dev& w, const
         const double cost = per_block * ((p.k_blocks + n - 1) / n) + 3.6 + bytes / 3e6;
         if (pinned || cost < best) { best = cost; splits = n; }
     }
-    if (splits > 1 && (!partial_room(scratch, sm_count / 2, s) || scratch.partial.bytes() < (size_t)tiles * splits * p.Mp * 128 * sizeof(float))) splits = 1;
+    const bool room = partial_room(scratch, sm_count / 2, s);         // (by an uncut call too)
+    if (splits > 1 && (!room || scratch.partial.bytes() < (size_t)tiles * splits * p.Mp * 128 * sizeof(float))) splits = 1;
     p.splits = splits;
     p.partial = scratch.partial.as<float>();
     CUtensorMap map_x;

@@ -60,3 +60,32 @@ def test_a_loaded_weight_takes_few_rows(ctx, tmp_path):
     a, sfa = (torch.from_numpy(v).cuda() for v in synth.nvfp4_tensor(5, 512, seed=96, stream=0))
     w2 = makepad_b200.load_weight(ctx, path)
     assert torch.equal(makepad_b200.QuantLinear(w)((a, sfa, 1.0)), makepad_b200.QuantLinear(w2)((a, sfa, 1.0)))
+
+
+@pytest.mark.parametrize("M", [16, 1000])
+def test_an_uncut_call_reserves_the_room_of_later_captures(M):
+    """The context's first call is one of few rows whose K is not cut; a captured call of few rows or of many, whose K is, then has the two
+    launches and the bits of the eager one."""
+    import makepad_b200
+    import torch
+    N, K = 4096, 14336
+    c2 = makepad_b200.Context(0)
+    small = makepad_b200.QuantLinear(makepad_b200.Nvfp4Weight(c2, *synth.nvfp4_tensor(8, 32, seed=97, stream=1), 1.0))
+    lin = makepad_b200.QuantLinear(makepad_b200.Nvfp4Weight(c2, *synth.nvfp4_tensor(N, K, seed=98, stream=1), 1.0))
+    rows = lambda m, k: (*(torch.from_numpy(v).cuda() for v in synth.nvfp4_tensor(m, k, seed=99, stream=0)), 0.5)
+    a, y = rows(M, K), torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
+    before = c2.launches
+    small(rows(5, 32))
+    torch.cuda.synchronize()
+    assert c2.launches - before == 1
+    graph = torch.cuda.CUDAGraph()
+    before = c2.launches
+    with torch.cuda.graph(graph):
+        lin.forward(a, out=y)
+    assert c2.launches - before == 2
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, lin(a))
+    assert c2.lib.mpq_context_poll_status(c2.h) == _lib.OK
+    del graph
+    c2.close()
