@@ -644,17 +644,15 @@ static int32_t q4_stream_forward(mpq_context* ctx, const Q4Dev& q, const Q4Strea
 // ---------------------------------------------------------------------------
 struct Q4RectPlan { int mt, depth, slice_chunks, nks, ntg; bool cluster; size_t smem; };
 
-// Clusters of `size` CTAs of the rectangle kernel (one per SM) that the device keeps resident at once.
-static int q4_rect_clusters(int device, int size)
+// most[size]: clusters of that many CTAs of the rectangle kernel (one per SM) that the device keeps resident at once.
+static void q4_rect_clusters(int device, int (&most)[Q4R_MAX_CLUSTER + 1])
 {
-    static int most[PerDeviceOnce::MAX_DEVICES][Q4R_MAX_CLUSTER + 1];
-    static PerDeviceOnce known;
-    int* n = most[device >= 0 && device < PerDeviceOnce::MAX_DEVICES ? device : 0];
-    if (known.needs(device)) {
+    static PerDeviceNumbers<Q4R_MAX_CLUSTER + 1> table;
+    table.get(device, most, [](int (&n)[Q4R_MAX_CLUSTER + 1]) {
         auto kern = q4_rect_kernel<4>;
         const size_t smem = (size_t)120 * 1024;            // more than half of an SM's, as the register file
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227 * 1024 - 1024));
-        for (int c = 2; c <= Q4R_MAX_CLUSTER; ++c) {
+        for (int c = 2; c <= Q4R_MAX_CLUSTER && e == cudaSuccess; ++c) {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(1024, (unsigned)c);
             cfg.blockDim = dim3(Q4R_THREADS);
@@ -664,13 +662,11 @@ static int q4_rect_clusters(int device, int size)
             at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = (unsigned)c; at[0].val.clusterDim.z = 1;
             cfg.attrs = at;
             cfg.numAttrs = 1;
-            int found = 0;
-            if (e != cudaSuccess || cudaOccupancyMaxActiveClusters(&found, kern, &cfg) != cudaSuccess) { cudaGetLastError(); found = 0; }
-            n[c] = found;
+            e = cudaOccupancyMaxActiveClusters(&n[c], kern, &cfg);
         }
-        known.mark(device);
-    }
-    return n[size];
+        if (e != cudaSuccess) cudaGetLastError();
+        return e == cudaSuccess;
+    });
 }
 
 static bool q4_rect_plan(const mpq_context* ctx, const Q4Dev& q, int M, Q4RectPlan* pl)
@@ -681,6 +677,8 @@ static bool q4_rect_plan(const mpq_context* ctx, const Q4Dev& q, int M, Q4RectPl
     const size_t per_chunk = (size_t)2 * mp * 128 + (size_t)2 * mp * 8;          // fragments + corrections
     const size_t wpart = (size_t)Q4R_WARPS * (4 * mt) * 32 * 4, bars = (size_t)Q4R_WARPS * Q4S_MAX_DEPTH * 8;
     const size_t total = (size_t)227 * 1024 - 1024;
+    int clusters[Q4R_MAX_CLUSTER + 1] = {};
+    if (ctx->q4_rect_cluster) q4_rect_clusters(ctx->device, clusters);
     // The deeper ring first (measured: two stages per warp with more K slices beat one stage with fewer);
     // MPQ_Q4_RECT_DEPTH pins the ring depth.
     for (int depth = ctx->q4_rect_depth ? std::min(ctx->q4_rect_depth, (int)Q4S_MAX_DEPTH) : 2; depth >= 1; --depth) {
@@ -703,8 +701,8 @@ static bool q4_rect_plan(const mpq_context* ctx, const Q4Dev& q, int M, Q4RectPl
             const int sl = ((q.nchunks + cand - 1) / cand + Q4R_G - 1) / Q4R_G * Q4R_G;
             const int real = (q.nchunks + sl - 1) / sl;
             if (real > sms) continue;                      // (cannot happen for K below a few million)
-            for (int cluster = 0; cluster <= (real > 1 && real <= Q4R_MAX_CLUSTER && ctx->q4_rect_cluster); ++cluster) {
-                const int room = cluster ? q4_rect_clusters(ctx->device, real) : sms / real;
+            for (int cluster = 0; cluster <= (real > 1 && real <= Q4R_MAX_CLUSTER); ++cluster) {
+                const int room = cluster ? clusters[real] : sms / real;
                 if (room < 1) continue;
                 const int tg = std::max(1, std::min(q.nrp, room)), tiles = (q.nrp + tg - 1) / tg;
                 const size_t smem = ring + per_chunk * sl + wpart + bars + (cluster ? 16 + (size_t)(tiles * mt + real - 1) / real * real * 512 : 0);

@@ -49,6 +49,52 @@ def test_per_device_flags_are_per_device():
         assert out.returncode == 0 and out.stdout.strip() == "0", out.stdout + out.stderr
 
 
+NUMBERS = r"""
+#include "per_device.h"
+#include <cstdio>
+#include <thread>
+#include <vector>
+int main()
+{
+    int bad = 0, asked = 0, v[3];
+    mpq::PerDeviceNumbers<3> table;
+    auto fails = [&](int (&n)[3]) { ++asked; n[0] = 7; return false; };
+    auto works = [&](int (&n)[3]) { ++asked; n[0] = n[1] = n[2] = 5; return true; };
+    table.get(2, v, fails);
+    bad += asked != 1 || v[0] || v[1] || v[2];                             // nothing is known, and nothing is kept
+    table.get(2, v, works);
+    bad += asked != 2 || v[0] != 5 || v[2] != 5;                           // a failed query is made again
+    table.get(2, v, fails);
+    bad += asked != 2 || v[0] != 5;                                        // a good one is not
+    table.get(3, v, works);
+    table.get(-1, v, works);
+    table.get(mpq::PerDeviceOnce::MAX_DEVICES, v, works);
+    bad += asked != 5;
+    mpq::PerDeviceNumbers<3> shared;                                       // several threads: one asks, all see whole rows
+    asked = 0;
+    std::vector<std::thread> threads;
+    std::vector<int> wrong(8);
+    for (int t = 0; t < 8; ++t)
+        threads.emplace_back([&, t] {
+            int n[3];
+            for (int i = 0; i < 1000; ++i) { shared.get(i & 1, n, works); wrong[t] += n[0] != 5 || n[1] != 5 || n[2] != 5; }
+        });
+    for (auto& t : threads) t.join();
+    for (int w : wrong) bad += w;
+    bad += asked != 2;
+    std::printf("%d\n", bad);
+    return bad;
+}
+"""
+
+
+def test_numbers_of_a_device_are_asked_for_again_where_the_query_failed():
+    _run(NUMBERS, "-pthread")
+    text = open(os.path.join(ROOT, "makepad_b200", "csrc", "mpq.cu")).read()
+    body = text[text.index("static void q4_rect_clusters("):]
+    assert "PerDeviceNumbers<" in body[:body.index("\n}")]
+
+
 def test_no_per_process_flag_guards_a_per_device_setting():
     """Every cudaFuncSetAttribute in the library sits behind PerDeviceOnce, none behind a plain static bool."""
     csrc = os.path.join(ROOT, "makepad_b200", "csrc")

@@ -49,6 +49,24 @@ def test_slices_of_the_rectangle_kernel(orc, N, K):
         c.close()
 
 
+# (28672 of K at 16 rows: more slices than a cluster holds)
+@pytest.mark.parametrize("N,K,M,slices,one", [(4096, 4096, 8, 0, 1), (4096, 4096, 8, 5, 1), (1000, 2112, 13, 3, 1), (33, 1120, 5, 2, 1), (300, 28672, 16, 0, 2)])
+def test_slices_are_added_by_a_cluster_or_by_a_second_launch(N, K, M, slices, one):
+    """One launch where the slices of a tile group are a cluster (nothing but the plan says that they are), two through memory."""
+    import makepad_b200
+    import torch
+    codes, scales = synth.q4_weight(N, K, seed=75)
+    xd = torch.from_numpy(synth.activations(M, K, seed=76)).cuda()
+    for cluster, launches in (("1", one), ("0", 2)):
+        c = _context(MPQ_Q4_RECT_CLUSTER=cluster, MPQ_Q4_RECT_NKS=str(slices))
+        w = makepad_b200.Q4Weight(c, codes, scales)
+        before = c.launches
+        makepad_b200.QuantLinear(w)(xd)
+        assert c.launches - before == launches, (cluster, slices)
+        w.destroy()
+        c.close()
+
+
 def test_slices_in_a_graph_and_on_two_streams(ctx, orc):
     """Clusters under capture, and two calls of one context in flight on two streams (they share no scratch)."""
     import makepad_b200
