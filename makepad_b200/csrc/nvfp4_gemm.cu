@@ -33,6 +33,7 @@
 #include <cstring>
 
 #include "nvfp4.cuh"
+#include "pdl.cuh"
 #include "swiglu.cuh"
 #include "per_device.h"
 #include "settle.cuh"
@@ -169,7 +170,7 @@ __device__ __forceinline__ void nvfp4_load16(const void* xin, int64_t at, float 
 // 13.4 -> 5.6.  (These times include what launching beside the kernel before saves, about 2 us of each.)
 // SWIGLU: the input is [R][2K] = [gate | up] and what is quantised is silu(gate) * up (fp32), never written to memory.
 template <bool BF16, bool SWIGLU>
-__global__ void nvfp4_quantize_kernel(const void* __restrict__ xin, int64_t R, int64_t K, float ts, uint8_t* __restrict__ codes,
+__global__ void nvfp4_quantize_kernel(const void* xin, int64_t R, int64_t K, float ts, uint8_t* __restrict__ codes,
                                       uint8_t* __restrict__ sf)
 {
     asm volatile("griddepcontrol.launch_dependents;");
@@ -844,7 +845,7 @@ static_assert(V2_SF_COL + Q_STAGES * V2_SF_COLS <= TMEM_COLS, "scale-factor buff
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(V2_THREADS, 1)
 nvfp4_gemm_pair_kernel_v2(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                           const __grid_constant__ CUtensorMap map_sfa, const __grid_constant__ CUtensorMap map_c, const PairParams p,
-                          const uint8_t* __restrict__ sfa, const uint8_t* __restrict__ sfb)
+                          const uint8_t* sfa, const uint8_t* sfb)
 {
     extern __shared__ unsigned char smem_dyn[];
     __shared__ uint32_t s_tmem_base;
@@ -1083,7 +1084,7 @@ __global__ void __launch_bounds__(224) nvfp4_pair_reduce_kernel(const PairParams
         const float4* src = reinterpret_cast<const float4*>(p.partial + ((size_t)t * p.splits * 256 + r) * BN) + q;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int s = 0; s < p.splits; ++s) {
-            const float4 u = __ldcs(src + (size_t)s * (256 * BN / 4));
+            const float4 u = load_once(src + (size_t)s * (256 * BN / 4));
             v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
         }
         const __nv_bfloat162 h0 = __floats2bfloat162_rn(v.x * p.scale, v.y * p.scale), h1 = __floats2bfloat162_rn(v.z * p.scale, v.w * p.scale);

@@ -44,12 +44,12 @@ __device__ __forceinline__ uint4 rows_sfx(const RowsParams& p, int m, int kb)
 {
     if (m >= p.M) return make_uint4(0, 0, 0, 0);
     const uint8_t* src = p.sfx + (size_t)m * (p.K / 16) + kb * 16;
-    if (p.sfx_wide) return __ldg(reinterpret_cast<const uint4*>(src));
+    if (p.sfx_wide) return *reinterpret_cast<const uint4*>(src);
     uint32_t w[4] = {0, 0, 0, 0};
     const int n = p.K / 16 - kb * 16;                      // even, as the row pitch: K is a multiple of 32
 #pragma unroll
     for (int j = 0; j < 8; ++j)
-        if (2 * j < n) w[j >> 1] |= (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(src) + j) << (16 * (j & 1));
+        if (2 * j < n) w[j >> 1] |= (uint32_t)reinterpret_cast<const unsigned short*>(src)[j] << (16 * (j & 1));
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(128) nvfp4_rows_reduce_kernel(const __grid_con
         float4 u[8];
 #pragma unroll
         for (int s = 0; s < 8; ++s)
-            if (s0 + s < p.splits) u[s] = __ldcs(src + (size_t)(s0 + s) * p.Mp * 32);
+            if (s0 + s < p.splits) u[s] = load_once(src + (size_t)(s0 + s) * p.Mp * 32);
 #pragma unroll
         for (int s = 0; s < 8; ++s)
             if (s0 + s < p.splits) { v.x += u[s].x; v.y += u[s].y; v.z += u[s].z; v.w += u[s].w; }

@@ -44,7 +44,7 @@ struct Q4GemmLaunch {
 // block.  With SWIGLU the row is silu(gate) * up of a [gate | up] row.  The row is kept in shared memory between the
 // search for its largest magnitude and the conversion (cached; else it is read, or computed, twice).
 template <bool SWIGLU>
-__global__ void __launch_bounds__(256) q4g_xstage_kernel(const float* __restrict__ X, int M, int Mt, int K, int nchunks, int cached,
+__global__ void __launch_bounds__(256) q4g_xstage_kernel(const float* X, int M, int Mt, int K, int nchunks, int cached,
                                                           unsigned char* __restrict__ XS, float* __restrict__ inv_sc)
 {
     extern __shared__ float4 s_row[];
@@ -54,8 +54,8 @@ __global__ void __launch_bounds__(256) q4g_xstage_kernel(const float* __restrict
     const int m = blockIdx.x, tid = threadIdx.x, t = m / Mt, r = m - t * Mt;
     const float4* g4 = reinterpret_cast<const float4*>(X + (size_t)m * (SWIGLU ? 2 * (size_t)K : (size_t)K));
     auto load = [&](int f) {
-        float4 v = __ldg(g4 + f);
-        if (SWIGLU) v = swiglu_f32x4(v, __ldg(g4 + K / 4 + f));
+        float4 v = g4[f];
+        if (SWIGLU) v = swiglu_f32x4(v, g4[K / 4 + f]);
         return v;
     };
     float sc = 1.f;
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(Q4G_THREADS, 1) q4_gemm_kernel(const __grid_co
 
 // y of the tiles that were cut (those from tile0 on): their pieces' slots added in order.  64 threads x float4 per (tile, row), four
 // rows of a tile per block; four slots on their way at a time, 32-bit divisions: it is bound by latency.
-__global__ void __launch_bounds__(256) q4g_reduce_kernel(const float* __restrict__ partial, int M, int Mt, int N, int nt, int nchunks, int W, int tile0,
+__global__ void __launch_bounds__(256) q4g_reduce_kernel(const float* partial, int M, int Mt, int N, int nt, int nchunks, int W, int tile0,
                                                           float* __restrict__ Y, int64_t ldy)
 {
     asm volatile("griddepcontrol.launch_dependents;");
@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(256) q4g_reduce_kernel(const float* __restrict
         float4 u[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            if (s + k <= pl) u[k] = __ldcs(src + ((size_t)(s + k) * 2 + (s + k == pf && second)) * (Q4G_SLOT / 4));
+            if (s + k <= pl) u[k] = load_once(src + ((size_t)(s + k) * 2 + (s + k == pf && second)) * (Q4G_SLOT / 4));
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (s + k <= pl) { v.x += u[k].x; v.y += u[k].y; v.z += u[k].z; v.w += u[k].w; }

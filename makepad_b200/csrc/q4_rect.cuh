@@ -16,6 +16,7 @@
 // rounding are those of the streaming kernel (q4.cuh), so both give the same accuracy.
 #pragma once
 #include "q4.cuh"
+#include "pdl.cuh"
 #include "settle.cuh"
 
 namespace mpq {
@@ -168,7 +169,7 @@ __global__ void __launch_bounds__(Q4R_THREADS, 1) q4_rect_kernel(const __grid_co
         const int m = q4s_tile_of(i, pk4, pk4_magic), f = i - m * pk4;
         const int64_t k = k0 + 4 * f;
         cache[it] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (i < total4 && m < p.M && k < p.K) cache[it] = __ldg(reinterpret_cast<const float4*>(p.X + (size_t)m * p.K + k));
+        if (i < total4 && m < p.M && k < p.K) cache[it] = *reinterpret_cast<const float4*>(p.X + (size_t)m * p.K + k);
     }
 #pragma unroll
     for (int it = 0; it < Q4R_CACHE; ++it) {
@@ -181,7 +182,7 @@ __global__ void __launch_bounds__(Q4R_THREADS, 1) q4_rect_kernel(const __grid_co
         const int m = q4s_tile_of(i, pk4, pk4_magic), f = i - m * pk4;
         const int64_t k = k0 + 4 * f;
         if (k < p.K) {
-            const float4 v = __ldg(reinterpret_cast<const float4*>(p.X + (size_t)m * p.K + k));
+            const float4 v = *reinterpret_cast<const float4*>(p.X + (size_t)m * p.K + k);
             mx = max(mx, __float_as_uint(v.x) & 0x7FFFFFFFu);
             mx = max(mx, __float_as_uint(v.y) & 0x7FFFFFFFu);
             mx = max(mx, __float_as_uint(v.z) & 0x7FFFFFFFu);
@@ -214,7 +215,7 @@ __global__ void __launch_bounds__(Q4R_THREADS, 1) q4_rect_kernel(const __grid_co
             const int m = q4s_tile_of(i, pk4, pk4_magic), f = i - m * pk4;
             const int64_t k = k0 + 4 * f;
             cache[it] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (i < total4 && m < p.M && k < p.K) cache[it] = __ldg(reinterpret_cast<const float4*>(p.X + (size_t)m * p.K + k));
+            if (i < total4 && m < p.M && k < p.K) cache[it] = *reinterpret_cast<const float4*>(p.X + (size_t)m * p.K + k);
         }
 #pragma unroll
         for (int it = 0; it < Q4R_CACHE; ++it) {
@@ -414,7 +415,7 @@ __global__ void __launch_bounds__(Q4R_THREADS, 1) q4_rect_kernel(const __grid_co
 // their way at a time, and no index needs a division.  Calls with the slices' loads one after the other / this form (us, in a graph):
 // 4096 x 4096 (eight slices) at 8 rows 10.1 / 8.9, at 16 13.0 / 11.9; 4096 x 11008 at 8 rows 14.7 / 14.0; 12288 x 4096 (four) at 8 14.8 / 14.4.
 constexpr int Q4R_REDUCE_LOADS = 8, Q4R_REDUCE_THREADS = 128;
-__global__ void __launch_bounds__(Q4R_REDUCE_THREADS) q4_rect_reduce_kernel(const float* __restrict__ partial, int nks, int M, int N, float* __restrict__ Y,
+__global__ void __launch_bounds__(Q4R_REDUCE_THREADS) q4_rect_reduce_kernel(const float* partial, int nks, int M, int N, float* __restrict__ Y,
                                                                             int64_t ldy)
 {
     asm volatile("griddepcontrol.launch_dependents;");
@@ -431,7 +432,7 @@ __global__ void __launch_bounds__(Q4R_REDUCE_THREADS) q4_rect_reduce_kernel(cons
             float4 u[Q4R_REDUCE_LOADS];
 #pragma unroll
             for (int k = 0; k < Q4R_REDUCE_LOADS; ++k)
-                if (k0 + k < nks) u[k] = __ldcs(reinterpret_cast<const float4*>(src + (k0 + k) * slice + n));
+                if (k0 + k < nks) u[k] = load_once(reinterpret_cast<const float4*>(src + (k0 + k) * slice + n));
 #pragma unroll
             for (int k = 0; k < Q4R_REDUCE_LOADS; ++k)
                 if (k0 + k < nks) v = k0 + k == 0 ? u[k] : make_float4(v.x + u[k].x, v.y + u[k].y, v.z + u[k].z, v.w + u[k].w);
@@ -445,7 +446,7 @@ __global__ void __launch_bounds__(Q4R_REDUCE_THREADS) q4_rect_reduce_kernel(cons
             float u[Q4R_REDUCE_LOADS];
 #pragma unroll
             for (int k = 0; k < Q4R_REDUCE_LOADS; ++k)
-                if (k0 + k < nks) u[k] = __ldcs(src + (k0 + k) * slice + n);
+                if (k0 + k < nks) u[k] = load_once(src + (k0 + k) * slice + n);
 #pragma unroll
             for (int k = 0; k < Q4R_REDUCE_LOADS; ++k)
                 if (k0 + k < nks) v = k0 + k == 0 ? u[k] : v + u[k];

@@ -47,6 +47,7 @@
 
 #include "q4.cuh"
 #include "q4_plan.h"
+#include "pdl.cuh"
 #include "settle.cuh"
 
 namespace mpq {
@@ -106,7 +107,7 @@ struct Q4ULaunch {
 // 64 rows 346 -> 339 us (another day 337 -> 334).  For plain rows the cluster's launch and barriers cost more than the reads (about 0.8 us of 19 at
 // short K).
 template <bool SWIGLU>
-__global__ void __launch_bounds__(256) q4u_xstage_kernel(const float* __restrict__ X, int M, int Mp, int K, int nchunks, int cached,
+__global__ void __launch_bounds__(256) q4u_xstage_kernel(const float* X, int M, int Mp, int K, int nchunks, int cached,
                                                           unsigned char* __restrict__ XS, float* __restrict__ inv_sc)
 {
     extern __shared__ float4 s_part[];
@@ -120,8 +121,8 @@ __global__ void __launch_bounds__(256) q4u_xstage_kernel(const float* __restrict
     const size_t row_off = (size_t)(m >> 3) * 1024 + (size_t)(m & 7) * 128;
     const float4* x4 = reinterpret_cast<const float4*>(X + (size_t)m * (SWIGLU ? 2 * (size_t)K : (size_t)K));
     auto load = [&](int f) {
-        float4 v = __ldg(x4 + f);
-        if (SWIGLU) v = swiglu_f32x4(v, __ldg(x4 + K / 4 + f));
+        float4 v = x4[f];
+        if (SWIGLU) v = swiglu_f32x4(v, x4[K / 4 + f]);
         return v;
     };
     float sc = 1.f;
@@ -643,7 +644,7 @@ __global__ void __launch_bounds__(Q4U_THREADS, 1) q4_umma_kernel(const __grid_co
 // of up to Q4U_REDUCE_LOADS pieces go out together.  Calls before / now (us, in a graph): 4096 x 4096 (16 pieces) at 17 rows 15.1 / 14.2, 64 rows
 // 18.9 / 18.0; 22016 x 4096 at 64 39.7 / 38.6; 1000 x 2112 at 20 11.3 / 10.7.
 constexpr int Q4U_REDUCE_LOADS = 8;
-__global__ void __launch_bounds__(32 * Q4U_TEAMS) q4u_reduce_kernel(const float* __restrict__ partial, int M, int N, int nchunks, int W,
+__global__ void __launch_bounds__(32 * Q4U_TEAMS) q4u_reduce_kernel(const float* partial, int M, int N, int nchunks, int W,
                                                                     float* __restrict__ Y, int64_t ldy)
 {
     asm volatile("griddepcontrol.launch_dependents;");
@@ -663,7 +664,7 @@ __global__ void __launch_bounds__(32 * Q4U_TEAMS) q4u_reduce_kernel(const float*
             float4 u[Q4U_REDUCE_LOADS];
 #pragma unroll
             for (int k = 0; k < Q4U_REDUCE_LOADS; ++k)
-                if (s + k < np) u[k] = __ldcs(reinterpret_cast<const float4*>(src + (s + k) * slice + n));
+                if (s + k < np) u[k] = load_once(reinterpret_cast<const float4*>(src + (s + k) * slice + n));
 #pragma unroll
             for (int k = 0; k < Q4U_REDUCE_LOADS; ++k)
                 if (s + k < np) { v.x += u[k].x; v.y += u[k].y; v.z += u[k].z; v.w += u[k].w; }
@@ -675,7 +676,7 @@ __global__ void __launch_bounds__(32 * Q4U_TEAMS) q4u_reduce_kernel(const float*
         const int n = (int)blockIdx.x * 128 * Q4U_TEAMS + c;
         if (n >= N) return;
         float v = 0.f;
-        for (int s = 0; s < np; ++s) v += __ldcs(src + s * slice + n);
+        for (int s = 0; s < np; ++s) v += load_once(src + s * slice + n);
         y[n] = v;
     }
 }

@@ -486,6 +486,25 @@ def test_no_cta_of_a_cluster_leaves_while_another_may_still_store_into_it():
     assert "return" not in kernel[kernel.index("barrier.cluster.arrive"):].replace("if (m >= p.M) return;", "")
 
 
+def test_what_an_earlier_kernel_writes_is_read_by_ordinary_loads():
+    """Kernels that start beside the one in front of them read its output behind griddepcontrol.wait, where only ordinary loads see it: no
+    __ldg, no load that the compiler may move (pdl.cuh has those for data read once), no const __restrict__ pointer to it."""
+    csrc = os.path.join(ROOT, "makepad_b200", "csrc")
+    kernels = 0
+    for f in sorted(os.listdir(csrc)):
+        if not f.endswith((".cu", ".cuh")):
+            continue
+        for kernel in re.split(r"(?=__global__ )", open(os.path.join(csrc, f)).read())[1:]:
+            kernel = kernel[:kernel.index("\n}")]
+            if "griddepcontrol.wait" in kernel:
+                kernels += 1
+                assert not re.search(r"__ld(g|cs|cg|ca|lu)\(", kernel), (f, kernel[:120])
+                assert not re.search(r"const \w+\* __restrict__", kernel[:kernel.index("{")]), (f, kernel[:120])
+    assert kernels == 15, kernels
+    rows = open(os.path.join(csrc, "nvfp4_rows.cuh")).read()               # (and in the helper of one of them)
+    assert not re.search(r"__ld(g|cs)\(", rows)
+
+
 def test_waits_for_staged_rows_begin_behind_the_kernels_before():
     """In the Q4 tcgen05 kernels the issuing warp and the workers wait for the kernels before (griddepcontrol.wait) ahead of their first
     bounded wait for what depends on the staged activations."""
