@@ -115,7 +115,7 @@ nvfp4_rows_kernel(const __grid_constant__ CUtensorMap map_first, const __grid_co
             int s = 0;
             uint32_t phase = 0;
             for (int i = ahead; i < count && !s_abort; ++i) {
-                if (!bar_wait(bar_empty + 8 * s, phase, RW_TRIES)) { atomicExch(p.status, 21); s_abort = 1; break; }
+                if (!bar_wait(bar_empty + 8 * s, phase, RW_TRIES)) { atomicExch(p.status, 25); s_abort = 1; break; }
                 load_w(i, s);
                 load_x(i, s);
                 if (++s == p.stages) { s = 0; phase ^= 1u; }

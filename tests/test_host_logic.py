@@ -505,6 +505,18 @@ def test_what_an_earlier_kernel_writes_is_read_by_ordinary_loads():
     assert not re.search(r"__ld(g|cs)\(", rows)
 
 
+def test_every_bounded_wait_has_a_code_of_its_own():
+    """mpq_context_poll_status reports a word and a code: the code names the wait that ran out."""
+    csrc = os.path.join(ROOT, "makepad_b200", "csrc")
+    codes = []
+    for f in os.listdir(csrc):
+        if f.endswith((".cu", ".cuh")):
+            text = open(os.path.join(csrc, f)).read()
+            codes += re.findall(r"atomicExch\((?:p\.)?status, (\d+)\)", text)
+            codes += set(re.findall(r"\bfail = ([1-9]\d*);", text))           # (a role with several waits for the same thing)
+    assert len(codes) > 25 and len(codes) == len(set(codes)), sorted(codes, key=int)
+
+
 def test_waits_for_staged_rows_begin_behind_the_kernels_before():
     """In the Q4 tcgen05 kernels the issuing warp and the workers wait for the kernels before (griddepcontrol.wait) ahead of their first
     bounded wait for what depends on the staged activations."""
