@@ -87,11 +87,12 @@ def test_gemm_matches_oracle(ctx, orc, M, N, K):
     assert np.mean(got == c16) > 0.99
 
 
-@pytest.mark.parametrize("kernel", ["single"])
+@pytest.mark.parametrize("kernel", ["single", "pair"])
 @pytest.mark.parametrize("M,N,K", [(128, 224, 256), (256, 448, 512), (100, 200, 320), (1, 8, 32), (640, 672, 2048),
-                                   (300, 224, 4096), (1200, 2912, 1024)])
+                                   (300, 224, 4096), (1200, 2912, 1024), (16, 448, 4096), (64, 232, 288)])
 def test_single_cta_kernel_matches_oracle(ctx, orc, kernel, M, N, K):
-    """The one-CTA-per-tile kernel, used where clusters of two cannot be scheduled (MPQ_FP4_KERNEL=single), computes the same GEMM."""
+    """The one-CTA-per-tile kernel, used where clusters of two cannot be scheduled (MPQ_FP4_KERNEL=single), and the one of CTA pairs, which
+    calls of up to 64 rows take where the weight has no tensor maps (pair), compute the same GEMM."""
     a, sfa = synth.nvfp4_tensor(M, K, seed=M + 2, stream=0)
     b, sfb = synth.nvfp4_tensor(N, K, seed=M + 2, stream=1)
     c32, c16 = orc.nvfp4_gemm(a, sfa, 0.5, b, sfb, 3.0)
@@ -321,12 +322,15 @@ def test_quantisation_at_the_rounding_boundaries(ctx, orc, ts):
         assert codes[:, :2].cpu().tolist() == [[0xF7, 0x80], [0x77, 0x77]] and sf.flatten().cpu().tolist() == [0x7E, 0x40]
 
 
-@pytest.mark.parametrize("M,N,K", [(1000, 4096, 14336), (300, 1024, 8192), (1, 4096, 8192), (257, 232, 6176)])
-def test_tiles_split_along_k(ctx, orc, M, N, K):
+@pytest.mark.parametrize("M,N,K,kernel", [(1000, 4096, 14336, None), (300, 1024, 8192, None), (1, 4096, 8192, None), (257, 232, 6176, None),
+                                          (1, 4096, 8192, "pair"), (16, 4096, 14336, "pair"), (64, 1024, 6176, "pair")])
+def test_tiles_split_along_k(ctx, orc, monkeypatch, M, N, K, kernel):
     """Shapes whose last (or only) wave of tiles is cut along K: sampled rows against the oracle, nothing written outside the
     output, the same bits twice."""
     import torch
     import makepad_b200
+    if kernel:
+        monkeypatch.setenv("MPQ_FP4_KERNEL", kernel)
     a, sfa = synth.nvfp4_tensor(M, K, seed=31, stream=0)
     b, sfb = synth.nvfp4_tensor(N, K, seed=31, stream=1)
     lin = makepad_b200.QuantLinear(makepad_b200.Nvfp4Weight(ctx, b, sfb, 2.0))
@@ -343,11 +347,15 @@ def test_tiles_split_along_k(ctx, orc, M, N, K):
     _check(orc, y[rows].view(torch.int16).cpu().numpy().view(np.uint16), c32)
 
 
-def test_a_graph_of_cut_tiles_replays_after_calls_that_need_more_scratch():
-    """4096 x 14336: 1000 rows need 28 partial tiles, 16 rows 57.  A graph of 1000 rows gives the same bits after eager calls of
-    16 rows and calls with another K (whose scale factors are re-tiled into scratch)."""
+@pytest.mark.parametrize("kernel", [None, "pair"])
+def test_a_graph_of_cut_tiles_replays_after_calls_that_need_more_scratch(monkeypatch, kernel):
+    """4096 x 14336: in the kernel of CTA pairs 1000 rows need 28 partial tiles, 16 rows 57 (the kernel of few rows, which takes them by default,
+    cuts K in eight).  A graph of 1000 rows gives the same bits after eager calls of 16 rows and calls with another K (whose scale factors are
+    re-tiled into scratch, with CTA pairs those of 64 rows too)."""
     import torch
     import makepad_b200
+    if kernel:
+        monkeypatch.setenv("MPQ_FP4_KERNEL", kernel)
     N, K = 4096, 14336
     c2 = makepad_b200.Context(0)
     lin = makepad_b200.QuantLinear(makepad_b200.Nvfp4Weight(c2, *synth.nvfp4_tensor(N, K, seed=61, stream=1), 1.0))
@@ -382,14 +390,15 @@ def test_a_graph_of_cut_tiles_replays_after_calls_that_need_more_scratch():
     c2.close()
 
 
+@pytest.mark.parametrize("kernel,M", [(None, 16), ("pair", 16), (None, 70)])
 @pytest.mark.parametrize("warm", ["larger", "other kernel"])
-def test_a_captured_gemm_cuts_its_tiles_like_an_eager_one(orc, monkeypatch, warm):
-    """16 rows of 4096 x 14336 want more room for partial tiles than 1000 rows do: captured after a warm-up with the larger M the
-    call still has two launches (GEMM, sum of the cut tiles) and the eager call's bits.  With no room reserved (the warm-up went
-    to the one-CTA kernel) the captured call keeps its tiles whole and agrees with the oracle."""
+def test_a_captured_gemm_cuts_its_tiles_like_an_eager_one(orc, monkeypatch, warm, kernel, M):
+    """16 and 70 rows of 4096 x 14336 want more room for partial tiles than 1000 rows do, in the kernel of CTA pairs and in the one of few rows:
+    captured after a warm-up with the larger M the call still has two launches (GEMM, sum of the cut tiles) and the eager call's bits.  With
+    no room reserved (the warm-up went to the one-CTA kernel) the captured call does not cut and agrees with the oracle."""
     import torch
     import makepad_b200
-    N, K, M = 4096, 14336, 16
+    N, K = 4096, 14336
     b, sfb = synth.nvfp4_tensor(N, K, seed=71, stream=1)
     a, sfa = synth.nvfp4_tensor(M, K, seed=71, stream=0)
     big = synth.nvfp4_tensor(1000, K, seed=72, stream=0)
@@ -401,6 +410,8 @@ def test_a_captured_gemm_cuts_its_tiles_like_an_eager_one(orc, monkeypatch, warm
     lin((torch.from_numpy(big[0]).cuda(), torch.from_numpy(big[1]).cuda(), 1.0))
     torch.cuda.synchronize()
     monkeypatch.delenv("MPQ_FP4_KERNEL", raising=False)
+    if kernel:
+        monkeypatch.setenv("MPQ_FP4_KERNEL", kernel)
     y = torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
     graph = torch.cuda.CUDAGraph()
     before = c2.launches
