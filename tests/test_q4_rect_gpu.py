@@ -68,21 +68,21 @@ def test_slices_are_added_by_a_cluster_or_by_a_second_launch(N, K, M, slices, on
 
 
 def test_slices_in_a_graph_and_on_two_streams(ctx, orc):
-    """Clusters under capture, and two calls of one context in flight on two streams (they share no scratch)."""
+    """Clusters under capture, and calls of two contexts in flight on two streams (the calls of one context are ordered)."""
     import makepad_b200
     import torch
     N, K, M = 4096, 4096, 8
     codes, scales = synth.q4_weight(N, K, seed=73)
-    w = makepad_b200.Q4Weight(ctx, codes, scales)
-    lin = makepad_b200.QuantLinear(w)
+    contexts = [makepad_b200.Context(0) for _ in range(2)]
+    lins = [makepad_b200.QuantLinear(makepad_b200.Q4Weight(c, codes, scales)) for c in contexts]
     xs = [torch.from_numpy(synth.activations(M, K, seed=74 + i)).cuda() for i in range(2)]
-    want = [lin(x) for x in xs]
+    want = [lin(x) for lin, x in zip(lins, xs)]
     torch.cuda.synchronize()
     side = torch.cuda.Stream()
     out = torch.empty_like(want[0])
     g = torch.cuda.CUDAGraph()
     with torch.cuda.graph(g, stream=side):
-        lin.forward(xs[0], out=out)
+        lins[0].forward(xs[0], out=out)
     out.zero_()
     g.replay()
     torch.cuda.synchronize()
@@ -92,8 +92,11 @@ def test_slices_in_a_graph_and_on_two_streams(ctx, orc):
     for k in range(8):
         for i, s in enumerate(streams):
             with torch.cuda.stream(s):
-                lin.forward(xs[i], out=outs[i][k])
+                lins[i].forward(xs[i], out=outs[i][k])
     torch.cuda.synchronize()
     assert all(torch.equal(o, want[i]) for i in range(2) for o in outs[i])
-    w.destroy()
-    assert ctx.lib.mpq_context_poll_status(ctx.h) == _lib.OK
+    del g
+    for lin, c in zip(lins, contexts):
+        assert c.lib.mpq_context_poll_status(c.h) == _lib.OK
+        lin.w.destroy()
+        c.close()
