@@ -456,11 +456,12 @@ __global__ void __launch_bounds__(Q4_THREADS) q4_linear_kernel(const Q4Launch p)
 // between two CTAs is finished through global scratch (q4s_cross_cta).
 //
 // What bounds it: up to about 10 MB per launch the fixed parts (prologue, staging of x, merge, the next launch's wait), else the run
-// itself, 43 cycles per unit and SM against 47..51 at the HBM rate.  One row takes copies of four chunks (G = 4): one barrier wait and one
-// refill for four units.  Before (two chunks per copy, waits in front of each copy's arithmetic, divisions in the prologue, one warp per shared tile
-// in the merge) / now, us per launch in a graph: 4096 x 4096 5.55 / 4.78, 12288 x 4096 8.6 / 7.85, 22016 x 4096 12.05 / 11.6, 4096 x 11008
-// 9.7 / 8.5, 1000 x 2112 6.4 / 5.3, 57344 x 8192 45.6 / 43.9, 2 rows of 4096 x 4096 7.1 / 6.6 (four chunks per copy: 6.8).  With the staging's
-// slots found once per thread and its maximum by reductions of a warp: 4.57, 7.7, 11.5, 8.3, 5.1, 43.6; 6.4.
+// itself.  One row takes copies of four chunks (G = 4): one barrier wait and one refill for four units.  Two chunks per copy, divisions in the
+// prologue, slots of the staging found per element, one warp per shared tile in the merge / this form, us per launch in a graph: 4096 x 4096 5.63 / 4.34,
+// 12288 x 4096 8.58 / 7.65, 22016 x 4096 11.6 / 10.7, 4096 x 11008 9.7 / 8.3, 1000 x 2112 6.5 / 5.2, 57344 x 8192 43.8 / 39.8, 128256 x 4096 46.5 / 42.0; 2 rows
+// of 4096 x 4096 7.3 / 6.3 (four chunks per copy: 0.2 more), of 22016 x 4096 13.4 / 13.2, of 128256 x 4096 48.1 / 48.4, of 152064 x 3584 49.5 / 51.2.
+// A look at the next copy's barrier ahead of the last unit's arithmetic and a predicated refill, which help the rectangle kernel, cost several rows
+// here 2..6 % (22016 x 4096 13.5, 49152 x 2048 13.2 -> 13.9) and gave one row nothing.
 constexpr int Q4S_WARPS = 16;                    // one CTA of sixteen warps per SM
 constexpr int Q4S_THREADS = Q4S_WARPS * 32;
 constexpr int Q4S_MAX_DEPTH = 8;                 // most ring stages per warp
@@ -695,6 +696,24 @@ __device__ __noinline__ void q4s_cross_cta(const Q4StreamLaunch& p, float v, int
     q4s_store_value(p, v, q, rp, lane);
 }
 
+// ... all four of them
+__device__ __forceinline__ void q4s_store_tile(const Q4StreamLaunch& p, const float (&v)[4], int rp, int lane)
+{
+    const int g = lane >> 2, t = lane & 3;
+    if (t >= p.M) return;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int n = rp * 32 + (q >> 1) * 16 + g + 8 * (q & 1);
+        if (n >= p.N) continue;
+        if (p.xworld > 0) {
+            const size_t e = (size_t)p.xrank * p.xslot + (size_t)t * p.N + n;
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+                if (r < p.xworld) st_tagged_sys(p.xpeer[r] + e, v[q], 1u);
+        } else p.Y[(size_t)t * p.ldy + n] = v[q];
+    }
+}
+
 // One float4 of x (element index 4f of activation row m) -> normalised hi/lo fp16 fragments in xs, block
 // corrections in cs.
 //   xs: uint4 [chunk][2M columns][4 t][2 blocks]   column 2m = hi, 2m+1 = lo of activation row m; the uint4 of
@@ -905,8 +924,7 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
         float v[4] = {acc[0][0] * fA, acc[0][1] * fB, acc[1][0] * fA, acc[1][1] * fB};
         const int r0 = tile_rp * gpr;
         if (gb <= r0 && r0 + gpr <= ge) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) q4s_store_value(p, v[q], q, tile_rp, lane);
+            q4s_store_tile(p, v, tile_rp, lane);
         } else {
             const int slot = tile_rp == first_rp ? 0 : 1;
 #pragma unroll
@@ -920,11 +938,9 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
     const long long cyc_loop0 = clock64();
 #endif
 
-    // The look at the next stage's barrier is a round trip of about 90 cycles: it is taken while this stage's last unit is multiplied.
-    bool ready = false;
     for (int j = 0; j < ngroups; ++j) {
         Q4S_CYC(c_w)
-        const bool arrived = ready || mbar_wait(bars_u32 + s * 8, parity, Q4S_SPIN_LIMIT);
+        const bool arrived = mbar_wait(bars_u32 + s * 8, parity, Q4S_SPIN_LIMIT);
         Q4S_CYC_ADD(cyc_wait, c_w)
         if (!arrived) {
             // Record it, issue nothing more, and give every copy still in flight the same generous bounded wait, so
@@ -936,8 +952,6 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
             timed_out = true;
             break;
         }
-        const int next_s = s + 1 == D ? 0 : s + 1;
-        const uint32_t next_parity = next_s ? parity : parity ^ 1u;
         const uint32_t st = s * STAGE_BYTES;
 #pragma unroll
         for (int q = 0; q < G; ++q) {
@@ -948,7 +962,6 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
             const float4 cf = make_float4(__uint_as_float(cfu.x), __uint_as_float(cfu.y), __uint_as_float(cfu.z), __uint_as_float(cfu.w));
             xsp += xstep;
             csp += cstep;
-            if (q == G - 1) ready = mbar_test(bars_u32 + next_s * 8, next_parity);
             const uint32_t wt[2][4] = {{w0.x, w0.y, w0.z, w0.w}, {w1.x, w1.y, w1.z, w1.w}};
             const uint32_t sw[2][2] = {{sv.x, sv.y}, {sv.z, sv.w}};
 #pragma unroll
@@ -971,8 +984,12 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
         ++cg;
         Q4S_CYC(c_r)
         __syncwarp();
-        bulk_refill(ring_u32 + s * STAGE_BYTES, gnext, STAGE_BYTES, bars_u32 + s * 8, l2pol, lane == 0 && j + D < ngroups);    // the stage just drained
-        gnext += STAGE_BYTES;
+        if (lane == 0 && j + D < ngroups) {                // refill the stage just drained
+            mbar_expect_tx(bars_u32 + s * 8, STAGE_BYTES);
+            bulk_g2s(ring_u32 + s * STAGE_BYTES, gnext, STAGE_BYTES, bars_u32 + s * 8, l2pol);
+            gnext += STAGE_BYTES;
+        }
+        __syncwarp();
         Q4S_CYC_ADD(cyc_refill, c_r)
 #ifdef MPQ_TRACE
         if (j == 0) cyc_first = clock64() - cyc_loop0;
@@ -985,8 +1002,7 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
             xsp = xs0;
             csp = cs0;
         }
-        s = next_s;
-        parity = next_parity;
+        if (++s == D) { s = 0; parity ^= 1u; }
     }
     if (cg != 0 && !timed_out) flush(rp);  // the run ended inside a row pair-tile
 #ifdef MPQ_TRACE
@@ -1000,30 +1016,53 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
     __syncthreads();
     Q4S_TRACE(6)
 
-    // ---- tiles shared between warps: add the parked partials in warp order.  Segment (w, slot) opens a tile if no segment before it
-    // belongs to the same one; four warps then add the tile's segments, one of its four values per lane each (one warp for all four, and a
-    // search for each segment, took 0.9..1.8 us).  The sharers are consecutive warps, and all but the first have the tile in slot 0.
+    // ---- tiles shared between warps: add the parked partials in warp order.  The sharers of a tile are consecutive warps, and all but the
+    // first have it in slot 0: segment (w, slot) opens a tile if the one before it belongs to another.  Up to four tiles are added by four
+    // warps each, one of the four values per lane: with up to sixteen sharers of one tile a warp for all of it took 0.7 us longer (4096 x 4096).  More
+    // tiles have few sharers each and are added by the warps that open them, in a loop that is short on purpose: every CTA goes through
+    // it once, and its time is that of fetching the instructions.  (Four warps per tile here, too: 100000 x 2048 20.1 instead of 19.1 us.  The vote over
+    // equal tiles by __match_any_sync: another 0.2 us with twelve tiles.)
     const int entry = wrp[lane >> 1][lane & 1];             // lane i holds segment i = (warp i/2, slot i%2)
-    const uint32_t peers = __match_any_sync(0xFFFFFFFFu, entry);
-    uint32_t openers = __ballot_sync(0xFFFFFFFFu, entry >= 0 && (peers & ((1u << lane) - 1u)) == 0);
-    const int cta_first_rp = q4s_tile_of(cta_gb, gpr, p.gpr_magic), q = warp & 3;
-    for (int skip = warp >> 2; openers; openers &= openers - 1u) {
-        if (skip--) continue;
-        skip = NW / 4 - 1;
-        const int first = __ffs(openers) - 1, my = __shfl_sync(0xFFFFFFFFu, entry, first), count = __popc(__shfl_sync(0xFFFFFFFFu, peers, first));
-        const float* src = wpart + q * 32 + lane;
-        float v = src[first * 128];
-        src += (first & ~1) * 128;
-        for (int k = 1; k < count; k += 8) {
-            float u[8];
+    const int up1 = __shfl_up_sync(0xFFFFFFFFu, entry, 1), up2 = __shfl_up_sync(0xFFFFFFFFu, entry, 2);
+    uint32_t openers = __ballot_sync(0xFFFFFFFFu, entry >= 0 && ((lane & 1) || lane == 0 || entry != (up1 >= 0 ? up1 : up2)));
+    const int cta_first_rp = q4s_tile_of(cta_gb, gpr, p.gpr_magic);
+    if (__popc(openers) <= NW / 4) {
+        const int q = warp & 3;
+        for (int skip = warp >> 2; openers; openers &= openers - 1u) {
+            if (skip--) continue;
+            skip = NW / 4 - 1;
+            const int first = __ffs(openers) - 1, my = __shfl_sync(0xFFFFFFFFu, entry, first), count = __popc(__ballot_sync(0xFFFFFFFFu, entry == my));
+            const float* src = wpart + q * 32 + lane;
+            float v = src[first * 128];
+            src += (first & ~1) * 128;
+            for (int k = 1; k < count; k += 8) {
+                float u[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) u[i] = k + i < count ? src[(k + i) * 256] : 0.f;
+                for (int i = 0; i < 8; ++i) u[i] = k + i < count ? src[(k + i) * 256] : 0.f;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v += u[i];
+                for (int i = 0; i < 8; ++i) v += u[i];
+            }
+            const int r0 = my * gpr, r1 = r0 + gpr;
+            if (cta_gb <= r0 && r1 <= cta_ge) q4s_store_value(p, v, q, my, lane);
+            else q4s_cross_cta(p, v, q, my, r0, r1, cta_first_rp, lane);
         }
-        const int r0 = my * gpr, r1 = r0 + gpr;
-        if (cta_gb <= r0 && r1 <= cta_ge) q4s_store_value(p, v, q, my, lane);
-        else q4s_cross_cta(p, v, q, my, r0, r1, cta_first_rp, lane);
+    } else {
+#pragma unroll
+        for (int slot = 0; slot < 2; ++slot) {
+            const int segment = warp * 2 + slot, my = __shfl_sync(0xFFFFFFFFu, entry, segment);
+            if (!(openers >> segment & 1u)) continue;
+            float v[4] = {0.f, 0.f, 0.f, 0.f};
+            uint32_t same = __ballot_sync(0xFFFFFFFFu, entry == my);
+            for (; same; same &= same - 1u) {
+                const float* src = wpart + (size_t)(__ffs(same) - 1) * 128 + lane;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) v[q] += src[q * 32];
+            }
+            const int r0 = my * gpr, r1 = r0 + gpr;
+            if (cta_gb <= r0 && r1 <= cta_ge) q4s_store_tile(p, v, my, lane);
+            else
+                for (int q = 0; q < 4; ++q) q4s_cross_cta(p, q == 0 ? v[0] : q == 1 ? v[1] : q == 2 ? v[2] : v[3], q, my, r0, r1, cta_first_rp, lane);
+        }
     }
 
     Q4S_TRACE(7)

@@ -42,3 +42,30 @@ def test_runs_of_the_streaming_kernel(orc, group):
         w.destroy()
     assert c.lib.mpq_context_poll_status(c.h) == _lib.OK
     c.close()
+
+
+@pytest.mark.parametrize("tile", ["1", "0"])
+@pytest.mark.parametrize("N,K", [(28456, 320), (28300, 1088), (50000, 128), (24000, 768)])
+def test_many_tiles_per_cta(orc, monkeypatch, N, K, tile):
+    """More than four tiles of a CTA are shared between its warps (fewer take another way through the merge); with equal runs (tile 0) its
+    first and last tile are shared with the neighbours as well."""
+    import makepad_b200
+    import torch
+    monkeypatch.setenv("MPQ_Q4_TILE", tile)
+    c = makepad_b200.Context(0)
+    codes, scales = synth.q4_weight(N, K, seed=64)
+    w = makepad_b200.Q4Weight(c, codes, scales)
+    lin = makepad_b200.QuantLinear(w)
+    for M in (1, 2, 4):
+        x = synth.activations(M, K, seed=65)
+        xd = torch.from_numpy(x).cuda()
+        buf = torch.full((M * N + 256,), 777.0, device="cuda")
+        y = buf[128:128 + M * N].view(M, N)
+        lin.forward(xd, out=y)
+        assert torch.equal(y, lin(xd))
+        rep = orc.err_report(y.cpu().numpy(), orc.q4_matmul_f64(codes, scales, x))
+        assert rep["floored_1e-2_rms"] < 1e-3 and rep["max_abs_over_rms"] < 2e-5, (N, K, M, rep)
+        assert (buf[:128] == 777.0).all() and (buf[128 + M * N:] == 777.0).all()
+    w.destroy()
+    assert c.lib.mpq_context_poll_status(c.h) == _lib.OK
+    c.close()
