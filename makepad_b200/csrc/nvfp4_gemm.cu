@@ -33,6 +33,7 @@
 #include <cstring>
 
 #include "nvfp4.cuh"
+#include "nvfp4_plan.h"
 #include "pdl.cuh"
 #include "swiglu.cuh"
 #include "per_device.h"
@@ -232,7 +233,6 @@ cudaError_t nvfp4_quantize_launch(const void* x, bool bf16, bool swiglu, int64_t
 // ---------------------------------------------------------------------------
 // geometry
 // ---------------------------------------------------------------------------
-constexpr int BM = 128, BN = 224, BK = 256;               // BK in elements
 
 // The same export for a WEIGHT, whose scale factors exist on the device only in the tiled order the GEMM
 // consumes (nvfp4_sf_tile_kernel with tiles of BN rows): reading them back from there proves the tiling pass.
@@ -838,7 +838,6 @@ constexpr int Q_STAGE_BYTES = A_BYTES + P_BH_BYTES + SFA_BYTES + SFB_BYTES;     
 constexpr int Q_OUT_COLS = 16;                                                  // columns per TMA store of one epilogue warp
 constexpr int Q_OUT_BYTES = 32 * Q_OUT_COLS * 2;                                // 1024: 32 rows of bf16, dense
 constexpr int Q_SMEM_BYTES = Q_STAGES * Q_STAGE_BYTES + 8 * Q_OUT_BYTES + 1024 + 256;
-constexpr int SPLIT_MIN_BLOCKS = 2;                                             // fewest K blocks of an item of a tile that is cut along K
 static_assert(V2_EPI_COLS % Q_OUT_COLS == 0 && (Q_OUT_COLS * 2) % 16 == 0, "store boxes tile the epilogue columns in 16-byte units");
 static_assert(V2_SF_COL + Q_STAGES * V2_SF_COLS <= TMEM_COLS, "scale-factor buffers must fit beside the accumulator");
 
@@ -1291,31 +1290,18 @@ static bool partial_room(Nvfp4Scratch& scratch, int pairs, cudaStream_t s)
 }
 
 // Up to RW_MAX_ROWS activation rows through nvfp4_rows_kernel.
-static int32_t nvfp4_rows_launch(Nvfp4Scratch& scratch, const Nvfp4Dev& w, const uint8_t* a_codes, const uint8_t* a_sf, float ta, int M, uint16_t* c, int device,
-                                 int sm_count, bool pdl, int pinned, cudaStream_t s, int* launches, std::string& err)
+static int32_t nvfp4_rows_launch(Nvfp4Scratch& scratch, const Nvfp4Dev& w, const RowsPlan& pl, const uint8_t* a_codes, const uint8_t* a_sf, float ta, int M, uint16_t* c,
+                                 int device, int sm_count, bool pdl, cudaStream_t s, int* launches, std::string& err)
 {
     RowsParams p;
-    p.M = M; p.Mp = (M + 15) / 16 * 16; p.N = (int)w.N; p.K = (int)w.K;
-    p.k_blocks = (int)((w.K + BK - 1) / BK); p.ksteps_pad = ksteps_padded(w.K);
+    p.M = M; p.Mp = pl.Mp; p.N = (int)w.N; p.K = (int)w.K;
+    p.k_blocks = pl.k_blocks; p.ksteps_pad = ksteps_padded(w.K);
     p.C = reinterpret_cast<__nv_bfloat16*>(c); p.sfx = a_sf; p.sfw = w.sf_tiled; p.scale = ta * w.tensor_scale; p.status = scratch.status;
     p.sfx_wide = w.K % 256 == 0;                           // (the array is 16-byte aligned)
-    const int n_tiles = (p.N + BN - 1) / BN, tiles = 2 * n_tiles - (p.N - (n_tiles - 1) * BN <= 128);        // (the last tile may have one atom)
-    const int stage = A_BYTES + p.Mp * (BK / 2) + SFA_BYTES;
+    const int tiles = pl.tiles, stage = A_BYTES + p.Mp * (BK / 2) + SFA_BYTES;
     p.stages = std::min(RW_MAX_STAGES, (RW_SMEM_MOST - 1024) / stage);
-    // Cuts of K, by estimated cost (us): a K block of a CTA; a second launch (1.5 of device time, and the host's 2.5 where it is the host that is
-    // waited for), and what the cuts write for it.  Never more CTAs than are resident at once: 8192 x 8192 at 16 rows, 32 K blocks, uncut 18.0, in four 11.0, in five (370 CTAs) 15.1.
-    // (pinned: as many cuts as that, as far as K goes)
-    const int most = pinned ? pinned : 16;
-    int splits = 1;
-    const double per_block = 0.44 + 0.0055 * p.Mp;
-    double best = pinned ? 1e30 : per_block * p.k_blocks;
-    for (int n = 2; n <= std::min(most, p.k_blocks / SPLIT_MIN_BLOCKS) && (pinned || tiles * n <= 2 * sm_count); ++n) {
-        const size_t bytes = (size_t)tiles * n * p.Mp * 128 * sizeof(float);
-        const double cost = per_block * ((p.k_blocks + n - 1) / n) + 3.6 + bytes / 3e6;
-        if (pinned || cost < best) { best = cost; splits = n; }
-    }
     const bool room = partial_room(scratch, sm_count / 2, s);         // (by an uncut call too)
-    if (splits > 1 && (!room || scratch.partial.bytes() < (size_t)tiles * splits * p.Mp * 128 * sizeof(float))) splits = 1;
+    const int splits = room && scratch.partial.bytes() >= rows_partial_bytes(pl) ? pl.splits : 1;
     p.splits = splits;
     p.partial = scratch.partial.as<float>();
     CUtensorMap map_x;
@@ -1359,15 +1345,20 @@ int32_t nvfp4_gemm_launch(Nvfp4Scratch& scratch, const Nvfp4Dev& w, const uint8_
         if (e == cudaSuccess) e = cudaMemset(scratch.status, 0, sizeof(int));
         if (e != cudaSuccess) { err = std::string("status allocation failed: ") + cudaGetErrorString(e); return MPQ_ERR_CUDA; }
     }
-    // MPQ_FP4_KERNEL=single forces the one-CTA kernel, pair the kernel of CTA pairs, rows=<n> so many cuts of K in the one of few rows, which
-    // the parity tests use to cover all
+    // MPQ_FP4_KERNEL=single forces the one-CTA kernel, pair the kernel of CTA pairs, rows=<n> the one of few rows (up to 64) with n cuts of K (0: its
+    // own choice), which the parity tests use to cover all
     const char* env = getenv("MPQ_FP4_KERNEL");
-    const bool single = env && strcmp(env, "single") == 0, pair = env && strcmp(env, "pair") == 0;
-    if (M <= RW_MAX_ROWS && w.mapped && !single && !pair)
-        return nvfp4_rows_launch(scratch, w, a_codes, a_sf, ta, (int)M, c, device, sm_count, pdl, env && strncmp(env, "rows=", 5) == 0 ? atoi(env + 5) : 0, s, launches, err);
+    const bool single = env && strcmp(env, "single") == 0, pair = env && strcmp(env, "pair") == 0, rows = env && strncmp(env, "rows=", 5) == 0;
     // The activations' scale factors are read straight from the canonical [M][K/16] array when a K block's 16 bytes per
     // row can be a TMA box (row pitch a multiple of 16 bytes); otherwise they are re-tiled first, like the weights'.
     const bool direct = K % 256 == 0 && (reinterpret_cast<uintptr_t>(a_sf) & 15u) == 0;
+    const int nclusters = single ? 0 : pair_v2_clusters(device, sm_count);
+    if (M <= RW_MAX_ROWS && w.mapped && !single && !pair) {
+        const RowsPlan pl = rows_plan((int)M, N, K, sm_count, rows ? atoi(env + 5) : 0);
+        // (re-tiled scale factors would be another launch, and scratch that a capture after a call of other rows might not have)
+        if (rows || !direct || nclusters == 0 || nvfp4_rows_pay(pl, pair_plan(M, N, K, nclusters), M))
+            return nvfp4_rows_launch(scratch, w, pl, a_codes, a_sf, ta, (int)M, c, device, sm_count, pdl, s, launches, err);
+    }
     cudaError_t e = cudaSuccess;
     if (!direct) {
         e = scratch.sfa_tiled.reserve(sf_tiled_bytes(M, K, BM, 2));
@@ -1382,32 +1373,20 @@ int32_t nvfp4_gemm_launch(Nvfp4Scratch& scratch, const Nvfp4Dev& w, const uint8_
         err = "cuTensorMapEncodeTiled failed (pointers must be 16-byte aligned, K a multiple of 32)";
         return MPQ_ERR_CUDA;
     }
-    // CTA pairs where clusters of two can be scheduled
-    const int nclusters = single ? 0 : pair_v2_clusters(device, sm_count);
-    if (nclusters > 0) {
+    if (nclusters > 0) {                                   // CTA pairs where clusters of two can be scheduled
         CUtensorMap map_bh, map_c;
         if (!make_map(&map_bh, w.codes, N, K, BN / 2) || !make_c_map(&map_c, c, M, N, Q_OUT_COLS)) { err = "cuTensorMapEncodeTiled failed for the CTA-pair kernel"; return MPQ_ERR_CUDA; }
         PairParams pp;
         pp.C = reinterpret_cast<__nv_bfloat16*>(c);
         pp.M = (int)M; pp.N = (int)N; pp.K = (int)K;
-        pp.m_pairs = (int)((M + 2 * BM - 1) / (2 * BM)); pp.n_tiles = (int)((N + BN - 1) / BN);
-        pp.k_blocks = (int)((K + BK - 1) / BK); pp.ksteps_pad = ksteps_padded(K);
+        const PairPlan pl = pair_plan(M, N, K, nclusters);
+        pp.m_pairs = pl.m_pairs; pp.n_tiles = pl.n_tiles;
+        pp.k_blocks = pl.k_blocks; pp.ksteps_pad = ksteps_padded(K);
         pp.scale = ta * w.tensor_scale;
         pp.status = scratch.status;
         pp.sfa_direct = direct ? 1 : 0;
-        // Full waves of tiles go whole; a last wave that leaves pairs idle may be cut along K.  The cut that costs least, by
-        // rates measured on 74 pairs (microseconds: a K block of a pair; the launch that adds the items and the fp32 epilogue;
-        // writing and adding the rows of one item); uncut unless it gains a microsecond.  GEMM and sum in a graph, 1000 x 4096 x 14336
-        // (2 tiles of 76 in the second wave): 47.6 -> 38.8 us; 16 x 1024 x 8192 (5 tiles): 17.2 -> 8.8; but 700 x 11008 x 4096 (2 of
-        // 150) cut into eighths of 16 K blocks: 24.9 -> 28.7, left whole.
-        const int tiles = pp.m_pairs * pp.n_tiles, last = tiles % nclusters;
-        const double rows = (double)M / (256.0 * pp.m_pairs);
-        int splits = 1;
-        double best = 0.42 * pp.k_blocks - 1.0;
-        for (int c = 2; last && c <= std::min(nclusters / last, pp.k_blocks / SPLIT_MIN_BLOCKS); ++c) {
-            const double cost = 0.42 * ((pp.k_blocks + c - 1) / c) + 5.0 + 0.08 * rows * last * c;
-            if (cost < best) { best = cost; splits = c; }
-        }
+        const int tiles = pl.tiles, last = pl.last;
+        int splits = pl.splits;
         if (!partial_room(scratch, nclusters, s)) splits = 1;      // (last * splits <= nclusters)
         pp.splits = splits;
         pp.whole = splits > 1 ? tiles - last : tiles;

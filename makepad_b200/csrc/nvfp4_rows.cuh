@@ -19,7 +19,7 @@
 
 namespace mpq {
 
-constexpr int RW_THREADS = 192, RW_MAX_ROWS = 64, RW_MAX_STAGES = 6, RW_TMEM_COLS = 256;
+constexpr int RW_THREADS = 192, RW_MAX_STAGES = 6, RW_TMEM_COLS = 256;
 constexpr int RW_SF_COLS = 32;                             // tensor-memory columns of a stage: [weights: 4 K steps x 4 | activations: 4 x 4]
 constexpr int RW_SMEM_MOST = 112 * 1024;
 // Tries of a suspended wait (up to 4 us each): the producer and the epilogue wait so, the others look all the time.  Eight shapes of 1 to 64 rows, all

@@ -461,6 +461,41 @@ def test_pages_for_host_rows_grow_in_doubling_steps():
     _run(PAGES)
 
 
+FP4 = r"""
+#include "nvfp4_plan.h"
+#include <cstdio>
+using namespace mpq;
+static bool rows(int M, int64_t N, int64_t K) { return nvfp4_rows_pay(rows_plan(M, N, K, 148, 0), pair_plan(M, N, K, 74), M); }
+int main()
+{
+    int bad = 0;
+    // one CTA more than a full wave, K too short for 64 rows, and their neighbours, as measured
+    bad += rows(64, 33264, 2048) || !rows(64, 33152, 2048) || rows(64, 33264, 14336) || !rows(64, 28672, 4096) || !rows(64, 57344, 4096);
+    bad += rows(64, 8192, 2048) || rows(64, 14336, 4096) || !rows(64, 4096, 4096) || !rows(64, 4096, 14336) || !rows(48, 14336, 4096);
+    for (int64_t N = 8; N < 200000; N += 8 * 61)
+        for (int64_t K = 32; K < 60000; K += 32 * 37)
+            for (int M : {1, 16, 17, 32, 33, 64}) {
+                const RowsPlan r = rows_plan(M, N, K, 148, 0);
+                const PairPlan p = pair_plan(M, N, K, 74);
+                bad += M <= 32 && !rows(M, N, K);
+                bad += r.splits < 1 || (r.splits > 1 && (r.tiles * r.splits > 296 || r.k_blocks / r.splits < SPLIT_MIN_BLOCKS));
+                bad += r.tiles * 96 > N + 224 || r.tiles * 128 < N || r.Mp % 16 || r.Mp < M;
+                bad += rows_partial_bytes(r) > (size_t)74 * 256 * BN * 4 && r.splits > 1;          // the room that is reserved
+                bad += p.splits < 1 || p.last * p.splits > 74 || (p.splits > 1 && p.k_blocks / p.splits < SPLIT_MIN_BLOCKS);
+                bad += !(r.cost > 0) || !(p.cost > 0);
+                const RowsPlan cut = rows_plan(M, N, K, 148, 3);
+                bad += cut.splits != (r.k_blocks >= 6 ? 3 : r.k_blocks >= 4 ? 2 : 1);
+            }
+    std::printf("%d\n", bad);
+    return bad;
+}
+"""
+
+
+def test_few_nvfp4_rows_go_to_the_kernel_that_is_faster():
+    _run(FP4)
+
+
 def test_every_kernel_that_can_give_up_a_wait_settles_before_it_ends():
     """A kernel whose roles share an abort flag waits for what was in flight behind its last CTA barrier, before tensor memory is freed."""
     kernels = 0
