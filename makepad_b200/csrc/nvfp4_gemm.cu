@@ -34,6 +34,8 @@
 
 #include "nvfp4.cuh"
 #include "nvfp4_plan.h"
+#include "nvfp4_ptx.cuh"
+#include "nvfp4_rows.cuh"
 #include "pdl.cuh"
 #include "swiglu.cuh"
 #include "per_device.h"
@@ -255,16 +257,11 @@ __global__ void nvfp4_dequant_tiled_kernel(const uint8_t* __restrict__ codes, co
     out[r * K + 2 * kb + 1] = e2m1_value(b >> 4) * s * ts;
 }
 constexpr int STAGES = 4;
-constexpr int A_BYTES = BM * BK / 2;                       // 16384
-constexpr int B_BYTES = BN * BK / 2;                       // 28672
-constexpr int SFA_BYTES = 4 * 512;                         // four K steps x one 128-row atom
-constexpr int SFB_BYTES = 4 * 2 * 512;                     // four K steps x two atoms (224 rows)
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES + SFA_BYTES + SFB_BYTES;   // 51200
 constexpr int OUT_COLS = 16;                               // columns per TMA store of one epilogue warp (one-CTA kernel)
 constexpr int OUT_BYTES = 32 * OUT_COLS * 2;               // 1024: 32 rows of bf16, dense
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 8 * OUT_BYTES + 1024 /*align*/ + 256 /*barriers*/;
 constexpr int TMEM_COLS = 512;
-constexpr uint32_t SPIN_LIMIT = 1u << 22;     // polls of one mbarrier before the kernel gives up and reports it
 
 // scale factors of `rows` rows, tiled for tiles of `tile_rows` rows (128 for A, 224 for B):
 // dst[tile][kstep][atom][512] with atom = local_row / 128, zero where row or K step is out of range.
@@ -345,144 +342,6 @@ int32_t nvfp4_weight_build(Nvfp4Dev& w, int64_t N, int64_t K, const uint8_t* cod
     if (e == cudaSuccess) nvfp4_weight_map(w);
     if (e != cudaSuccess) { err = std::string("NVFP4 weight build failed: ") + cudaGetErrorString(e); return MPQ_ERR_CUDA; }
     return MPQ_OK;
-}
-
-// ---------------------------------------------------------------------------
-// PTX wrappers
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t s2u(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void bar_expect_tx(uint32_t bar, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void bar_arrive(uint32_t bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-// bounded wait: false when the limit ran out
-__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, uint32_t limit)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        ".reg .u32 n;\n\t"
-        "mov.u32 n, 0;\n\t"
-        "W_LOOP:\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "@p bra W_DONE;\n\t"
-        "add.u32 n, n, 1;\n\t"
-        "setp.lt.u32 p, n, %3;\n\t"
-        "@p bra W_LOOP;\n\t"
-        "mov.u32 %0, 0;\n\t"
-        "bra W_END;\n\t"
-        "W_DONE:\n\t"
-        "mov.u32 %0, 1;\n\t"
-        "W_END:\n\t"
-        "}"
-        : "=r"(ok) : "r"(bar), "r"(parity), "r"(limit) : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar)
-{
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar)
-{
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint32_t bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tc_mma_nvf4(uint32_t d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t sfa,
-                                            uint32_t sfb, uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %6, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%4], [%5], p;\n\t"
-        "}"
-        ::"r"(d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&r)[32])
-{
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void tc_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t* r)
-{
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr) : "memory");
-}
-// registers -> this warp's 32 TMEM lanes: thread l writes lane l, register j goes to column +j
-__device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t* r)
-{
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-                   "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
-}
-__device__ __forceinline__ void tc_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// TMA tile store shared -> global (rows and columns beyond the tensor are clipped); completion is tracked per thread
-// by bulk groups
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int y, uint32_t src)
-{
-    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x), "r"(y), "r"(src) : "memory");
-    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-}
-__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-__device__ __forceinline__ bool bar_test(uint32_t bar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-// bounded spin on a phase parity without suspending the thread: for the hand-offs whose latency is on the critical path
-__device__ __forceinline__ bool bar_spin(uint32_t bar, uint32_t parity, uint32_t limit)
-{
-    for (uint32_t n = 0; n < limit; ++n) {
-        uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (ok) return true;
-    }
-    return false;
-}
-
-// K-major operand tile, SWIZZLE_128B: rows are 128 bytes, 8-row groups 1024 bytes apart
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr)
-{
-    uint64_t d = 0;
-    d |= (uint64_t)((addr >> 4) & 0x3FFF);          // start address
-    d |= (uint64_t)1 << 16;                         // leading byte offset field (unused for swizzled K-major): 1
-    d |= (uint64_t)(1024 >> 4) << 32;               // stride byte offset: 8 rows * 128 B
-    d |= (uint64_t)1 << 46;                         // descriptor version for sm_100
-    d |= (uint64_t)2 << 61;                         // SWIZZLE_128B
-    return d;
 }
 
 struct GemmParams {
@@ -1090,10 +949,6 @@ __global__ void __launch_bounds__(224) nvfp4_pair_reduce_kernel(const PairParams
         *reinterpret_cast<uint2*>(p.C + (size_t)m * p.N + n) = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
     }
 }
-
-}  // namespace mpq
-#include "nvfp4_rows.cuh"              // nvfp4_rows_kernel, on the helpers above
-namespace mpq {
 
 // ---------------------------------------------------------------------------
 // measured ceiling of the FP4 tensor pipe

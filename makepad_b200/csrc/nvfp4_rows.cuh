@@ -1,6 +1,6 @@
 // NVFP4 GEMM of few activation rows (up to 64): the WEIGHTS are the M = 128 operand.
 //
-// With a handful of rows the GEMM streams the weights once, and the tiles of the kernels above are wrong for that: 256 activation rows of which 16
+// With a handful of rows the GEMM streams the weights once, and the tiles of the kernels for more rows are wrong for that: 256 activation rows of which 16
 // exist, half of a 224-column tile per CTA, no weight fetched before the kernels in front have ended.  Here a CTA takes 128 or 96
 // weight rows (the two scale-factor atoms of a 224-row tile, which are in the order that the M operand's scales have, too) and a range of
 // K blocks; the N = 16..64 operand is the activation.  A CTA keeps to less than half of an SM's shared memory and tensor memory, so that two are
@@ -14,17 +14,24 @@
 // and 16 rows of 14336 x 4096 stream 3.2 TB/s.  CTA pairs / this kernel (us, GEMM alone in a graph): 14336 x 4096 at 1 row 43 / 10.0 (64 pairs
 // asked for one row of 256), 16 14.7 / 10.4, 64 15.1 / 14.5; 28672 x 4096 at 16 24.1 / 13.9, 64 24.0 / 16.6; 4096 x 14336 at 16 16.7 / 10.7, 64 19.5 / 13.2;
 // 4096 x 4096 at 16 10.5 / 6.0; 8192 x 8192 at 16 18.7 / 11.0, 64 16.6 / 13.9; 1024 x 1024 at 16 5.9 / 4.6.
-// Part of nvfp4_gemm.cu, whose geometry and PTX wrappers it uses.
 #pragma once
+#include <cuda.h>
+#include <cuda_bf16.h>
+
+#include "nvfp4_plan.h"
+#include "nvfp4_ptx.cuh"
+#include "pdl.cuh"
+#include "settle.cuh"
 
 namespace mpq {
 
-constexpr int RW_THREADS = 192, RW_MAX_STAGES = 6, RW_TMEM_COLS = 256;
+constexpr int RW_THREADS = 192, RW_MAX_STAGES = 5, RW_TMEM_COLS = 256;
 constexpr int RW_SF_COLS = 32;                             // tensor-memory columns of a stage: [weights: 4 K steps x 4 | activations: 4 x 4]
 constexpr int RW_SMEM_MOST = 112 * 1024;
 // Tries of a suspended wait (up to 4 us each): the producer and the epilogue wait so, the others look all the time.  Eight shapes of 1 to 64 rows, all
 // spinning / this: 28672 x 4096 at 16 rows 14.0 / 13.85 us, 4096 x 14336 10.2 / 10.0, 4096 x 4096 5.84 / 5.73, the rest within 0.5 %.
 constexpr uint32_t RW_TRIES = 1u << 17;
+static_assert((RW_SMEM_MOST - 1024) / (A_BYTES + 16 * (BK / 2) + SFA_BYTES) == RW_MAX_STAGES, "the ring of the fewest rows is the longest");
 static_assert(RW_MAX_ROWS + RW_MAX_STAGES * RW_SF_COLS <= RW_TMEM_COLS, "accumulator and scale factors of two CTAs must fit in tensor memory");
 
 struct RowsParams {

@@ -499,13 +499,13 @@ def test_few_nvfp4_rows_go_to_the_kernel_that_is_faster():
 def test_every_kernel_that_can_give_up_a_wait_settles_before_it_ends():
     """A kernel whose roles share an abort flag waits for what was in flight behind its last CTA barrier, before tensor memory is freed."""
     kernels = 0
-    for f in ("q4_umma.cuh", "q4_gemm.cuh", "nvfp4_gemm.cu"):
+    for f in ("q4_umma.cuh", "q4_gemm.cuh", "nvfp4_gemm.cu", "nvfp4_rows.cuh"):
         text = open(os.path.join(ROOT, "makepad_b200", "csrc", f)).read()
         for body in text.split("volatile int s_abort;")[1:]:
             kernels += 1
             end = body[:body.index("tcgen05.dealloc")]
             assert "settle_after_timeout(s_abort);" in end[end.rindex("__syncthreads();"):], f
-    assert kernels == 4
+    assert kernels == 5
 
 
 def test_no_cta_of_a_cluster_leaves_while_another_may_still_store_into_it():
