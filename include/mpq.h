@@ -124,7 +124,8 @@ int32_t mpq_weight_destroy(mpq_weight* w);
  * row-major device arrays, 16-byte aligned.  Any M >= 1: one row, and up to
  * four rows while M * K < 16384, is one launch of the streaming kernel; up to
  * 16 rows otherwise one pass of the rectangle kernel (weights read once,
- * only a K slice of x staged per CTA) plus a small reduction; 17..64 rows
+ * only a K slice of x staged per CTA), one launch where its K slices are
+ * added inside a cluster and a small reduction behind it elsewhere; 17..64 rows
  * the tcgen05 kernel; above that the tcgen05 kernel on tiles of 256 weight
  * rows x up to 128 activation rows, or, up to 128 rows of a large weight, two
  * slabs of 64 rows (each: activation staging, main kernel, reduction of the
@@ -165,8 +166,9 @@ int32_t mpq_q4_linear_forward(mpq_context* ctx, const mpq_weight* w, const float
  * that a kernel sets non-zero when one of its bounded waits runs out. */
 int32_t mpq_q4_linear_forward_static(mpq_context* ctx, const mpq_weight* w, const float* x_dev, int64_t M,
                                      float* y_dev, int32_t* status_dev, void* stream);
-/* Convenience end-to-end call with HOST buffers: copies X up, runs, copies Y
- * back and synchronises. */
+/* Convenience end-to-end call with HOST buffers: brings X up (rows of up to
+ * 512 KB in ordinary memory through page-locked pages that the context keeps),
+ * runs, brings Y back and synchronises.  Calls on one context take turns. */
 int32_t mpq_q4_linear_forward_host(mpq_context* ctx, const mpq_weight* w, const float* x_host, int64_t M,
                                    float* y_host);
 
@@ -221,15 +223,17 @@ int32_t mpq_q4_linear_forward_swiglu(mpq_context* ctx, const mpq_weight* w, cons
 /* ---- NVFP4 GEMM ---------------------------------------------------------- */
 /* C[M][N] (bf16 bits, row-major) = bf16( tsA * tsB * sum_k A~[m,k] * B~[n,k] ).
  * A is canonical NVFP4 on the device: codes [M][K/2], sf [M][K/16]; any
- * M >= 1.  When K is a multiple of 256 the kernel reads the activation scale
- * factors straight from that array; otherwise they are first re-tiled on the
- * GPU inside this call (counted in its time) into scratch the context owns.
- * Where the last wave of output tiles would leave SMs idle, its tiles may be
- * cut along K; their fp32 sums lie in scratch (17 MB on 148 SMs) that the
- * context's first call outside a capture reserves.  Without it (no such call,
+ * M >= 1.  Up to 32 rows, and up to 64 where that is the faster way, a kernel
+ * with the weights as the tensor core's M operand reads the activation scale
+ * factors straight from that array.  Other calls go to tiles of 256 activation
+ * rows: they read it directly when K is a multiple of 256; otherwise the scale
+ * factors are first re-tiled on the GPU inside this call (counted in its time)
+ * into scratch the context owns.
+ * Where output tiles would leave SMs idle, they may be cut along K; their fp32
+ * sums lie in scratch (17 MB on 148 SMs) that the context's first call outside
+ * a capture reserves, whether it cuts tiles or not.  Without it (no such call,
  * or no memory) tiles stay whole: slower, and with other last bits.
- * C must not overlap A (it is written with TMA tile stores while other tiles
- * are still being read). */
+ * C must not overlap A (it is written while other tiles are still being read). */
 int32_t mpq_nvfp4_gemm_forward(mpq_context* ctx, const mpq_weight* w,
                                const uint8_t* a_codes_dev, const uint8_t* a_sf_dev, float a_tensor_scale,
                                int64_t M, uint16_t* c_bf16_dev, void* stream);

@@ -1040,7 +1040,9 @@ static int q4_gemm_route(const mpq_context* ctx, const Q4Dev& q, int64_t M)
 
 // The streaming kernel stages ALL of x in every CTA, the rectangle kernel only a K slice of it: measured on the 7B shapes,
 // from about 16 K staged elements (4 rows of K = 4096, 2 rows of K = 11008) the rectangle kernel is the faster one for
-// several rows (4096 x 11008 at 4 rows: 11.9 against 22.8 us).  One row always streams.
+// several rows (4096 x 11008 at 4 rows: 11.9 against 22.8 us).  One row always streams.  Today's rectangle kernel is the faster one for 2 and
+// 3 rows of a shorter K, too (streaming / rectangle, us: 4096 x 4096 at 3 rows 7.6 / 6.1, 22016 x 4096 at 3 14.4 / 13.1, 1000 x 2112 at 2 6.6 / 4.3); the line stays
+// because the call without allocation, which only streams, is held to the bits of this one.
 static bool q4_prefers_stream(const mpq_context* ctx, const Q4Dev& q, int64_t M)
 {
     if (M > ctx->q4_stream_max_m) return false;

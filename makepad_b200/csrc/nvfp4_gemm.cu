@@ -11,7 +11,7 @@
 // K is consumed in blocks of 256 elements = 128 bytes per row = one 128-byte-swizzle atom = four tcgen05.mma
 // (K = 64 each).  Two kernels share that geometry: nvfp4_gemm_pair_kernel_v2 (default; a cluster of two CTAs on
 // 256 x 224 tiles with tcgen05 cta_group::2) and nvfp4_gemm_kernel_v2 (one CTA per tile, used where clusters of
-// two cannot be scheduled).  Up to 64 activation rows go to nvfp4_rows_kernel (nvfp4_rows.cuh).
+// two cannot be scheduled).  Up to 32 activation rows, and most calls of up to 64, go to nvfp4_rows_kernel (nvfp4_rows.cuh).
 //
 // ROLES (both kernels).  warp 0: TMA producer.  warp 1: TMEM allocation, MMA issue.  warps 2..9: epilogue
 // (tcgen05.ld of the whole accumulator into registers, release, then scale -> bf16 -> global).  warps 10..13:

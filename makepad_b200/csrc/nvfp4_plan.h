@@ -66,7 +66,8 @@ inline PairPlan pair_plan(int64_t M, int64_t N, int64_t K, int nclusters)
 // Whether a call of up to RW_MAX_ROWS rows goes to nvfp4_rows_kernel, where both kernels can take it.  It does up to 32 rows; above, unless
 // CTA pairs are estimated to be a twentieth and a microsecond faster: where a few CTAs more than a full wave make a second one, and where
 // K is short and 64 rows take their time in the epilogue.  The estimates were fitted to 668 measured calls (16 to 64 rows, 512 to 98304 weight
-// rows, K 512 to 14336; median error 3 % of this kernel's, 5 % of the other's).  CTA pairs / this kernel, us in a graph, 64 rows: 33264 x 2048 (297
+// rows, K 512 to 14336; median error 3 % of this kernel's, 5 % of the other's, whose few rows meet in L2 now and then: 34816 x 4096 at 48 rows takes pairs 23 us
+// where 27 are estimated and taken here).  CTA pairs / this kernel, us in a graph, 64 rows: 33264 x 2048 (297
 // tiles) 14.8 / 20.3, 33152 x 2048 (296) 15.8 / 11.8, 8192 x 2048 7.3 / 9.6, 14336 x 4096 12.8 / 14.6, 4096 x 4096 9.9 / 9.0, 57344 x 4096 36.7 / 33.0.
 inline bool nvfp4_rows_pay(const RowsPlan& rows, const PairPlan& pair, int64_t M)
 {

@@ -1,4 +1,4 @@
-// NVFP4 GEMM of few activation rows (up to 64): the WEIGHTS are the M = 128 operand.
+// NVFP4 GEMM of few activation rows (up to 32, most calls of up to 64): the WEIGHTS are the M = 128 operand.
 //
 // With a handful of rows the GEMM streams the weights once, and the tiles of the kernels for more rows are wrong for that: 256 activation rows of which 16
 // exist, half of a 224-column tile per CTA, no weight fetched before the kernels in front have ended.  Here a CTA takes 128 or 96
@@ -11,9 +11,10 @@
 // With few weight rows K is cut; the fp32 sums of the cuts go to [item][row of x][128] and nvfp4_rows_reduce_kernel adds them in order.
 //
 // What bounds it: a K block of a CTA takes about half a microsecond (copies, scale factors, MMAs, one after the other in a ring of four or five),
-// and 16 rows of 14336 x 4096 stream 3.2 TB/s.  CTA pairs / this kernel (us, GEMM alone in a graph): 14336 x 4096 at 1 row 43 / 10.0 (64 pairs
-// asked for one row of 256), 16 14.7 / 10.4, 64 15.1 / 14.5; 28672 x 4096 at 16 24.1 / 13.9, 64 24.0 / 16.6; 4096 x 14336 at 16 16.7 / 10.7, 64 19.5 / 13.2;
-// 4096 x 4096 at 16 10.5 / 6.0; 8192 x 8192 at 16 18.7 / 11.0, 64 16.6 / 13.9; 1024 x 1024 at 16 5.9 / 4.6.
+// and 16 rows of 14336 x 4096 stream 3.3 TB/s, of 28672 x 4096 4.8.  CTA pairs / this kernel (us, GEMM alone in a graph): 14336 x 4096 at 1 row 42.4 / 9.7 (64
+// pairs ask for one row of 256), 16 15.1 / 10.1, 64 13.1 / 14.6; 28672 x 4096 at 16 34.3 / 13.6, 64 19.5 / 16.0; 4096 x 14336 at 16 15.4 / 9.7, 64 17.8 / 12.8;
+// 4096 x 4096 at 16 10.1 / 5.7, 64 10.2 / 9.2; 8192 x 8192 at 16 17.8 / 10.3, 64 15.5 / 13.8; 1024 x 1024 at 16 5.6 / 4.2, 64 5.6 / 6.5.  Which of the two a
+// call of 33 to 64 rows takes: nvfp4_rows_pay (nvfp4_plan.h).
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>

@@ -457,11 +457,13 @@ __global__ void __launch_bounds__(Q4_THREADS) q4_linear_kernel(const Q4Launch p)
 //
 // What bounds it: up to about 10 MB per launch the fixed parts (prologue, staging of x, merge, the next launch's wait), else the run
 // itself.  One row takes copies of four chunks (G = 4): one barrier wait and one refill for four units.  Two chunks per copy, divisions in the
-// prologue, slots of the staging found per element, one warp per shared tile in the merge / this form, us per launch in a graph: 4096 x 4096 5.63 / 4.34,
-// 12288 x 4096 8.58 / 7.65, 22016 x 4096 11.6 / 10.7, 4096 x 11008 9.7 / 8.3, 1000 x 2112 6.5 / 5.2, 57344 x 8192 43.8 / 39.8, 128256 x 4096 46.5 / 42.0; 2 rows
-// of 4096 x 4096 7.3 / 6.3 (four chunks per copy: 0.2 more), of 22016 x 4096 13.4 / 13.2, of 128256 x 4096 48.1 / 48.4, of 152064 x 3584 49.5 / 51.2.
+// prologue, slots of the staging found per element, one warp per shared tile in the merge / this form, us per launch in a graph of weights that L2
+// does not hold: 4096 x 4096 5.6 / 4.6, 12288 x 4096 8.5 / 7.5, 22016 x 4096 11.6 / 10.6, 4096 x 11008 9.6 / 8.2, 1000 x 2112 6.5 / 5.3, 57344 x 8192 44.7 / 41.2,
+// 128256 x 4096 47.4 / 45.5; 2 rows of 4096 x 4096 7.1 / 6.4 (four chunks per copy: 0.2 more), of 22016 x 4096 13.4 / 13.1, of 128256 x 4096 49.0 / 49.8.
+// Over 70 shapes of 30000 to 250002 rows one row gains 3.5 %, two 0.1 %, four 1.6 %; the worst are those of 152000 x 3584 (1, 2, 4 rows 48.7 / 49.9, 50.2 / 53.2,
+// 54.8 / 56.0), where the order of the tiles over the SMs matters: spread evenly 48.2, 51.0, 55.2, and other shapes slower for it.
 // A look at the next copy's barrier ahead of the last unit's arithmetic and a predicated refill, which help the rectangle kernel, cost several rows
-// here 2..6 % (22016 x 4096 13.5, 49152 x 2048 13.2 -> 13.9) and gave one row nothing.
+// here 2..6 % (22016 x 4096 13.1 -> 13.5, 49152 x 2048 13.2 -> 14.2) and gave one row nothing.
 constexpr int Q4S_WARPS = 16;                    // one CTA of sixteen warps per SM
 constexpr int Q4S_THREADS = Q4S_WARPS * 32;
 constexpr int Q4S_MAX_DEPTH = 8;                 // most ring stages per warp
@@ -1018,9 +1020,9 @@ __global__ void __launch_bounds__(Q4S_THREADS, 1) q4_stream_kernel(const __grid_
 
     // ---- tiles shared between warps: add the parked partials in warp order.  The sharers of a tile are consecutive warps, and all but the
     // first have it in slot 0: segment (w, slot) opens a tile if the one before it belongs to another.  Up to four tiles are added by four
-    // warps each, one of the four values per lane: with up to sixteen sharers of one tile a warp for all of it took 0.7 us longer (4096 x 4096).  More
+    // warps each, one of the four values per lane: with up to sixteen sharers of one tile a warp for all of it took 0.6 us longer (4096 x 4096).  More
     // tiles have few sharers each and are added by the warps that open them, in a loop that is short on purpose: every CTA goes through
-    // it once, and its time is that of fetching the instructions.  (Four warps per tile here, too: 100000 x 2048 20.1 instead of 19.1 us.  The vote over
+    // it once, and its time is that of fetching the instructions.  (Four warps per tile here, too: 100000 x 2048 20.8 instead of 19.5 us.  The vote over
     // equal tiles by __match_any_sync: another 0.2 us with twelve tiles.)
     const int entry = wrp[lane >> 1][lane & 1];             // lane i holds segment i = (warp i/2, slot i%2)
     const int up1 = __shfl_up_sync(0xFFFFFFFFu, entry, 1), up2 = __shfl_up_sync(0xFFFFFFFFu, entry, 2);

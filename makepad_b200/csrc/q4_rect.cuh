@@ -31,10 +31,10 @@ constexpr int Q4R_MAX_CLUSTER = 8;                        // K slices of a clust
 constexpr uint32_t Q4R_SUM_TRIES = 1u << 17;              // tries (up to 4 us each) of the wait for the slices that the other CTAs send: half a second
 
 // What bounds it: up to about 10 MB of weights the fixed parts, above that the legacy tensor path and the FP pipes from about eight rows.
-// Slices always through memory, one warp per shared tile in the last phase, divisions in prologue and staging, a barrier look in front of
-// every copy's arithmetic / this form, us per call in a graph: 4096 x 4096 at 4 rows 8.2 / 6.2, 8 10.15 / 7.7, 16 13.0 / 11.0; 12288 x 4096 at 8
-// 14.8 / 13.1; 22016 x 4096 at 8 20.1 / 18.1, 16 30.9 / 29.4; 4096 x 11008 at 8 14.6 / 13.2; 1000 x 2112 at 13 9.2 / 5.9; 57344 x 8192 at 8 66.6 / 65.2.
-// With the staging's slots found once per thread: 22016 x 4096 at 8 17.8, 4096 x 11008 at 8 12.8, 2000 x 6016 at 8 7.26 / 7.04.
+// Slices always through memory, one warp per shared tile in the last phase, divisions in prologue and staging, slots of the staging found per
+// element, a barrier look in front of every copy's arithmetic / this form, us per call in a graph of weights that L2 does not hold: 4096 x 4096 at 4 rows
+// 8.3 / 6.4, 8 10.3 / 7.8, 16 13.1 / 11.0; 12288 x 4096 at 8 14.6 / 12.9; 22016 x 4096 at 8 19.8 / 17.2, 16 30.6 / 28.8; 4096 x 11008 at 8 14.4 / 12.9; 1000 x 2112 at 13
+// 9.3 / 6.2; 57344 x 8192 at 8 69.8 / 68.8.  0.1 us of each is the price of ordinary loads of x (pdl.cuh); the cluster barrier at the end costs nothing that shows.
 
 struct Q4RectLaunch {
     const uint4* stream;
